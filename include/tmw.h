@@ -337,6 +337,41 @@ TMW_API int tmw_decode_split_static(const tmw_cache_desc* cache, const void* q, 
                             const int64_t o_stride[2], const int32_t* pos, int32_t splits, void* stream);
 
 /*
+ * The model around the attention as one table, for the calls that run all of it.  One tmw_block per layer
+ * (titans_core/blocks/titan_block.py:41-102): weights as torch.nn.Linear stores them ([out, in] contiguous), norm scales
+ * [d_model], biases [n] or NULL, and the layer's ring cache (tmw_cache_desc).
+ */
+typedef struct tmw_block {
+    const void *norm_attn, *w_qkv, *w_out;
+    const void *norm_mlp, *w_fc1, *b_fc1, *w_fc2, *b_fc2;
+    void *k_ring, *v_ring;
+    const void *k_pers, *v_pers;
+    float cache_scale; /* 0 selects 1/sqrt(head_dim) */
+} tmw_block;
+
+typedef struct tmw_stack_desc {
+    int32_t dtype; /* TMW_BF16 or TMW_F16: every tensor of the model */
+    int32_t batch, layers, d_model, heads, head_dim, d_ff, window, n_persistent, vocab, max_positions;
+    float eps;                   /* of every RMSNorm */
+    const void *embed_tokens;    /* [vocab, d_model] */
+    const void *embed_positions; /* [max_positions, d_model] */
+    const void *norm;            /* final norm, [d_model] */
+    const void *head;            /* [vocab, d_model] */
+} tmw_stack_desc;
+
+/*
+ * One decode step of the whole model: token_ids [batch] int64 and pos [batch] int32 (device) -> logits [batch, vocab].
+ * Every block runs RMSNorm -> QKV -> tmw_decode on its ring -> output projection + residual -> RMSNorm -> MLP + residual
+ * (titan_block.py:92-100, blocks/mlp.py:58-65), then the final norm and the head; what the reference's generation
+ * helper gets from a full re-forward per token (examples/train_math.py:146-161).  head_dim 64 or 128, d_ff a multiple of
+ * 32.  `workspace`: device memory of tmw_decode_step_workspace() bytes, used until the call's kernels have finished;
+ * ids or positions outside the tables are clamped and reported by tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).
+ */
+TMW_API size_t tmw_decode_step_workspace(const tmw_stack_desc* desc);
+TMW_API int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, const int32_t* pos,
+                    void* logits, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Residual add + RMSNorm over contiguous rows [rows, dim] (dim a multiple of 8, pointers 16-byte aligned):
  *     h = x + residual          (residual may be NULL: h = x)
  *     sum_out = h               (sum_out may be NULL, and may be x itself: the residual stream in place)

@@ -1,0 +1,87 @@
+"""The whole decode step as one library call (``tmw_decode_step``) against the same step module by module: every row
+count at which the products change their kernel, both head sizes, a vocabulary that is no multiple of eight."""
+
+import pytest
+import torch
+
+from titanmac_b200 import TitanMAC, TitanMACConfig, _native, _stack
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def make(dtype, heads, dh, window, Np, vocab, layers=2, seed=0):
+    D = heads * dh
+    cfg = TitanMACConfig(vocab_size=vocab, d_model=D, n_heads=heads, n_layers=layers, d_ff=3 * D + 32, max_seq_len=256,
+                         window_size=window, n_persistent=Np, use_block_sparse=False)
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    with torch.device(DEV):
+        model = TitanMAC(cfg).eval()
+    with torch.no_grad():
+        for name, prm in model.named_parameters():
+            prm.normal_(1.0 if name.endswith("scale") else 0.0, 0.1 if name.endswith(("scale", "bias")) else 0.04, generator=g)
+    return model.to(dtype), g
+
+
+@pytest.mark.parametrize("B,dtype,heads,dh,window,Np,vocab,t", [
+    (1, torch.bfloat16, 10, 64, 512, 16, 1003, 200),   # one sequence, a ragged vocabulary
+    (8, torch.float16, 4, 128, 70, 0, 5000, 20),       # ring not full yet, no persistent rows
+    (16, torch.bfloat16, 2, 64, 33, 5, 512, 100),
+    (17, torch.bfloat16, 6, 64, 20, 3, 776, 61),       # the second row tile holds one row
+    (32, torch.float16, 3, 128, 64, 16, 333, 64),
+    (33, torch.bfloat16, 2, 64, 8, 1, 1000, 0),        # first token; tcgen05 products from here on
+    (129, torch.bfloat16, 10, 64, 17, 16, 99, 40),     # two tiles of 128 rows, a ragged vocabulary
+    (256, torch.float16, 8, 64, 40, 8, 1024, 41),
+])
+def test_step_equals_module_by_module(B, dtype, heads, dh, window, Np, vocab, t, monkeypatch):
+    model, g = make(dtype, heads, dh, window, Np, vocab)
+    ids = torch.randint(0, vocab, (B,), generator=g, device=DEV)
+    pos = torch.randint(max(0, t - 3), t + 1, (B,), generator=g, device=DEV, dtype=torch.int32)
+    sets = []
+    for _ in range(2):
+        sets.append(model.new_caches(B, DEV, dtype))
+    for a, b in zip(*sets):
+        for x, y in zip((a.k_ring, a.v_ring, a.k_pers, a.v_pers), (b.k_ring, b.v_ring, b.k_pers, b.v_pers)):
+            x.normal_(0.0, 0.5, generator=g)
+            y.copy_(x)
+    assert _stack.table_of(model) is not None
+    got = model.decode_step(ids, pos, sets[0])
+    _native.poll_status(torch.device(DEV))
+    monkeypatch.setattr(_stack, "table_of", lambda m: None)
+    want = model.decode_step(ids, pos, sets[1])
+    tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
+    assert got.shape == want.shape == (B, vocab)
+    assert ((got.float() - want.float()).norm() / want.float().norm()).item() <= tol
+    for a, b in zip(*sets):
+        for x, y in ((a.k_ring, b.k_ring), (a.v_ring, b.v_ring)):
+            assert ((x.float() - y.float()).norm() / y.float().norm()).item() <= tol
+
+
+def test_table_follows_the_model():
+    """A moved parameter, a replaced module, a hook: the step never uses what the model no longer is."""
+    model, g = make(torch.bfloat16, 2, 64, 16, 2, 128)
+    caches = model.new_caches(3, DEV, torch.bfloat16)
+    ids = torch.tensor([1, 2, 3], device=DEV)
+    pos = torch.zeros(3, dtype=torch.int32, device=DEV)
+    before = model.decode_step(ids, pos, caches)
+    lin = torch.nn.Linear(128, 128, bias=False, device=DEV, dtype=torch.bfloat16)
+    model.layers[1].attention.out_proj = lin
+    replaced = model.decode_step(ids, pos, caches)
+    assert not torch.equal(before, replaced)
+    with torch.no_grad():
+        lin.weight = torch.nn.Parameter(lin.weight * 2)
+    assert not torch.equal(replaced, model.decode_step(ids, pos, caches))
+    seen = []
+    handle = model.layers[0].mlp.register_forward_hook(lambda *a: seen.append(1))
+    model.decode_step(ids, pos, caches)
+    handle.remove()
+    assert seen == [1] and _stack.table_of(model) is not None
+
+
+def test_ids_outside_the_table_are_reported():
+    model, _ = make(torch.bfloat16, 2, 64, 16, 2, 128)
+    caches = model.new_caches(2, DEV, torch.bfloat16)
+    model.decode_step(torch.tensor([5, 128], device=DEV), torch.zeros(2, dtype=torch.int32, device=DEV), caches)
+    with pytest.raises(_native.TmwError):
+        _native.poll_status(torch.device(DEV))
+    _native.poll_status(torch.device(DEV))

@@ -38,6 +38,19 @@ int* device_status_word() {
     return cache[dev].load(std::memory_order_acquire);
 }
 
+int sm_count() {
+    constexpr int kMaxDevices = 64;
+    static int cache[kMaxDevices] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
+    if (cache[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        cache[dev] = n;
+    }
+    return cache[dev];
+}
+
 // One side stream and two events per device, made on first use and kept for the life of the process (make
 // that first use outside stream capture).  Calls that use them are serialised on the host by `mutex`.
 SideStream* side_stream_of_current_device() {

@@ -130,23 +130,8 @@ int launch_add_rmsnorm(long long rows, int dim, const void* x, const void* res, 
 
 // ---- exact GELU --------------------------------------------------------------------------------------
 // 0.5 x (1 + erf(x / sqrt 2)), the default nn.GELU() of the reference's MLP (titans_core/blocks/mlp.py:58-65).
-// erf by Abramowitz & Stegun 7.1.26 (|error| <= 1.5e-7, below fp32 rounding of the result): a reciprocal,
-// five multiply-adds and one exp2 instead of the branchy library erff, so that the kernel stays bound by
-// HBM (one read, one write) and not by arithmetic.
-__device__ __forceinline__ float gelu_erf(float x) {
-    const float z = fabsf(x) * 0.70710678118654752f;
-    const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
-    float poly = fmaf(1.061405429f, t, -1.453152027f);
-    poly = fmaf(poly, t, 1.421413741f);
-    poly = fmaf(poly, t, -0.284496736f);
-    poly = fmaf(poly, t, 0.254829592f);
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-z * z * 1.4426950408889634f));
-    const float erfc_z = poly * t * e;  // 1 - erf(z), z >= 0
-    const float erf_abs = 1.0f - erfc_z;
-    return 0.5f * x * (1.0f + copysignf(erf_abs, x));
-}
-
+// erf by the rational approximation of gelu_erf (tmw_common.cuh), so that the kernel stays bound by HBM (one read, one
+// write) and not by arithmetic.
 constexpr int kGeluUnroll = 4;  // 16-byte loads in flight per thread
 
 template <typename T>

@@ -11,10 +11,10 @@
 // ONE warp (no block-level merge, all pairs resident at once, so no wave
 // quantisation); with few pairs a whole CTA of 8 warps shares one pair.
 //
-// 16-bit caches with more than half a pair per SM take decode_stream_kernel further
-// down instead: the same arithmetic fed from shared memory, which bulk asynchronous
-// copies keep filled three chunks ahead (measured on B200, 2560 pairs, window 512:
-// 60 us against 68 us; 5120 pairs: 105 us against 129 us, the bandwidth of a plain copy).
+// 16-bit caches with head_dim 64 or 128 take one of two other kernels further down: decode_stream_kernel with many
+// pairs - the same arithmetic fed from shared memory, which bulk asynchronous copies keep filled three chunks ahead
+// (measured on B200, 2560 pairs, window 512: 60 us against 68 us; 5120 pairs: 105 us against 129 us, the bandwidth of
+// a plain copy) - and decode_cluster_kernel with few.
 #include <math_constants.h>
 
 #include <cstdio>
@@ -22,10 +22,6 @@
 #include <atomic>
 
 #include "tmw_common.cuh"
-
-#ifndef TMW_DECODE_STREAM
-#define TMW_DECODE_STREAM 1
-#endif
 
 namespace tmw {
 namespace {
@@ -48,6 +44,7 @@ struct DecodeParams {
     float* scratch;          // [pairs][splits][DH + 2] partial results (accumulator, running maximum, sum)
     unsigned int* counters;  // [pairs] arrivals of a pair's CTAs; zero between launches
     int* status;             // device status word (bounded waits of the streaming kernel report here)
+    int cluster;             // decode_cluster_kernel: CTAs per pair
 };
 
 // 8 consecutive elements as raw bits, loaded through the read-only path without keeping
@@ -399,6 +396,7 @@ decode_stream_kernel(const DecodeParams p) {
     extern __shared__ __align__(128) unsigned char stream_smem[];
 
     constexpr int NW = WPP == 1 ? 2 : WPP;  // warps per CTA
+    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int pair = WPP == 1 ? blockIdx.x * 2 + warp : blockIdx.x;
     const int wslot = WPP == 1 ? 0 : warp;  // which share of the chunks this warp scans
@@ -458,8 +456,10 @@ decode_stream_kernel(const DecodeParams p) {
         asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      ::"r"(dst + kStreamChunkBytes), "l"(vsrc), "r"(bytes), "r"(bar) : "memory");
     };
+    // (ring rows and positions are nothing that an earlier kernel of the chain writes, see pdl_wait)
     if (lane == 0)
         for (int n = 0; n < min(kStreamStages, my_chunks); ++n) issue(n);
+    pdl_wait();
 
     // the new token (every lane group computes its score, group 0 owns it)
     float qreg[8];
@@ -633,8 +633,205 @@ decode_stream_kernel(const DecodeParams p) {
     }
 }
 
+// -----------------------------------------------------------------------------------------------------
+// Few pairs (small batches): a cluster of up to eight CTAs of four warps shares one pair's keys, each lane holding up
+// to six rows of K and of V in registers, and merges through distributed shared memory - no scratch memory, no
+// counters.  One CTA per pair left 138 of 148 SMs idle for a single sequence of ten heads and scanned its 529 keys in
+// three dependent rounds.
+// The loads depend on nothing the launch in front writes, so they are issued before pdl_wait().
+// -----------------------------------------------------------------------------------------------------
+constexpr int kClusterWarps = 4;
+
+template <typename T, int DH>
+__global__ void __launch_bounds__(kClusterWarps * 32, 5) decode_cluster_kernel(const DecodeParams p) {
+    constexpr int U = 6;           // row loads in flight per lane, for K and again for V
+    constexpr int LPK = DH / 8;    // lanes per key row
+    constexpr int RPW = 32 / LPK;  // key rows per warp per load instruction
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cs = p.cluster, pair = blockIdx.x / cs, rank = blockIdx.x % cs;
+    const int b = pair / p.heads, h = pair % p.heads;
+    const int sub = lane % LPK, grp = lane / LPK;
+    int t = p.pos[b];
+    if (t < 0) {  // see decode_kernel
+        if (lane == 0) atomicCAS(p.status, 0, (int)TMW_ERR_INVALID_ARGUMENT);
+        t = 0;
+    }
+    const int slot_new = t % p.slots;
+    const int n_keys = p.np + min(t + 1, p.slots) - 1;  // persistent rows, then the older ring slots in slot order
+    const long long ring_bh = ((long long)b * p.heads + h) * p.slots * DH;
+    T* kr = static_cast<T*>(p.k_ring) + ring_bh;
+    T* vr = static_cast<T*>(p.v_ring) + ring_bh;
+    const T* kp = static_cast<const T*>(p.k_pers) + (long long)h * p.np * DH;
+    const T* vp = static_cast<const T*>(p.v_pers) + (long long)h * p.np * DH;
+    const int first = (rank * kClusterWarps + warp) * RPW + grp;  // this lane group's first key
+    const int stride = cs * kClusterWarps * RPW;
+    Raw8<T> kraw[U], vraw[U];
+    auto load_k = [&](int u, int i) {
+        if (i < p.np) kraw[u].load(kp + (long long)i * DH + sub * 8);
+        else if (i < n_keys) kraw[u].load(kr + (long long)(i - p.np + (i - p.np >= slot_new)) * DH + sub * 8);
+    };
+    auto load_v = [&](int u, int i) {
+        if (i < p.np) vraw[u].load(vp + (long long)i * DH + sub * 8);
+        else if (i < n_keys) vraw[u].load(vr + (long long)(i - p.np + (i - p.np >= slot_new)) * DH + sub * 8);
+    };
+#pragma unroll
+    for (int u = 0; u < U; ++u) load_k(u, first + u * stride);
+#pragma unroll
+    for (int u = 0; u < U; ++u) load_v(u, first + u * stride);
+    pdl_wait();
+
+    const T* kn = static_cast<const T*>(p.k_new) + b * p.ns[0] + h * p.ns[1];
+    const T* vn = static_cast<const T*>(p.v_new) + b * p.ns[0] + h * p.ns[1];
+    float qreg[8], m, l, acc[8];
+    load8<T>(static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1] + sub * 8, qreg);
+    {
+        // the new token: taken by the first lane group of the pair, which also writes it into its ring slot
+        float kf[8], vf[8];
+        load8<T>(kn + sub * 8, kf);
+        load8<T>(vn + sub * 8, vf);
+        float part = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part = fmaf(qreg[e], kf[e], part);
+#pragma unroll
+        for (int off = 1; off < LPK; off <<= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+        const bool owner = first == 0;
+        m = owner ? part * p.scale_log2 : -CUDART_INF_F;
+        l = owner ? 1.f : 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = owner ? vf[e] : 0.f;
+        if (owner) {
+            store8<T>(kr + (long long)slot_new * DH + sub * 8, kf);
+            store8<T>(vr + (long long)slot_new * DH + sub * 8, vf);
+        }
+    }
+    // (the loop runs the same number of times in every lane group of a warp)
+    for (int i0 = first; i0 - grp < n_keys; i0 += U * stride) {
+        float s[U], tmax = -CUDART_INF_F;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float part = 0.f;
+            const bool ok = i0 + u * stride < n_keys;
+            if (ok) {
+                float kf[8];
+                kraw[u].unpack(kf);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) part = fmaf(qreg[e], kf[e], part);
+            }
+#pragma unroll
+            for (int off = 1; off < LPK; off <<= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+            s[u] = ok ? part * p.scale_log2 : -CUDART_INF_F;
+            tmax = fmaxf(tmax, s[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_k(u, i0 + (U + u) * stride);
+        if (tmax > -CUDART_INF_F) {
+            const float m_new = fmaxf(m, tmax);
+            const float alpha = exp2f(m - m_new);
+            m = m_new;
+            l *= alpha;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] *= alpha;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + u * stride < n_keys) {
+                    const float pj = exp2f(s[u] - m);
+                    l += pj;
+                    float vf[8];
+                    vraw[u].unpack(vf);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] = fmaf(pj, vf[e], acc[e]);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_v(u, i0 + (U + u) * stride);
+    }
+    // merge: lane groups by shuffles, warps through shared memory, CTAs through each other's
+#pragma unroll
+    for (int off = LPK; off < 32; off <<= 1) {
+        const float m_o = __shfl_xor_sync(0xffffffffu, m, off);
+        const float l_o = __shfl_xor_sync(0xffffffffu, l, off);
+        const float m_new = fmaxf(m, m_o);
+        const float a = m_new > -CUDART_INF_F ? exp2f(m - m_new) : 0.f;
+        const float a_o = m_new > -CUDART_INF_F ? exp2f(m_o - m_new) : 0.f;
+        l = l * a + l_o * a_o;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float acc_o = __shfl_xor_sync(0xffffffffu, acc[e], off);
+            acc[e] = acc[e] * a + acc_o * a_o;
+        }
+        m = m_new;
+    }
+    __shared__ float wpart[kClusterWarps][DH + 2];  // per warp: accumulator, maximum, sum
+    __shared__ float cpart[DH + 2];                 // per CTA
+    if (grp == 0) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wpart[warp][sub * 8 + e] = acc[e];
+        if (sub == 0) {
+            wpart[warp][DH] = m;
+            wpart[warp][DH + 1] = l;
+        }
+    }
+    __syncthreads();
+    float m_all = -CUDART_INF_F, l_all = 0.f, a_all = 0.f;  // of output column tid
+    if (tid < DH) {
+#pragma unroll
+        for (int w = 0; w < kClusterWarps; ++w) m_all = fmaxf(m_all, wpart[w][DH]);
+#pragma unroll
+        for (int w = 0; w < kClusterWarps; ++w) {
+            const float f = m_all > -CUDART_INF_F ? exp2f(wpart[w][DH] - m_all) : 0.f;
+            l_all = fmaf(wpart[w][DH + 1], f, l_all);
+            a_all = fmaf(wpart[w][tid], f, a_all);
+        }
+    }
+    if (cs > 1) {
+        if (tid < DH) cpart[tid] = a_all;
+        if (tid == 0) {
+            cpart[DH] = m_all;
+            cpart[DH + 1] = l_all;
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0 && tid < DH) {
+            // all of the peers' values are requested before the first is used: one trip through the cluster's network
+            const uint32_t base = smem_u32(cpart);
+            float pm[8], pl[8], pa[8];
+#pragma unroll
+            for (int r = 1; r < 8; ++r) {
+                pm[r] = -CUDART_INF_F;
+                pl[r] = pa[r] = 0.f;
+                if (r < cs) {
+                    uint32_t peer;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(base), "r"(r));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pm[r]) : "r"(peer + DH * 4) : "memory");
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pl[r]) : "r"(peer + (DH + 1) * 4) : "memory");
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pa[r]) : "r"(peer + tid * 4) : "memory");
+                }
+            }
+            const float m_own = m_all;
+#pragma unroll
+            for (int r = 1; r < 8; ++r) m_all = fmaxf(m_all, pm[r]);
+            const float f0 = exp2f(m_own - m_all);  // the new token is in rank 0's share: m_all is finite
+            l_all *= f0;
+            a_all *= f0;
+#pragma unroll
+            for (int r = 1; r < 8; ++r) {
+                const float f = exp2f(pm[r] - m_all);
+                l_all = fmaf(pl[r], f, l_all);
+                a_all = fmaf(pa[r], f, a_all);
+            }
+        }
+    }
+    if (rank == 0 && tid < DH)
+        (static_cast<T*>(p.o) + b * p.os[0] + h * p.os[1])[tid] = from_f32<T>(a_all / l_all);
+    if (cs > 1) {  // nobody's shared memory goes away while rank 0 may still read it
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
 template <typename T, int DH, int WPP>
-int launch_decode_stream(const DecodeParams& p, cudaStream_t stream) {
+int launch_decode_stream(const DecodeParams& p, cudaStream_t stream, bool pdl) {
     if constexpr (sizeof(T) == 2 && (DH == 64 || DH == 128)) {
         auto kern = decode_stream_kernel<T, DH, WPP>;
         // nine 64-thread CTAs with 24 KB each per SM: ask for the largest shared-memory carve-out, once per
@@ -649,9 +846,8 @@ int launch_decode_stream(const DecodeParams& p, cudaStream_t stream) {
             if (dev >= 0 && dev < 64) configured[dev] = true;
         }
         const int pairs = p.batch * p.heads;
-        if (WPP == 1) kern<<<(pairs + 1) / 2, 64, stream_smem_bytes(2), stream>>>(p);
-        else kern<<<pairs, WPP * 32, stream_smem_bytes(WPP), stream>>>(p);
-        TMW_CUDA_TRY(cudaGetLastError());
+        if (WPP == 1) TMW_CUDA_TRY(launch_ex(kern, dim3((pairs + 1) / 2), dim3(64), stream_smem_bytes(2), stream, pdl, 1, p));
+        else TMW_CUDA_TRY(launch_ex(kern, dim3(pairs), dim3(WPP * 32), stream_smem_bytes(WPP), stream, pdl, 1, p));
         return TMW_OK;
     } else {
         return TMW_ERR_UNSUPPORTED;
@@ -687,27 +883,37 @@ __global__ void cache_fill_kernel(const FillParams p) {
 }
 
 template <typename T, int DH>
-int launch_decode_shape(const DecodeParams& p, cudaStream_t stream) {
+int launch_decode_shape(const DecodeParams& p0, cudaStream_t stream, bool pdl) {
+    DecodeParams p = p0;
     const int pairs = p.batch * p.heads;
     if (p.splits > 0) {
         decode_kernel<T, DH, 4, true><<<pairs * p.splits, 128, 0, stream>>>(p);
         TMW_CUDA_TRY(cudaGetLastError());
         return TMW_OK;
     }
-    int sms = 148;
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // 16-bit caches whose rows are whole 16-byte units at 16-byte aligned addresses take the streaming variant
-    constexpr bool kStreamShape = sizeof(T) == 2 && (DH == 64 || DH == 128);
-    const bool aligned = (((uintptr_t)p.k_ring | (uintptr_t)p.v_ring | (uintptr_t)p.k_pers | (uintptr_t)p.v_pers) & 15) == 0;
-    if (TMW_DECODE_STREAM && kStreamShape && aligned) {
-        // every shape runs as a single wave: 2 pairs per CTA x 9 CTAs per SM, 1 pair per 2-warp CTA x 9, or
-        // 1 pair per 4-warp CTA x 4 (measured, us per layer at window 512: 2560 pairs 60, 800 pairs 20.8,
-        // 640 pairs 18.5, 480 pairs 14.3, 320 pairs 11.8, 160 pairs 8.9)
-        if (pairs > 9 * sms) return launch_decode_stream<T, DH, 1>(p, stream);
-        if (pairs > 4 * sms) return launch_decode_stream<T, DH, 2>(p, stream);
-        if (pairs > sms / 2) return launch_decode_stream<T, DH, 4>(p, stream);
+    const int sms = sm_count();
+    // 16-bit caches whose rows are whole 16-byte units at 16-byte aligned addresses
+    if constexpr (sizeof(T) == 2 && (DH == 64 || DH == 128)) {
+        if ((((uintptr_t)p.k_ring | (uintptr_t)p.v_ring | (uintptr_t)p.k_pers | (uintptr_t)p.v_pers) & 15) == 0) {
+            // every shape runs as a single wave: 2 pairs per CTA x 9 CTAs per SM, 1 pair per 2-warp CTA x 9, or
+            // 1 pair per 4-warp CTA x 4 (measured, us per layer at window 512: 2560 pairs 60, 800 pairs 20.8,
+            // 640 pairs 18.5, 500 pairs 11.5)
+            if (pairs > 9 * sms) return launch_decode_stream<T, DH, 1>(p, stream, pdl);
+            if (pairs > 4 * sms) return launch_decode_stream<T, DH, 2>(p, stream, pdl);
+            if (pairs > 2 * sms + sms / 2) return launch_decode_stream<T, DH, 4>(p, stream, pdl);
+            // few pairs: CTAs of a cluster share a pair, five to an SM; eight only where that is less than one per SM
+            // (in a chain, us per layer at window 512, clusters of 2 | 4 | 8: 160 pairs 10.1 | 7.8 | -, 80 pairs
+            // - | 6.9 | 9.0; 320 pairs 10.9 against 10.4 of the streaming kernel, whose shared memory keeps the next
+            // launch out: 480 us a step against 530; 500 pairs 17.5 against 11.5)
+            p.cluster = 1;
+            while (p.cluster < 4 && pairs * p.cluster * 2 <= 5 * sms) p.cluster *= 2;
+            if (pairs * 8 <= sms) p.cluster = 8;
+            TMW_CUDA_TRY(launch_ex(decode_cluster_kernel<T, DH>, dim3(pairs * p.cluster), dim3(kClusterWarps * 32), 0, stream,
+                                   pdl, p.cluster, p));
+            return TMW_OK;
+        }
     }
+    if (pdl) return TMW_ERR_UNSUPPORTED;  // the kernels below do not take part in a chain of dependent launches
     if (pairs > 9 * sms) {
         decode_kernel<T, DH, 1><<<(pairs + 1) / 2, 64, 0, stream>>>(p);
     } else if (pairs > 4 * sms) {
@@ -722,14 +928,14 @@ int launch_decode_shape(const DecodeParams& p, cudaStream_t stream) {
 }
 
 template <typename T>
-int launch_decode_dh(const DecodeParams& p, int dh, cudaStream_t stream) {
+int launch_decode_dh(const DecodeParams& p, int dh, cudaStream_t stream, bool pdl) {
     switch (dh) {
-        case 8: return launch_decode_shape<T, 8>(p, stream);
-        case 16: return launch_decode_shape<T, 16>(p, stream);
-        case 32: return launch_decode_shape<T, 32>(p, stream);
-        case 64: return launch_decode_shape<T, 64>(p, stream);
-        case 128: return launch_decode_shape<T, 128>(p, stream);
-        case 256: return launch_decode_shape<T, 256>(p, stream);
+        case 8: return launch_decode_shape<T, 8>(p, stream, pdl);
+        case 16: return launch_decode_shape<T, 16>(p, stream, pdl);
+        case 32: return launch_decode_shape<T, 32>(p, stream, pdl);
+        case 64: return launch_decode_shape<T, 64>(p, stream, pdl);
+        case 128: return launch_decode_shape<T, 128>(p, stream, pdl);
+        case 256: return launch_decode_shape<T, 256>(p, stream, pdl);
         default: return TMW_ERR_UNSUPPORTED;
     }
 }
@@ -738,7 +944,7 @@ int launch_decode_dh(const DecodeParams& p, int dh, cudaStream_t stream) {
 
 int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, const void* v_new, void* o,
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,
-                  int splits, float* scratch, unsigned int* counters, cudaStream_t stream) {
+                  int splits, float* scratch, unsigned int* counters, cudaStream_t stream, bool pdl) {
     if (c.batch == 0 || c.heads == 0) return TMW_OK;
     if ((long long)c.batch * c.heads > (1LL << 30)) return TMW_ERR_TOO_LARGE;
     DecodeParams p;
@@ -746,15 +952,15 @@ int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, con
     p.q = q; p.k_new = k_new; p.v_new = v_new; p.o = o; p.pos = pos;
     for (int i = 0; i < 2; ++i) { p.qs[i] = qs[i]; p.ns[i] = ns[i]; p.os[i] = os[i]; }
     p.batch = c.batch; p.heads = c.heads; p.slots = c.window + 1; p.np = c.n_persistent;
-    p.splits = splits; p.scratch = scratch; p.counters = counters;
+    p.splits = splits; p.scratch = scratch; p.counters = counters; p.cluster = 1;
     p.status = device_status_word();
     if (p.status == nullptr) return TMW_ERR_CUDA;
     const float scale = c.scale != 0.f ? c.scale : 1.0f / sqrtf((float)c.head_dim);
     p.scale_log2 = scale * 1.4426950408889634f;
     switch (c.dtype) {
-        case TMW_F32: return launch_decode_dh<float>(p, c.head_dim, stream);
-        case TMW_BF16: return launch_decode_dh<__nv_bfloat16>(p, c.head_dim, stream);
-        case TMW_F16: return launch_decode_dh<__half>(p, c.head_dim, stream);
+        case TMW_F32: return launch_decode_dh<float>(p, c.head_dim, stream, pdl);
+        case TMW_BF16: return launch_decode_dh<__nv_bfloat16>(p, c.head_dim, stream, pdl);
+        case TMW_F16: return launch_decode_dh<__half>(p, c.head_dim, stream, pdl);
         default: return TMW_ERR_UNSUPPORTED;
     }
 }

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 #include "tmw_common.cuh"
 
 namespace tmw {
@@ -49,21 +50,6 @@ struct GemmParams {
     const void* bias;    // [n] in the dtype of the operands, or nullptr
     int* status;
 };
-
-// Exact (erf-based) GELU, 0.5 x (1 + erf(x / sqrt 2)), with erf from the rational approximation 7.1.26 of
-// Abramowitz & Stegun (absolute error below 1.5e-7, i.e. fp32 rounding noise against the 16-bit result): one
-// reciprocal, one exponential and a degree-5 polynomial instead of the library's branchy erff - the epilogue of
-// a 128 x 256 tile evaluates it 32 768 times and must stay shorter than the tile's matrix products.
-__device__ __forceinline__ float gelu_erf(float x) {
-    const float z = fabsf(x) * 0.70710678118654752f;
-    const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
-    float poly = fmaf(1.061405429f, t, -1.453152027f);
-    poly = fmaf(poly, t, 1.421413741f);
-    poly = fmaf(poly, t, -0.284496736f);
-    poly = fmaf(poly, t, 0.254829592f);
-    const float erf_abs = 1.0f - poly * t * __expf(-z * z);  // erf(|x| / sqrt 2)
-    return 0.5f * x * (1.0f + copysignf(erf_abs, x));
-}
 
 template <int BN, bool BF16>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -470,82 +456,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // ---------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    });
-    return fn;
-}
-
-// Map over a row-major [rows, cols] matrix with leading dimension ld (elements): boxes of box_rows x box_cols.
-// Encoded maps are kept per host thread, keyed by everything that goes into them.
-struct Map2dKey {
-    const void* base;
-    int64_t ld;
-    int32_t dtype, rows, cols, box_rows, box_cols, swizzle;
-    bool operator==(const Map2dKey& o) const {
-        return base == o.base && ld == o.ld && dtype == o.dtype && rows == o.rows && cols == o.cols &&
-               box_rows == o.box_rows && box_cols == o.box_cols && swizzle == o.swizzle;
-    }
-};
-bool make_map_2d(CUtensorMap* map, const void* base, int dtype, int rows, int cols, int64_t ld, int box_rows,
-                 int box_cols, CUtensorMapSwizzle swizzle) {
-    constexpr int kEntries = 64;
-    struct Cache { Map2dKey key[kEntries]; CUtensorMap map[kEntries]; bool used[kEntries] = {false}; int next = 0; };
-    static thread_local Cache cache;
-    const Map2dKey key{base, ld, dtype, rows, cols, box_rows, box_cols, (int32_t)swizzle};
-    for (int i = 0; i < kEntries; ++i)
-        if (cache.used[i] && cache.key[i] == key) {
-            *map = cache.map[i];
-            return true;
-        }
-    EncodeTiledFn fn = encode_fn();
-    if (fn == nullptr) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    const CUtensorMapDataType dt = dtype == TMW_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    const CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        char text[96];
-        snprintf(text, sizeof(text), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-        set_error_text(text);
-        return false;
-    }
-    const int slot = cache.next;
-    cache.next = (cache.next + 1) % kEntries;
-    cache.key[slot] = key;
-    cache.map[slot] = *map;
-    cache.used[slot] = true;
-    return true;
-}
-
-int sm_count() {
-    constexpr int kMaxDevices = 64;
-    static int cache[kMaxDevices] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
-    if (cache[dev] == 0) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cache[dev] = n;
-    }
-    return cache[dev];
-}
-
 template <int BN>
 int launch_gemm(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream) {
     using L = GemmSmem<BN>;

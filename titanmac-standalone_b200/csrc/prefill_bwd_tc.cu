@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 #include "tmw_common.cuh"
 
 namespace tmw {
@@ -558,74 +559,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
 // ---------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    });
-    return fn;
-}
-
-struct Strides4 {
-    int64_t row, head, batch;
-    bool heads_first;
-    bool ok;  // positive multiples of 16 bytes below 2^40 bytes: what a tensor map accepts
-};
-Strides4 strides_of(int batch, int heads, int rows, int dh, const int64_t stride[3]) {
-    Strides4 m;
-    m.row = rows > 1 ? stride[2] : dh;
-    m.head = heads > 1 ? stride[1] : m.row * rows;
-    const int64_t inner_span = m.head * heads > m.row * rows ? m.head * heads : m.row * rows;
-    m.batch = batch > 1 ? stride[0] : inner_span;
-    m.heads_first = m.head < m.row;
-    const int64_t limit = ((int64_t)1 << 40) / 2;
-    m.ok = m.row > 0 && m.head > 0 && m.batch > 0 && m.row < limit && m.head < limit && m.batch < limit &&
-           m.row % 8 == 0 && m.head % 8 == 0 && m.batch % 8 == 0;
-    return m;
-}
-
-// map over a [batch, heads, rows, dh] tensor: boxes of box_rows rows x 64 columns of one (batch, head), 128-byte swizzle
-bool make_map4(CUtensorMap* map, const void* base, int dtype, int batch, int heads, int rows, int dh, const Strides4& m,
-               int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (fn == nullptr) return false;
-    cuuint64_t dims[4], strides[3];
-    cuuint32_t box[4];
-    dims[0] = (cuuint64_t)dh;
-    box[0] = 64;
-    if (m.heads_first) {
-        dims[1] = (cuuint64_t)heads; strides[0] = (cuuint64_t)m.head * 2; box[1] = 1;
-        dims[2] = (cuuint64_t)rows;  strides[1] = (cuuint64_t)m.row * 2;  box[2] = (cuuint32_t)box_rows;
-    } else {
-        dims[1] = (cuuint64_t)rows;  strides[0] = (cuuint64_t)m.row * 2;  box[1] = (cuuint32_t)box_rows;
-        dims[2] = (cuuint64_t)heads; strides[1] = (cuuint64_t)m.head * 2; box[2] = 1;
-    }
-    dims[3] = (cuuint64_t)batch;
-    strides[2] = (cuuint64_t)m.batch * 2;
-    box[3] = 1;
-    const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
-    const CUtensorMapDataType dt = dtype == TMW_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    const CUresult r = fn(map, dt, 4, const_cast<void*>(base), dims, strides, box, elem_strides,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        char text[96];
-        snprintf(text, sizeof(text), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-        set_error_text(text);
-        return false;
-    }
-    return true;
-}
-
 // Stream-ordered scratch memory comes from a pool of the library's own (one per device, created on first use,
 // kept for the life of the process): freed blocks stay in the pool, so a call costs no trip to the driver's
 // allocator after the first, and the device's default pool and its settings are left alone.
@@ -661,17 +594,17 @@ int launch_bwd_tc(const tmw_prefill_desc& d, const void* q, const void* k, const
                   const float* lse, void* dq, void* dk, void* dv, cudaStream_t stream, int window_block) {
     using L = BwdSmem<DH>;
     const int B = d.batch, H = d.heads, R = d.q_rows;
-    const Strides4 sq = strides_of(B, H, R, DH, d.q_stride), sk = strides_of(B, H, R, DH, d.k_stride);
-    const Strides4 sv = strides_of(B, H, R, DH, d.v_stride), so = strides_of(B, H, R, DH, d.o_stride);
+    const MapStrides sq = map_strides(B, H, R, DH, d.q_stride), sk = map_strides(B, H, R, DH, d.k_stride);
+    const MapStrides sv = map_strides(B, H, R, DH, d.v_stride), so = map_strides(B, H, R, DH, d.o_stride);
     constexpr int CW = Geo<DH>::kCW;
     // row-tile maps (boxes of 128 rows; also the outputs) and column-tile maps (boxes of CW rows)
     CUtensorMap mq, mk, mv, mdo, mdq, mdk, mdv, cq, ck, cv, cdo;
-    if (!make_map4(&mq, q, d.dtype, B, H, R, DH, sq, BT) || !make_map4(&mk, k, d.dtype, B, H, R, DH, sk, BT) ||
-        !make_map4(&mv, v, d.dtype, B, H, R, DH, sv, BT) || !make_map4(&mdo, d_o, d.dtype, B, H, R, DH, so, BT) ||
-        !make_map4(&mdq, dq, d.dtype, B, H, R, DH, sq, BT) || !make_map4(&mdk, dk, d.dtype, B, H, R, DH, sk, BT) ||
-        !make_map4(&mdv, dv, d.dtype, B, H, R, DH, sv, BT) || !make_map4(&cq, q, d.dtype, B, H, R, DH, sq, CW) ||
-        !make_map4(&ck, k, d.dtype, B, H, R, DH, sk, CW) || !make_map4(&cv, v, d.dtype, B, H, R, DH, sv, CW) ||
-        !make_map4(&cdo, d_o, d.dtype, B, H, R, DH, so, CW))
+    if (!make_map_4d(&mq, q, d.dtype, B, H, R, DH, sq, BT) || !make_map_4d(&mk, k, d.dtype, B, H, R, DH, sk, BT) ||
+        !make_map_4d(&mv, v, d.dtype, B, H, R, DH, sv, BT) || !make_map_4d(&mdo, d_o, d.dtype, B, H, R, DH, so, BT) ||
+        !make_map_4d(&mdq, dq, d.dtype, B, H, R, DH, sq, BT) || !make_map_4d(&mdk, dk, d.dtype, B, H, R, DH, sk, BT) ||
+        !make_map_4d(&mdv, dv, d.dtype, B, H, R, DH, sv, BT) || !make_map_4d(&cq, q, d.dtype, B, H, R, DH, sq, CW) ||
+        !make_map_4d(&ck, k, d.dtype, B, H, R, DH, sk, CW) || !make_map_4d(&cv, v, d.dtype, B, H, R, DH, sv, CW) ||
+        !make_map_4d(&cdo, d_o, d.dtype, B, H, R, DH, so, CW))
         return TMW_ERR_CUDA;
     BwdParams p;
     p.rows = R; p.window = d.window; p.np = d.n_persistent;
@@ -735,10 +668,10 @@ bool prefill_backward_tc_supports(const tmw_prefill_desc& d) {
     if (d.head_dim != 64 && d.head_dim != 128) return false;
     if (d.batch > 65535 || d.heads > 65535) return false;
     if ((int64_t)d.q_rows + d.window + 2 * BT >= (int64_t)1 << 29) return false;  // (+ a block size of up to 2^20)
-    return strides_of(d.batch, d.heads, d.q_rows, d.head_dim, d.q_stride).ok &&
-           strides_of(d.batch, d.heads, d.q_rows, d.head_dim, d.k_stride).ok &&
-           strides_of(d.batch, d.heads, d.q_rows, d.head_dim, d.v_stride).ok &&
-           strides_of(d.batch, d.heads, d.q_rows, d.head_dim, d.o_stride).ok;
+    return map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.q_stride).ok &&
+           map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.k_stride).ok &&
+           map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.v_stride).ok &&
+           map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.o_stride).ok;
 }
 
 int launch_prefill_backward_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o,

@@ -36,6 +36,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "tensor_map.cuh"
 #include "tmw_common.cuh"
 
 namespace tmw {
@@ -991,114 +992,6 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 // ---------------------------------------------------------------------------------
 // Host side: tensor maps and launch
 // ---------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    });
-    return fn;
-}
-
-// Strides (in elements) that the tensor maps of a [batch, heads, rows, dh] tensor use.  The stride of an
-// extent-1 axis is never used for addressing; it gets a harmless valid value.
-struct MapStrides {
-    int64_t row, head, batch;
-    bool heads_first;  // the head axis has the smaller stride and comes before the row axis in the map
-};
-MapStrides map_strides(int batch, int heads, int rows, int dh, const int64_t stride[3]) {
-    MapStrides m;
-    m.row = rows > 1 ? stride[2] : dh;
-    m.head = heads > 1 ? stride[1] : m.row * rows;
-    const int64_t inner_span = m.head * heads > m.row * rows ? m.head * heads : m.row * rows;
-    m.batch = batch > 1 ? stride[0] : inner_span;
-    m.heads_first = m.head < m.row;
-    return m;
-}
-
-// What cuTensorMapEncodeTiled accepts: strides that are positive multiples of 16 bytes below 2^40 bytes.
-// (Broadcast views with a zero stride and the like go to the CUDA-core kernel.)
-bool map_strides_ok(const MapStrides& m) {
-    const int64_t limit = ((int64_t)1 << 40) / 2;
-    return m.row > 0 && m.head > 0 && m.batch > 0 && m.row < limit && m.head < limit && m.batch < limit &&
-           m.row % 8 == 0 && m.head % 8 == 0 && m.batch % 8 == 0;
-}
-
-// Encoded maps are kept per host thread, keyed by everything that goes into them: a caller that runs the same
-// buffers again (a layer inside a captured or repeated step) pays for the six driver calls once.
-struct MapKey {
-    const void* base;
-    int64_t row, head, batch_stride;
-    int32_t dtype, batch, heads, rows, dh, box_rows;
-    bool operator==(const MapKey& o) const {
-        return base == o.base && row == o.row && head == o.head && batch_stride == o.batch_stride && dtype == o.dtype &&
-               batch == o.batch && heads == o.heads && rows == o.rows && dh == o.dh && box_rows == o.box_rows;
-    }
-};
-struct MapCache {
-    static constexpr int kEntries = 64;
-    MapKey key[kEntries];
-    CUtensorMap map[kEntries];
-    bool used[kEntries] = {false};
-    int next = 0;
-};
-
-// Map over rows [0, rows) of a [batch, heads, *, dh] tensor laid out by `m`: a box of box_rows rows x 64
-// columns of one (batch, head).  Rows of a box at or beyond `rows` are filled with zeros on load and dropped
-// on store.  Returns false on failure.
-bool make_map(CUtensorMap* map, const void* base, int dtype, int batch, int heads, int rows, int dh,
-              const MapStrides& m, int box_rows) {
-    static thread_local MapCache cache;
-    const MapKey key{base, m.row, m.head, m.batch, dtype, batch, heads, rows, dh, box_rows};
-    for (int i = 0; i < MapCache::kEntries; ++i)
-        if (cache.used[i] && cache.key[i] == key) {
-            *map = cache.map[i];
-            return true;
-        }
-    EncodeTiledFn fn = encode_fn();
-    if (fn == nullptr) return false;
-    cuuint64_t dims[4];
-    cuuint64_t strides[3];
-    cuuint32_t box[4];
-    dims[0] = (cuuint64_t)dh;
-    box[0] = 64;
-    if (m.heads_first) {
-        dims[1] = (cuuint64_t)heads; strides[0] = (cuuint64_t)m.head * 2; box[1] = 1;
-        dims[2] = (cuuint64_t)rows;  strides[1] = (cuuint64_t)m.row * 2;  box[2] = (cuuint32_t)box_rows;
-    } else {
-        dims[1] = (cuuint64_t)rows;  strides[0] = (cuuint64_t)m.row * 2;  box[1] = (cuuint32_t)box_rows;
-        dims[2] = (cuuint64_t)heads; strides[1] = (cuuint64_t)m.head * 2; box[2] = 1;
-    }
-    dims[3] = (cuuint64_t)batch;
-    strides[2] = (cuuint64_t)m.batch * 2;
-    box[3] = 1;
-    const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
-    const CUtensorMapDataType dt = dtype == TMW_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    const CUresult r = fn(map, dt, 4, const_cast<void*>(base), dims, strides, box, elem_strides,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        char text[96];
-        snprintf(text, sizeof(text), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-        set_error_text(text);
-        return false;
-    }
-    const int slot = cache.next;
-    cache.next = (cache.next + 1) % MapCache::kEntries;
-    cache.key[slot] = key;
-    cache.map[slot] = *map;
-    cache.used[slot] = true;
-    return true;
-}
-
 int np_pad_of(int np) { return np > 0 ? ((np + 15) / 16) * 16 : 0; }
 
 template <int DH, int KS, int VS, int TILES, int RS>
@@ -1115,12 +1008,12 @@ int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const voi
     // np_pad are zero-filled instead of being read from the first sequence rows (whatever those hold - even
     // Inf or NaN bits of a buffer that is still being filled - must not reach 0 x V in the P V product).
     const int np_rows = d.n_persistent > 0 ? d.n_persistent : 1;
-    if (!make_map(&mq, q, d.dtype, d.batch, d.heads, d.q_rows, DH, sq, BM) ||
-        !make_map(&mk, k, d.dtype, d.batch, d.heads, d.k_rows, DH, sk, BN) ||
-        !make_map(&mv, v, d.dtype, d.batch, d.heads, d.k_rows, DH, sv, BN) ||
-        !make_map(&mo, o, d.dtype, d.batch, d.heads, d.q_rows, DH, so, BM) ||
-        !make_map(&mkp, k, d.dtype, d.batch, d.heads, np_rows, DH, sk, np_pad > 0 ? np_pad : 16) ||
-        !make_map(&mvp, v, d.dtype, d.batch, d.heads, np_rows, DH, sv, np_pad > 0 ? np_pad : 16))
+    if (!make_map_4d(&mq, q, d.dtype, d.batch, d.heads, d.q_rows, DH, sq, BM) ||
+        !make_map_4d(&mk, k, d.dtype, d.batch, d.heads, d.k_rows, DH, sk, BN) ||
+        !make_map_4d(&mv, v, d.dtype, d.batch, d.heads, d.k_rows, DH, sv, BN) ||
+        !make_map_4d(&mo, o, d.dtype, d.batch, d.heads, d.q_rows, DH, so, BM) ||
+        !make_map_4d(&mkp, k, d.dtype, d.batch, d.heads, np_rows, DH, sk, np_pad > 0 ? np_pad : 16) ||
+        !make_map_4d(&mvp, v, d.dtype, d.batch, d.heads, np_rows, DH, sv, np_pad > 0 ? np_pad : 16))
         return TMW_ERR_CUDA;
     TcParams p;
     p.q_rows = d.q_rows; p.k_rows = d.k_rows; p.window = d.window; p.np = d.n_persistent; p.np_pad = np_pad;
@@ -1175,10 +1068,10 @@ bool prefill_tc_supports(const tmw_prefill_desc& d, const void*, const void*, co
     // positions are combined in 32-bit arithmetic inside the kernel
     if ((int64_t)d.q_pos0 + d.q_rows + d.window + 4 * BN >= (int64_t)1 << 30) return false;
     // layouts a tensor map cannot describe
-    if (!map_strides_ok(map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.q_stride)) ||
-        !map_strides_ok(map_strides(d.batch, d.heads, d.k_rows, d.head_dim, d.k_stride)) ||
-        !map_strides_ok(map_strides(d.batch, d.heads, d.k_rows, d.head_dim, d.v_stride)) ||
-        !map_strides_ok(map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.o_stride)))
+    if (!map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.q_stride).ok ||
+        !map_strides(d.batch, d.heads, d.k_rows, d.head_dim, d.k_stride).ok ||
+        !map_strides(d.batch, d.heads, d.k_rows, d.head_dim, d.v_stride).ok ||
+        !map_strides(d.batch, d.heads, d.q_rows, d.head_dim, d.o_stride).ok)
         return false;
     return true;
 }

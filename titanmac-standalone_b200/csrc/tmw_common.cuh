@@ -88,6 +88,21 @@ __device__ __forceinline__ void store8<__half>(__half* p, const float (&in)[8]) 
     *reinterpret_cast<uint4*>(p) = raw;
 }
 
+// Exact (erf-based) GELU, 0.5 x (1 + erf(x / sqrt 2)), with erf from the rational approximation 7.1.26 of
+// Abramowitz & Stegun (absolute error below 1.5e-7, i.e. fp32 rounding noise against a 16-bit result): one reciprocal,
+// one exponential and a degree-5 polynomial instead of the library's branchy erff, which is longer than the products
+// or loads it sits behind.
+__device__ __forceinline__ float gelu_erf(float x) {
+    const float z = fabsf(x) * 0.70710678118654752f;
+    const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
+    float poly = fmaf(1.061405429f, t, -1.453152027f);
+    poly = fmaf(poly, t, 1.421413741f);
+    poly = fmaf(poly, t, -0.284496736f);
+    poly = fmaf(poly, t, 0.254829592f);
+    const float erf_abs = 1.0f - poly * t * __expf(-z * z);  // erf(|x| / sqrt 2)
+    return 0.5f * x * (1.0f + copysignf(erf_abs, x));
+}
+
 __host__ __device__ inline size_t dtype_size(int dtype) { return dtype == TMW_F32 ? 4 : 2; }
 
 // Position of the first sequence key that the sequence query at position `pos` (>= np) sees.
@@ -117,6 +132,43 @@ struct SideStream {
     std::mutex mutex;
 };
 SideStream* side_stream_of_current_device();  // nullptr if it cannot be made
+
+// ---- programmatic dependent launch ---------------------------------------------------
+// A chain of small kernels spends more time on launch, drain and cold loads than on work.  A kernel of such a chain
+// triggers the launch of its successor at once (launching takes about 2.5 us), loads what no kernel of the chain writes
+// (weights, cache rows) and then waits until its predecessor has finished - which has waited for its own.  The first
+// kernel of a chain is an ordinary launch: what the stream held before is complete when the chain starts.
+// Without the launch attribute both calls are no-ops.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// launch with the dependent-launch attribute and / or a cluster of `cluster` CTAs along x
+template <typename P>
+cudaError_t launch_ex(void (*kern)(P), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, int cluster,
+                      const P& params) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kern, params);
+}
+
+int sm_count();  // of the current device, asked once per device
 
 #define TMW_CUDA_TRY(expr)                                   \
     do {                                                     \
@@ -161,7 +213,7 @@ int launch_prefill_backward_tc(const tmw_prefill_desc& d, const void* q, const v
 bool prefill_tc_supports(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o);
 int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, const void* v_new, void* o,
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,
-                  int splits, float* scratch, unsigned int* counters, cudaStream_t stream);
+                  int splits, float* scratch, unsigned int* counters, cudaStream_t stream, bool pdl = false);
 
 // layout of the split-decode scratch memory: partial results, then (16-byte aligned) one counter per pair
 inline size_t decode_partials_bytes(int batch, int heads, int head_dim, int splits) {
@@ -170,6 +222,11 @@ inline size_t decode_partials_bytes(int batch, int heads, int head_dim, int spli
 }
 int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c,
                   cudaStream_t stream);
+// links of a chain of dependent launches (see pdl_wait): a product of up to a few hundred rows (epi: 0 = store, 1 = GELU,
+// 2 = added to c, which is read and written; n and k multiples of 8, contiguous rows), and the RMSNorm in front of it
+int launch_rows_tc(int dtype, int m, int n, int k, const void* a, const void* w, const void* bias, void* c, int epi,
+                   cudaStream_t stream);
+int launch_rows_norm(int dtype, int rows, int dim, const void* x, const void* gain, float eps, void* y, cudaStream_t stream);
 int launch_cache_fill(const tmw_cache_desc& c, const void* k, const void* v, const int64_t ks[3],
                       const int64_t vs[3], int rows, int t0, cudaStream_t stream);
 

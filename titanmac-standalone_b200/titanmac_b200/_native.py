@@ -7,6 +7,7 @@ or to the CPU.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import os
@@ -88,6 +89,24 @@ class LinearDesc(ctypes.Structure):
         ("lda", ctypes.c_int64),
         ("ldw", ctypes.c_int64),
         ("ldc", ctypes.c_int64),
+    ]
+
+
+class Block(ctypes.Structure):
+    """One layer of the whole-model calls (tmw_block)."""
+
+    _fields_ = [(n, ctypes.c_void_p) for n in ("norm_attn", "w_qkv", "w_out", "norm_mlp", "w_fc1", "b_fc1", "w_fc2", "b_fc2",
+                                               "k_ring", "v_ring", "k_pers", "v_pers")] + [("cache_scale", ctypes.c_float)]
+
+
+class StackDesc(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int32) for n in ("dtype", "batch", "layers", "d_model", "heads", "head_dim", "d_ff", "window",
+                                              "n_persistent", "vocab", "max_positions")] + [
+        ("eps", ctypes.c_float),
+        ("embed_tokens", ctypes.c_void_p),
+        ("embed_positions", ctypes.c_void_p),
+        ("norm", ctypes.c_void_p),
+        ("head", ctypes.c_void_p),
     ]
 
 
@@ -179,6 +198,11 @@ SIGNATURES = {
          ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64),
          ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p],
     ),
+    "tmw_decode_step_workspace": (ctypes.c_size_t, [ctypes.POINTER(StackDesc)]),
+    "tmw_decode_step": (
+        ctypes.c_int,
+        [ctypes.POINTER(StackDesc), ctypes.POINTER(Block)] + [ctypes.c_void_p] * 4 + [ctypes.c_size_t, ctypes.c_void_p],
+    ),
     "tmw_halo_push": (
         ctypes.c_int,
         [ctypes.POINTER(HaloCopy), ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
@@ -244,6 +268,14 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
 
 def _stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_no_guard = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """``torch.cuda.device(device)``, for nothing where that device is the current one already."""
+    return _no_guard if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _bhrd_strides(t: torch.Tensor) -> Sequence[int]:
@@ -389,6 +421,7 @@ class RingCache:
         self.window, self.n_persistent = window, n_persistent
         self.slots = window + 1
         self.dtype, self.device, self.scale = dtype, torch.device(device), scale
+        self.geometry = (batch, heads, head_dim, window, n_persistent, dtype)
         nbytes = lib().tmw_cache_ring_bytes(_DTYPES[dtype], batch, heads, head_dim, window)
         elems = nbytes // torch.empty((), dtype=dtype).element_size()
         assert elems == batch * heads * self.slots * head_dim

@@ -1,0 +1,184 @@
+"""The model as the flat table that the whole-model calls of libtmw take (``tmw_block`` / ``tmw_stack_desc``).
+
+A step of a few rows is bound by its host work when every norm, product and attention call is issued from Python, so
+``TitanMAC`` hands the library one table per call.  The table is built once and holds addresses only: before every use
+it is checked against the modules it was built from, and rebuilt when a parameter has moved or a module has been
+replaced.  A model that the table cannot describe - another type of module in a known place, hooks, fp32, an active
+dropout - has no table, and its modules are called one by one.
+"""
+
+from __future__ import annotations
+
+import ctypes
+import weakref
+from typing import List, Optional
+
+import torch
+import torch.nn as nn
+from torch.nn.modules import module as _nn_module
+
+from . import _native
+
+
+def _global_hooks() -> bool:
+    return bool(_nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks)
+
+
+class ModelTable:
+    """Addresses of a ``TitanMAC``'s parameters and how to tell that they still hold."""
+
+    def __init__(self, model):
+        from .attn.windowed_attention import WindowedAttention
+        from .blocks.titan_block import MLPBlock, RMSNorm, TitanBlock
+
+        self.ok = False
+        self._params: list = []    # (parameter dict of a module, name, address)
+        self._children: list = []  # (child dict of a module, name, child)
+        self._modules: list = []
+        self._dropouts: list = []
+        self.dtype = model.embed_tokens.weight.dtype
+        self.device = model.embed_tokens.weight.device
+        if self.dtype not in (torch.bfloat16, torch.float16) or self.device.type != "cuda":
+            return
+        c = model.config
+
+        def take(parent: nn.Module, name: str, *types) -> Optional[nn.Module]:
+            child = parent._modules.get(name)
+            self._children.append((parent._modules, name, child))
+            if type(child) not in types:
+                return None
+            if isinstance(child, nn.Dropout):
+                self._dropouts.append(child)
+            self._modules.append(child)
+            return child
+
+        def address(mod: nn.Module, name: str, shape) -> Optional[int]:
+            prm = mod._parameters.get(name)
+            if prm is None or prm.dtype != self.dtype or tuple(prm.shape) != tuple(shape) or not prm.is_contiguous() \
+                    or prm.device != self.device or prm.data_ptr() % 16:
+                return None
+            self._params.append((mod._parameters, name, prm.data_ptr()))
+            return prm.data_ptr()
+
+        def optional(mod: nn.Module, name: str, shape):
+            if mod._parameters.get(name) is None:
+                self._params.append((mod._parameters, name, 0))
+                return 0
+            return address(mod, name, shape)
+
+        D, V = c.d_model, c.vocab_size
+        layers = take(model, "layers", nn.ModuleList)
+        tops = (take(model, "embed_tokens", nn.Embedding), take(model, "embed_positions", nn.Embedding),
+                take(model, "norm", RMSNorm), take(model, "lm_head", nn.Linear))
+        if layers is None or len(layers) == 0 or any(t is None for t in tops) or tops[3].bias is not None:
+            return
+        F = layers[0].mlp.d_ff if type(layers[0]) is TitanBlock and type(layers[0].mlp) is MLPBlock else 0
+        found: List[Optional[int]] = []
+        self.blocks = (_native.Block * len(layers))()
+        for i in range(len(layers)):
+            block = take(layers, str(i), TitanBlock)
+            if block is None:
+                return
+            attn, mlp = take(block, "attention", WindowedAttention), take(block, "mlp", MLPBlock)
+            norms = (take(block, "norm_attn", RMSNorm), take(block, "norm_mlp", RMSNorm))
+            if attn is None or mlp is None or None in norms or any(n.eps != c.norm_eps for n in norms):
+                return
+            if (attn.n_heads, attn.d_head, attn.window_size, attn.num_persistent) != (c.n_heads, c.d_head, c.window_size,
+                                                                                     c.n_persistent) or mlp.d_ff != F:
+                return
+            qkv, out = take(attn, "qkv_proj", nn.Linear), take(attn, "out_proj", nn.Linear)
+            fc1, fc2 = take(mlp, "fc1", nn.Linear), take(mlp, "fc2", nn.Linear)
+            if None in (qkv, out, fc1, fc2) or qkv.bias is not None or out.bias is not None:
+                return
+            if take(attn, "dropout", nn.Identity, nn.Dropout) is None or take(mlp, "dropout", nn.Identity, nn.Dropout) is None \
+                    or take(mlp, "activation", nn.GELU) is None or mlp.activation.approximate != "none":
+                return
+            b = self.blocks[i]
+            values = dict(norm_attn=address(norms[0], "scale", (D,)), norm_mlp=address(norms[1], "scale", (D,)),
+                          w_qkv=address(qkv, "weight", (3 * D, D)), w_out=address(out, "weight", (D, D)),
+                          w_fc1=address(fc1, "weight", (F, D)), w_fc2=address(fc2, "weight", (D, F)),
+                          b_fc1=optional(fc1, "bias", (F,)), b_fc2=optional(fc2, "bias", (D,)))
+            found += values.values()
+            for name, value in values.items():
+                setattr(b, name, value or None)
+        d = self.desc = _native.StackDesc()
+        top = (address(tops[0], "weight", (V, D)), address(tops[1], "weight", (c.max_seq_len, D)), address(tops[2], "scale", (D,)),
+               address(tops[3], "weight", (V, D)))
+        if None in found or None in top or tops[2].eps != c.norm_eps or tops[0].max_norm is not None \
+                or tops[1].max_norm is not None:
+            return
+        d.embed_tokens, d.embed_positions, d.norm, d.head = top
+        d.dtype = _native._DTYPES[self.dtype]
+        d.layers, d.d_model, d.heads, d.head_dim, d.d_ff = len(layers), D, c.n_heads, c.d_head, F
+        d.window, d.n_persistent, d.vocab, d.max_positions, d.eps = c.window_size, c.n_persistent, V, c.max_seq_len, c.norm_eps
+        self.geometry = (c.n_heads, c.d_head, c.window_size, c.n_persistent, self.dtype)
+        self.supported = c.d_head in (64, 128) and F % 32 == 0
+        self.workspace_bytes: dict = {}  # batch -> bytes
+        self.ok = True
+
+    def holds(self) -> bool:
+        """Whether the modules are still the ones, and their parameters still where, the table says."""
+        dtype = self.dtype
+        for d, name, child in self._children:
+            if d.get(name) is not child:
+                return False
+        for d, name, ptr in self._params:
+            prm = d.get(name)
+            if prm is None:
+                if ptr:
+                    return False
+            elif prm.data_ptr() != ptr or prm.dtype is not dtype:
+                return False
+        return True
+
+    def plain_call(self) -> bool:
+        """Whether calling the modules would do nothing but compute: no hooks, no active dropout."""
+        for m in self._modules:
+            if m._forward_hooks or m._forward_pre_hooks:
+                return False
+        for m in self._dropouts:
+            if m.training and m.p > 0:
+                return False
+        return not _global_hooks()
+
+
+# not an attribute of the model: copies and pickles of a model do not carry addresses
+_tables: "weakref.WeakKeyDictionary[nn.Module, ModelTable]" = weakref.WeakKeyDictionary()
+
+
+def table_of(model) -> Optional[ModelTable]:
+    """The model's table if it can be used right now, else None."""
+    table = _tables.get(model)
+    if table is None or not table.holds():
+        table = _tables[model] = ModelTable(model)
+    return table if table.ok and table.supported and table.plain_call() else None
+
+
+def decode_step(table: ModelTable, token_ids: torch.Tensor, pos: torch.Tensor, caches) -> Optional[torch.Tensor]:
+    """``tmw_decode_step``; None where the arguments are not what that call takes."""
+    B = token_ids.shape[0]
+    device = table.device
+    if (B == 0 or token_ids.dtype != torch.int64 or pos.dtype != torch.int32 or token_ids.dim() != 1 or pos.shape != (B,)
+            or token_ids.device != device or pos.device != device or len(caches) != len(table.blocks)):
+        return None
+    token_ids, pos = token_ids.contiguous(), pos.contiguous()
+    geometry = (B,) + table.geometry
+    blocks = type(table.blocks).from_buffer_copy(table.blocks)  # (the table is shared by all threads)
+    for b, c in zip(blocks, caches):
+        if c.geometry != geometry or c.k_ring.device != device:
+            return None
+        b.k_ring, b.v_ring = c.k_ring.data_ptr(), c.v_ring.data_ptr()
+        b.k_pers, b.v_pers = c.k_pers.data_ptr(), c.v_pers.data_ptr()
+        b.cache_scale = c.scale
+    d = _native.StackDesc.from_buffer_copy(table.desc)
+    d.batch = B
+    lib = _native.lib()
+    nbytes = table.workspace_bytes.get(B)
+    if nbytes is None:
+        nbytes = table.workspace_bytes[B] = lib.tmw_decode_step_workspace(ctypes.byref(d))
+    workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    logits = torch.empty((B, d.vocab), dtype=table.dtype, device=device)
+    with _native._on(device):
+        _native.check(lib.tmw_decode_step(ctypes.byref(d), blocks, token_ids.data_ptr(), pos.data_ptr(),
+                                          logits.data_ptr(), workspace.data_ptr(), nbytes, _native._stream_ptr(device)))
+    return logits

@@ -28,7 +28,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .. import _native
+from .. import _native, _stack
 from ..blocks.titan_block import RMSNorm, TitanBlock
 
 
@@ -148,6 +148,11 @@ class TitanMAC(nn.Module):
         """One new token per sequence.  ``token_ids [B]``, ``pos [B] int32`` = its index in the sequence
         (the prompt occupied 0..T-1).  Returns logits ``[B, V]``; ``pos`` is not modified."""
         self._need_windowed()
+        table = _stack.table_of(self)
+        if table is not None:  # the whole step as one call (tmw_decode_step)
+            logits = _stack.decode_step(table, token_ids, pos, caches)
+            if logits is not None:
+                return logits
         c = self.config
         B = token_ids.shape[0]
         x = self.embed_tokens(token_ids) + self.embed_positions(pos.long())
