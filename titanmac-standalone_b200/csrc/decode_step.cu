@@ -483,7 +483,7 @@ int decode_step_t(const tmw_stack_desc& d, const tmw_block* blocks, const int64_
     auto normed = [&](const void* gain, const void* w, const void* bias, int n, void* c, int epi) {
         if (tc) {
             const int rc = launch_rows_norm(d.dtype, B, D, x, gain, d.eps, y, stream);
-            return rc != TMW_OK ? rc : launch_rows_tc(d.dtype, B, n, D, y, w, bias, c, epi, stream);
+            return rc != TMW_OK ? rc : launch_rows_tc(d.dtype, B, n, D, y, w, bias, c, epi, stream, true);
         }
         p.a = x; p.lda = D; p.k = D; p.w = w; p.bias = bias; p.n = n; p.c = c; p.ldc = n;
         p.gain = gain; p.ss_in = ss; p.ss_parts = parts; p.ss_out = nullptr;
@@ -492,7 +492,7 @@ int decode_step_t(const tmw_stack_desc& d, const tmw_block* blocks, const int64_
                                : launch_rows<T, true, EPI_STORE>(p, &unused, stream);
     };
     auto back = [&](const void* a, int k, const void* w, const void* bias) {
-        if (tc) return launch_rows_tc(d.dtype, B, D, k, a, w, bias, x, EPI_RESIDUAL, stream);
+        if (tc) return launch_rows_tc(d.dtype, B, D, k, a, w, bias, x, EPI_RESIDUAL, stream, true);
         p.a = a; p.lda = k; p.k = k; p.w = w; p.bias = bias; p.n = D; p.c = x; p.ldc = D; p.ss_out = ss;
         return launch_rows<T, false, EPI_RESIDUAL>(p, &parts, stream);
     };

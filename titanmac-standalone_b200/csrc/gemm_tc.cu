@@ -14,7 +14,7 @@
 // the device status word.
 #include <cuda.h>
 
-#include <cstdio>
+#include <cmath>
 #include <mutex>
 
 #include "tc_ptx.cuh"
@@ -34,8 +34,11 @@ constexpr int kGemmThreads = 32 * (2 + kEpiWarps);
 
 template <int BN>
 struct GemmSmem {
-    static constexpr int kStageA = GM * GK * 2;
-    static constexpr int kStageB = BN * GK * 2;
+    // 64-wide slices of K per stage: a tcgen05.commit costs the issuing thread about 220 cycles, which the products of
+    // one slice cover only where the tile is wide (K = 2560, us: 128 columns 10.4 -> 8.7, 32 columns 9.3 -> 7.0)
+    static constexpr int kSlices = BN <= 128 ? 2 : 1;
+    static constexpr int kStageA = kSlices * GM * GK * 2;
+    static constexpr int kStageB = kSlices * BN * GK * 2;
     static constexpr int kStage = kStageA + kStageB;
     static constexpr int kOut = GM * BN * 2;  // staging of one output tile: BN / 32 panels of 128 rows x 64 bytes
     static constexpr int kStages = (232448 - 2048 - kOut) / kStage;
@@ -74,7 +77,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = (p.n + BN - 1) / BN, m_tiles = (p.m + GM - 1) / GM;
     const int tiles = n_tiles * m_tiles;
-    const int k_blocks = (p.k + GK - 1) / GK;
+    const int k_blocks = (p.k + L::kSlices * GK - 1) / (L::kSlices * GK);
 
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
@@ -97,48 +100,57 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    constexpr int SL = L::kSlices;
     if (warp == 0) {
         // ---------------- producer ----------------
-        int n = 0;  // stages filled so far
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            const int row0 = (tile / n_tiles) * GM, col0 = (tile % n_tiles) * BN;
-            for (int kb = 0; kb < k_blocks; ++kb, ++n) {
-                const int s = n % S;
-                mbar_wait(empty(s), ((n / S) & 1) ^ 1, abort_flag, p.status);
-                if (lane == 0) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t parity = 1;
+            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+                const int row0 = (tile / n_tiles) * GM, col0 = (tile % n_tiles) * BN;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    mbar_wait(empty(s), parity, abort_flag, p.status);
                     mbar_expect_tx(full(s), L::kStage);
                     const uint32_t dst = smem_base + s * L::kStage;
-                    tma_load_2d(dst, &map_a, full(s), kb * GK, row0);
-                    tma_load_2d(dst + L::kStageA, &map_w, full(s), kb * GK, col0);
+#pragma unroll
+                    for (int u = 0; u < SL; ++u) {  // (slices beyond K arrive as zeros)
+                        tma_load_2d(dst + u * (GM * GK * 2), &map_a, full(s), (kb * SL + u) * GK, row0);
+                        tma_load_2d(dst + L::kStageA + u * (BN * GK * 2), &map_w, full(s), (kb * SL + u) * GK, col0);
+                    }
+                    if (++s == S) { s = 0; parity ^= 1u; }
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- tensor-core issue ----------------
-        const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, BN);
-        int n = 0, t = 0;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
-            const int buf = t & 1;
-            mbar_wait(acc_empty(buf), ((t >> 1) & 1) ^ 1, abort_flag, p.status);  // the epilogue has drained it
-            tc_fence_after();
-            const uint32_t d_tmem = tmem_base + buf * BN;
-            for (int kb = 0; kb < k_blocks; ++kb, ++n) {
-                const int s = n % S;
-                mbar_wait(full(s), (n / S) & 1, abort_flag, p.status);
+        if (elect_one()) {
+            const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, BN);
+            int s = 0, t = 0;
+            uint32_t parity = 0;
+            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
+                const int buf = t & 1;
+                mbar_wait(acc_empty(buf), ((t >> 1) & 1) ^ 1, abort_flag, p.status);  // the epilogue has drained it
                 tc_fence_after();
-                if (lane == 0) {
+                const uint32_t d_tmem = tmem_base + buf * BN;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    mbar_wait(full(s), parity, abort_flag, p.status);
+                    tc_fence_after();
                     const uint64_t a_desc = kmajor_desc(smem_base + s * L::kStage);
                     const uint64_t b_desc = kmajor_desc(smem_base + s * L::kStage + L::kStageA);
 #pragma unroll
-                    for (int kk = 0; kk < GK / 16; ++kk)
-                        mma_ss(d_tmem, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                    for (int u = 0; u < SL; ++u)
+#pragma unroll
+                        for (int kk = 0; kk < GK / 16; ++kk)
+                            mma_ss(d_tmem, a_desc + u * (GM * GK * 2 / 16) + 2 * kk, b_desc + u * (BN * GK * 2 / 16) + 2 * kk,
+                                   idesc, (kb | u | kk) ? 1u : 0u);
                     tc_commit(empty(s));  // the stage is free once these products have read it
                     if (kb == k_blocks - 1) tc_commit(acc_full(buf));
+                    if (++s == S) { s = 0; parity ^= 1u; }
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else {
         // ---------------- epilogue ----------------
         const int g = warp & 3;             // lane group of tensor memory this warp may read
@@ -219,7 +231,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 tma_store_commit();
             }
         }
-        if (epi_leader) tma_store_wait_all();
+        if (epi_leader) tma_store_wait_read();  // (the stores themselves complete with the grid)
     }
 
     tc_fence_before();
@@ -315,51 +327,51 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ---------------- producer (both CTAs) ----------------
-        int n = 0;
-        for (int tile = pair; tile < tiles; tile += pairs) {
-            const int row0 = (tile / n_tiles) * (2 * GM) + (int)rank * GM;
-            // each CTA supplies half of the tile's columns (the box is BN / 2 rows; a narrow tile uses its first rows)
-            const int col0 = (tile % n_tiles) * BN + (int)rank * (n_of(tile) / 2);
-            for (int kb = 0; kb < k_blocks; ++kb, ++n) {
-                const int s = n % S;
-                mbar_wait(empty(s), ((n / S) & 1) ^ 1, abort_flag, p.status);
-                if (lane == 0) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t parity = 1;
+            for (int tile = pair; tile < tiles; tile += pairs) {
+                const int row0 = (tile / n_tiles) * (2 * GM) + (int)rank * GM;
+                // each CTA supplies half of the tile's columns (the box is BN / 2 rows; a narrow tile uses its first rows)
+                const int col0 = (tile % n_tiles) * BN + (int)rank * (n_of(tile) / 2);
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    mbar_wait(empty(s), parity, abort_flag, p.status);
                     if (rank == 0) mbar_expect_tx(full(s), 2 * L::kStage);  // both CTAs' bytes
                     const uint32_t bar0 = map_to_cta(full(s), 0);
                     const uint32_t dst = smem_base + s * L::kStage;
                     tma_load_2d_pair(dst, &map_a, bar0, kb * GK, row0);
                     tma_load_2d_pair(dst + L::kStageA, &map_w, bar0, kb * GK, col0);
+                    if (++s == S) { s = 0; parity ^= 1u; }
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- tensor-core issue (first CTA of the pair only) ----------------
-        if (rank == 0) {
-            int n = 0, t = 0;
+        if (rank == 0 && elect_one()) {
+            int s = 0, t = 0;
+            uint32_t parity = 0;
             for (int tile = pair; tile < tiles; tile += pairs, ++t) {
                 const int buf = t & 1;
                 const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, (uint32_t)n_of(tile), 2 * GM);
                 mbar_wait(acc_empty(buf), ((t >> 1) & 1) ^ 1, abort_flag, p.status);
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < k_blocks; ++kb, ++n) {
-                    const int s = n % S;
-                    mbar_wait(full(s), (n / S) & 1, abort_flag, p.status);
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    mbar_wait(full(s), parity, abort_flag, p.status);
                     tc_fence_after();
-                    if (lane == 0) {
-                        const uint64_t a_desc = kmajor_desc(smem_base + s * L::kStage);
-                        const uint64_t b_desc = kmajor_desc(smem_base + s * L::kStage + L::kStageA);
+                    const uint64_t a_desc = kmajor_desc(smem_base + s * L::kStage);
+                    const uint64_t b_desc = kmajor_desc(smem_base + s * L::kStage + L::kStageA);
 #pragma unroll
-                        for (int kk = 0; kk < GK / 16; ++kk)
-                            mma_ss_pair(d_tmem, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
-                        tc_commit_pair(empty(s));
-                        if (kb == k_blocks - 1) tc_commit_pair(acc_full(buf));
-                    }
-                    __syncwarp();
+                    for (int kk = 0; kk < GK / 16; ++kk)
+                        mma_ss_pair(d_tmem, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                    tc_commit_pair(empty(s));
+                    if (kb == k_blocks - 1) tc_commit_pair(acc_full(buf));
+                    if (++s == S) { s = 0; parity ^= 1u; }
                 }
             }
         }
+        __syncwarp();
     } else {
         // ---------------- epilogue (both CTAs, each its own 128 rows) ----------------
         const int g = warp & 3;
@@ -437,7 +449,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 tma_store_commit();
             }
         }
-        if (epi_leader) tma_store_wait_all();
+        if (epi_leader) tma_store_wait_read();  // (the stores themselves complete with the grid)
     }
 
     tc_fence_before();
@@ -545,23 +557,40 @@ int launch_gemm_pair(const tmw_linear_desc& d, const void* a, const void* w, con
 
 }  // namespace
 
+// Which kernel: the one whose waves of tiles take the least time, with what each was measured to need (us): a launch
+// without its K, what a 64-wide slice of K takes where a tile is alone on the chip, and where all SMs stream operands.  A
+// long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 6.5 us against 8.2).  The pair kernel moves the fewest operand bytes per product and wins wherever it has enough
+// tiles: measured at K = 640 for 1056 | 2528 | 8256 | 32 896 rows of N = 1920, pair | 128 | 64 columns: 9.3 | 12.6 | 21.3 |
+// 68.8, 6.3 | 11.4 | 24.1 | 82.5, 7.1 | 11.7 | 29.0 us.
 int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream) {
-    const int m_tiles = (d.m + GM - 1) / GM;
-    if (m_tiles <= 2) {
-        // Few rows (a decode step): the weights are streamed once and the work is spread by narrow column tiles -
-        // the widest tile that still gives most SMs a tile of their own.
-        const int want = sm_count() * 2 / 3;
-        auto tiles = [&](int bn) { return m_tiles * ((d.n + bn - 1) / bn); };
-        if (tiles(256) >= want) return launch_gemm<256>(d, a, w, bias, c, stream);
-        if (tiles(128) >= want) return launch_gemm<128>(d, a, w, bias, c, stream);
-        if (tiles(64) >= want) return launch_gemm<64>(d, a, w, bias, c, stream);
-        return launch_gemm<32>(d, a, w, bias, c, stream);
+    struct Variant { int rows, cols, units; float launch, alone, full; };
+    const int sms = sm_count();
+    const Variant variants[] = {{2 * GM, 256, sms / 2, 6.1f, 0.28f, 0.46f}, {GM, 256, sms, 5.0f, 0.305f, 0.54f},
+                                {GM, 128, sms, 4.2f, 0.167f, 0.306f},       {GM, 64, sms, 3.7f, 0.128f, 0.186f},
+                                {GM, 32, sms, 3.5f, 0.117f, 0.135f}};
+    const float slices = (float)((d.k + GK - 1) / GK);
+    if (slices >= 16.f && 2 * ((d.m + GM - 1) / GM) * ((d.n + 31) / 32) <= sms && d.lda == d.k && d.ldw == d.k && d.ldc == d.n)
+        return launch_rows_tc(d.dtype, d.m, d.n, d.k, a, w, bias, c, d.epilogue, stream, false);
+    int best = 0;
+    float least = 0.f;
+    for (int i = 0; i < 5; ++i) {
+        const Variant& v = variants[i];
+        // (the pair kernel's last tile of a row multiplies only the columns that exist)
+        const float cols = i == 0 ? (float)((d.n + 31) / 32) / 8.f : (float)((d.n + v.cols - 1) / v.cols);
+        const float load = (float)((d.m + v.rows - 1) / v.rows) * cols / (float)v.units;
+        const float t = v.launch + slices * (load <= 1.f ? v.alone + (v.full - v.alone) * load : v.full * ceilf(load));
+        if (i == 0 || t < least) {
+            best = i;
+            least = t;
+        }
     }
-    // Many rows: CTA pairs on 256 x 256 tiles, the shape that moves the fewest operand bytes per product.  That
-    // stream (L2 -> shared memory) is what bounds the kernel, so the wide tile wins even where the last tile of a
-    // row is partly empty: measured at M = 32 896, K = 640 for N = 1920 / 640 with tiles of 256 | 192 | 160 | 128
-    // columns: 71.9 | 77.4 | 85.6 | 103.8 us and 31.0 | 33.1 | 33.2 | 39.4 us.
-    return launch_gemm_pair<256>(d, a, w, bias, c, stream);
+    switch (best) {
+        case 0: return launch_gemm_pair<256>(d, a, w, bias, c, stream);
+        case 1: return launch_gemm<256>(d, a, w, bias, c, stream);
+        case 2: return launch_gemm<128>(d, a, w, bias, c, stream);
+        case 3: return launch_gemm<64>(d, a, w, bias, c, stream);
+        default: return launch_gemm<32>(d, a, w, bias, c, stream);
+    }
 }
 
 }  // namespace tmw

@@ -230,7 +230,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
 
     if (warp == 0) {
         // ---------------- producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(bar(BAR_R_FULL), 2 * L::kTile);
             int c1, c2;
             coords(kR1, r0, c1, c2);
@@ -243,7 +243,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         for (int n = 0; n < n_cols; ++n) {
             const int s = n % kColStages;
             mbar_wait(bar(BAR_C_EMPTY + s), ((n / kColStages) & 1) ^ 1, abort_flag, p.status);
-            if (lane == 0) {
+            if (elect_one()) {
                 mbar_expect_tx(bar(BAR_C_FULL + s), 2 * L::kCTile);
                 const uint32_t dst = smem_base + L::kC + s * 2 * L::kCTile;
                 const int row = col_tile(n) * CW;
@@ -288,9 +288,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         // warp 2:  Y = R2 C2^T,  then  dK += dS^T Q  or  dQ += dS K           (dS lies over Y)
         // The products of one thread execute in issue order, so each warp's next X / Y overwrites the P / dS that
         // its own earlier product has consumed.  Two issuing threads because one thread feeds the pipe with short
-        // products (N = 64, K = 16) at well below the rate the pipe runs them.  (The whole warp runs the loop and
-        // computes the operands; one lane issues - a lone lane inside a divergent branch issues markedly slower.)
-        const bool leader = lane == 0;
+        // products (N = 64, K = 16) at well below the rate the pipe runs them.  (elect_one has what
+        // it costs to pick that thread by its lane number.)
+        if (elect_one()) {  // one thread runs the whole role
         const bool second = warp == 2;
         const uint32_t fmt = BF16 ? 1u : 0u;
         const uint32_t idesc_xy = idesc_kmajor(fmt, CW);
@@ -312,10 +312,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             for (int kk = 0; kk < DH / 16; ++kk) {
                 const uint64_t ad = kmajor_desc(r_addr + (kk / 4) * L::kSub + (kk % 4) * 32);
                 const uint64_t bd = kmajor_desc(c_tile + (kk / 4) * L::kCSub + (kk % 4) * 32);
-                if (leader) mma_ss(tmem_base + (second ? kY : kX), ad, bd, idesc_xy, kk > 0 ? 1u : 0u);
+                mma_ss(tmem_base + (second ? kY : kX), ad, bd, idesc_xy, kk > 0 ? 1u : 0u);
             }
-            if (leader) tc_commit(bar(BAR_XY_FULL));
-            __syncwarp();
+            tc_commit(bar(BAR_XY_FULL));
             // (the next column tile has usually landed: seeing it now takes that wait off the path hand-over ->
             // products of this tile -> X / Y of the next)
             if (n + 1 < n_cols)
@@ -331,14 +330,12 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
                 const uint32_t acc = n > 0 ? 1u : 0u;
 #pragma unroll
                 for (int kk = 0; kk < CW / 16; ++kk) {
-                    if (leader) mma_ts(d_acc, a_base + packed_col(kk), b0 + kk * 128, idesc_acc, kk > 0 ? 1u : acc);
+                    mma_ts(d_acc, a_base + packed_col(kk), b0 + kk * 128, idesc_acc, kk > 0 ? 1u : acc);
                 }
             }
-            if (leader) {
-                tc_commit(bar(BAR_C_EMPTY + s));
-                if (n == n_cols - 1) tc_commit(bar(BAR_ACC_DONE));
-            }
-            __syncwarp();
+            tc_commit(bar(BAR_C_EMPTY + s));
+            if (n == n_cols - 1) tc_commit(bar(BAR_ACC_DONE));
+        }
         }
     } else if (warp >= 4) {
         // ---------------- element-wise warps: two threads per row of the tile, half of the columns each ----------------
@@ -544,6 +541,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         }
     }
 
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

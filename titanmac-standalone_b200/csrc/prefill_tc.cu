@@ -36,11 +36,14 @@
 #include <mutex>
 #include <type_traits>
 
+#include "tc_ptx.cuh"
 #include "tensor_map.cuh"
 #include "tmw_common.cuh"
 
 namespace tmw {
 namespace {
+
+using namespace ptx;
 
 // Threads and register budget per query tiles of a CTA.  Two tiles: 384 threads launched with 168 registers
 // (one CTA per SM).  One tile: 256 threads launched with 128 registers (two CTAs per SM).  The four
@@ -62,7 +65,6 @@ struct Budget {
 };
 constexpr int BM = 128;  // query rows per tile
 constexpr int BN = 128;  // keys per tile
-constexpr long long kWaitLimitCycles = 2000000000LL;  // about one second
 // The two softmax groups of a two-tile CTA take turns with their exponentials for head_dim 128 (measured: +10 %
 // at head_dim 128 / window 1024, -6 % at head_dim 64 / window 512, where it is off).
 template <int DH>
@@ -135,83 +137,12 @@ __device__ __forceinline__ void flag_wait(const int* flag, int value, long long 
 }
 
 // ---------------------------------------------------------------------------------
-// PTX wrappers
+// PTX wrappers beyond tc_ptx.cuh
 // ---------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Bounded wait.  `abort_flag` lives in shared memory; once it is set nobody waits any more.  The first
-// wait that expires on the device also records where it was: status[1] = shared-memory offset of the
-// barrier and parity, status[2] = blockIdx.x | blockIdx.y << 16, status[3] = blockIdx.z | warp << 16.
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
-    if (mbar_try_wait(bar, parity)) return;
-    const long long t0 = clock64();
-    uint32_t spins = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if ((++spins & 63u) == 0u) {
-            if (*abort_flag) return;
-            if (clock64() - t0 > kWaitLimitCycles) {
-                *abort_flag = 1;
-                if (atomicCAS(status, 0, (int)TMW_ERR_DEVICE_TIMEOUT) == 0) {
-                    status[1] = (int)((bar & 0xffffu) | (parity << 16));
-                    status[2] = (int)(blockIdx.x | (blockIdx.y << 16));
-                    status[3] = (int)(blockIdx.z | ((threadIdx.x >> 5) << 16));
-                }
-                return;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2,
-                                            int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map),
-                 "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
 __device__ __forceinline__ void tma_store_commit_and_wait() {
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    tma_store_commit();
+    tma_store_wait_read();
 }
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void named_barrier_sync(int id, int threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -237,70 +168,9 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return d;
 }
 
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-#define TMW_R8(a, o)                                                                                        \
-    "=r"(a[o + 0]), "=r"(a[o + 1]), "=r"(a[o + 2]), "=r"(a[o + 3]), "=r"(a[o + 4]), "=r"(a[o + 5]),        \
-        "=r"(a[o + 6]), "=r"(a[o + 7])
 #define TMW_I8(a, o)                                                                                        \
     "r"(a[o + 0]), "r"(a[o + 1]), "r"(a[o + 2]), "r"(a[o + 3]), "r"(a[o + 4]), "r"(a[o + 5]), "r"(a[o + 6]), \
         "r"(a[o + 7])
-
-// 32 lanes x 32 consecutive columns: thread t of the warp gets lane (base lane + t)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : TMW_R8(r, 0), TMW_R8(r, 8), TMW_R8(r, 16), TMW_R8(r, 24)
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : TMW_R8(r, 0), TMW_R8(r, 8)
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-        ::"r"(taddr), TMW_I8(r, 0)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-        ::"r"(taddr), TMW_I8(r, 0), TMW_I8(r, 8)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -489,14 +359,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     if (warp < 4) {
         // register budget: see Budget
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Budget<TILES, RS>::kRegsService) : "memory");
-        // Every role warp runs its loop with all 32 lanes (so the warp never splits into a running
-        // lane and 31 lanes parked at the final barrier); one lane issues the asynchronous operations.
-        const bool leader = lane == 0;
         if (warp == 0) {
             // ---------------- producer: Q tiles, then K tiles ----------------
 #pragma unroll
             for (int t = 0; t < TILES; ++t) {
-                if (plan.qt[t].rows == 0 || !leader) continue;
+                if (plan.qt[t].rows == 0 || !elect_one()) continue;
                 mbar_expect_tx(bar(BAR_Q_FULL + t), L::kTileBytes);
                 int c1, c2;
                 coords(0, (blockIdx.x * TILES + t) * BM, c1, c2);
@@ -513,7 +380,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     halo_seen = true;
                 }
                 mbar_wait(bar(BAR_K_EMPTY + s), ((n / KS) & 1) ^ 1, abort_flag, p.status);
-                if (leader) {
+                if (elect_one()) {
                     mbar_expect_tx(bar(BAR_K_FULL + s), L::kTileBytes);
                     int c1, c2;
                     coords(1, p.np + plan.anchor + x * BN - p.k_pos0, c1, c2);
@@ -528,7 +395,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             // (the persistent maps end at row np: rows np .. np_pad - 1 of the tile arrive as zeros)
             if (p.np > 0 && p.pers_flag != nullptr)
                 flag_wait(p.pers_flag, p.flag_value, p.flag_wait_limit, abort_flag, p.status);
-            if (p.np > 0 && leader) {
+            if (p.np > 0 && elect_one()) {
                 mbar_expect_tx(bar(BAR_KP_FULL), 2 * pers_bytes);
                 int c1, c2;
                 coords(1, 0, c1, c2);
@@ -548,7 +415,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     halo_seen = true;
                 }
                 mbar_wait(bar(BAR_V_EMPTY + s), ((n / VS) & 1) ^ 1, abort_flag, p.status);
-                if (leader) {
+                if (elect_one()) {
                     mbar_expect_tx(bar(BAR_V_FULL + s), L::kTileBytes);
                     int c1, c2;
                     coords(2, p.np + plan.anchor + x * BN - p.k_pos0, c1, c2);
@@ -558,7 +425,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 }
                 __syncwarp();
             }
-        } else if (warp - 2 < TILES) {
+        } else if (warp - 2 < TILES && elect_one()) {  // (one thread runs the whole role, see elect_one)
             // ---------------- tensor-core issue: warp 2 drives query tile 0, warp 3 query tile 1 ----------------
             // Each warp issues, for its own query tile, QK of item i+1 right after PV of item i (P aliases S, and
             // tcgen05 operations of one thread execute in issue order).  A K/V stage is free again once BOTH
@@ -600,11 +467,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 while (kn < n_stop || vn < n_stop) {
                     if (kn < n_stop && kn <= vn) {
                         mbar_wait(bar(BAR_K_FULL + k_stage), k_par, abort_flag, p.status);
-                        if (leader) mbar_arrive(bar(BAR_K_EMPTY + k_stage));
+                        mbar_arrive(bar(BAR_K_EMPTY + k_stage));
                         k_advance();
                     } else {
                         mbar_wait(bar(BAR_V_FULL + v_stage), v_par, abort_flag, p.status);
-                        if (leader) mbar_arrive(bar(BAR_V_EMPTY + v_stage));
+                        mbar_arrive(bar(BAR_V_EMPTY + v_stage));
                         v_advance();
                     }
                 }
@@ -619,10 +486,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 for (int kk = 0; kk < DH / 16; ++kk) {
                     const uint64_t ad = desc_of(a_lo + (kk / 4) * (L::kSubTileBytes >> 4) + (kk % 4) * 2);
                     const uint64_t bd = desc_of(b_lo + (kk / 4) * b_sub + (kk % 4) * 2);
-                    if (leader) mma_ss(s_tmem, ad, bd, idesc_qk_pers, kk > 0 ? 1u : 0u);
+                    mma_ss(s_tmem, ad, bd, idesc_qk_pers, kk > 0 ? 1u : 0u);
                 }
-                if (leader) tc_commit(s_bar);
-                __syncwarp();
+                tc_commit(s_bar);
             };
             // QK of the window tile under the K cursor (waits for the tile, releases its stage)
             auto qk_win = [&]() {
@@ -634,13 +500,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 for (int kk = 0; kk < DH / 16; ++kk) {
                     const uint64_t ad = desc_of(a_lo + (kk / 4) * (L::kSubTileBytes >> 4) + (kk % 4) * 2);
                     const uint64_t bd = desc_of(b_lo + (kk / 4) * (L::kSubTileBytes >> 4) + (kk % 4) * 2);
-                    if (leader) mma_ss(s_tmem, ad, bd, idesc_qk_win, kk > 0 ? 1u : 0u);
+                    mma_ss(s_tmem, ad, bd, idesc_qk_win, kk > 0 ? 1u : 0u);
                 }
-                if (leader) {
-                    tc_commit(s_bar);
-                    tc_commit(e_bar);
-                }
-                __syncwarp();
+                tc_commit(s_bar);
+                tc_commit(e_bar);
                 k_advance();
             };
             auto pv_pers = [&]() {
@@ -648,9 +511,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 tc_fence_after();
                 for (int kk = 0; kk < p.np_pad / 16; ++kk) {
                     const uint64_t bd = desc_of(b_lo + kk * 128);
-                    if (leader) mma_ts(o_tmem, p_tmem + kk * 8, bd, idesc_pv, kk > 0 ? 1u : 0u);
+                    mma_ts(o_tmem, p_tmem + kk * 8, bd, idesc_pv, kk > 0 ? 1u : 0u);
                 }
-                __syncwarp();
             };
             // PV of the window tile under the V cursor; acc0 = 0 only for the very first product of the tile
             auto pv_win = [&](uint32_t acc0) {
@@ -662,10 +524,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
                 for (int kk = 0; kk < BN / 16; ++kk) {
                     const uint64_t bd = desc_of(b_lo + kk * 128);
-                    if (leader) mma_ts(o_tmem, p_tmem + kk * 8, bd, idesc_pv, kk > 0 ? 1u : acc0);
+                    mma_ts(o_tmem, p_tmem + kk * 8, bd, idesc_pv, kk > 0 ? 1u : acc0);
                 }
-                if (leader) tc_commit(e_bar);
-                __syncwarp();
+                tc_commit(e_bar);
                 v_advance();
             };
 
@@ -684,10 +545,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     mbar_wait(p_bar, i & 1, abort_flag, p.status);
                     if (i < q.has_pers) pv_pers(); else pv_win(i > 0 ? 1u : 0u);
                     if (TM::kSplitP) {
-                        if (leader) tc_commit(bar(i + 1 < q.n_items ? BAR_PV_DONE + t : BAR_O_DONE + t));
+                        tc_commit(bar(i + 1 < q.n_items ? BAR_PV_DONE + t : BAR_O_DONE + t));
                     } else {
                         if (i + 1 < q.n_items) qk_win();
-                        else if (leader) tc_commit(bar(BAR_O_DONE + t));
+                        else tc_commit(bar(BAR_O_DONE + t));
                     }
                 }
             }
@@ -975,6 +836,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
     }
 
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

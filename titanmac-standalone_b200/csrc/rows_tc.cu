@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kTcThreads) rows_tc_kernel(const __grid_consta
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kBars + 16 * S + 16);
 
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     const int cs = p.cluster, rank = (int)blockIdx.x % cs, n0 = (int)(blockIdx.x / cs) * BN, m0 = blockIdx.y * 128;
     const int blocks = (p.k + 63) / 64;
     const int b_lo = blocks * rank / cs, nb = blocks * (rank + 1) / cs - b_lo;  // this CTA's 64-wide slices of k
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kTcThreads) rows_tc_kernel(const __grid_consta
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 4) {
-        if (lane == 0) {
+        if (elect_one()) {
             for (int i = 0; i < nb && i < S; ++i) {  // weights of the first stages: nobody's output
                 mbar_expect_tx(full(i), L::kStage);
                 tma_load_2d(smem_base + i * L::kStage + L::kA, &args.map_w, full(i), (b_lo + i) * 64, n0);
@@ -100,22 +100,23 @@ __global__ void __launch_bounds__(kTcThreads) rows_tc_kernel(const __grid_consta
         }
         __syncwarp();
     } else if (warp == 5) {
-        const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, BN);
-        for (int i = 0; i < nb; ++i) {
-            const int s = i % S;
-            mbar_wait(full(s), (i / S) & 1, abort_flag, p.status);
-            tc_fence_after();
-            const uint64_t ad = kmajor_desc(smem_base + s * L::kStage);
-            const uint64_t wd = kmajor_desc(smem_base + s * L::kStage + L::kA);
-            if (lane == 0) {
+        if (elect_one()) {
+            const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, BN);
+            for (int i = 0; i < nb; ++i) {
+                const int s = i % S;
+                mbar_wait(full(s), (i / S) & 1, abort_flag, p.status);
+                tc_fence_after();
+                const uint64_t ad = kmajor_desc(smem_base + s * L::kStage);
+                const uint64_t wd = kmajor_desc(smem_base + s * L::kStage + L::kA);
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) mma_ss(tmem, ad + 2 * kk, wd + 2 * kk, idesc, (i | kk) ? 1u : 0u);
-                tc_commit(empty(s));
-                if (i == nb - 1) tc_commit(done);
+                if (i + S < nb) tc_commit(empty(s));  // (a stage that is not filled again needs no hand-back)
             }
-            __syncwarp();
+            tc_commit(done);
         }
+        __syncwarp();
     }
+
     // ---- epilogue: CS threads per row, BN / CS columns each (one CTA: one thread per row), eight columns at a time ----
     const int rows_r = 128 / cs, cols_t = BN / cs;
     const int row = rank * rows_r + (int)threadIdx.x / cs, col0 = ((int)threadIdx.x % cs) * cols_t;
@@ -263,7 +264,7 @@ int launch_rows_norm(int dtype, int rows, int dim, const void* x, const void* ga
 }
 
 int launch_rows_tc(int dtype, int m, int n, int k, const void* a, const void* w, const void* bias, void* c, int epi,
-                   cudaStream_t stream) {
+                   cudaStream_t stream, bool pdl) {
     RowsTcArgs args;
     // 32 columns per tile, and the k of a tile over as many CTAs as fill the chip once (a CTA keeps at least two slices
     // of 64): one step of 16 layers for 64 | 128 | 256 rows took 784 | 1093 | 1461 us, with 64 columns 865 | 1261 | 1629
@@ -283,7 +284,7 @@ int launch_rows_tc(int dtype, int m, int n, int k, const void* a, const void* w,
     auto run = [&](auto kern, int smem) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), smem);
         if (rc != TMW_OK) return rc;
-        TMW_CUDA_TRY(launch_ex(kern, grid, dim3(kTcThreads), smem, stream, true, p.cluster, args));
+        TMW_CUDA_TRY(launch_ex(kern, grid, dim3(kTcThreads), smem, stream, pdl, p.cluster, args));
         return TMW_OK;
     };
     auto pick = [&](auto bf16) -> int {

@@ -14,6 +14,16 @@ constexpr long long kWaitLimitCycles = 2000000000LL;  // about one second
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// True in one lane of the (whole, converged) warp, in a way the compiler can see: the operands of TMA and tcgen05
+// instructions live in uniform registers, and inside a branch on `lane == 0` every one of them is issued through a loop
+// over the possibly different values of the lanes.  Measured on one SM: four tcgen05.mma and two commits take 400
+// cycles of the issuing thread behind `lane == 0` and 100 behind elect.sync; two TMA loads 400 and 240.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }

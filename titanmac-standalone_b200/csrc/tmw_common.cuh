@@ -225,7 +225,7 @@ int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const 
 // links of a chain of dependent launches (see pdl_wait): a product of up to a few hundred rows (epi: 0 = store, 1 = GELU,
 // 2 = added to c, which is read and written; n and k multiples of 8, contiguous rows), and the RMSNorm in front of it
 int launch_rows_tc(int dtype, int m, int n, int k, const void* a, const void* w, const void* bias, void* c, int epi,
-                   cudaStream_t stream);
+                   cudaStream_t stream, bool pdl);
 int launch_rows_norm(int dtype, int rows, int dim, const void* x, const void* gain, float eps, void* y, cudaStream_t stream);
 int launch_cache_fill(const tmw_cache_desc& c, const void* k, const void* v, const int64_t ks[3],
                       const int64_t vs[3], int rows, int t0, cudaStream_t stream);
