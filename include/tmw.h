@@ -344,20 +344,53 @@ TMW_API int tmw_decode_split_static(const tmw_cache_desc* cache, const void* q, 
 typedef struct tmw_block {
     const void *norm_attn, *w_qkv, *w_out;
     const void *norm_mlp, *w_fc1, *b_fc1, *w_fc2, *b_fc2;
-    void *k_ring, *v_ring;
-    const void *k_pers, *v_pers;
+    const void *conv_q, *conv_k, *conv_v; /* depthwise filters [d_model, taps] of the block-sparse class, else NULL */
+    void *k_ring, *v_ring;                /* NULL where a call keeps no keys and values */
+    void *k_pers, *v_pers;
     float cache_scale; /* 0 selects 1/sqrt(head_dim) */
 } tmw_block;
 
 typedef struct tmw_stack_desc {
     int32_t dtype; /* TMW_BF16 or TMW_F16: every tensor of the model */
     int32_t batch, layers, d_model, heads, head_dim, d_ff, window, n_persistent, vocab, max_positions;
+    int32_t block_size;          /* 0: WindowedAttention, else BlockSparseAttention with that block size */
+    int32_t conv_taps;           /* 0: no convolutions */
     float eps;                   /* of every RMSNorm */
     const void *embed_tokens;    /* [vocab, d_model] */
     const void *embed_positions; /* [max_positions, d_model] */
+    const void *persistent;      /* [n_persistent, d_model] or NULL (tmw_stack_forward) */
     const void *norm;            /* final norm, [d_model] */
     const void *head;            /* [vocab, d_model] */
 } tmw_stack_desc;
+
+/*
+ * The attention module over full sequences as one call: y = (attention(x w_qkvᵀ, after the depthwise convolutions where
+ * conv_taps > 0)) w_outᵀ for x, y [batch, rows, heads * head_dim] contiguous - WindowedAttention.forward
+ * (windowed_attention.py:277-334), or with block_size > 0 BlockSparseAttention.forward (block_sparse_attention.py:201-343).
+ * 16-bit types.  `workspace`: device memory of tmw_attention_workspace() bytes, used until the call's kernels have finished.
+ */
+typedef struct tmw_attention_desc {
+    int32_t dtype, batch, rows, heads, head_dim, window, n_persistent;
+    int32_t block_size; /* 0: per-token window */
+    int32_t conv_taps;  /* 0: no convolutions; else conv_q, conv_k, conv_v are [heads * head_dim, conv_taps] */
+    float scale;        /* 0 selects 1/sqrt(head_dim) */
+} tmw_attention_desc;
+
+TMW_API size_t tmw_attention_workspace(const tmw_attention_desc* desc);
+TMW_API int tmw_attention_forward(const tmw_attention_desc* desc, const void* x, const void* w_qkv, const void* conv_q,
+                          const void* conv_k, const void* conv_v, const void* w_out, void* y, void* workspace,
+                          size_t workspace_bytes, void* stream);
+
+/*
+ * The whole model over token_ids [batch, tokens] (int64, device): embeddings with the persistent rows in front
+ * (titans_core/models/titanmac.py:554-619), the blocks, the final norm and the head.  logits: [batch, n_persistent + tokens,
+ * vocab], or with last_only [batch, vocab] of the last token.  Blocks whose k_ring is not NULL keep their keys and values
+ * as tmw_cache_fill does (and the persistent rows' in k_pers, v_pers): a prompt that decode steps continue.  d_ff and vocab
+ * multiples of 8, tokens <= max_positions; ids outside the table are clamped and reported by tmw_poll_status.
+ */
+TMW_API size_t tmw_stack_workspace(const tmw_stack_desc* desc, int32_t tokens);
+TMW_API int tmw_stack_forward(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, int32_t tokens,
+                      int32_t last_only, void* logits, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * One decode step of the whole model: token_ids [batch] int64 and pos [batch] int32 (device) -> logits [batch, vocab].

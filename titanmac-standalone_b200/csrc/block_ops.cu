@@ -26,8 +26,10 @@ int resident_ctas(K kernel, int threads) {
 // (it comes out of L1/L2: the same warp has just read or written it).
 template <typename T, int NV>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-add_rmsnorm_kernel(const T* x, const T* __restrict__ res, const T* __restrict__ scale, float eps,
-                   T* sum_out, T* __restrict__ y, long long rows, int dim) {
+add_rmsnorm_kernel(const T* x, const T* res, const T* __restrict__ scale, float eps, T* sum_out, T* y, long long rows,
+                   int dim) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * kWarpsPerBlock;
     // a resident grid: every warp walks over rows (a block that lives for one row per warp spends most of
@@ -53,13 +55,27 @@ add_rmsnorm_kernel(const T* x, const T* __restrict__ res, const T* __restrict__ 
 
     float keep[NV > 0 ? NV : 1][8];
     float ss = 0.f;
-    if (NV > 0) {
+    if constexpr (NV > 0) {
+        // (all loads before the first store, which may be to the same rows)
+        Vec8<T> xv[NV], rv[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+            if (lane + j * 32 < nvec) {
+                xv[j].load(xr + (lane + j * 32) * 8);
+                if (rr != nullptr) rv[j].load(rr + (lane + j * 32) * 8);
+            }
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             const int v = lane + j * 32;
             if (v < nvec) {
-                load_h(v, keep[j]);
-                if (sr != nullptr && rr != nullptr) store8<T>(sr + v * 8, keep[j]);
+                xv[j].unpack(keep[j]);
+                if (rr != nullptr) {
+                    float r[8];
+                    rv[j].unpack(r);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) keep[j][i] = to_f32<T>(from_f32<T>(keep[j][i] + r[i]));
+                    if (sr != nullptr) store8<T>(sr + v * 8, keep[j]);
+                }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) ss = fmaf(keep[j][i], keep[j][i], ss);
             }
@@ -102,8 +118,8 @@ add_rmsnorm_kernel(const T* x, const T* __restrict__ res, const T* __restrict__ 
 }
 
 template <typename T>
-int launch_add_rmsnorm(long long rows, int dim, const void* x, const void* res, const void* scale, float eps,
-                       void* sum_out, void* y, cudaStream_t stream) {
+int launch_add_rmsnorm_t(long long rows, int dim, const void* x, const void* res, const void* scale, float eps,
+                         void* sum_out, void* y, cudaStream_t stream, bool pdl) {
     const long long want = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
     const int nv = (dim / 8 + 31) / 32;
     // one resident wave: every warp walks over its rows, nothing waits for a slot
@@ -112,9 +128,9 @@ int launch_add_rmsnorm(long long rows, int dim, const void* x, const void* res, 
         static int wave = 0;                                                                                 \
         if (wave == 0) wave = resident_ctas(add_rmsnorm_kernel<T, N>, kWarpsPerBlock * 32);                  \
         const unsigned blocks = (unsigned)(want < wave ? want : wave);                                       \
-        add_rmsnorm_kernel<T, N><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(                                \
-            static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(scale), eps,        \
-            static_cast<T*>(sum_out), static_cast<T*>(y), rows, dim);                                        \
+        TMW_CUDA_TRY(launch_ex(add_rmsnorm_kernel<T, N>, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, stream, pdl, 1,      \
+                               static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(scale), eps,  \
+                               static_cast<T*>(sum_out), static_cast<T*>(y), rows, dim));                                \
     }
     switch (nv) {
         case 1: TMW_NORM_CASE(1); break;
@@ -124,7 +140,6 @@ int launch_add_rmsnorm(long long rows, int dim, const void* x, const void* res, 
         default: TMW_NORM_CASE(0); break;
     }
 #undef TMW_NORM_CASE
-    TMW_CUDA_TRY(cudaGetLastError());
     return TMW_OK;
 }
 
@@ -173,19 +188,27 @@ int launch_gelu(long long n, const void* x, void* y, cudaStream_t stream) {
 constexpr int kConvStrip = 64;
 constexpr int kConvThreads = 128;
 
+// The filters [channels, taps] in up to three arrays of `per` channels each (Q, K and V keep theirs apart).
+struct ConvWeights {
+    const void* w[3];
+    int per;
+};
+
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(kConvThreads)
-dwconv_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, int rows, int channels) {
+dwconv_kernel(const T* __restrict__ x, const ConvWeights f, T* __restrict__ y, int rows, int channels) {
     const int vec = blockIdx.x * kConvThreads + threadIdx.x;  // which group of 8 channels
     if (vec * 8 >= channels) return;
     const int t0 = blockIdx.y * kConvStrip;
     const int t1 = min(rows, t0 + kConvStrip);
     const long long base = (long long)blockIdx.z * rows * channels + vec * 8;
+    const int part = vec * 8 / f.per, first = vec * 8 - part * f.per;  // (`per` is a multiple of 8)
+    const T* w = static_cast<const T*>(part == 0 ? f.w[0] : part == 1 ? f.w[1] : f.w[2]);
     float wr[TAPS][8];
 #pragma unroll
     for (int c = 0; c < 8; ++c)
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) wr[j][c] = to_f32<T>(w[(long long)(vec * 8 + c) * TAPS + j]);
+        for (int j = 0; j < TAPS; ++j) wr[j][c] = to_f32<T>(w[(long long)(first + c) * TAPS + j]);
     float hist[TAPS][8];  // hist[j] = x[t - (TAPS-1) + j]
 #pragma unroll
     for (int j = 0; j < TAPS - 1; ++j) {
@@ -216,10 +239,9 @@ dwconv_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ 
 }
 
 template <typename T, int TAPS>
-int launch_dwconv_taps(int batch, int rows, int channels, const void* x, const void* w, void* y, cudaStream_t stream) {
+int launch_dwconv_taps(int batch, int rows, int channels, const void* x, const ConvWeights& w, void* y, cudaStream_t stream) {
     const dim3 grid((channels / 8 + kConvThreads - 1) / kConvThreads, (rows + kConvStrip - 1) / kConvStrip, batch);
-    dwconv_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), static_cast<const T*>(w),
-                                                              static_cast<T*>(y), rows, channels);
+    dwconv_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), w, static_cast<T*>(y), rows, channels);
     TMW_CUDA_TRY(cudaGetLastError());
     return TMW_OK;
 }
@@ -332,8 +354,8 @@ int launch_dwconv_bwd(int batch, int rows, int channels, int taps, const void* x
 }
 
 template <typename T>
-int launch_dwconv(int batch, int rows, int channels, int taps, const void* x, const void* w, void* y,
-                  cudaStream_t stream) {
+int launch_dwconv_t(int batch, int rows, int channels, int taps, const void* x, const ConvWeights& w, void* y,
+                    cudaStream_t stream) {
     switch (taps) {
         case 1: return launch_dwconv_taps<T, 1>(batch, rows, channels, x, w, y, stream);
         case 2: return launch_dwconv_taps<T, 2>(batch, rows, channels, x, w, y, stream);
@@ -348,6 +370,28 @@ int launch_dwconv(int batch, int rows, int channels, int taps, const void* x, co
 }
 
 }  // namespace
+
+int launch_add_rmsnorm(int dtype, long long rows, int dim, const void* x, const void* residual, const void* scale, float eps,
+                       void* sum_out, void* y, cudaStream_t stream, bool pdl) {
+    switch (dtype) {
+        case TMW_F32: return launch_add_rmsnorm_t<float>(rows, dim, x, residual, scale, eps, sum_out, y, stream, pdl);
+        case TMW_BF16: return launch_add_rmsnorm_t<__nv_bfloat16>(rows, dim, x, residual, scale, eps, sum_out, y, stream, pdl);
+        default: return launch_add_rmsnorm_t<__half>(rows, dim, x, residual, scale, eps, sum_out, y, stream, pdl);
+    }
+}
+
+int launch_dwconv(int dtype, int batch, int rows, int channels, int taps, const void* x, const void* const* w, int n_w, void* y,
+                  cudaStream_t stream) {
+    ConvWeights f;
+    f.per = channels / n_w;
+    for (int i = 0; i < 3; ++i) f.w[i] = w[i < n_w ? i : 0];
+    switch (dtype) {
+        case TMW_F32: return launch_dwconv_t<float>(batch, rows, channels, taps, x, f, y, stream);
+        case TMW_BF16: return launch_dwconv_t<__nv_bfloat16>(batch, rows, channels, taps, x, f, y, stream);
+        default: return launch_dwconv_t<__half>(batch, rows, channels, taps, x, f, y, stream);
+    }
+}
+
 }  // namespace tmw
 
 extern "C" int tmw_causal_dwconv(int32_t dtype, int32_t batch, int32_t rows, int32_t channels, int32_t taps,
@@ -366,12 +410,7 @@ extern "C" int tmw_causal_dwconv(int32_t dtype, int32_t batch, int32_t rows, int
         return TMW_ERR_INVALID_ARGUMENT;
     }
     if (batch > 65535 || (rows + kConvStrip - 1) / kConvStrip > 65535) return TMW_ERR_TOO_LARGE;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    switch (dtype) {
-        case TMW_F32: return launch_dwconv<float>(batch, rows, channels, taps, x, weight, y, s);
-        case TMW_BF16: return launch_dwconv<__nv_bfloat16>(batch, rows, channels, taps, x, weight, y, s);
-        default: return launch_dwconv<__half>(batch, rows, channels, taps, x, weight, y, s);
-    }
+    return launch_dwconv(dtype, batch, rows, channels, taps, x, &weight, 1, y, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tmw_causal_dwconv_backward(int32_t dtype, int32_t batch, int32_t rows, int32_t channels, int32_t taps,
@@ -436,10 +475,5 @@ extern "C" int tmw_add_rmsnorm(int32_t dtype, int64_t rows, int32_t dim, const v
         return TMW_ERR_INVALID_ARGUMENT;
     }
     if (rows == 0) return TMW_OK;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    switch (dtype) {
-        case TMW_F32: return launch_add_rmsnorm<float>(rows, dim, x, residual, scale, eps, sum_out, y, s);
-        case TMW_BF16: return launch_add_rmsnorm<__nv_bfloat16>(rows, dim, x, residual, scale, eps, sum_out, y, s);
-        default: return launch_add_rmsnorm<__half>(rows, dim, x, residual, scale, eps, sum_out, y, s);
-    }
+    return launch_add_rmsnorm(dtype, rows, dim, x, residual, scale, eps, sum_out, y, static_cast<cudaStream_t>(stream));
 }

@@ -861,13 +861,29 @@ struct FillParams {
     const void* v;
     long long ks[3], vs[3];
     int heads, slots, dh, rows, first_row, t0;
+    const void *pers_k, *pers_v;  // optional: rows of the first sequence for the persistent arrays
+    void *k_pers, *v_pers;
+    int np;
 };
 
 // One thread per 8-element chunk of a kept row; rows [first_row, rows) are kept.
 template <typename T>
 __global__ void cache_fill_kernel(const FillParams p) {
+    pdl_trigger();
+    pdl_wait();
     const int h = blockIdx.y, b = blockIdx.z;
     const int chunks_per_row = p.dh / 8;
+    if (p.pers_k != nullptr && b == 0) {
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < p.np * chunks_per_row; c += gridDim.x * blockDim.x) {
+            const int i = c / chunks_per_row, col = (c % chunks_per_row) * 8;
+            const long long dst = ((long long)h * p.np + i) * p.dh + col;
+            float tmp[8];
+            load8<T>(static_cast<const T*>(p.pers_k) + h * p.ks[1] + (long long)i * p.ks[2] + col, tmp);
+            store8<T>(static_cast<T*>(p.k_pers) + dst, tmp);
+            load8<T>(static_cast<const T*>(p.pers_v) + h * p.vs[1] + (long long)i * p.vs[2] + col, tmp);
+            store8<T>(static_cast<T*>(p.v_pers) + dst, tmp);
+        }
+    }
     const int n = (p.rows - p.first_row) * chunks_per_row;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
         const int i = p.first_row + c / chunks_per_row;
@@ -966,7 +982,8 @@ int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, con
 }
 
 int launch_cache_fill(const tmw_cache_desc& c, const void* k, const void* v, const int64_t ks[3],
-                      const int64_t vs[3], int rows, int t0, cudaStream_t stream) {
+                      const int64_t vs[3], int rows, int t0, cudaStream_t stream, const void* pers_k, const void* pers_v,
+                      bool pdl) {
     if (c.batch == 0 || c.heads == 0 || rows == 0) return TMW_OK;
     if (c.batch > 65535 || c.heads > 65535) return TMW_ERR_TOO_LARGE;
     FillParams p;
@@ -975,15 +992,16 @@ int launch_cache_fill(const tmw_cache_desc& c, const void* k, const void* v, con
     p.heads = c.heads; p.slots = c.window + 1; p.dh = c.head_dim; p.rows = rows;
     p.first_row = rows > p.slots ? rows - p.slots : 0;
     p.t0 = t0;
+    p.pers_k = pers_k; p.pers_v = pers_v;
+    p.k_pers = const_cast<void*>(c.k_pers); p.v_pers = const_cast<void*>(c.v_pers); p.np = c.n_persistent;
     const int n = (rows - p.first_row) * (c.head_dim / 8);
-    dim3 grid((n + 255) / 256, c.heads, c.batch);
+    const dim3 grid((n + 255) / 256, c.heads, c.batch), block(256);
     switch (c.dtype) {
-        case TMW_F32: cache_fill_kernel<float><<<grid, 256, 0, stream>>>(p); break;
-        case TMW_BF16: cache_fill_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p); break;
-        case TMW_F16: cache_fill_kernel<__half><<<grid, 256, 0, stream>>>(p); break;
+        case TMW_F32: TMW_CUDA_TRY(launch_ex(cache_fill_kernel<float>, grid, block, 0, stream, pdl, 1, p)); break;
+        case TMW_BF16: TMW_CUDA_TRY(launch_ex(cache_fill_kernel<__nv_bfloat16>, grid, block, 0, stream, pdl, 1, p)); break;
+        case TMW_F16: TMW_CUDA_TRY(launch_ex(cache_fill_kernel<__half>, grid, block, 0, stream, pdl, 1, p)); break;
         default: return TMW_ERR_UNSUPPORTED;
     }
-    TMW_CUDA_TRY(cudaGetLastError());
     return TMW_OK;
 }
 

@@ -51,6 +51,7 @@ struct GemmParams {
     int m, n, k;
     int epilogue;        // tmw_epilogue
     const void* bias;    // [n] in the dtype of the operands, or nullptr
+    int drain;           // a dependent launch follows: the stores have to be complete when the kernel ends
     int* status;
 };
 
@@ -99,6 +100,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();  // (with its tensor memory in hand: a dependent that took it first would wait for this CTA forever)
+    pdl_wait();
 
     constexpr int SL = L::kSlices;
     if (warp == 0) {
@@ -231,7 +234,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 tma_store_commit();
             }
         }
-        if (epi_leader) tma_store_wait_read();  // (the stores themselves complete with the grid)
+        if (epi_leader) {
+            if (p.drain) tma_store_wait_all();
+            else tma_store_wait_read();  // (the stores themselves complete with the grid)
+        }
     }
 
     tc_fence_before();
@@ -324,6 +330,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     cluster_sync();  // the partner's barriers exist before anything is signalled across
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();  // (with its tensor memory in hand: a dependent that took it first would wait for this CTA forever)
+    pdl_wait();
 
     if (warp == 0) {
         // ---------------- producer (both CTAs) ----------------
@@ -449,7 +457,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 tma_store_commit();
             }
         }
-        if (epi_leader) tma_store_wait_read();  // (the stores themselves complete with the grid)
+        if (epi_leader) {
+            if (p.drain) tma_store_wait_all();
+            else tma_store_wait_read();  // (the stores themselves complete with the grid)
+        }
     }
 
     tc_fence_before();
@@ -469,7 +480,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // Host side
 // ---------------------------------------------------------------------------------
 template <int BN>
-int launch_gemm(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream) {
+int launch_gemm(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream,
+                int chain) {
     using L = GemmSmem<BN>;
     CUtensorMap ma, mw, mc;
     if (!make_map_2d(&ma, a, d.dtype, d.m, d.k, d.lda, GM, GK, CU_TENSOR_MAP_SWIZZLE_128B) ||
@@ -480,6 +492,7 @@ int launch_gemm(const tmw_linear_desc& d, const void* a, const void* w, const vo
     p.m = d.m; p.n = d.n; p.k = d.k;
     p.epilogue = d.epilogue;
     p.bias = bias;
+    p.drain = chain & kChainFollowed;
     p.status = device_status_word();
     if (p.status == nullptr) return TMW_ERR_CUDA;
     const int tiles = ((d.m + GM - 1) / GM) * ((d.n + BN - 1) / BN);
@@ -487,13 +500,11 @@ int launch_gemm(const tmw_linear_desc& d, const void* a, const void* w, const vo
     auto run = [&](auto kern) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), L::kTotal);
         if (rc != TMW_OK) return rc;
-        kern<<<grid, kGemmThreads, L::kTotal, stream>>>(ma, mw, mc, p);
+        TMW_CUDA_TRY(launch_ex(kern, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, chain & kChainDependent, 1, ma, mw, mc, p));
         return TMW_OK;
     };
     const int st = d.dtype == TMW_BF16 ? run(gemm_tc_kernel<BN, true>) : run(gemm_tc_kernel<BN, false>);
-    if (st != TMW_OK) return st;
-    TMW_CUDA_TRY(cudaGetLastError());
-    return TMW_OK;
+    return st;
 }
 
 // How many CTA pairs of the kernel the device runs at once (asked once per kernel and device).
@@ -526,7 +537,7 @@ int max_active_pairs(const void* kern, int smem_bytes) {
 
 template <int BN>
 int launch_gemm_pair(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, int chain) {
     using L = PairSmem<BN>;
     CUtensorMap ma, mw, mc;
     if (!make_map_2d(&ma, a, d.dtype, d.m, d.k, d.lda, GM, GK, CU_TENSOR_MAP_SWIZZLE_128B) ||
@@ -537,6 +548,7 @@ int launch_gemm_pair(const tmw_linear_desc& d, const void* a, const void* w, con
     p.m = d.m; p.n = d.n; p.k = d.k;
     p.epilogue = d.epilogue;
     p.bias = bias;
+    p.drain = chain & kChainFollowed;
     p.status = device_status_word();
     if (p.status == nullptr) return TMW_ERR_CUDA;
     const int tiles = ((d.m + 2 * GM - 1) / (2 * GM)) * ((d.n + BN - 1) / BN);
@@ -546,13 +558,11 @@ int launch_gemm_pair(const tmw_linear_desc& d, const void* a, const void* w, con
         if (rc != TMW_OK) return rc;
         const int resident = max_active_pairs(fn, L::kTotal);
         const int pairs = tiles < resident ? tiles : resident;
-        kern<<<2 * pairs, kGemmThreads, L::kTotal, stream>>>(ma, mw, mc, p);
+        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kGemmThreads), L::kTotal, stream, chain & kChainDependent, 1, ma, mw, mc, p));
         return TMW_OK;
     };
     const int st = d.dtype == TMW_BF16 ? run(gemm_tc_pair_kernel<BN, true>) : run(gemm_tc_pair_kernel<BN, false>);
-    if (st != TMW_OK) return st;
-    TMW_CUDA_TRY(cudaGetLastError());
-    return TMW_OK;
+    return st;
 }
 
 }  // namespace
@@ -562,7 +572,8 @@ int launch_gemm_pair(const tmw_linear_desc& d, const void* a, const void* w, con
 // long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 6.5 us against 8.2).  The pair kernel moves the fewest operand bytes per product and wins wherever it has enough
 // tiles: measured at K = 640 for 1056 | 2528 | 8256 | 32 896 rows of N = 1920, pair | 128 | 64 columns: 9.3 | 12.6 | 21.3 |
 // 68.8, 6.3 | 11.4 | 24.1 | 82.5, 7.1 | 11.7 | 29.0 us.
-int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream) {
+int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream,
+                  int chain) {
     struct Variant { int rows, cols, units; float launch, alone, full; };
     const int sms = sm_count();
     const Variant variants[] = {{2 * GM, 256, sms / 2, 6.1f, 0.28f, 0.46f}, {GM, 256, sms, 5.0f, 0.305f, 0.54f},
@@ -570,7 +581,7 @@ int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const 
                                 {GM, 32, sms, 3.5f, 0.117f, 0.135f}};
     const float slices = (float)((d.k + GK - 1) / GK);
     if (slices >= 16.f && 2 * ((d.m + GM - 1) / GM) * ((d.n + 31) / 32) <= sms && d.lda == d.k && d.ldw == d.k && d.ldc == d.n)
-        return launch_rows_tc(d.dtype, d.m, d.n, d.k, a, w, bias, c, d.epilogue, stream, false);
+        return launch_rows_tc(d.dtype, d.m, d.n, d.k, a, w, bias, c, d.epilogue, stream, chain & kChainDependent);
     int best = 0;
     float least = 0.f;
     for (int i = 0; i < 5; ++i) {
@@ -585,11 +596,11 @@ int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const 
         }
     }
     switch (best) {
-        case 0: return launch_gemm_pair<256>(d, a, w, bias, c, stream);
-        case 1: return launch_gemm<256>(d, a, w, bias, c, stream);
-        case 2: return launch_gemm<128>(d, a, w, bias, c, stream);
-        case 3: return launch_gemm<64>(d, a, w, bias, c, stream);
-        default: return launch_gemm<32>(d, a, w, bias, c, stream);
+        case 0: return launch_gemm_pair<256>(d, a, w, bias, c, stream, chain);
+        case 1: return launch_gemm<256>(d, a, w, bias, c, stream, chain);
+        case 2: return launch_gemm<128>(d, a, w, bias, c, stream, chain);
+        case 3: return launch_gemm<64>(d, a, w, bias, c, stream, chain);
+        default: return launch_gemm<32>(d, a, w, bias, c, stream, chain);
     }
 }
 

@@ -97,6 +97,7 @@ struct TcParams {
     int all_keys;     // 1: every query row of the call sees every key row, unmasked
     int dim_order;  // bit i set: tensor i (0=q,1=k,2=v,3=o) has its head axis before its row axis in the map
     float scale_log2;
+    int drain;  // a dependent launch follows: the stores have to be complete when the kernel ends
     int* status;
     float* lse;  // optional [batch, heads, q_rows]: log2 of the row's softmax denominator, in the scaled-by-log2(e) domain
     // Sequence-sharded call whose K/V buffer is filled by other GPUs (tmw_halo_push): key rows [0, np) may be read
@@ -139,9 +140,10 @@ __device__ __forceinline__ void flag_wait(const int* flag, int value, long long 
 // ---------------------------------------------------------------------------------
 // PTX wrappers beyond tc_ptx.cuh
 // ---------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_store_commit_and_wait() {
+__device__ __forceinline__ void tma_store_commit_and_wait(bool drain) {
     tma_store_commit();
-    tma_store_wait_read();
+    if (drain) tma_store_wait_all();
+    else tma_store_wait_read();
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
@@ -350,6 +352,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();  // (with its tensor memory in hand: a dependent that took it first would wait for this CTA forever)
+    pdl_wait();
 
     // coordinate order of each tensor map: (dh, rows, heads, batch) or (dh, heads, rows, batch)
     auto coords = [&](int which, int row, int& c1, int& c2) {
@@ -831,7 +835,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 coords(3, (blockIdx.x * TILES + t) * BM, c1, c2);
                 for (int u = 0; u < NSUB; ++u)
                     tma_store_4d(&map_o, smem_u32(stage + u * L::kSubTileBytes), u * 64, c1, c2, batch);
-                tma_store_commit_and_wait();
+                tma_store_commit_and_wait(p.drain);
             }
         }
     }
@@ -858,7 +862,7 @@ int np_pad_of(int np) { return np > 0 ? ((np + 15) / 16) * 16 : 0; }
 
 template <int DH, int KS, int VS, int TILES, int RS>
 int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o, cudaStream_t stream,
-              int window_block, bool all_keys, float* lse, const tmw_halo_wait* wait) {
+              int window_block, bool all_keys, float* lse, const tmw_halo_wait* wait, int chain) {
     using L = TcSmem<DH, KS, VS, TILES>;
     const int np_pad = np_pad_of(d.n_persistent);
     CUtensorMap mq, mk, mv, mo, mkp, mvp;
@@ -883,6 +887,7 @@ int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const voi
     p.window_plan = d.window + (window_block > 0 ? window_block - 1 : 0);
     p.all_keys = all_keys ? 1 : 0;
     p.lse = lse;
+    p.drain = chain & kChainFollowed;
     p.pers_flag = wait != nullptr ? wait->pers_flag : nullptr;
     p.halo_flag = wait != nullptr ? wait->halo_flag : nullptr;
     p.flag_value = wait != nullptr ? wait->value : 0;
@@ -901,7 +906,7 @@ int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const voi
     auto run = [&](auto kern) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), smem_bytes);
         if (rc != TMW_OK) return rc;
-        kern<<<grid, kThreadsTc, smem_bytes, stream>>>(mq, mk, mv, mo, mkp, mvp, p);
+        TMW_CUDA_TRY(launch_ex(kern, grid, dim3(kThreadsTc), smem_bytes, stream, chain & kChainDependent, 1, mq, mk, mv, mo, mkp, mvp, p));
         return TMW_OK;
     };
     int st;
@@ -909,9 +914,7 @@ int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const voi
         st = general ? run(prefill_tc_kernel<DH, KS, VS, true, TILES, true, RS>) : run(prefill_tc_kernel<DH, KS, VS, true, TILES, false, RS>);
     else
         st = general ? run(prefill_tc_kernel<DH, KS, VS, false, TILES, true, RS>) : run(prefill_tc_kernel<DH, KS, VS, false, TILES, false, RS>);
-    if (st != TMW_OK) return st;
-    TMW_CUDA_TRY(cudaGetLastError());
-    return TMW_OK;
+    return st;
 }
 
 constexpr int kMaxDynamicSmem = 232448;  // 227 KB per CTA on sm_100
@@ -939,7 +942,7 @@ bool prefill_tc_supports(const tmw_prefill_desc& d, const void*, const void*, co
 }
 
 int launch_prefill_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
-                      cudaStream_t stream, int window_block, bool all_keys, float* lse, const tmw_halo_wait* wait) {
+                      cudaStream_t stream, int window_block, bool all_keys, float* lse, const tmw_halo_wait* wait, int chain) {
     if (d.head_dim == 64) {
         // One query tile per CTA and two CTAs per SM when two such CTAs fit into shared memory (they do
         // unless there are many persistent keys): independent CTAs drift apart, so one CTA's exponentials,
@@ -949,12 +952,12 @@ int launch_prefill_tc(const tmw_prefill_desc& d, const void* q, const void* k, c
             // query tile has enough key tiles for that to outweigh the exchange between the two threads: measured
             // on 8 x 10 heads x 4112 rows, window 128 | 512 | 2048: 91.0 | 141.5 | 293.9 us against 87.2 | 152.6 | 300.9.
             if (d.window >= 192)
-                return launch_tc<64, 3, 2, 1, 2>(d, q, k, v, o, stream, window_block, all_keys, lse, wait);
-            return launch_tc<64, 3, 2, 1, 1>(d, q, k, v, o, stream, window_block, all_keys, lse, wait);
+                return launch_tc<64, 3, 2, 1, 2>(d, q, k, v, o, stream, window_block, all_keys, lse, wait, chain);
+            return launch_tc<64, 3, 2, 1, 1>(d, q, k, v, o, stream, window_block, all_keys, lse, wait, chain);
         }
-        return launch_tc<64, 3, 3, 2, 1>(d, q, k, v, o, stream, window_block, all_keys, lse, wait);
+        return launch_tc<64, 3, 3, 2, 1>(d, q, k, v, o, stream, window_block, all_keys, lse, wait, chain);
     }
-    return launch_tc<128, 2, 2, 2, 1>(d, q, k, v, o, stream, window_block, all_keys, lse, wait);
+    return launch_tc<128, 2, 2, 2, 1>(d, q, k, v, o, stream, window_block, all_keys, lse, wait, chain);
 }
 
 }  // namespace tmw

@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(kTcThreads) rows_tc_kernel(const __grid_consta
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + L::kBars + 16 * S + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kBars + 16 * S + 16);
 
-    pdl_trigger();
     const int warp = threadIdx.x >> 5;
     const int cs = p.cluster, rank = (int)blockIdx.x % cs, n0 = (int)(blockIdx.x / cs) * BN, m0 = blockIdx.y * 128;
     const int blocks = (p.k + 63) / 64;
@@ -80,6 +79,7 @@ __global__ void __launch_bounds__(kTcThreads) rows_tc_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_trigger();  // (with its tensor memory in hand: a dependent that took it first would wait for this CTA forever)
 
     if (warp == 4) {
         if (elect_one()) {

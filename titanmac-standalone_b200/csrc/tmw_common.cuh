@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <utility>
 
 #include "tmw.h"
 
@@ -105,6 +106,17 @@ __device__ __forceinline__ float gelu_erf(float x) {
 
 __host__ __device__ inline size_t dtype_size(int dtype) { return dtype == TMW_F32 ? 4 : 2; }
 
+// Eight consecutive elements as raw bits: half the registers of their fp32 values for 16-bit types.
+template <typename T>
+struct Vec8 {
+    uint4 raw[sizeof(T) / 2];
+    __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T) / 2; ++i) raw[i] = reinterpret_cast<const uint4*>(p)[i];
+    }
+    __device__ __forceinline__ void unpack(float (&out)[8]) const { load8<T>(reinterpret_cast<const T*>(raw), out); }
+};
+
 // Position of the first sequence key that the sequence query at position `pos` (>= np) sees.
 // block == 0: the query and its `window` predecessors (WindowedAttention, windowed_attention.py:136-150).
 // block  > 0: the left edge moves in steps of `block` rows - the query in block b of the sequence sees the
@@ -139,13 +151,18 @@ SideStream* side_stream_of_current_device();  // nullptr if it cannot be made
 // (weights, cache rows) and then waits until its predecessor has finished - which has waited for its own.  The first
 // kernel of a chain is an ordinary launch: what the stream held before is complete when the chain starts.
 // Without the launch attribute both calls are no-ops.
+// What another kernel of the chain writes must not be read through a `const __restrict__` pointer: the compiler takes such
+// loads for invariant and moves them in front of pdl_wait().
+// A kernel that stores through TMA has to see its stores complete, not just read, before it ends if a dependent follows:
+// what it leaves in flight an ordinary launch waits for, pdl_wait() does not.
+enum : int { kChainDependent = 1, kChainFollowed = 2, kChainLink = 3 };  // a launch's place in a chain (0: none)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // launch with the dependent-launch attribute and / or a cluster of `cluster` CTAs along x
-template <typename P>
-cudaError_t launch_ex(void (*kern)(P), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, int cluster,
-                      const P& params) {
+template <typename... P, typename... A>
+cudaError_t launch_ex(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, int cluster,
+                      A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -165,7 +182,7 @@ cudaError_t launch_ex(void (*kern)(P), dim3 grid, dim3 block, size_t smem, cudaS
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kern, params);
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
 int sm_count();  // of the current device, asked once per device
@@ -193,7 +210,7 @@ int launch_prefill_simt(const tmw_prefill_desc& d, const void* q, const void* k,
                         cudaStream_t stream, int window_block = 0, bool all_keys = false, float* lse = nullptr);
 int launch_prefill_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
                       cudaStream_t stream, int window_block = 0, bool all_keys = false, float* lse = nullptr,
-                      const tmw_halo_wait* wait = nullptr);
+                      const tmw_halo_wait* wait = nullptr, int chain = 0);
 // window_block / pers_global select the mask of the block-sparse class (see first_visible_pos; pers_global: the
 // persistent query rows see every key, and lse comes as [batch, heads, rows - np] followed by [batch, heads, np])
 int launch_prefill_backward(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o,
@@ -221,13 +238,20 @@ inline size_t decode_partials_bytes(int batch, int heads, int head_dim, int spli
     return (n + 15) & ~(size_t)15;
 }
 int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c,
+                  cudaStream_t stream, int chain = 0);
+int launch_add_rmsnorm(int dtype, long long rows, int dim, const void* x, const void* residual, const void* scale, float eps,
+                       void* sum_out, void* y, cudaStream_t stream, bool pdl = false);
+// w: the filters of channels [0, c/n), [c/n, 2c/n), ... in n arrays [c/n, taps]
+int launch_dwconv(int dtype, int batch, int rows, int channels, int taps, const void* x, const void* const* w, int n_w, void* y,
                   cudaStream_t stream);
 // links of a chain of dependent launches (see pdl_wait): a product of up to a few hundred rows (epi: 0 = store, 1 = GELU,
 // 2 = added to c, which is read and written; n and k multiples of 8, contiguous rows), and the RMSNorm in front of it
 int launch_rows_tc(int dtype, int m, int n, int k, const void* a, const void* w, const void* bias, void* c, int epi,
                    cudaStream_t stream, bool pdl);
 int launch_rows_norm(int dtype, int rows, int dim, const void* x, const void* gain, float eps, void* y, cudaStream_t stream);
+// pers_k / pers_v (optional): rows [0, n_persistent) of the first sequence at these addresses go into k_pers / v_pers
 int launch_cache_fill(const tmw_cache_desc& c, const void* k, const void* v, const int64_t ks[3],
-                      const int64_t vs[3], int rows, int t0, cudaStream_t stream);
+                      const int64_t vs[3], int rows, int t0, cudaStream_t stream, const void* pers_k = nullptr,
+                      const void* pers_v = nullptr, bool pdl = false);
 
 }  // namespace tmw

@@ -96,18 +96,24 @@ class Block(ctypes.Structure):
     """One layer of the whole-model calls (tmw_block)."""
 
     _fields_ = [(n, ctypes.c_void_p) for n in ("norm_attn", "w_qkv", "w_out", "norm_mlp", "w_fc1", "b_fc1", "w_fc2", "b_fc2",
-                                               "k_ring", "v_ring", "k_pers", "v_pers")] + [("cache_scale", ctypes.c_float)]
+                                               "conv_q", "conv_k", "conv_v", "k_ring", "v_ring", "k_pers", "v_pers")] + [("cache_scale", ctypes.c_float)]
 
 
 class StackDesc(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int32) for n in ("dtype", "batch", "layers", "d_model", "heads", "head_dim", "d_ff", "window",
-                                              "n_persistent", "vocab", "max_positions")] + [
+                                              "n_persistent", "vocab", "max_positions", "block_size", "conv_taps")] + [
         ("eps", ctypes.c_float),
         ("embed_tokens", ctypes.c_void_p),
         ("embed_positions", ctypes.c_void_p),
+        ("persistent", ctypes.c_void_p),
         ("norm", ctypes.c_void_p),
         ("head", ctypes.c_void_p),
     ]
+
+
+class AttentionDesc(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int32) for n in ("dtype", "batch", "rows", "heads", "head_dim", "window", "n_persistent",
+                                              "block_size", "conv_taps")] + [("scale", ctypes.c_float)]
 
 
 EPILOGUE_NONE, EPILOGUE_GELU = 0, 1
@@ -197,6 +203,17 @@ SIGNATURES = {
         [ctypes.POINTER(CacheDesc), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
          ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64),
          ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p],
+    ),
+    "tmw_attention_workspace": (ctypes.c_size_t, [ctypes.POINTER(AttentionDesc)]),
+    "tmw_attention_forward": (
+        ctypes.c_int,
+        [ctypes.POINTER(AttentionDesc)] + [ctypes.c_void_p] * 8 + [ctypes.c_size_t, ctypes.c_void_p],
+    ),
+    "tmw_stack_workspace": (ctypes.c_size_t, [ctypes.POINTER(StackDesc), ctypes.c_int32]),
+    "tmw_stack_forward": (
+        ctypes.c_int,
+        [ctypes.POINTER(StackDesc), ctypes.POINTER(Block), ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
+         ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p],
     ),
     "tmw_decode_step_workspace": (ctypes.c_size_t, [ctypes.POINTER(StackDesc)]),
     "tmw_decode_step": (

@@ -10,6 +10,7 @@ dropout - has no table, and its modules are called one by one.
 from __future__ import annotations
 
 import ctypes
+import math
 import weakref
 from typing import List, Optional
 
@@ -28,6 +29,7 @@ class ModelTable:
     """Addresses of a ``TitanMAC``'s parameters and how to tell that they still hold."""
 
     def __init__(self, model):
+        from .attn.block_sparse_attention import BlockSparseAttention
         from .attn.windowed_attention import WindowedAttention
         from .blocks.titan_block import MLPBlock, RMSNorm, TitanBlock
 
@@ -36,6 +38,7 @@ class ModelTable:
         self._children: list = []  # (child dict of a module, name, child)
         self._modules: list = []
         self._dropouts: list = []
+        self._attentions: list = []
         self.dtype = model.embed_tokens.weight.dtype
         self.device = model.embed_tokens.weight.device
         if self.dtype not in (torch.bfloat16, torch.float16) or self.device.type != "cuda":
@@ -79,13 +82,24 @@ class ModelTable:
             block = take(layers, str(i), TitanBlock)
             if block is None:
                 return
-            attn, mlp = take(block, "attention", WindowedAttention), take(block, "mlp", MLPBlock)
+            attn, mlp = take(block, "attention", WindowedAttention, BlockSparseAttention), take(block, "mlp", MLPBlock)
             norms = (take(block, "norm_attn", RMSNorm), take(block, "norm_mlp", RMSNorm))
             if attn is None or mlp is None or None in norms or any(n.eps != c.norm_eps for n in norms):
                 return
-            if (attn.n_heads, attn.d_head, attn.window_size, attn.num_persistent) != (c.n_heads, c.d_head, c.window_size,
-                                                                                     c.n_persistent) or mlp.d_ff != F:
+            windowed = type(attn) is WindowedAttention
+            np_attn = attn.num_persistent if windowed else attn.n_persistent
+            if (attn.n_heads, attn.d_head, attn.window_size, np_attn) != (c.n_heads, c.d_head, c.window_size,
+                                                                          c.n_persistent) or mlp.d_ff != F:
                 return
+            kind = (0, 0)
+            if not windowed:
+                if attn.scale != 1.0 / math.sqrt(c.d_head):
+                    return
+                kind = (attn.block_size, attn.conv_q.kernel_size[0] if attn.use_conv else 0)
+            if i > 0 and kind != self.kind:
+                return
+            self.kind = kind
+            self._attentions.append(attn)
             qkv, out = take(attn, "qkv_proj", nn.Linear), take(attn, "out_proj", nn.Linear)
             fc1, fc2 = take(mlp, "fc1", nn.Linear), take(mlp, "fc2", nn.Linear)
             if None in (qkv, out, fc1, fc2) or qkv.bias is not None or out.bias is not None:
@@ -98,22 +112,33 @@ class ModelTable:
                           w_qkv=address(qkv, "weight", (3 * D, D)), w_out=address(out, "weight", (D, D)),
                           w_fc1=address(fc1, "weight", (F, D)), w_fc2=address(fc2, "weight", (D, F)),
                           b_fc1=optional(fc1, "bias", (F,)), b_fc2=optional(fc2, "bias", (D,)))
+            for name in ("conv_q", "conv_k", "conv_v") if kind[1] else ():
+                conv = take(attn, name, nn.Conv1d)
+                if conv is None or conv.bias is not None:
+                    return
+                values[name] = address(conv, "weight", (D, 1, kind[1]))
             found += values.values()
             for name, value in values.items():
                 setattr(b, name, value or None)
         d = self.desc = _native.StackDesc()
         top = (address(tops[0], "weight", (V, D)), address(tops[1], "weight", (c.max_seq_len, D)), address(tops[2], "scale", (D,)),
                address(tops[3], "weight", (V, D)))
-        if None in found or None in top or tops[2].eps != c.norm_eps or tops[0].max_norm is not None \
+        pers = 0
+        if c.n_persistent > 0:
+            pers = address(model, "persistent_tokens", (c.n_persistent, D))
+        if None in found or None in top or pers is None or tops[2].eps != c.norm_eps or tops[0].max_norm is not None \
                 or tops[1].max_norm is not None:
             return
         d.embed_tokens, d.embed_positions, d.norm, d.head = top
+        d.persistent = pers or None
+        d.block_size, d.conv_taps = self.kind
         d.dtype = _native._DTYPES[self.dtype]
         d.layers, d.d_model, d.heads, d.head_dim, d.d_ff = len(layers), D, c.n_heads, c.d_head, F
         d.window, d.n_persistent, d.vocab, d.max_positions, d.eps = c.window_size, c.n_persistent, V, c.max_seq_len, c.norm_eps
         self.geometry = (c.n_heads, c.d_head, c.window_size, c.n_persistent, self.dtype)
-        self.supported = c.d_head in (64, 128) and F % 32 == 0
-        self.workspace_bytes: dict = {}  # batch -> bytes
+        self.decodes = c.d_head in (64, 128) and F % 32 == 0 and self.kind == (0, 0)
+        self.forwards = V % 8 == 0 and F % 8 == 0 and D % 8 == 0 and c.d_head % 8 == 0 and self.kind[1] <= 8
+        self.workspace_bytes: dict = {}  # (batch, tokens) -> bytes; tokens = -1: a decode step
         self.ok = True
 
     def holds(self) -> bool:
@@ -139,6 +164,9 @@ class ModelTable:
         for m in self._dropouts:
             if m.training and m.p > 0:
                 return False
+        for m in self._attentions:
+            if m.algo != _native.ALGO_AUTO or m.core_events is not None or not m.causal or (m.training and m.dropout_p > 0):
+                return False
         return not _global_hooks()
 
 
@@ -151,34 +179,114 @@ def table_of(model) -> Optional[ModelTable]:
     table = _tables.get(model)
     if table is None or not table.holds():
         table = _tables[model] = ModelTable(model)
-    return table if table.ok and table.supported and table.plain_call() else None
+    return table if table.ok and table.plain_call() else None
+
+
+def _attach(blocks, caches, geometry, device) -> bool:
+    for b, c in zip(blocks, caches):
+        if c.geometry != geometry or c.k_ring.device != device:
+            return False
+        b.k_ring, b.v_ring = c.k_ring.data_ptr(), c.v_ring.data_ptr()
+        b.k_pers, b.v_pers = c.k_pers.data_ptr(), c.v_pers.data_ptr()
+        b.cache_scale = c.scale
+    return True
+
+
+def forward(table: ModelTable, token_ids: torch.Tensor, caches=None) -> Optional[torch.Tensor]:
+    """``tmw_stack_forward``: logits of every row (persistent rows first), or, with ``caches`` to fill, of the last one
+    only; None where the arguments are not what that call takes."""
+    device = table.device
+    if not table.forwards or token_ids.dtype != torch.int64 or token_ids.dim() != 2 or token_ids.device != device:
+        return None
+    B, T = token_ids.shape
+    d = _native.StackDesc.from_buffer_copy(table.desc)
+    if B == 0 or T == 0 or T > d.max_positions or B * (T + d.n_persistent) >= 1 << 31:
+        return None
+    token_ids = token_ids.contiguous()
+    blocks = type(table.blocks).from_buffer_copy(table.blocks)
+    if caches is not None and (len(caches) != len(blocks) or not _attach(blocks, caches, (B,) + table.geometry, device)):
+        return None
+    d.batch = B
+    lib = _native.lib()
+    nbytes = table.workspace_bytes.get((B, T))
+    if nbytes is None:
+        if len(table.workspace_bytes) > 256:
+            table.workspace_bytes.clear()
+        nbytes = table.workspace_bytes[B, T] = lib.tmw_stack_workspace(ctypes.byref(d), T)
+    workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    shape = (B, d.vocab) if caches is not None else (B, T + d.n_persistent, d.vocab)
+    logits = torch.empty(shape, dtype=table.dtype, device=device)
+    with _native._on(device):
+        _native.check(lib.tmw_stack_forward(ctypes.byref(d), blocks, token_ids.data_ptr(), T, int(caches is not None),
+                                            logits.data_ptr(), workspace.data_ptr(), nbytes, _native._stream_ptr(device)))
+    return logits
 
 
 def decode_step(table: ModelTable, token_ids: torch.Tensor, pos: torch.Tensor, caches) -> Optional[torch.Tensor]:
     """``tmw_decode_step``; None where the arguments are not what that call takes."""
     B = token_ids.shape[0]
     device = table.device
-    if (B == 0 or token_ids.dtype != torch.int64 or pos.dtype != torch.int32 or token_ids.dim() != 1 or pos.shape != (B,)
+    if (not table.decodes or B == 0 or token_ids.dtype != torch.int64 or pos.dtype != torch.int32 or token_ids.dim() != 1 or pos.shape != (B,)
             or token_ids.device != device or pos.device != device or len(caches) != len(table.blocks)):
         return None
     token_ids, pos = token_ids.contiguous(), pos.contiguous()
     geometry = (B,) + table.geometry
     blocks = type(table.blocks).from_buffer_copy(table.blocks)  # (the table is shared by all threads)
-    for b, c in zip(blocks, caches):
-        if c.geometry != geometry or c.k_ring.device != device:
-            return None
-        b.k_ring, b.v_ring = c.k_ring.data_ptr(), c.v_ring.data_ptr()
-        b.k_pers, b.v_pers = c.k_pers.data_ptr(), c.v_pers.data_ptr()
-        b.cache_scale = c.scale
+    if not _attach(blocks, caches, geometry, device):
+        return None
     d = _native.StackDesc.from_buffer_copy(table.desc)
     d.batch = B
     lib = _native.lib()
-    nbytes = table.workspace_bytes.get(B)
+    nbytes = table.workspace_bytes.get((B, -1))
     if nbytes is None:
-        nbytes = table.workspace_bytes[B] = lib.tmw_decode_step_workspace(ctypes.byref(d))
+        nbytes = table.workspace_bytes[B, -1] = lib.tmw_decode_step_workspace(ctypes.byref(d))
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
     logits = torch.empty((B, d.vocab), dtype=table.dtype, device=device)
     with _native._on(device):
         _native.check(lib.tmw_decode_step(ctypes.byref(d), blocks, token_ids.data_ptr(), pos.data_ptr(),
                                           logits.data_ptr(), workspace.data_ptr(), nbytes, _native._stream_ptr(device)))
     return logits
+
+
+def _plain_weight(mod: nn.Module, kind, dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """The weight of a submodule that is nothing but a ``kind`` without bias and hooks, contiguous and of that dtype."""
+    if type(mod) is not kind or mod._forward_hooks or mod._forward_pre_hooks:
+        return None
+    p = mod._parameters
+    w = p["weight"]
+    return w if p["bias"] is None and w.dtype is dtype and w.is_contiguous() else None
+
+
+def attention_forward(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float) -> Optional[torch.Tensor]:
+    """An attention module's forward as one ``tmw_attention_forward``; None where that call does not apply."""
+    dtype = x.dtype
+    if (dtype is not torch.bfloat16 and dtype is not torch.float16) or attn.algo or attn.core_events is not None \
+            or not x.is_contiguous():
+        return None
+    B, L, D = x.shape
+    mods = attn._modules
+    w_qkv, w_out = _plain_weight(mods["qkv_proj"], nn.Linear, dtype), _plain_weight(mods["out_proj"], nn.Linear, dtype)
+    if w_qkv is None or w_out is None or B * L == 0 or D % 8 or attn.d_head % 8 or _global_hooks():
+        return None
+    conv, taps = (None, None, None), 0
+    if block_size and attn.use_conv:
+        ws = [_plain_weight(mods[n], nn.Conv1d, dtype) for n in ("conv_q", "conv_k", "conv_v")]
+        taps = ws[0].shape[2] if ws[0] is not None else 0
+        if not 1 <= taps <= 8 or any(w is None or w.shape != (D, 1, taps) for w in ws):
+            return None
+        conv = tuple(w.data_ptr() for w in ws)
+    d = _native.AttentionDesc(_native._DTYPES[dtype], B, L, attn.n_heads, attn.d_head, attn.window_size, n_persistent, block_size,
+                              taps, scale)
+    lib = _native.lib()
+    ref = ctypes.byref(d)
+    device = x.device
+    nbytes = lib.tmw_attention_workspace(ref)
+    y = torch.empty_like(x)
+    workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    px, pq, po = x.data_ptr(), w_qkv.data_ptr(), w_out.data_ptr()
+    if (px | pq | po) % 16 or w_qkv.device != device:
+        return None
+    with _native._on(device):
+        _native.check(lib.tmw_attention_forward(ref, px, pq, *conv, po, y.data_ptr(), workspace.data_ptr(), nbytes,
+                                                _native._stream_ptr(device)))
+    return y

@@ -26,7 +26,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from .. import _native
+from .. import _native, _stack
 
 
 class _CausalDwConv(torch.autograd.Function):
@@ -134,6 +134,9 @@ class BlockSparseAttention(nn.Module):
         B, L, D = x.shape
         if self.n_persistent >= L:
             raise ValueError(f"n_persistent ({self.n_persistent}) must be < seq_len ({L})")
+        y = _stack.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)  # the module as one call
+        if y is not None:
+            return self.dropout(y)
         qkv = _native.project(self.qkv_proj, x)
         if self.use_conv:
             qkv = _native.causal_dwconv(qkv, self.stacked_conv_weight())

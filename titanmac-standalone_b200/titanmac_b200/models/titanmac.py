@@ -74,6 +74,24 @@ class TitanMAC(nn.Module):
     def forward(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None,
                 attention_mask: Optional[torch.Tensor] = None) -> Dict[str, torch.Tensor]:
         Np = self.config.n_persistent
+        logits = None
+        if not torch.is_grad_enabled() or not any(p.requires_grad for p in self.parameters()):
+            table = _stack.table_of(self)
+            if table is not None:  # the whole forward as one call (tmw_stack_forward)
+                logits = _stack.forward(table, input_ids)
+        if logits is None:
+            logits = self._forward_modules(input_ids)
+        logits = logits[:, Np:, :] if Np > 0 else logits
+        out = {"logits": logits}
+        if labels is not None:
+            shift_logits = logits[..., :-1, :].contiguous()
+            shift_labels = labels[..., 1:].contiguous()
+            out["loss"] = F.cross_entropy(shift_logits.reshape(-1, self.config.vocab_size), shift_labels.reshape(-1),
+                                          reduction="mean", ignore_index=-100)
+        return out
+
+    def _forward_modules(self, input_ids: torch.Tensor) -> torch.Tensor:
+        """Logits of every row, persistent rows first, module by module."""
         x = self._embed(input_ids)
         # Same wiring as TitanBlock.forward, with every residual add folded into the RMSNorm that follows it
         # (one kernel): the MLP output of a layer is added by the next layer's first norm, or by the final norm.
@@ -87,15 +105,7 @@ class TitanMAC(nn.Module):
             x, h = layer.norm_mlp.add_forward(x, a, inplace=True)
             pending = layer.mlp(h)
         h = self.norm(x) if pending is None else self.norm.add_forward(x, pending, inplace=True)[1]
-        logits = _native.project(self.lm_head, h)
-        logits = logits[:, Np:, :] if Np > 0 else logits
-        out = {"logits": logits}
-        if labels is not None:
-            shift_logits = logits[..., :-1, :].contiguous()
-            shift_labels = labels[..., 1:].contiguous()
-            out["loss"] = F.cross_entropy(shift_logits.reshape(-1, self.config.vocab_size), shift_labels.reshape(-1),
-                                          reduction="mean", ignore_index=-100)
-        return out
+        return _native.project(self.lm_head, h)
 
     # --------------------------------------------------------------- generation --
     def _need_windowed(self) -> None:
@@ -116,9 +126,14 @@ class TitanMAC(nn.Module):
         self._need_windowed()
         B, T = input_ids.shape
         Np = self.config.n_persistent
-        x = self._embed(input_ids)
         if caches is None:
-            caches = self.new_caches(B, x.device, x.dtype)
+            caches = self.new_caches(B, input_ids.device, self.embed_tokens.weight.dtype)
+        table = _stack.table_of(self)
+        if table is not None:  # the prompt as one call (tmw_stack_forward)
+            logits = _stack.forward(table, input_ids, caches)
+            if logits is not None:
+                return logits, caches
+        x = self._embed(input_ids)
         pending = None
         for layer, cache in zip(self.layers, caches):
             attn = layer.attention
