@@ -393,6 +393,53 @@ TMW_API int tmw_stack_forward(const tmw_stack_desc* desc, const tmw_block* block
                       int32_t last_only, void* logits, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * Training in 16-bit types: forward that keeps what the backward needs in `saved` (device memory of the size the
+ * *_train_saved call gives, to be handed on unchanged), and backward.  Replaces what autograd records and replays through
+ * WindowedAttention / BlockSparseAttention (see tmw_prefill_backward) and, for the whole model, through
+ * titans_core/models/titanmac.py:554-662 with its blocks.  `scratch` is used until the call's kernels have finished.
+ * Gradients are written (not added to); the bias and convolution entries are NULL where the model has none.  d_model at
+ * most 2048 for the whole model, otherwise the limits of tmw_stack_forward.
+ */
+typedef struct tmw_block_grads {
+    void *norm_attn, *w_qkv, *w_out;
+    void *norm_mlp, *w_fc1, *b_fc1, *w_fc2, *b_fc2;
+    void *conv_q, *conv_k, *conv_v;
+} tmw_block_grads;
+
+typedef struct tmw_stack_grads {
+    void *embed_tokens, *head; /* the same array for tied weights */
+    void *embed_positions, *persistent, *norm;
+} tmw_stack_grads;
+
+TMW_API size_t tmw_attention_train_saved(const tmw_attention_desc* desc);
+TMW_API size_t tmw_attention_train_scratch(const tmw_attention_desc* desc);
+TMW_API int tmw_attention_train_forward(const tmw_attention_desc* desc, const void* x, const void* w_qkv, const void* conv_q,
+                                const void* conv_k, const void* conv_v, const void* w_out, void* y, void* saved,
+                                size_t saved_bytes, void* stream);
+TMW_API int tmw_attention_train_backward(const tmw_attention_desc* desc, const void* x, const void* w_qkv, const void* conv_q,
+                                 const void* conv_k, const void* conv_v, const void* w_out, const void* dy, const void* saved,
+                                 void* dx, const tmw_block_grads* grads, void* scratch, size_t scratch_bytes, void* stream);
+
+TMW_API size_t tmw_stack_train_saved(const tmw_stack_desc* desc, int32_t tokens);
+TMW_API size_t tmw_stack_train_scratch(const tmw_stack_desc* desc, int32_t tokens);
+TMW_API int tmw_stack_train_forward(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, int32_t tokens,
+                            void* logits, void* saved, size_t saved_bytes, void* stream);
+TMW_API int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_block* blocks, const tmw_stack_grads* grads,
+                             const tmw_block_grads* block_grads, const int64_t* token_ids, int32_t tokens,
+                             const void* d_logits, const void* saved, void* scratch, size_t scratch_bytes, void* stream);
+
+/*
+ * Shifted cross-entropy (titanmac.py:674-684) over logits [batch, n_persistent + tokens, vocab]: row n_persistent + t of a
+ * sequence predicts labels[t + 1]; label -100 does not count, nor do the persistent rows and the last.  With d_logits
+ * NULL: *loss (in dtype) = the mean over the counted rows, `stats` (4 + 2 * rows floats) filled for the backward.  Else the
+ * backward: d_logits = softmax gradient times *grad (in dtype), zero on rows that do not count.  vocab a multiple of 8;
+ * labels outside the vocabulary do not count and are reported by tmw_poll_status.
+ */
+TMW_API int tmw_cross_entropy(int32_t dtype, int32_t batch, int32_t tokens, int32_t n_persistent, int32_t vocab,
+                      const void* logits, const int64_t* labels, void* loss, float* stats, const void* grad, void* d_logits,
+                      void* stream);
+
+/*
  * One decode step of the whole model: token_ids [batch] int64 and pos [batch] int32 (device) -> logits [batch, vocab].
  * Every block runs RMSNorm -> QKV -> tmw_decode on its ring -> output projection + residual -> RMSNorm -> MLP + residual
  * (titan_block.py:92-100, blocks/mlp.py:58-65), then the final norm and the head; what the reference's generation

@@ -74,7 +74,7 @@ SideStream* side_stream_of_current_device() {
 
 // the opt-in to more than 48 KB of dynamic shared memory is per kernel and per device: made once
 int allow_shared_memory(const void* kern, int bytes) {
-    constexpr int kMaxDevices = 64, kMaxKernels = 32;
+    constexpr int kMaxDevices = 64, kMaxKernels = 256;
     struct Entry { const void* kern; int allowed[kMaxDevices]; };
     static std::mutex mutex;
     static Entry table[kMaxKernels] = {};

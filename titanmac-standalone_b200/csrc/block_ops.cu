@@ -252,18 +252,20 @@ int launch_dwconv_taps(int batch, int rows, int channels, const void* x, const C
 // [channels, TAPS] (zero on entry) with atomics.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(kConvThreads)
-dwconv_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ dy, T* __restrict__ dx,
+dwconv_bwd_kernel(const T* __restrict__ x, const ConvWeights f, const T* __restrict__ dy, T* __restrict__ dx,
                   float* __restrict__ dw, int rows, int channels) {
     const int vec = blockIdx.x * kConvThreads + threadIdx.x;
     if (vec * 8 >= channels) return;
     const int t0 = blockIdx.y * kConvStrip;
     const int t1 = min(rows, t0 + kConvStrip);
     const long long base = (long long)blockIdx.z * rows * channels + vec * 8;
+    const int part = vec * 8 / f.per, first = vec * 8 - part * f.per;
+    const T* w = static_cast<const T*>(part == 0 ? f.w[0] : part == 1 ? f.w[1] : f.w[2]);
     float wr[TAPS][8];
 #pragma unroll
     for (int c = 0; c < 8; ++c)
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) wr[j][c] = to_f32<T>(w[(long long)(vec * 8 + c) * TAPS + j]);
+        for (int j = 0; j < TAPS; ++j) wr[j][c] = to_f32<T>(w[(long long)(first + c) * TAPS + j]);
     // ---- dx: bottom-up, ahead[m] = dy[t + m]
     float ahead[TAPS][8];
 #pragma unroll
@@ -327,10 +329,10 @@ dwconv_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __r
 }
 
 template <typename T, int TAPS>
-int launch_dwconv_bwd_taps(int batch, int rows, int channels, const void* x, const void* w, const void* dy, void* dx,
+int launch_dwconv_bwd_taps(int batch, int rows, int channels, const void* x, const ConvWeights& w, const void* dy, void* dx,
                            float* dw, cudaStream_t stream) {
     const dim3 grid((channels / 8 + kConvThreads - 1) / kConvThreads, (rows + kConvStrip - 1) / kConvStrip, batch);
-    dwconv_bwd_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), static_cast<const T*>(w),
+    dwconv_bwd_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), w,
                                                                   static_cast<const T*>(dy), static_cast<T*>(dx), dw,
                                                                   rows, channels);
     TMW_CUDA_TRY(cudaGetLastError());
@@ -338,7 +340,7 @@ int launch_dwconv_bwd_taps(int batch, int rows, int channels, const void* x, con
 }
 
 template <typename T>
-int launch_dwconv_bwd(int batch, int rows, int channels, int taps, const void* x, const void* w, const void* dy,
+int launch_dwconv_bwd(int batch, int rows, int channels, int taps, const void* x, const ConvWeights& w, const void* dy,
                       void* dx, float* dw, cudaStream_t stream) {
     switch (taps) {
         case 1: return launch_dwconv_bwd_taps<T, 1>(batch, rows, channels, x, w, dy, dx, dw, stream);
@@ -392,6 +394,18 @@ int launch_dwconv(int dtype, int batch, int rows, int channels, int taps, const 
     }
 }
 
+int launch_dwconv_backward(int dtype, int batch, int rows, int channels, int taps, const void* x, const void* const* w, int n_w,
+                           const void* dy, void* dx, float* dw, cudaStream_t stream) {
+    ConvWeights f;
+    f.per = channels / n_w;
+    for (int i = 0; i < 3; ++i) f.w[i] = w[i < n_w ? i : 0];
+    switch (dtype) {
+        case TMW_F32: return launch_dwconv_bwd<float>(batch, rows, channels, taps, x, f, dy, dx, dw, stream);
+        case TMW_BF16: return launch_dwconv_bwd<__nv_bfloat16>(batch, rows, channels, taps, x, f, dy, dx, dw, stream);
+        default: return launch_dwconv_bwd<__half>(batch, rows, channels, taps, x, f, dy, dx, dw, stream);
+    }
+}
+
 }  // namespace tmw
 
 extern "C" int tmw_causal_dwconv(int32_t dtype, int32_t batch, int32_t rows, int32_t channels, int32_t taps,
@@ -425,12 +439,7 @@ extern "C" int tmw_causal_dwconv_backward(int32_t dtype, int32_t batch, int32_t 
         return TMW_ERR_INVALID_ARGUMENT;
     if ((((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) != 0) return TMW_ERR_INVALID_ARGUMENT;
     if (batch > 65535 || (rows + kConvStrip - 1) / kConvStrip > 65535) return TMW_ERR_TOO_LARGE;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    switch (dtype) {
-        case TMW_F32: return launch_dwconv_bwd<float>(batch, rows, channels, taps, x, weight, dy, dx, dw, s);
-        case TMW_BF16: return launch_dwconv_bwd<__nv_bfloat16>(batch, rows, channels, taps, x, weight, dy, dx, dw, s);
-        default: return launch_dwconv_bwd<__half>(batch, rows, channels, taps, x, weight, dy, dx, dw, s);
-    }
+    return launch_dwconv_backward(dtype, batch, rows, channels, taps, x, &weight, 1, dy, dx, dw, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tmw_gelu(int32_t dtype, int64_t n, const void* x, void* y, void* stream) {

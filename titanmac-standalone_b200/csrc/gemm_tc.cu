@@ -15,6 +15,7 @@
 #include <cuda.h>
 
 #include <cmath>
+#include <type_traits>
 #include <mutex>
 
 #include "tc_ptx.cuh"
@@ -49,13 +50,75 @@ struct GemmSmem {
 
 struct GemmParams {
     int m, n, k;
-    int epilogue;        // tmw_epilogue
+    int epilogue;        // GemmEpilogue
     const void* bias;    // [n] in the dtype of the operands, or nullptr
+    void* aux;           // [m, n] beside the output (see GemmEpilogue), contiguous
+    float* partial;      // k cut into `splits` ranges: their fp32 sums go to [splits][m][n] here instead of to the output
+    int splits;
     int drain;           // a dependent launch follows: the stores have to be complete when the kernel ends
     int* status;
 };
 
-template <int BN, bool BF16>
+// 32 accumulator columns of one row -> the values to be stored (bias, then the epilogue)
+template <bool BF16>
+__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, int row, int col) {
+    using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+    if (p.bias != nullptr) {
+        // bias of 32 columns: 64 bytes, the same for every row (broadcast loads)
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+            if (col + j < p.n) {  // n is a multiple of 8
+                float b8[8];
+                load8<T>(static_cast<const T*>(p.bias) + col + j, b8);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
+            }
+    }
+    if (p.epilogue == GEMM_GELU) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
+    } else if (p.epilogue > GEMM_GELU && row < p.m) {
+        T* aux = static_cast<T*>(p.aux) + (long long)row * p.n + col;
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+            if (col + j < p.n) {
+                float x[8];
+                if (p.epilogue == GEMM_GELU_KEEP) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = to_f32<T>(from_f32<T>(v[j + e]));
+                    store8<T>(aux + j, x);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[j + e] = gelu_erf(x[e]);
+                } else {
+                    load8<T>(aux + j, x);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        v[j + e] = p.epilogue == GEMM_ADD ? x[e] + to_f32<T>(from_f32<T>(v[j + e])) : v[j + e] * gelu_slope(x[e]);
+                }
+            }
+    }
+}
+
+// the fp32 sums of a k range
+__device__ __forceinline__ void store_partial(const float (&v)[32], const GemmParams& p, int split, int row, int col) {
+    if (row >= p.m) return;
+    float* dst = p.partial + ((long long)split * p.m + row) * p.n + col;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4)
+        if (col + j < p.n) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+}
+
+// An operand tile of R rows (of the product: M or N) x 64 k-elements in shared memory, 128 bytes per swizzled row.
+// K-major (the matrix is [R, k] row-major): R rows of 64 k.  MN-major (the matrix is [k, R]): R / 64 sub-tiles of 64 k-rows
+// x 64 columns.
+template <int R, bool MN>
+__device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
+    return MN ? mnmajor_desc(addr, 64 * 128) : kmajor_desc(addr);
+}
+template <bool MN>
+constexpr uint64_t kStepDesc = MN ? 128 : 2;  // 16 k-elements on, in units of 16 bytes
+
+template <int BN, bool BF16, bool AMN, bool BMN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
@@ -77,7 +140,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = (p.n + BN - 1) / BN, m_tiles = (p.m + GM - 1) / GM;
-    const int tiles = n_tiles * m_tiles;
+    const int tiles = n_tiles * m_tiles * p.splits;  // (tile, k range)
     const int k_blocks = (p.k + L::kSlices * GK - 1) / (L::kSlices * GK);
 
     if (threadIdx.x == 0) {
@@ -110,15 +173,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int s = 0;
             uint32_t parity = 1;
             for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-                const int row0 = (tile / n_tiles) * GM, col0 = (tile % n_tiles) * BN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                const int mn = tile / p.splits, split = tile % p.splits;
+                const int row0 = (mn / n_tiles) * GM, col0 = (mn % n_tiles) * BN;
+                const int kb1 = k_blocks * (split + 1) / p.splits;
+                for (int kb = k_blocks * split / p.splits; kb < kb1; ++kb) {
                     mbar_wait(empty(s), parity, abort_flag, p.status);
                     mbar_expect_tx(full(s), L::kStage);
                     const uint32_t dst = smem_base + s * L::kStage;
 #pragma unroll
                     for (int u = 0; u < SL; ++u) {  // (slices beyond K arrive as zeros)
-                        tma_load_2d(dst + u * (GM * GK * 2), &map_a, full(s), (kb * SL + u) * GK, row0);
-                        tma_load_2d(dst + L::kStageA + u * (BN * GK * 2), &map_w, full(s), (kb * SL + u) * GK, col0);
+                        const int k0 = (kb * SL + u) * GK;
+                        const uint32_t da = dst + u * (GM * GK * 2), db = dst + L::kStageA + u * (BN * GK * 2);
+                        if (AMN) {
+#pragma unroll
+                            for (int c = 0; c < GM / 64; ++c) tma_load_2d(da + c * 8192, &map_a, full(s), row0 + c * 64, k0);
+                        } else {
+                            tma_load_2d(da, &map_a, full(s), k0, row0);
+                        }
+                        if (BMN) {
+#pragma unroll
+                            for (int c = 0; c < BN / 64; ++c) tma_load_2d(db + c * 8192, &map_w, full(s), col0 + c * 64, k0);
+                        } else {
+                            tma_load_2d(db, &map_w, full(s), k0, col0);
+                        }
                     }
                     if (++s == S) { s = 0; parity ^= 1u; }
                 }
@@ -128,7 +205,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1) {
         // ---------------- tensor-core issue ----------------
         if (elect_one()) {
-            const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, BN);
+            const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, BN) | (AMN ? 1u << 15 : 0u) | (BMN ? 1u << 16 : 0u);
             int s = 0, t = 0;
             uint32_t parity = 0;
             for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
@@ -136,19 +213,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 mbar_wait(acc_empty(buf), ((t >> 1) & 1) ^ 1, abort_flag, p.status);  // the epilogue has drained it
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                const int split = tile % p.splits, kb0 = k_blocks * split / p.splits, kb1 = k_blocks * (split + 1) / p.splits;
+                for (int kb = kb0; kb < kb1; ++kb) {
                     mbar_wait(full(s), parity, abort_flag, p.status);
                     tc_fence_after();
-                    const uint64_t a_desc = kmajor_desc(smem_base + s * L::kStage);
-                    const uint64_t b_desc = kmajor_desc(smem_base + s * L::kStage + L::kStageA);
+                    const uint64_t a_desc = tile_desc<GM, AMN>(smem_base + s * L::kStage);
+                    const uint64_t b_desc = tile_desc<BN, BMN>(smem_base + s * L::kStage + L::kStageA);
 #pragma unroll
                     for (int u = 0; u < SL; ++u)
 #pragma unroll
                         for (int kk = 0; kk < GK / 16; ++kk)
-                            mma_ss(d_tmem, a_desc + u * (GM * GK * 2 / 16) + 2 * kk, b_desc + u * (BN * GK * 2 / 16) + 2 * kk,
-                                   idesc, (kb | u | kk) ? 1u : 0u);
+                            mma_ss(d_tmem, a_desc + u * (GM * GK * 2 / 16) + kStepDesc<AMN> * kk,
+                                   b_desc + u * (BN * GK * 2 / 16) + kStepDesc<BMN> * kk, idesc, (kb > kb0 || (u | kk)) ? 1u : 0u);
                     tc_commit(empty(s));  // the stage is free once these products have read it
-                    if (kb == k_blocks - 1) tc_commit(acc_full(buf));
+                    if (kb == kb1 - 1) tc_commit(acc_full(buf));
                     if (++s == S) { s = 0; parity ^= 1u; }
                 }
             }
@@ -168,7 +246,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int t = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
             const int buf = t & 1;
-            const int row0 = (tile / n_tiles) * GM, col0 = (tile % n_tiles) * BN;
+            const int mn = tile / p.splits, row0 = (mn / n_tiles) * GM, col0 = (mn % n_tiles) * BN;
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
             // the previous tile's store must have read the staging buffer before it is overwritten
@@ -190,23 +268,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-                if (p.bias != nullptr) {
-                    // bias of 32 columns: 64 bytes, the same for every row (broadcast loads)
-#pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        if (col + j < p.n) {  // n is a multiple of 8
-                            float b8[8];
-                            if (BF16) load8<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.bias) + col + j, b8);
-                            else load8<__half>(static_cast<const __half*>(p.bias) + col + j, b8);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
-                        }
-                    }
+                if (p.partial != nullptr) {
+                    store_partial(v, p, tile % p.splits, row0 + row, col);
+                    continue;
                 }
-                if (p.epilogue == TMW_EPILOGUE_GELU) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
-                }
+                finish_panel<BF16>(v, p, row0 + row, col);
                 // 32 columns = 64 bytes = four 16-byte chunks of this row in panel pn (64-byte swizzle)
                 uint8_t* prow = stage + pn * (GM * 64) + row * 64;
 #pragma unroll
@@ -227,7 +293,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             fence_proxy_async_smem();
             named_barrier_sync(2, kEpiWarps * 32);
-            if (epi_leader) {
+            if (epi_leader && p.partial == nullptr) {
                 for (int pn = 0; pn < kPanels; ++pn)
                     if (col0 + pn * kPanel < p.n)
                         tma_store_2d(&map_c, smem_u32(stage + pn * (GM * 64)), col0 + pn * kPanel, row0);
@@ -275,7 +341,7 @@ struct PairSmem {
     static_assert(kStage % 1024 == 0 && kStageA % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
 
-template <int BN, bool BF16>
+template <int BN, bool BF16, bool AMN, bool BMN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
@@ -300,12 +366,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const uint32_t rank = cluster_ctarank();  // 0: issues the products, 1: partner
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int n_tiles = (p.n + BN - 1) / BN, m_tiles = (p.m + 2 * GM - 1) / (2 * GM);
-    const int tiles = n_tiles * m_tiles;
+    const int tiles = n_tiles * m_tiles * p.splits;  // (tile, k range)
     const int k_blocks = (p.k + GK - 1) / GK;
     // columns a tile multiplies: BN, or for the last tile of a row what is left of N (in steps of 32) - a product
     // over columns that do not exist would cost its full time
     auto n_of = [&](int tile) -> int {
-        const int rem = p.n - (tile % n_tiles) * BN;
+        const int rem = p.n - (tile / p.splits % n_tiles) * BN;
         return rem >= BN ? BN : (rem + 31) / 32 * 32;
     };
 
@@ -339,16 +405,29 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int s = 0;
             uint32_t parity = 1;
             for (int tile = pair; tile < tiles; tile += pairs) {
-                const int row0 = (tile / n_tiles) * (2 * GM) + (int)rank * GM;
+                const int mn = tile / p.splits, split = tile % p.splits;
+                const int row0 = (mn / n_tiles) * (2 * GM) + (int)rank * GM;
                 // each CTA supplies half of the tile's columns (the box is BN / 2 rows; a narrow tile uses its first rows)
-                const int col0 = (tile % n_tiles) * BN + (int)rank * (n_of(tile) / 2);
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                const int col0 = (mn % n_tiles) * BN + (int)rank * (n_of(tile) / 2);
+                const int kb1 = k_blocks * (split + 1) / p.splits;
+                for (int kb = k_blocks * split / p.splits; kb < kb1; ++kb) {
                     mbar_wait(empty(s), parity, abort_flag, p.status);
                     if (rank == 0) mbar_expect_tx(full(s), 2 * L::kStage);  // both CTAs' bytes
                     const uint32_t bar0 = map_to_cta(full(s), 0);
                     const uint32_t dst = smem_base + s * L::kStage;
-                    tma_load_2d_pair(dst, &map_a, bar0, kb * GK, row0);
-                    tma_load_2d_pair(dst + L::kStageA, &map_w, bar0, kb * GK, col0);
+                    if (AMN) {
+#pragma unroll
+                        for (int c = 0; c < GM / 64; ++c) tma_load_2d_pair(dst + c * 8192, &map_a, bar0, row0 + c * 64, kb * GK);
+                    } else {
+                        tma_load_2d_pair(dst, &map_a, bar0, kb * GK, row0);
+                    }
+                    if (BMN) {
+#pragma unroll
+                        for (int c = 0; c < BN / 128; ++c)
+                            tma_load_2d_pair(dst + L::kStageA + c * 8192, &map_w, bar0, col0 + c * 64, kb * GK);
+                    } else {
+                        tma_load_2d_pair(dst + L::kStageA, &map_w, bar0, kb * GK, col0);
+                    }
                     if (++s == S) { s = 0; parity ^= 1u; }
                 }
             }
@@ -361,20 +440,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             uint32_t parity = 0;
             for (int tile = pair; tile < tiles; tile += pairs, ++t) {
                 const int buf = t & 1;
-                const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, (uint32_t)n_of(tile), 2 * GM);
+                const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, (uint32_t)n_of(tile), 2 * GM) | (AMN ? 1u << 15 : 0u) |
+                                       (BMN ? 1u << 16 : 0u);
                 mbar_wait(acc_empty(buf), ((t >> 1) & 1) ^ 1, abort_flag, p.status);
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                const int split = tile % p.splits, kb0 = k_blocks * split / p.splits, kb1 = k_blocks * (split + 1) / p.splits;
+                for (int kb = kb0; kb < kb1; ++kb) {
                     mbar_wait(full(s), parity, abort_flag, p.status);
                     tc_fence_after();
-                    const uint64_t a_desc = kmajor_desc(smem_base + s * L::kStage);
-                    const uint64_t b_desc = kmajor_desc(smem_base + s * L::kStage + L::kStageA);
+                    const uint64_t a_desc = tile_desc<GM, AMN>(smem_base + s * L::kStage);
+                    const uint64_t b_desc = tile_desc<BN / 2, BMN>(smem_base + s * L::kStage + L::kStageA);
 #pragma unroll
                     for (int kk = 0; kk < GK / 16; ++kk)
-                        mma_ss_pair(d_tmem, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                        mma_ss_pair(d_tmem, a_desc + kStepDesc<AMN> * kk, b_desc + kStepDesc<BMN> * kk, idesc,
+                                    (kb > kb0 || kk) ? 1u : 0u);
                     tc_commit_pair(empty(s));
-                    if (kb == k_blocks - 1) tc_commit_pair(acc_full(buf));
+                    if (kb == kb1 - 1) tc_commit_pair(acc_full(buf));
                     if (++s == S) { s = 0; parity ^= 1u; }
                 }
             }
@@ -391,7 +473,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         int t = 0;
         for (int tile = pair; tile < tiles; tile += pairs, ++t) {
             const int buf = t & 1;
-            const int row0 = (tile / n_tiles) * (2 * GM) + (int)rank * GM, col0 = (tile % n_tiles) * BN;
+            const int mn = tile / p.splits;
+            const int row0 = (mn / n_tiles) * (2 * GM) + (int)rank * GM, col0 = (mn % n_tiles) * BN;
             // the tile's panels of 32 columns, split between the two warps of a lane group
             const int panels = n_of(tile) / kPanel, half_panels = (panels + 1) / 2;
             const int panel0 = half == 0 ? 0 : half_panels;
@@ -415,22 +498,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-                if (p.bias != nullptr) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        if (col + j < p.n) {
-                            float b8[8];
-                            if (BF16) load8<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.bias) + col + j, b8);
-                            else load8<__half>(static_cast<const __half*>(p.bias) + col + j, b8);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
-                        }
-                    }
+                if (p.partial != nullptr) {
+                    store_partial(v, p, tile % p.splits, row0 + row, col);
+                    continue;
                 }
-                if (p.epilogue == TMW_EPILOGUE_GELU) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
-                }
+                finish_panel<BF16>(v, p, row0 + row, col);
                 uint8_t* prow = stage + pn * (GM * 64) + row * 64;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -450,7 +522,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
             fence_proxy_async_smem();
             named_barrier_sync(2, kEpiWarps * 32);
-            if (epi_leader && row0 < p.m) {
+            if (epi_leader && row0 < p.m && p.partial == nullptr) {
                 for (int pn = 0; pn < kPanels; ++pn)
                     if (col0 + pn * kPanel < p.n)
                         tma_store_2d(&map_c, smem_u32(stage + pn * (GM * 64)), col0 + pn * kPanel, row0);
@@ -479,32 +551,57 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // ---------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------
+bool make_maps(const GemmCall& g, int b_rows, CUtensorMap* ma, CUtensorMap* mb, CUtensorMap* mc) {
+    const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
+    return (g.a_mn ? make_map_2d(ma, g.a, g.dtype, g.k, g.m, g.lda, GK, 64, sw) : make_map_2d(ma, g.a, g.dtype, g.m, g.k, g.lda, GM, GK, sw)) &&
+           (g.b_mn ? make_map_2d(mb, g.b, g.dtype, g.k, g.n, g.ldb, GK, 64, sw)
+                   : make_map_2d(mb, g.b, g.dtype, g.n, g.k, g.ldb, b_rows, GK, sw)) &&
+           make_map_2d(mc, g.c, g.dtype, g.m, g.n, g.ldc, GM, kPanel, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
+int gemm_params(const GemmCall& g, GemmParams* p) {
+    p->m = g.m; p->n = g.n; p->k = g.k;
+    p->epilogue = g.epilogue;
+    p->bias = g.bias;
+    p->aux = g.aux;
+    p->splits = g.splits;
+    p->partial = g.splits > 1 ? g.partial : nullptr;
+    p->drain = g.chain & kChainFollowed;
+    p->status = device_status_word();
+    return p->status == nullptr ? TMW_ERR_CUDA : TMW_OK;
+}
+
+// `with` is called with the kernel of the call's data type and operand layouts
+template <typename K00, typename K01, typename K11, typename F>
+int with_layout(const GemmCall& g, K00 k00, K01 k01, K11 k11, F with) {
+    if (!g.a_mn) return g.b_mn ? with(k01) : with(k00);
+    return g.b_mn ? with(k11) : TMW_ERR_UNSUPPORTED;
+}
+
 template <int BN>
-int launch_gemm(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream,
-                int chain) {
+int launch_gemm(const GemmCall& g, cudaStream_t stream) {
     using L = GemmSmem<BN>;
-    CUtensorMap ma, mw, mc;
-    if (!make_map_2d(&ma, a, d.dtype, d.m, d.k, d.lda, GM, GK, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map_2d(&mw, w, d.dtype, d.n, d.k, d.ldw, BN, GK, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map_2d(&mc, c, d.dtype, d.m, d.n, d.ldc, GM, kPanel, CU_TENSOR_MAP_SWIZZLE_64B))
-        return TMW_ERR_CUDA;
+    CUtensorMap ma, mb, mc;
     GemmParams p;
-    p.m = d.m; p.n = d.n; p.k = d.k;
-    p.epilogue = d.epilogue;
-    p.bias = bias;
-    p.drain = chain & kChainFollowed;
-    p.status = device_status_word();
-    if (p.status == nullptr) return TMW_ERR_CUDA;
-    const int tiles = ((d.m + GM - 1) / GM) * ((d.n + BN - 1) / BN);
+    if (!make_maps(g, BN, &ma, &mb, &mc)) return TMW_ERR_CUDA;
+    if (gemm_params(g, &p) != TMW_OK) return TMW_ERR_CUDA;
+    const int tiles = ((g.m + GM - 1) / GM) * ((g.n + BN - 1) / BN) * g.splits;
     const int grid = tiles < sm_count() ? tiles : sm_count();
     auto run = [&](auto kern) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), L::kTotal);
         if (rc != TMW_OK) return rc;
-        TMW_CUDA_TRY(launch_ex(kern, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, chain & kChainDependent, 1, ma, mw, mc, p));
+        TMW_CUDA_TRY(launch_ex(kern, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, mc, p));
         return TMW_OK;
     };
-    const int st = d.dtype == TMW_BF16 ? run(gemm_tc_kernel<BN, true>) : run(gemm_tc_kernel<BN, false>);
-    return st;
+    if constexpr (BN == 64 || BN == 128) {
+        return g.dtype == TMW_BF16 ? with_layout(g, gemm_tc_kernel<BN, true, false, false>, gemm_tc_kernel<BN, true, false, true>,
+                                                 gemm_tc_kernel<BN, true, true, true>, run)
+                                   : with_layout(g, gemm_tc_kernel<BN, false, false, false>, gemm_tc_kernel<BN, false, false, true>,
+                                                 gemm_tc_kernel<BN, false, true, true>, run);
+    } else {
+        if (g.a_mn || g.b_mn) return TMW_ERR_UNSUPPORTED;
+        return g.dtype == TMW_BF16 ? run(gemm_tc_kernel<BN, true, false, false>) : run(gemm_tc_kernel<BN, false, false, false>);
+    }
 }
 
 // How many CTA pairs of the kernel the device runs at once (asked once per kernel and device).
@@ -536,72 +633,111 @@ int max_active_pairs(const void* kern, int smem_bytes) {
 }
 
 template <int BN>
-int launch_gemm_pair(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c,
-                     cudaStream_t stream, int chain) {
+int launch_gemm_pair(const GemmCall& g, cudaStream_t stream) {
     using L = PairSmem<BN>;
-    CUtensorMap ma, mw, mc;
-    if (!make_map_2d(&ma, a, d.dtype, d.m, d.k, d.lda, GM, GK, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map_2d(&mw, w, d.dtype, d.n, d.k, d.ldw, BN / 2, GK, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map_2d(&mc, c, d.dtype, d.m, d.n, d.ldc, GM, kPanel, CU_TENSOR_MAP_SWIZZLE_64B))
-        return TMW_ERR_CUDA;
+    CUtensorMap ma, mb, mc;
     GemmParams p;
-    p.m = d.m; p.n = d.n; p.k = d.k;
-    p.epilogue = d.epilogue;
-    p.bias = bias;
-    p.drain = chain & kChainFollowed;
-    p.status = device_status_word();
-    if (p.status == nullptr) return TMW_ERR_CUDA;
-    const int tiles = ((d.m + 2 * GM - 1) / (2 * GM)) * ((d.n + BN - 1) / BN);
+    if (!make_maps(g, BN / 2, &ma, &mb, &mc)) return TMW_ERR_CUDA;
+    if (gemm_params(g, &p) != TMW_OK) return TMW_ERR_CUDA;
+    const int tiles = ((g.m + 2 * GM - 1) / (2 * GM)) * ((g.n + BN - 1) / BN) * g.splits;
     auto run = [&](auto kern) -> int {
         const void* fn = reinterpret_cast<const void*>(kern);
         const int rc = allow_shared_memory(fn, L::kTotal);
         if (rc != TMW_OK) return rc;
         const int resident = max_active_pairs(fn, L::kTotal);
         const int pairs = tiles < resident ? tiles : resident;
-        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kGemmThreads), L::kTotal, stream, chain & kChainDependent, 1, ma, mw, mc, p));
+        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kGemmThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, mc, p));
         return TMW_OK;
     };
-    const int st = d.dtype == TMW_BF16 ? run(gemm_tc_pair_kernel<BN, true>) : run(gemm_tc_pair_kernel<BN, false>);
-    return st;
+    return g.dtype == TMW_BF16
+               ? with_layout(g, gemm_tc_pair_kernel<BN, true, false, false>, gemm_tc_pair_kernel<BN, true, false, true>,
+                             gemm_tc_pair_kernel<BN, true, true, true>, run)
+               : with_layout(g, gemm_tc_pair_kernel<BN, false, false, false>, gemm_tc_pair_kernel<BN, false, false, true>,
+                             gemm_tc_pair_kernel<BN, false, true, true>, run);
+}
+
+// What a kernel was measured to need (us): a launch without its K, what a 64-wide slice of K takes where a tile is alone on
+// the chip, and where all SMs stream operands.  The pair kernel moves the fewest operand bytes per product and wins
+// wherever it has enough tiles: measured at K = 640 for 1056 | 2528 | 8256 | 32 896 rows of N = 1920, pair | 128 | 64
+// columns: 9.3 | 12.6 | 21.3 | 68.8, 6.3 | 11.4 | 24.1 | 82.5, 7.1 | 11.7 | 29.0 us.
+struct Variant {
+    int rows, cols;
+    float launch, alone, full;
+};
+constexpr Variant kVariants[] = {{2 * GM, 256, 6.1f, 0.28f, 0.46f}, {GM, 256, 5.0f, 0.305f, 0.54f}, {GM, 128, 4.2f, 0.167f, 0.306f},
+                                 {GM, 64, 3.7f, 0.128f, 0.186f},    {GM, 32, 3.5f, 0.117f, 0.135f}};
+
+float variant_cost(int i, const GemmCall& g, int splits) {
+    const Variant& v = kVariants[i];
+    const float slices = (float)((g.k + GK - 1) / GK) / (float)splits;
+    // (the pair kernel's last tile of a row multiplies only the columns that exist)
+    const float cols = i == 0 ? (float)((g.n + 31) / 32) / 8.f : (float)((g.n + v.cols - 1) / v.cols);
+    const float load = (float)((g.m + v.rows - 1) / v.rows) * cols * (float)splits / (float)(i == 0 ? sm_count() / 2 : sm_count());
+    return v.launch + slices * (load <= 1.f ? v.alone + (v.full - v.alone) * load : v.full * ceilf(load));
+}
+
+int launch_variant(int i, const GemmCall& g, cudaStream_t stream) {
+    switch (i) {
+        case 0: return launch_gemm_pair<256>(g, stream);
+        case 1: return launch_gemm<256>(g, stream);
+        case 2: return launch_gemm<128>(g, stream);
+        case 3: return launch_gemm<64>(g, stream);
+        default: return launch_gemm<32>(g, stream);
+    }
 }
 
 }  // namespace
 
-// Which kernel: the one whose waves of tiles take the least time, with what each was measured to need (us): a launch
-// without its K, what a 64-wide slice of K takes where a tile is alone on the chip, and where all SMs stream operands.  A
-// long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 6.5 us against 8.2).  The pair kernel moves the fewest operand bytes per product and wins wherever it has enough
-// tiles: measured at K = 640 for 1056 | 2528 | 8256 | 32 896 rows of N = 1920, pair | 128 | 64 columns: 9.3 | 12.6 | 21.3 |
-// 68.8, 6.3 | 11.4 | 24.1 | 82.5, 7.1 | 11.7 | 29.0 us.
-int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream,
-                  int chain) {
-    struct Variant { int rows, cols, units; float launch, alone, full; };
-    const int sms = sm_count();
-    const Variant variants[] = {{2 * GM, 256, sms / 2, 6.1f, 0.28f, 0.46f}, {GM, 256, sms, 5.0f, 0.305f, 0.54f},
-                                {GM, 128, sms, 4.2f, 0.167f, 0.306f},       {GM, 64, sms, 3.7f, 0.128f, 0.186f},
-                                {GM, 32, sms, 3.5f, 0.117f, 0.135f}};
-    const float slices = (float)((d.k + GK - 1) / GK);
-    if (slices >= 16.f && 2 * ((d.m + GM - 1) / GM) * ((d.n + 31) / 32) <= sms && d.lda == d.k && d.ldw == d.k && d.ldc == d.n)
-        return launch_rows_tc(d.dtype, d.m, d.n, d.k, a, w, bias, c, d.epilogue, stream, chain & kChainDependent);
-    int best = 0;
+int launch_gemm_call(const GemmCall& call, cudaStream_t stream) {
+    GemmCall g = call;
+    g.splits = 1;
+    // a long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 6.5 us against 8.2)
+    if (!g.a_mn && !g.b_mn && g.epilogue <= GEMM_ADD && g.k >= 16 * GK && 2 * ((g.m + GM - 1) / GM) * ((g.n + 31) / 32) <= sm_count() &&
+        g.lda == g.k && g.ldb == g.k && g.ldc == g.n && (g.epilogue != GEMM_ADD || g.aux == g.c))
+        return launch_rows_tc(g.dtype, g.m, g.n, g.k, g.a, g.b, g.bias, g.c, g.epilogue, stream, g.chain & kChainDependent);
+    int best = -1;
     float least = 0.f;
     for (int i = 0; i < 5; ++i) {
-        const Variant& v = variants[i];
-        // (the pair kernel's last tile of a row multiplies only the columns that exist)
-        const float cols = i == 0 ? (float)((d.n + 31) / 32) / 8.f : (float)((d.n + v.cols - 1) / v.cols);
-        const float load = (float)((d.m + v.rows - 1) / v.rows) * cols / (float)v.units;
-        const float t = v.launch + slices * (load <= 1.f ? v.alone + (v.full - v.alone) * load : v.full * ceilf(load));
-        if (i == 0 || t < least) {
+        if ((g.a_mn || g.b_mn) && (i == 1 || i == 4)) continue;  // built for the layouts of a backward pass: 256 x 256, 128, 64
+        const float t = variant_cost(i, g, 1);
+        if (best < 0 || t < least) {
             best = i;
             least = t;
         }
     }
-    switch (best) {
-        case 0: return launch_gemm_pair<256>(d, a, w, bias, c, stream, chain);
-        case 1: return launch_gemm<256>(d, a, w, bias, c, stream, chain);
-        case 2: return launch_gemm<128>(d, a, w, bias, c, stream, chain);
-        case 3: return launch_gemm<64>(d, a, w, bias, c, stream, chain);
-        default: return launch_gemm<32>(d, a, w, bias, c, stream, chain);
+    return launch_variant(best, g, stream);
+}
+
+// A product with a long k and a small output (a weight gradient: k = rows of the batch): k is cut into as many ranges as
+// pays, each leaving fp32 sums in `partial`, and *splits says how many (1: the output itself was written).  Every range
+// costs a trip of m x n fp32 values through memory and back, at about 4 TB/s, and a launch.
+int launch_gemm_splitk(const GemmCall& call, size_t partial_bytes, int* splits, cudaStream_t stream) {
+    GemmCall g = call;
+    const size_t out = (size_t)g.m * g.n * sizeof(float);
+    int best = 0, best_s = 1;
+    float least = 0.f;
+    for (int i = 0; i < 4; ++i) {
+        if (i == 1) continue;
+        for (int s = 1; s <= 32 && (s == 1 || (s * out <= partial_bytes && g.k >= s * 4 * GK)); ++s) {
+            const float t = variant_cost(i, g, s) + (s > 1 ? 2.5f + 2.f * (float)(s * out) / 4e6f : 0.f);
+            if ((i == 0 && s == 1) || t < least) {
+                best = i;
+                best_s = s;
+                least = t;
+            }
+        }
     }
+    *splits = g.splits = best_s;
+    return launch_variant(best, g, stream);
+}
+
+int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream,
+                  int chain) {
+    GemmCall g;
+    g.dtype = d.dtype; g.m = d.m; g.n = d.n; g.k = d.k;
+    g.a = a; g.lda = d.lda; g.b = w; g.ldb = d.ldw; g.c = c; g.ldc = d.ldc;
+    g.bias = bias; g.epilogue = d.epilogue; g.chain = chain;
+    return launch_gemm_call(g, stream);
 }
 
 }  // namespace tmw

@@ -104,6 +104,19 @@ __device__ __forceinline__ float gelu_erf(float x) {
     return 0.5f * x * (1.0f + copysignf(erf_abs, x));
 }
 
+// derivative of gelu_erf: Phi(x) + x phi(x)
+__device__ __forceinline__ float gelu_slope(float x) {
+    const float z = fabsf(x) * 0.70710678118654752f;
+    const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
+    float poly = fmaf(1.061405429f, t, -1.453152027f);
+    poly = fmaf(poly, t, 1.421413741f);
+    poly = fmaf(poly, t, -0.284496736f);
+    poly = fmaf(poly, t, 0.254829592f);
+    const float e = __expf(-z * z);  // exp(-x^2 / 2)
+    const float erf_abs = 1.0f - poly * t * e;
+    return 0.5f * (1.0f + copysignf(erf_abs, x)) + 0.3989422804014327f * x * e;
+}
+
 __host__ __device__ inline size_t dtype_size(int dtype) { return dtype == TMW_F32 ? 4 : 2; }
 
 // Eight consecutive elements as raw bits: half the registers of their fp32 values for 16-bit types.
@@ -227,6 +240,11 @@ bool prefill_backward_tc_supports(const tmw_prefill_desc& d);
 int launch_prefill_backward_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o,
                                const void* d_o, const float* lse, void* dq, void* dk, void* dv, cudaStream_t stream,
                                int window_block = 0);
+int launch_dwconv_backward(int dtype, int batch, int rows, int channels, int taps, const void* x, const void* const* w, int n_w,
+                           const void* dy, void* dx, float* dw, cudaStream_t stream);
+// x = embedded rows (persistent rows first), y = RMSNorm(x): see stack_forward.cu
+int launch_embed_seq(const tmw_stack_desc& d, const int64_t* token_ids, int tokens, const void* gain, void* x, void* y,
+                     cudaStream_t stream);
 bool prefill_tc_supports(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o);
 int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, const void* v_new, void* o,
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,
@@ -237,6 +255,27 @@ inline size_t decode_partials_bytes(int batch, int heads, int head_dim, int spli
     const size_t n = (size_t)batch * heads * splits * ((size_t)head_dim + 2) * sizeof(float);
     return (n + 15) & ~(size_t)15;
 }
+// c[m, n] = epilogue(sum_k a(m, k) b(n, k)): a is [m, k] row-major, or [k, m] with a_mn; b is [n, k], or [k, n] with b_mn
+// (a_mn needs b_mn)
+enum GemmEpilogue {
+    GEMM_NONE = 0,
+    GEMM_GELU = 1,       // gelu(v)
+    GEMM_ADD = 2,        // aux + round(v)
+    GEMM_GELU_KEEP = 3,  // aux = round(v), c = gelu(aux)
+    GEMM_GELU_GRAD = 4   // v * gelu'(aux)
+};
+struct GemmCall {
+    int dtype = 0, m = 0, n = 0, k = 0;
+    const void *a = nullptr, *b = nullptr, *bias = nullptr;
+    void *c = nullptr, *aux = nullptr;  // aux: [m, n] contiguous
+    long long lda = 0, ldb = 0, ldc = 0;
+    bool a_mn = false, b_mn = false;
+    int epilogue = GEMM_NONE, chain = 0;
+    int splits = 1;
+    float* partial = nullptr;
+};
+int launch_gemm_call(const GemmCall& g, cudaStream_t stream);
+int launch_gemm_splitk(const GemmCall& g, size_t partial_bytes, int* splits, cudaStream_t stream);
 int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c,
                   cudaStream_t stream, int chain = 0);
 int launch_add_rmsnorm(int dtype, long long rows, int dim, const void* x, const void* residual, const void* scale, float eps,

@@ -116,6 +116,15 @@ class AttentionDesc(ctypes.Structure):
                                               "block_size", "conv_taps")] + [("scale", ctypes.c_float)]
 
 
+class BlockGrads(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("norm_attn", "w_qkv", "w_out", "norm_mlp", "w_fc1", "b_fc1", "w_fc2", "b_fc2",
+                                               "conv_q", "conv_k", "conv_v")]
+
+
+class StackGrads(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("embed_tokens", "head", "embed_positions", "persistent", "norm")]
+
+
 EPILOGUE_NONE, EPILOGUE_GELU = 0, 1
 HALO_MAX_COPIES = 8
 
@@ -215,6 +224,30 @@ SIGNATURES = {
         [ctypes.POINTER(StackDesc), ctypes.POINTER(Block), ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
          ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p],
     ),
+    "tmw_attention_train_saved": (ctypes.c_size_t, [ctypes.POINTER(AttentionDesc)]),
+    "tmw_attention_train_scratch": (ctypes.c_size_t, [ctypes.POINTER(AttentionDesc)]),
+    "tmw_attention_train_forward": (
+        ctypes.c_int,
+        [ctypes.POINTER(AttentionDesc)] + [ctypes.c_void_p] * 8 + [ctypes.c_size_t, ctypes.c_void_p],
+    ),
+    "tmw_attention_train_backward": (
+        ctypes.c_int,
+        [ctypes.POINTER(AttentionDesc)] + [ctypes.c_void_p] * 9 + [ctypes.POINTER(BlockGrads), ctypes.c_void_p, ctypes.c_size_t,
+                                                                   ctypes.c_void_p],
+    ),
+    "tmw_stack_train_saved": (ctypes.c_size_t, [ctypes.POINTER(StackDesc), ctypes.c_int32]),
+    "tmw_stack_train_scratch": (ctypes.c_size_t, [ctypes.POINTER(StackDesc), ctypes.c_int32]),
+    "tmw_stack_train_forward": (
+        ctypes.c_int,
+        [ctypes.POINTER(StackDesc), ctypes.POINTER(Block), ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p,
+         ctypes.c_size_t, ctypes.c_void_p],
+    ),
+    "tmw_stack_train_backward": (
+        ctypes.c_int,
+        [ctypes.POINTER(StackDesc), ctypes.POINTER(Block), ctypes.POINTER(StackGrads), ctypes.POINTER(BlockGrads), ctypes.c_void_p,
+         ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p],
+    ),
+    "tmw_cross_entropy": (ctypes.c_int, [ctypes.c_int32] * 5 + [ctypes.c_void_p] * 7),
     "tmw_decode_step_workspace": (ctypes.c_size_t, [ctypes.POINTER(StackDesc)]),
     "tmw_decode_step": (
         ctypes.c_int,

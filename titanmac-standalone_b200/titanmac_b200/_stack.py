@@ -39,6 +39,7 @@ class ModelTable:
         self._modules: list = []
         self._dropouts: list = []
         self._attentions: list = []
+        self._places: list = []
         self.dtype = model.embed_tokens.weight.dtype
         self.device = model.embed_tokens.weight.device
         if self.dtype not in (torch.bfloat16, torch.float16) or self.device.type != "cuda":
@@ -120,6 +121,11 @@ class ModelTable:
             found += values.values()
             for name, value in values.items():
                 setattr(b, name, value or None)
+            homes = dict(norm_attn=(norms[0], "scale"), norm_mlp=(norms[1], "scale"), w_qkv=(qkv, "weight"), w_out=(out, "weight"),
+                         w_fc1=(fc1, "weight"), w_fc2=(fc2, "weight"), b_fc1=(fc1, "bias"), b_fc2=(fc2, "bias"))
+            for name in ("conv_q", "conv_k", "conv_v") if kind[1] else ():
+                homes[name] = (attn._modules[name], "weight")
+            self._places += [((i, name), (m._parameters, key)) for name, (m, key) in homes.items()]
         d = self.desc = _native.StackDesc()
         top = (address(tops[0], "weight", (V, D)), address(tops[1], "weight", (c.max_seq_len, D)), address(tops[2], "scale", (D,)),
                address(tops[3], "weight", (V, D)))
@@ -130,14 +136,30 @@ class ModelTable:
                 or tops[1].max_norm is not None:
             return
         d.embed_tokens, d.embed_positions, d.norm, d.head = top
+        tops_at = dict(embed_tokens=(tops[0], "weight"), embed_positions=(tops[1], "weight"), norm=(tops[2], "scale"),
+                       head=(tops[3], "weight"))
+        if pers:
+            tops_at["persistent"] = (model, "persistent_tokens")
+        self._places += [((-1, name), (m._parameters, key)) for name, (m, key) in tops_at.items()]
         d.persistent = pers or None
         d.block_size, d.conv_taps = self.kind
         d.dtype = _native._DTYPES[self.dtype]
         d.layers, d.d_model, d.heads, d.head_dim, d.d_ff = len(layers), D, c.n_heads, c.d_head, F
         d.window, d.n_persistent, d.vocab, d.max_positions, d.eps = c.window_size, c.n_persistent, V, c.max_seq_len, c.norm_eps
+        # unique parameters as (dictionary, name), and each one's places in the structures: (layer or -1, field)
+        self.slots, self.roles, at = [], [], {}
+        for place, (d_, name) in self._places:
+            prm = d_.get(name)
+            if prm is not None:
+                if id(prm) not in at:
+                    at[id(prm)] = len(self.slots)
+                    self.slots.append((d_, name))
+                    self.roles.append([])
+                self.roles[at[id(prm)]].append(place)
         self.geometry = (c.n_heads, c.d_head, c.window_size, c.n_persistent, self.dtype)
         self.decodes = c.d_head in (64, 128) and F % 32 == 0 and self.kind == (0, 0)
         self.forwards = V % 8 == 0 and F % 8 == 0 and D % 8 == 0 and c.d_head % 8 == 0 and self.kind[1] <= 8
+        self.trains = self.forwards and D <= 2048
         self.workspace_bytes: dict = {}  # (batch, tokens) -> bytes; tokens = -1: a decode step
         self.ok = True
 
@@ -257,8 +279,9 @@ def _plain_weight(mod: nn.Module, kind, dtype: torch.dtype) -> Optional[torch.Te
     return w if p["bias"] is None and w.dtype is dtype and w.is_contiguous() else None
 
 
-def attention_forward(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float) -> Optional[torch.Tensor]:
-    """An attention module's forward as one ``tmw_attention_forward``; None where that call does not apply."""
+def attention_plan(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float):
+    """``(AttentionDesc, w_qkv, w_out, convolution weights)`` if the module's forward on ``x`` is nothing but what the library
+    computes in one call, else None."""
     dtype = x.dtype
     if (dtype is not torch.bfloat16 and dtype is not torch.float16) or attn.algo or attn.core_events is not None \
             or not x.is_contiguous():
@@ -268,25 +291,32 @@ def attention_forward(attn: nn.Module, x: torch.Tensor, n_persistent: int, block
     w_qkv, w_out = _plain_weight(mods["qkv_proj"], nn.Linear, dtype), _plain_weight(mods["out_proj"], nn.Linear, dtype)
     if w_qkv is None or w_out is None or B * L == 0 or D % 8 or attn.d_head % 8 or _global_hooks():
         return None
-    conv, taps = (None, None, None), 0
+    conv, taps = (), 0
     if block_size and attn.use_conv:
-        ws = [_plain_weight(mods[n], nn.Conv1d, dtype) for n in ("conv_q", "conv_k", "conv_v")]
-        taps = ws[0].shape[2] if ws[0] is not None else 0
-        if not 1 <= taps <= 8 or any(w is None or w.shape != (D, 1, taps) for w in ws):
+        conv = tuple(_plain_weight(mods[n], nn.Conv1d, dtype) for n in ("conv_q", "conv_k", "conv_v"))
+        taps = conv[0].shape[2] if conv[0] is not None else 0
+        if not 1 <= taps <= 8 or any(w is None or w.shape != (D, 1, taps) for w in conv):
             return None
-        conv = tuple(w.data_ptr() for w in ws)
-    d = _native.AttentionDesc(_native._DTYPES[dtype], B, L, attn.n_heads, attn.d_head, attn.window_size, n_persistent, block_size,
-                              taps, scale)
+    if (x.data_ptr() | w_qkv.data_ptr() | w_out.data_ptr()) % 16 or w_qkv.device != x.device:
+        return None
+    return _native.AttentionDesc(_native._DTYPES[dtype], B, L, attn.n_heads, attn.d_head, attn.window_size, n_persistent, block_size,
+                                 taps, scale), w_qkv, w_out, conv
+
+
+def attention_forward(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float) -> Optional[torch.Tensor]:
+    """An attention module's forward as one ``tmw_attention_forward``; None where that call does not apply."""
+    plan = attention_plan(attn, x, n_persistent, block_size, scale)
+    if plan is None:
+        return None
+    d, w_qkv, w_out, conv = plan
     lib = _native.lib()
     ref = ctypes.byref(d)
     device = x.device
     nbytes = lib.tmw_attention_workspace(ref)
     y = torch.empty_like(x)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    px, pq, po = x.data_ptr(), w_qkv.data_ptr(), w_out.data_ptr()
-    if (px | pq | po) % 16 or w_qkv.device != device:
-        return None
+    conv_ptrs = tuple(w.data_ptr() for w in conv) if conv else (None, None, None)
     with _native._on(device):
-        _native.check(lib.tmw_attention_forward(ref, px, pq, *conv, po, y.data_ptr(), workspace.data_ptr(), nbytes,
-                                                _native._stream_ptr(device)))
+        _native.check(lib.tmw_attention_forward(ref, x.data_ptr(), w_qkv.data_ptr(), *conv_ptrs, w_out.data_ptr(), y.data_ptr(),
+                                                workspace.data_ptr(), nbytes, _native._stream_ptr(device)))
     return y

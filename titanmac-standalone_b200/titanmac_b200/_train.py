@@ -1,0 +1,179 @@
+"""Training steps in 16-bit types as single autograd nodes over the whole-model and whole-module calls of libtmw.
+
+``TitanMAC`` and the attention modules use them when every part is what the library computes (see ``_stack.ModelTable``);
+anything else - fp32, frozen parameters, hooks, autocast - keeps the graph of the modules themselves.
+"""
+
+from __future__ import annotations
+
+import ctypes
+from typing import Optional
+
+import torch
+from torch.autograd.function import once_differentiable
+
+from . import _native, _stack
+
+
+def _autocast() -> bool:
+    return torch.is_autocast_enabled("cuda")
+
+
+class _StackTrain(torch.autograd.Function):
+    """``ids [B, T]`` → logits of every row ``[B, Np + T, V]``."""
+
+    @staticmethod
+    def forward(ctx, table, ids: torch.Tensor, *params: torch.Tensor) -> torch.Tensor:
+        d = _native.StackDesc.from_buffer_copy(table.desc)
+        B, T = ids.shape
+        d.batch = B
+        lib, ref, device = _native.lib(), ctypes.byref(d), ids.device
+        nbytes = lib.tmw_stack_train_saved(ref, T)
+        saved = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        logits = torch.empty((B, T + d.n_persistent, d.vocab), dtype=table.dtype, device=device)
+        with _native._on(device):
+            _native.check(lib.tmw_stack_train_forward(ref, table.blocks, ids.data_ptr(), T, logits.data_ptr(), saved.data_ptr(),
+                                                      nbytes, _native._stream_ptr(device)))
+        ctx.desc, ctx.roles = d, table.roles
+        ctx.save_for_backward(ids, saved, *params)
+        return logits
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, d_logits: torch.Tensor):
+        ids, saved, *params = ctx.saved_tensors
+        d = _native.StackDesc.from_buffer_copy(ctx.desc)
+        d_logits = d_logits.contiguous()
+        # the parameters' addresses as they are now, and their gradients'
+        blocks, block_grads = (_native.Block * d.layers)(), (_native.BlockGrads * d.layers)()
+        grads, out = _native.StackGrads(), []
+        for prm, roles in zip(params, ctx.roles):
+            grad = torch.empty_like(prm, memory_format=torch.contiguous_format)
+            out.append(grad)
+            p, g = prm.data_ptr(), grad.data_ptr()
+            for layer, name in roles:
+                if layer < 0:
+                    setattr(d, name, p)
+                    setattr(grads, name, g)
+                else:
+                    setattr(blocks[layer], name, p)
+                    setattr(block_grads[layer], name, g)
+        lib, ref, device, T = _native.lib(), ctypes.byref(d), ids.device, ids.shape[1]
+        nbytes = lib.tmw_stack_train_scratch(ref, T)
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        with _native._on(device):
+            _native.check(lib.tmw_stack_train_backward(ref, blocks, ctypes.byref(grads), block_grads, ids.data_ptr(), T,
+                                                       d_logits.data_ptr(), saved.data_ptr(), scratch.data_ptr(), nbytes,
+                                                       _native._stream_ptr(device)))
+        return (None, None, *out)
+
+
+def stack_forward(model, input_ids: torch.Tensor) -> Optional[torch.Tensor]:
+    """Logits of every row with a gradient to every parameter, or None where that takes the modules themselves."""
+    table = _stack.table_of(model)
+    if table is None or not table.trains or _autocast() or input_ids.dtype != torch.int64 or input_ids.dim() != 2 \
+            or input_ids.device != table.device:
+        return None
+    B, T = input_ids.shape
+    if B == 0 or T == 0 or T > table.desc.max_positions or B * (T + table.desc.n_persistent) >= (1 << 31) // 8:
+        return None
+    params = [d[name] for d, name in table.slots]
+    if not all(p.requires_grad for p in params):
+        return None
+    return _StackTrain.apply(table, input_ids.contiguous(), *params)
+
+
+class _ShiftedCrossEntropy(torch.autograd.Function):
+    """Mean cross-entropy of ``logits [B, Np + T, V]``, row ``Np + t`` against ``labels[:, t + 1]`` (-100: not counted)."""
+
+    @staticmethod
+    def forward(ctx, logits: torch.Tensor, labels: torch.Tensor, n_persistent: int) -> torch.Tensor:
+        B, L, V = logits.shape
+        loss = torch.empty((), dtype=logits.dtype, device=logits.device)
+        stats = torch.empty(4 + 2 * B * L, dtype=torch.float32, device=logits.device)
+        with _native._on(logits.device):
+            _native.check(_native.lib().tmw_cross_entropy(_native._DTYPES[logits.dtype], B, L - n_persistent, n_persistent, V,
+                                                          logits.data_ptr(), labels.data_ptr(), loss.data_ptr(), stats.data_ptr(),
+                                                          None, None, _native._stream_ptr(logits.device)))
+        ctx.save_for_backward(logits, labels, stats)
+        ctx.n_persistent = n_persistent
+        return loss
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, grad: torch.Tensor):
+        logits, labels, stats = ctx.saved_tensors
+        B, L, V = logits.shape
+        d_logits = torch.empty_like(logits)
+        grad = grad.contiguous()
+        with _native._on(logits.device):
+            _native.check(_native.lib().tmw_cross_entropy(_native._DTYPES[logits.dtype], B, L - ctx.n_persistent, ctx.n_persistent,
+                                                          V, logits.data_ptr(), labels.data_ptr(), None, stats.data_ptr(),
+                                                          grad.data_ptr(), d_logits.data_ptr(), _native._stream_ptr(logits.device)))
+        return d_logits, None, None
+
+
+def shifted_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, n_persistent: int) -> Optional[torch.Tensor]:
+    """``logits``: every row, persistent rows first.  None where the library's kernel does not apply."""
+    B, L, V = logits.shape
+    if (logits.dtype not in (torch.bfloat16, torch.float16) or not logits.is_cuda or not logits.is_contiguous() or V % 8
+            or logits.data_ptr() % 16 or labels.dtype != torch.int64 or labels.shape != (B, L - n_persistent)
+            or labels.device != logits.device or B == 0 or L == n_persistent or _autocast()):
+        return None
+    return _ShiftedCrossEntropy.apply(logits, labels.contiguous(), n_persistent)
+
+
+class _AttentionTrain(torch.autograd.Function):
+    """An attention module's forward and backward: ``x [B, L, D]``, its projections and (block-sparse) convolutions."""
+
+    @staticmethod
+    def forward(ctx, desc, x: torch.Tensor, w_qkv: torch.Tensor, w_out: torch.Tensor, *conv: torch.Tensor) -> torch.Tensor:
+        lib, ref, device = _native.lib(), ctypes.byref(desc), x.device
+        nbytes = lib.tmw_attention_train_saved(ref)
+        saved = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        y = torch.empty_like(x)
+        with _native._on(device):
+            _native.check(lib.tmw_attention_train_forward(ref, x.data_ptr(), w_qkv.data_ptr(), *_conv_ptrs(conv), w_out.data_ptr(),
+                                                          y.data_ptr(), saved.data_ptr(), nbytes, _native._stream_ptr(device)))
+        ctx.desc = desc
+        ctx.save_for_backward(x, saved, w_qkv, w_out, *conv)
+        return y
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dy: torch.Tensor):
+        x, saved, w_qkv, w_out, *conv = ctx.saved_tensors
+        dy = dy.contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        lib, ref, device = _native.lib(), ctypes.byref(ctx.desc), x.device
+        nbytes = lib.tmw_attention_train_scratch(ref)
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        dx = torch.empty_like(x)
+        weights = (w_qkv, w_out, *conv)
+        out = [torch.empty_like(w) for w in weights]
+        grads = _native.BlockGrads()
+        for name, g in zip(("w_qkv", "w_out", "conv_q", "conv_k", "conv_v"), out):
+            setattr(grads, name, g.data_ptr())
+        with _native._on(device):
+            _native.check(lib.tmw_attention_train_backward(ref, x.data_ptr(), w_qkv.data_ptr(), *_conv_ptrs(conv), w_out.data_ptr(),
+                                                           dy.data_ptr(), saved.data_ptr(), dx.data_ptr(), ctypes.byref(grads),
+                                                           scratch.data_ptr(), nbytes, _native._stream_ptr(device)))
+        need = ctx.needs_input_grad
+        return (None, dx if need[1] else None, *(g if n else None for g, n in zip(out, need[2:])))
+
+
+def _conv_ptrs(conv):
+    return tuple(w.data_ptr() for w in conv) if conv else (None, None, None)
+
+
+def attention_forward(attn, x: torch.Tensor, n_persistent: int, block_size: int, scale: float) -> Optional[torch.Tensor]:
+    """The module's forward as one autograd node, or None where that takes its parts."""
+    if _autocast():
+        return None
+    x = x.contiguous()
+    plan = _stack.attention_plan(attn, x, n_persistent, block_size, scale)
+    if plan is None:
+        return None
+    desc, w_qkv, w_out, conv = plan
+    return _AttentionTrain.apply(desc, x, w_qkv, w_out, *conv)

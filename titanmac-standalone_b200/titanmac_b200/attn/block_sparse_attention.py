@@ -26,7 +26,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from .. import _native, _stack
+from .. import _native, _stack, _train
 
 
 class _CausalDwConv(torch.autograd.Function):
@@ -117,6 +117,9 @@ class BlockSparseAttention(nn.Module):
         B, L, D = x.shape
         if self.n_persistent >= L:
             raise ValueError(f"n_persistent ({self.n_persistent}) must be < seq_len ({L})")
+        y = _train.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)
+        if y is not None:
+            return self.dropout(y)
         qkv = self.qkv_proj(x)
         if self.use_conv:
             qkv = _CausalDwConv.apply(qkv, self.stacked_conv_weight())

@@ -28,7 +28,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .. import _native, _stack
+from .. import _native, _stack, _train
 from ..blocks.titan_block import RMSNorm, TitanBlock
 
 
@@ -74,20 +74,25 @@ class TitanMAC(nn.Module):
     def forward(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None,
                 attention_mask: Optional[torch.Tensor] = None) -> Dict[str, torch.Tensor]:
         Np = self.config.n_persistent
-        logits = None
-        if not torch.is_grad_enabled() or not any(p.requires_grad for p in self.parameters()):
+        rows = None  # logits of every row, persistent rows first
+        if torch.is_grad_enabled() and any(p.requires_grad for p in self.parameters()):
+            rows = _train.stack_forward(self, input_ids)  # one autograd node
+        else:
             table = _stack.table_of(self)
             if table is not None:  # the whole forward as one call (tmw_stack_forward)
-                logits = _stack.forward(table, input_ids)
-        if logits is None:
-            logits = self._forward_modules(input_ids)
-        logits = logits[:, Np:, :] if Np > 0 else logits
+                rows = _stack.forward(table, input_ids)
+        if rows is None:
+            rows = self._forward_modules(input_ids)
+        logits = rows[:, Np:, :] if Np > 0 else rows
         out = {"logits": logits}
         if labels is not None:
-            shift_logits = logits[..., :-1, :].contiguous()
-            shift_labels = labels[..., 1:].contiguous()
-            out["loss"] = F.cross_entropy(shift_logits.reshape(-1, self.config.vocab_size), shift_labels.reshape(-1),
-                                          reduction="mean", ignore_index=-100)
+            loss = _train.shifted_cross_entropy(rows, labels, Np)
+            if loss is None:
+                shift_logits = logits[..., :-1, :].contiguous()
+                shift_labels = labels[..., 1:].contiguous()
+                loss = F.cross_entropy(shift_logits.reshape(-1, self.config.vocab_size), shift_labels.reshape(-1),
+                                       reduction="mean", ignore_index=-100)
+            out["loss"] = loss
         return out
 
     def _forward_modules(self, input_ids: torch.Tensor) -> torch.Tensor:
