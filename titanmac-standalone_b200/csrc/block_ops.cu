@@ -182,11 +182,20 @@ int launch_gelu(long long n, const void* x, void* y, cudaStream_t stream) {
 // ---- causal depthwise convolution along the rows ---------------------------------------------------------
 // y[b, t, c] = sum_j w[c, j] * x[b, t - (TAPS-1) + j, c]: the Conv1d(groups = channels, padding = TAPS-1),
 // trimmed to the input length, that the reference's block-sparse attention applies to Q, K and V
-// (titans_core/attn/block_sparse_attention.py:77-92, 241-256).  One thread owns 8 adjacent channels and
-// walks down a strip of rows with the last TAPS rows in registers: x is read once (plus TAPS-1 rows per
-// strip), y written once.
-constexpr int kConvStrip = 64;
-constexpr int kConvThreads = 128;
+// (titans_core/attn/block_sparse_attention.py:77-92, 241-256).  Bound by HBM (or L2) where the tensors are large and by the
+// length of a thread's chain of loads where they are not: a warp owns 32 x 8 adjacent channels and a strip of rows, four
+// rows requested at a time (one thread walking 64 rows one by one took 18.8 us for 8241 x 1920 values of 16 bits and 14.9 us
+// for 2112 x 768).  The taps - 1 rows in front of a warp's own come out of L1 or L2.
+constexpr int kConvWarps = 8;   // warps per CTA, one below the other
+constexpr int kConvThreads = 32 * kConvWarps;
+constexpr int kConvBatch = 4;   // rows in flight per thread
+constexpr int kConvMinRows = 8, kConvMaxRows = 16;  // rows per warp
+
+// eight rows per warp, or sixteen where that still leaves every SM two CTAs (fewer filter loads and rows read twice)
+int conv_rows_per_warp(int batch, int rows, int channels) {
+    const long long ctas = (long long)batch * ((channels + 255) / 256) * ((rows + kConvWarps * kConvMaxRows - 1) / (kConvWarps * kConvMaxRows));
+    return ctas >= 2 * sm_count() ? kConvMaxRows : kConvMinRows;
+}
 
 // The filters [channels, taps] in up to three arrays of `per` channels each (Q, K and V keep theirs apart).
 struct ConvWeights {
@@ -194,22 +203,34 @@ struct ConvWeights {
     int per;
 };
 
+// the filters of 8 adjacent channels: 8 * TAPS adjacent values
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(kConvThreads)
-dwconv_kernel(const T* __restrict__ x, const ConvWeights f, T* __restrict__ y, int rows, int channels) {
-    const int vec = blockIdx.x * kConvThreads + threadIdx.x;  // which group of 8 channels
-    if (vec * 8 >= channels) return;
-    const int t0 = blockIdx.y * kConvStrip;
-    const int t1 = min(rows, t0 + kConvStrip);
-    const long long base = (long long)blockIdx.z * rows * channels + vec * 8;
-    const int part = vec * 8 / f.per, first = vec * 8 - part * f.per;  // (`per` is a multiple of 8)
-    const T* w = static_cast<const T*>(part == 0 ? f.w[0] : part == 1 ? f.w[1] : f.w[2]);
-    float wr[TAPS][8];
+__device__ __forceinline__ void load_filters(const ConvWeights& f, int channel, float (&wr)[TAPS][8]) {
+    const int part = channel / f.per, first = channel - part * f.per;  // (`per` is a multiple of 8)
+    const T* w = static_cast<const T*>(part == 0 ? f.w[0] : part == 1 ? f.w[1] : f.w[2]) + (long long)first * TAPS;
+    float v[TAPS][8];
+    if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < TAPS; ++i) load8<T>(w + i * 8, v[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < TAPS * 8; ++i) v[i / 8][i % 8] = to_f32<T>(w[i]);
+    }
 #pragma unroll
     for (int c = 0; c < 8; ++c)
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) wr[j][c] = to_f32<T>(w[(long long)(first + c) * TAPS + j]);
-    float hist[TAPS][8];  // hist[j] = x[t - (TAPS-1) + j]
+        for (int j = 0; j < TAPS; ++j) wr[j][c] = v[(c * TAPS + j) / 8][(c * TAPS + j) % 8];
+}
+
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(kConvThreads)
+dwconv_kernel(const T* __restrict__ x, const ConvWeights f, T* __restrict__ y, int rows, int channels, int per_warp) {
+    const int vec = blockIdx.x * 32 + (threadIdx.x & 31);  // which group of 8 channels
+    const int t0 = (blockIdx.y * kConvWarps + (threadIdx.x >> 5)) * per_warp, t1 = min(rows, t0 + per_warp);
+    if (vec * 8 >= channels || t0 >= rows) return;
+    const long long base = (long long)blockIdx.z * rows * channels + vec * 8;
+    float wr[TAPS][8], hist[TAPS][8];  // hist[j] = x[t - (TAPS-1) + j]
+    load_filters<T, TAPS>(f, vec * 8, wr);
 #pragma unroll
     for (int j = 0; j < TAPS - 1; ++j) {
         const int t = t0 - (TAPS - 1) + j;
@@ -220,121 +241,143 @@ dwconv_kernel(const T* __restrict__ x, const ConvWeights f, T* __restrict__ y, i
             for (int c = 0; c < 8; ++c) hist[j + 1][c] = 0.f;
         }
     }
-    for (int t = t0; t < t1; ++t) {
+    for (int tb = t0; tb < t1; tb += kConvBatch) {
+        Vec8<T> raw[kConvBatch];
 #pragma unroll
-        for (int j = 0; j < TAPS - 1; ++j)
+        for (int u = 0; u < kConvBatch; ++u)
+            if (tb + u < t1) raw[u].load(x + base + (long long)(tb + u) * channels);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) hist[j][c] = hist[j + 1][c];
-        load8<T>(x + base + (long long)t * channels, hist[TAPS - 1]);
-        float out[8];
+        for (int u = 0; u < kConvBatch; ++u)
+            if (tb + u < t1) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            float a = 0.f;
+                for (int j = 0; j < TAPS - 1; ++j)
 #pragma unroll
-            for (int j = 0; j < TAPS; ++j) a = fmaf(wr[j][c], hist[j][c], a);
-            out[c] = a;
-        }
-        store8<T>(y + base + (long long)t * channels, out);
+                    for (int c = 0; c < 8; ++c) hist[j][c] = hist[j + 1][c];
+                raw[u].unpack(hist[TAPS - 1]);
+                float out[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    float a = 0.f;
+#pragma unroll
+                    for (int j = 0; j < TAPS; ++j) a = fmaf(wr[j][c], hist[j][c], a);
+                    out[c] = a;
+                }
+                store8<T>(y + base + (long long)(tb + u) * channels, out);
+            }
     }
 }
 
 template <typename T, int TAPS>
 int launch_dwconv_taps(int batch, int rows, int channels, const void* x, const ConvWeights& w, void* y, cudaStream_t stream) {
-    const dim3 grid((channels / 8 + kConvThreads - 1) / kConvThreads, (rows + kConvStrip - 1) / kConvStrip, batch);
-    dwconv_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), w, static_cast<T*>(y), rows, channels);
+    const int per_warp = conv_rows_per_warp(batch, rows, channels), strip = kConvWarps * per_warp;
+    const dim3 grid((channels / 8 + 31) / 32, (rows + strip - 1) / strip, batch);
+    dwconv_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), w, static_cast<T*>(y), rows, channels,
+                                                              per_warp);
     TMW_CUDA_TRY(cudaGetLastError());
     return TMW_OK;
 }
 
-// Backward of the convolution.  dx[t] = sum_j w[j] dy[t + (TAPS-1) - j] looks ahead, so a thread walks its strip
-// of rows from the bottom up with the TAPS rows dy[t .. t+TAPS-1] in registers.  dw[c][j] = sum over batch and rows
-// of dy[t][c] x[t - (TAPS-1) + j][c]: a thread accumulates its strip's share and adds it to an fp32 buffer
-// [channels, TAPS] (zero on entry) with atomics.
+// Backward of the convolution in one pass over x and dy: dx[t] = sum_j w[j] dy[t + (TAPS-1) - j] from the TAPS rows of dy at
+// and behind t, dw[c][j] = sum over batch and rows of dy[t][c] x[t - (TAPS-1) + j][c] from the TAPS rows of x up to t.  The
+// filter's gradient is added up over the CTA's warps in shared memory and from there, with atomics, into an fp32 buffer
+// [channels, TAPS] (zero on entry).  (2112 x 768 values: 34.3 us as two passes over strips of 64 rows, 11.3 us.)
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(kConvThreads)
 dwconv_bwd_kernel(const T* __restrict__ x, const ConvWeights f, const T* __restrict__ dy, T* __restrict__ dx,
-                  float* __restrict__ dw, int rows, int channels) {
-    const int vec = blockIdx.x * kConvThreads + threadIdx.x;
-    if (vec * 8 >= channels) return;
-    const int t0 = blockIdx.y * kConvStrip;
-    const int t1 = min(rows, t0 + kConvStrip);
+                  float* __restrict__ dw, int rows, int channels, int per_warp) {
+    __shared__ float sums[256 * TAPS];  // [tap][channel of the CTA]
+    constexpr int kBatch = TAPS <= 4 ? kConvBatch : 1;  // (registers)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int vec = blockIdx.x * 32 + lane;
+    const int t0 = (blockIdx.y * kConvWarps + warp) * per_warp, t1 = min(rows, t0 + per_warp);
+    const bool live = vec * 8 < channels && t0 < rows;
     const long long base = (long long)blockIdx.z * rows * channels + vec * 8;
-    const int part = vec * 8 / f.per, first = vec * 8 - part * f.per;
-    const T* w = static_cast<const T*>(part == 0 ? f.w[0] : part == 1 ? f.w[1] : f.w[2]);
-    float wr[TAPS][8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) wr[j][c] = to_f32<T>(w[(long long)(first + c) * TAPS + j]);
-    // ---- dx: bottom-up, ahead[m] = dy[t + m]
-    float ahead[TAPS][8];
-#pragma unroll
-    for (int m = 0; m < TAPS - 1; ++m) {  // the state "before" row t1 - 1: dy[t1 + m]
-        if (t1 + m < rows) {
-            load8<T>(dy + base + (long long)(t1 + m) * channels, ahead[m]);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) ahead[m][c] = 0.f;
-        }
-    }
-    for (int t = t1 - 1; t >= t0; --t) {
-#pragma unroll
-        for (int m = TAPS - 1; m >= 1; --m)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) ahead[m][c] = ahead[m - 1][c];
-        load8<T>(dy + base + (long long)t * channels, ahead[0]);
-        float out[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            float a = 0.f;
-#pragma unroll
-            for (int j = 0; j < TAPS; ++j) a = fmaf(wr[j][c], ahead[TAPS - 1 - j][c], a);
-            out[c] = a;
-        }
-        store8<T>(dx + base + (long long)t * channels, out);
-    }
-    // ---- dw: top-down like the forward, hist[j] = x[t - (TAPS-1) + j]
-    float hist[TAPS][8], acc[TAPS][8];
+    float acc[TAPS][8];
 #pragma unroll
     for (int j = 0; j < TAPS; ++j)
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[j][c] = 0.f;
+    if (live) {
+        float wr[TAPS][8], hist[TAPS][8], ahead[TAPS][8];  // hist[j] = x[t - (TAPS-1) + j], ahead[m] = dy[t + m]
+        load_filters<T, TAPS>(f, vec * 8, wr);
+        auto row_or_zero = [&](const T* src, int t, float (&out)[8]) {
+            if (t >= 0 && t < rows) {
+                load8<T>(src + base + (long long)t * channels, out);
+            } else {
 #pragma unroll
-    for (int j = 0; j < TAPS - 1; ++j) {
-        const int t = t0 - (TAPS - 1) + j;
-        if (t >= 0) {
-            load8<T>(x + base + (long long)t * channels, hist[j + 1]);
-        } else {
+                for (int c = 0; c < 8; ++c) out[c] = 0.f;
+            }
+        };
 #pragma unroll
-            for (int c = 0; c < 8; ++c) hist[j + 1][c] = 0.f;
+        for (int j = 0; j < TAPS - 1; ++j) {
+            row_or_zero(x, t0 - (TAPS - 1) + j, hist[j + 1]);
+            row_or_zero(dy, t0 + j, ahead[j + 1]);
+        }
+        for (int tb = t0; tb < t1; tb += kBatch) {
+            Vec8<T> xr[kBatch], dr[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                if (tb + u < t1) xr[u].load(x + base + (long long)(tb + u) * channels);
+                if (tb + u + TAPS - 1 < rows) dr[u].load(dy + base + (long long)(tb + u + TAPS - 1) * channels);
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (tb + u < t1) {
+#pragma unroll
+                    for (int j = 0; j < TAPS - 1; ++j)
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            hist[j][c] = hist[j + 1][c];
+                            ahead[j][c] = ahead[j + 1][c];
+                        }
+                    xr[u].unpack(hist[TAPS - 1]);
+                    if (tb + u + TAPS - 1 < rows) {
+                        dr[u].unpack(ahead[TAPS - 1]);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) ahead[TAPS - 1][c] = 0.f;
+                    }
+                    float out[8];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        float a = 0.f;
+#pragma unroll
+                        for (int j = 0; j < TAPS; ++j) {
+                            a = fmaf(wr[j][c], ahead[TAPS - 1 - j][c], a);
+                            acc[j][c] = fmaf(ahead[0][c], hist[j][c], acc[j][c]);
+                        }
+                        out[c] = a;
+                    }
+                    store8<T>(dx + base + (long long)(tb + u) * channels, out);
+                }
         }
     }
-    for (int t = t0; t < t1; ++t) {
+    for (int w = 0; w < kConvWarps; ++w) {
+        if (warp == w) {
 #pragma unroll
-        for (int j = 0; j < TAPS - 1; ++j)
+            for (int j = 0; j < TAPS; ++j)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) hist[j][c] = hist[j + 1][c];
-        load8<T>(x + base + (long long)t * channels, hist[TAPS - 1]);
-        float g[8];
-        load8<T>(dy + base + (long long)t * channels, g);
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) acc[j][c] = fmaf(g[c], hist[j][c], acc[j][c]);
+                for (int c = 0; c < 8; ++c) {
+                    float* p = sums + j * 256 + c * 32 + lane;
+                    *p = w ? *p + acc[j][c] : acc[j][c];
+                }
+        }
+        __syncthreads();
     }
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) atomicAdd(dw + (long long)(vec * 8 + c) * TAPS + j, acc[j][c]);
+    for (int i = threadIdx.x; i < 256 * TAPS; i += kConvThreads) {
+        const int j = i / 256, c = i % 256 / 32, channel = (blockIdx.x * 32 + i % 32) * 8 + c;
+        if (channel < channels) atomicAdd(dw + (long long)channel * TAPS + j, sums[i]);
+    }
 }
 
 template <typename T, int TAPS>
 int launch_dwconv_bwd_taps(int batch, int rows, int channels, const void* x, const ConvWeights& w, const void* dy, void* dx,
                            float* dw, cudaStream_t stream) {
-    const dim3 grid((channels / 8 + kConvThreads - 1) / kConvThreads, (rows + kConvStrip - 1) / kConvStrip, batch);
+    const int per_warp = conv_rows_per_warp(batch, rows, channels), strip = kConvWarps * per_warp;
+    const dim3 grid((channels / 8 + 31) / 32, (rows + strip - 1) / strip, batch);
     dwconv_bwd_kernel<T, TAPS><<<grid, kConvThreads, 0, stream>>>(static_cast<const T*>(x), w,
                                                                   static_cast<const T*>(dy), static_cast<T*>(dx), dw,
-                                                                  rows, channels);
+                                                                  rows, channels, per_warp);
     TMW_CUDA_TRY(cudaGetLastError());
     return TMW_OK;
 }
@@ -423,7 +466,7 @@ extern "C" int tmw_causal_dwconv(int32_t dtype, int32_t batch, int32_t rows, int
         set_error_text("tmw_causal_dwconv: x and y must be 16-byte aligned");
         return TMW_ERR_INVALID_ARGUMENT;
     }
-    if (batch > 65535 || (rows + kConvStrip - 1) / kConvStrip > 65535) return TMW_ERR_TOO_LARGE;
+    if (batch > 65535 || (rows + kConvWarps * kConvMinRows - 1) / (kConvWarps * kConvMinRows) > 65535) return TMW_ERR_TOO_LARGE;
     return launch_dwconv(dtype, batch, rows, channels, taps, x, &weight, 1, y, static_cast<cudaStream_t>(stream));
 }
 
@@ -438,7 +481,7 @@ extern "C" int tmw_causal_dwconv_backward(int32_t dtype, int32_t batch, int32_t 
     if (x == nullptr || weight == nullptr || dy == nullptr || dx == nullptr || dw == nullptr || dx == dy)
         return TMW_ERR_INVALID_ARGUMENT;
     if ((((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) != 0) return TMW_ERR_INVALID_ARGUMENT;
-    if (batch > 65535 || (rows + kConvStrip - 1) / kConvStrip > 65535) return TMW_ERR_TOO_LARGE;
+    if (batch > 65535 || (rows + kConvWarps * kConvMinRows - 1) / (kConvWarps * kConvMinRows) > 65535) return TMW_ERR_TOO_LARGE;
     return launch_dwconv_backward(dtype, batch, rows, channels, taps, x, &weight, 1, dy, dx, dw, static_cast<cudaStream_t>(stream));
 }
 
