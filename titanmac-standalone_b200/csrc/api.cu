@@ -171,6 +171,64 @@ int validate_decode_call(const tmw_cache_desc* cache, const void* q, const void*
     return TMW_OK;
 }
 
+// `chain`: the place of the call's launches in a chain of dependent launches (tensor-core path; see kChainLink)
+int prefill_block_sparse(const tmw_prefill_desc* desc, int block_size, const void* q, const void* k, const void* v, void* o,
+                         float* lse, cudaStream_t s, int chain) {
+    const int rc = validate_prefill(desc, q, k, v, o);
+    if (rc != TMW_OK) return rc;
+    if (block_size <= 0 || block_size > (1 << 20)) {
+        set_error_text("tmw_prefill_block_sparse: block_size must be positive (at most 2^20)");
+        return TMW_ERR_INVALID_ARGUMENT;
+    }
+    if (desc->q_pos0 != 0 || desc->k_pos0 != desc->n_persistent || desc->q_rows != desc->k_rows) {
+        set_error_text("tmw_prefill_block_sparse: whole sequences only (q_pos0 = 0, k_pos0 = n_persistent, q_rows = k_rows)");
+        return TMW_ERR_UNSUPPORTED;
+    }
+    if (desc->batch == 0 || desc->heads == 0 || desc->q_rows == 0) return TMW_OK;
+    tmw_prefill_desc d = *desc;
+    const bool tc_ok = prefill_tc_supports(d, q, k, v, o) && (int64_t)d.q_rows + d.window + block_size < ((int64_t)1 << 29);
+    if (d.algo == TMW_ALGO_TCGEN05 && !tc_ok) return TMW_ERR_UNSUPPORTED;
+    const bool use_tc = d.algo != TMW_ALGO_SIMT && tc_ok;
+    const int np = d.n_persistent;
+    // the log-sum-exp comes in two planes: [batch, heads, L - np] for the sequence rows (first launch), then
+    // [batch, heads, np] for the persistent rows (second launch)
+    float* lse_pers = lse != nullptr ? lse + (size_t)d.batch * d.heads * (d.q_rows - np) : nullptr;
+    if (np == 0)
+        return use_tc ? launch_prefill_tc(d, q, k, v, o, s, block_size, lse, nullptr, chain)
+                      : launch_prefill_simt(d, q, k, v, o, s, block_size, false, lse);
+    // Two independent launches: the sequence rows [np, L) with the block-granular window, and the np persistent query rows,
+    // which see every key.
+    tmw_prefill_desc seq = d, pers = d;
+    const size_t esz = dtype_size(d.dtype);
+    seq.q_rows = d.q_rows - np;
+    seq.q_pos0 = np;
+    const void* q_seq = static_cast<const char*>(q) + (size_t)np * d.q_stride[2] * esz;
+    void* o_seq = static_cast<char*>(o) + (size_t)np * d.o_stride[2] * esz;
+    pers.q_rows = np;
+    if (use_tc) {
+        const int st = launch_pers_rows(pers, q, k, v, o, lse_pers, s, chain & kChainDependent);
+        return st != TMW_OK ? st : launch_prefill_tc(seq, q_seq, k, v, o_seq, s, block_size, lse, nullptr, chain | kChainDependent);
+    }
+    // On CUDA cores the persistent rows occupy only batch x heads CTAs for a long time: they run on a side stream of the
+    // library between two events (a fork / join that stream capture accepts as well).
+    auto launch = [&](const tmw_prefill_desc& dd, const void* qq, void* oo, cudaStream_t st, bool all_keys) {
+        return launch_prefill_simt(dd, qq, k, v, oo, st, block_size, all_keys, all_keys ? lse_pers : lse);
+    };
+    SideStream* side = side_stream_of_current_device();
+    if (side == nullptr) {  // no side stream: one after the other
+        const int st = launch(seq, q_seq, o_seq, s, false);
+        return st != TMW_OK ? st : launch(pers, q, o, s, true);
+    }
+    std::lock_guard<std::mutex> lock(side->mutex);
+    TMW_CUDA_TRY(cudaEventRecord(side->fork, s));
+    TMW_CUDA_TRY(cudaStreamWaitEvent(side->stream, side->fork, 0));
+    int st = launch(pers, q, o, side->stream, true);
+    TMW_CUDA_TRY(cudaEventRecord(side->join, side->stream));
+    const int st2 = launch(seq, q_seq, o_seq, s, false);
+    TMW_CUDA_TRY(cudaStreamWaitEvent(s, side->join, 0));
+    return st != TMW_OK ? st : st2;
+}
+
 }  // namespace tmw
 
 extern "C" {
@@ -221,7 +279,7 @@ int tmw_prefill_halo(const tmw_prefill_desc* desc, const void* q, const void* k,
         tmw::set_error_text("tmw_prefill_halo: only the tensor-core kernel polls the flags (bf16 / f16, head_dim 64 or 128)");
         return TMW_ERR_UNSUPPORTED;
     }
-    return tmw::launch_prefill_tc(*desc, q, k, v, o, static_cast<cudaStream_t>(stream), 0, false, nullptr, wait);
+    return tmw::launch_prefill_tc(*desc, q, k, v, o, static_cast<cudaStream_t>(stream), 0, nullptr, wait);
 }
 
 int tmw_prefill_lse(const tmw_prefill_desc* desc, const void* q, const void* k, const void* v, void* o, float* lse,
@@ -233,7 +291,7 @@ int tmw_prefill_lse(const tmw_prefill_desc* desc, const void* q, const void* k, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool tc_ok = tmw::prefill_tc_supports(*desc, q, k, v, o);
     if (desc->algo == TMW_ALGO_TCGEN05 && !tc_ok) return TMW_ERR_UNSUPPORTED;
-    if (desc->algo != TMW_ALGO_SIMT && tc_ok) return tmw::launch_prefill_tc(*desc, q, k, v, o, s, 0, false, lse);
+    if (desc->algo != TMW_ALGO_SIMT && tc_ok) return tmw::launch_prefill_tc(*desc, q, k, v, o, s, 0, lse);
     return tmw::launch_prefill_simt(*desc, q, k, v, o, s, 0, false, lse);
 }
 
@@ -292,57 +350,7 @@ int tmw_prefill_block_sparse_backward(const tmw_prefill_desc* desc, int32_t bloc
 
 int tmw_prefill_block_sparse_lse(const tmw_prefill_desc* desc, int32_t block_size, const void* q, const void* k,
                                  const void* v, void* o, float* lse, void* stream) {
-    const int rc = tmw::validate_prefill(desc, q, k, v, o);
-    if (rc != TMW_OK) return rc;
-    if (block_size <= 0 || block_size > (1 << 20)) {
-        tmw::set_error_text("tmw_prefill_block_sparse: block_size must be positive (at most 2^20)");
-        return TMW_ERR_INVALID_ARGUMENT;
-    }
-    if (desc->q_pos0 != 0 || desc->k_pos0 != desc->n_persistent || desc->q_rows != desc->k_rows) {
-        tmw::set_error_text("tmw_prefill_block_sparse: whole sequences only (q_pos0 = 0, k_pos0 = n_persistent, q_rows = k_rows)");
-        return TMW_ERR_UNSUPPORTED;
-    }
-    if (desc->batch == 0 || desc->heads == 0 || desc->q_rows == 0) return TMW_OK;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    tmw_prefill_desc d = *desc;
-    const bool tc_ok = tmw::prefill_tc_supports(d, q, k, v, o) && (int64_t)d.q_rows + d.window + block_size < ((int64_t)1 << 29);
-    if (d.algo == TMW_ALGO_TCGEN05 && !tc_ok) return TMW_ERR_UNSUPPORTED;
-    const bool use_tc = d.algo != TMW_ALGO_SIMT && tc_ok;
-    const int np = d.n_persistent;
-    // the log-sum-exp comes in two planes: [batch, heads, L - np] for the sequence rows (first launch), then
-    // [batch, heads, np] for the persistent rows (second launch)
-    float* lse_pers = lse != nullptr ? lse + (size_t)d.batch * d.heads * (d.q_rows - np) : nullptr;
-    auto launch = [&](const tmw_prefill_desc& dd, const void* qq, void* oo, cudaStream_t st, bool all_keys) {
-        float* l = all_keys ? lse_pers : lse;
-        return use_tc ? tmw::launch_prefill_tc(dd, qq, k, v, oo, st, block_size, all_keys, l)
-                      : tmw::launch_prefill_simt(dd, qq, k, v, oo, st, block_size, all_keys, l);
-    };
-    if (np == 0) return launch(d, q, o, s, false);
-    // Two independent launches: the sequence rows [np, L) with the block-granular window, and the np
-    // persistent query rows, which see every key (one query tile per (batch, head) walking over all key
-    // tiles - it occupies only batch x heads CTAs for a long time).  They write different rows, so the
-    // second one runs on a side stream of the library between two events (a fork / join that stream
-    // capture accepts as well).
-    tmw_prefill_desc seq = d, pers = d;
-    const size_t esz = tmw::dtype_size(d.dtype);
-    seq.q_rows = d.q_rows - np;
-    seq.q_pos0 = np;
-    const void* q_seq = static_cast<const char*>(q) + (size_t)np * d.q_stride[2] * esz;
-    void* o_seq = static_cast<char*>(o) + (size_t)np * d.o_stride[2] * esz;
-    pers.q_rows = np;
-    tmw::SideStream* side = tmw::side_stream_of_current_device();
-    if (side == nullptr) {  // no side stream: one after the other
-        const int st = launch(seq, q_seq, o_seq, s, false);
-        return st != TMW_OK ? st : launch(pers, q, o, s, true);
-    }
-    std::lock_guard<std::mutex> lock(side->mutex);
-    TMW_CUDA_TRY(cudaEventRecord(side->fork, s));
-    TMW_CUDA_TRY(cudaStreamWaitEvent(side->stream, side->fork, 0));
-    int st = launch(pers, q, o, side->stream, true);
-    TMW_CUDA_TRY(cudaEventRecord(side->join, side->stream));
-    const int st2 = launch(seq, q_seq, o_seq, s, false);
-    TMW_CUDA_TRY(cudaStreamWaitEvent(s, side->join, 0));
-    return st != TMW_OK ? st : st2;
+    return tmw::prefill_block_sparse(desc, block_size, q, k, v, o, lse, static_cast<cudaStream_t>(stream), 0);
 }
 
 int tmw_linear(const tmw_linear_desc* d, const void* a, const void* w, const void* bias, void* c, void* stream) {

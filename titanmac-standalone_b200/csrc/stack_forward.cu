@@ -134,13 +134,15 @@ tmw_prefill_desc core_desc(const tmw_attention_desc& a) {
     return d;
 }
 
-int core(const tmw_attention_desc& a, const void* qkv, void* o, cudaStream_t stream) {
+// *link: whether the launch behind may be a dependent one
+int core(const tmw_attention_desc& a, const void* qkv, void* o, bool* link, cudaStream_t stream) {
     const tmw_prefill_desc d = core_desc(a);
     const int64_t D = (int64_t)a.heads * a.head_dim, esz = (int64_t)dtype_size(a.dtype);
     const char* q = static_cast<const char*>(qkv);
     const void *k = q + D * esz, *v = q + 2 * D * esz;
-    if (a.block_size > 0) return tmw_prefill_block_sparse(&d, a.block_size, q, k, v, o, stream);
-    if (prefill_tc_supports(d, q, k, v, o)) return launch_prefill_tc(d, q, k, v, o, stream, 0, false, nullptr, nullptr, kChainLink);
+    *link = prefill_tc_supports(d, q, k, v, o);
+    if (a.block_size > 0) return prefill_block_sparse(&d, a.block_size, q, k, v, o, nullptr, stream, kChainLink);
+    if (*link) return launch_prefill_tc(d, q, k, v, o, stream, 0, nullptr, nullptr, kChainLink);
     return tmw_prefill(&d, q, k, v, o, stream);
 }
 
@@ -180,9 +182,9 @@ int attention(const tmw_attention_desc& a, const void* x, const void* w_qkv, con
         rc = launch_dwconv(a.dtype, a.batch, a.rows, 3 * D, a.conv_taps, qkv, conv, 3, conv_out, stream);
         qkv = conv_out;
     }
-    if (rc == TMW_OK) rc = core(a, qkv, o, stream);
-    // (the block-sparse core ends in a wait for a side stream: an ordinary launch behind it)
-    const int link = (a.block_size > 0 ? 0 : kChainDependent) | (last ? 0 : kChainFollowed);
+    bool dependent = false;
+    if (rc == TMW_OK) rc = core(a, qkv, o, &dependent, stream);
+    const int link = (dependent ? kChainDependent : 0) | (last ? 0 : kChainFollowed);
     if (rc == TMW_OK) rc = linear(a.dtype, rows, D, D, o, w_out, nullptr, y, TMW_EPILOGUE_NONE, stream, link);
     return rc;
 }

@@ -143,6 +143,27 @@ __host__ __device__ inline int first_visible_pos(int pos, int np, int window, in
     return lo > np ? lo : np;
 }
 
+// d += a b for one 16 x 8 x 16 tile (mma.sync: tiles of a few rows, which tcgen05's 64 or 128 would waste)
+template <typename T>
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                          uint32_t b1);
+template <>
+__device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                         uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <>
+__device__ __forceinline__ void mma_16816<__half>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                  uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---- host-side plumbing shared by the entry points ---------------------------------
 void set_cuda_error(cudaError_t e, const char* where);
 void set_error_text(const char* text);
@@ -222,8 +243,11 @@ int validate_decode_call(const tmw_cache_desc* cache, const void* q, const void*
 int launch_prefill_simt(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
                         cudaStream_t stream, int window_block = 0, bool all_keys = false, float* lse = nullptr);
 int launch_prefill_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
-                      cudaStream_t stream, int window_block = 0, bool all_keys = false, float* lse = nullptr,
-                      const tmw_halo_wait* wait = nullptr, int chain = 0);
+                      cudaStream_t stream, int window_block = 0, float* lse = nullptr, const tmw_halo_wait* wait = nullptr,
+                      int chain = 0);
+// the query rows of the call see every key row, unmasked (16-bit types, head_dim 64 / 128): see pers_rows.cu
+int launch_pers_rows(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o, float* lse,
+                     cudaStream_t stream, bool pdl);
 // window_block / pers_global select the mask of the block-sparse class (see first_visible_pos; pers_global: the
 // persistent query rows see every key, and lse comes as [batch, heads, rows - np] followed by [batch, heads, np])
 int launch_prefill_backward(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o,
@@ -245,6 +269,9 @@ int launch_dwconv_backward(int dtype, int batch, int rows, int channels, int tap
 // x = embedded rows (persistent rows first), y = RMSNorm(x): see stack_forward.cu
 int launch_embed_seq(const tmw_stack_desc& d, const int64_t* token_ids, int tokens, const void* gain, void* x, void* y,
                      cudaStream_t stream);
+// tmw_prefill_block_sparse_lse as links of a chain of dependent launches
+int prefill_block_sparse(const tmw_prefill_desc* desc, int block_size, const void* q, const void* k, const void* v, void* o,
+                         float* lse, cudaStream_t s, int chain);
 bool prefill_tc_supports(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, const void* o);
 int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, const void* v_new, void* o,
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,

@@ -120,9 +120,9 @@ int attention_forward(const Dims& d, const void* x, const AttentionWeights& w, c
     if (rc != TMW_OK) return rc;
     const tmw_prefill_desc c = core_desc(d);
     const char *q = a.conv, *k = q + 2ll * D, *v = q + 4ll * D;
-    const bool link = d.block == 0 && prefill_tc_supports(c, q, k, v, a.o);
-    if (d.block > 0) rc = tmw_prefill_block_sparse_lse(&c, d.block, q, k, v, a.o, a.lse, s);
-    else if (link) rc = launch_prefill_tc(c, q, k, v, a.o, s, 0, false, a.lse, nullptr, d.taps > 0 ? kChainFollowed : kChainLink);
+    const bool link = prefill_tc_supports(c, q, k, v, a.o);
+    if (d.block > 0) rc = prefill_block_sparse(&c, d.block, q, k, v, a.o, a.lse, s, kChainLink);
+    else if (link) rc = launch_prefill_tc(c, q, k, v, a.o, s, 0, a.lse, nullptr, kChainLink);
     else rc = tmw_prefill_lse(&c, q, k, v, a.o, a.lse, s);
     if (rc != TMW_OK) return rc;
     return product(d, R, D, D, a.o, w.w_out, nullptr, y, residual != nullptr ? GEMM_ADD : GEMM_NONE, residual,
