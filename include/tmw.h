@@ -452,6 +452,15 @@ TMW_API int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* blocks,
                     void* logits, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * Greedy generation from the logits [batch, vocab] of the last prompt token (overwritten): `tokens` times the first index of
+ * each row's largest logit, and between them tmw_decode_step.  token_ids [batch] and pos [batch] (the index of the first
+ * generated token) are the steps' device buffers; the i-th choice of sequence b goes to out[b * out_stride + i].  Replaces
+ * the loop of the reference's generation helper (examples/train_math.py:146-161).
+ */
+TMW_API int tmw_generate(const tmw_stack_desc* desc, const tmw_block* blocks, void* logits, int32_t tokens, int64_t* token_ids,
+                 int32_t* pos, int64_t* out, int64_t out_stride, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Residual add + RMSNorm over contiguous rows [rows, dim] (dim a multiple of 8, pointers 16-byte aligned):
  *     h = x + residual          (residual may be NULL: h = x)
  *     sum_out = h               (sum_out may be NULL, and may be x itself: the residual stream in place)

@@ -85,3 +85,33 @@ def test_ids_outside_the_table_are_reported():
     with pytest.raises(_native.TmwError):
         _native.poll_status(torch.device(DEV))
     _native.poll_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("B,vocab,new", [(1, 1003, 5), (3, 512, 1), (40, 776, 9), (2, 8, 0)])
+def test_generate_equals_argmax_over_steps(B, vocab, new):
+    """``tmw_generate`` against a loop of ``decode_step`` and ``argmax``."""
+    model, g = make(torch.bfloat16, 2, 64, 20, 3, vocab)
+    ids = torch.randint(0, vocab, (B, 11), generator=g, device=DEV)
+    got = model.generate(ids, new)
+    logits, caches = model.prefill(ids)
+    want = [ids]
+    pos = torch.full((B,), 11, dtype=torch.int32, device=DEV)
+    for _ in range(new):
+        want.append(logits.argmax(-1)[:, None])
+        logits = model.decode_step(want[-1][:, 0], pos, caches)
+        pos += 1
+    assert torch.equal(got, torch.cat(want, dim=1))
+
+
+def test_greedy_choice_of_ties_and_nan():
+    model, _ = make(torch.bfloat16, 2, 64, 20, 0, 5000, layers=1)
+    logits = torch.zeros(4, 5000, dtype=torch.bfloat16, device=DEV)
+    logits[0, 4321] = logits[0, 17] = 2.0
+    logits[1] = -0.0
+    logits[1, 600:] = 0.0
+    logits[2, 900], logits[2, 100], logits[2, 3] = float("nan"), float("nan"), float("inf")
+    logits[3] = -1.0
+    logits[3, 4999] = -0.5
+    ids = torch.zeros(4, 1, dtype=torch.int64, device=DEV)
+    out = _stack.generate(_stack.table_of(model), ids, logits.clone(), model.new_caches(4, DEV, torch.bfloat16), 1)
+    assert out[:, 1].tolist() == [17, 0, 100, 4999] == logits.argmax(-1).tolist()

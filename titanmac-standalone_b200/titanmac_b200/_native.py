@@ -253,6 +253,11 @@ SIGNATURES = {
         ctypes.c_int,
         [ctypes.POINTER(StackDesc), ctypes.POINTER(Block)] + [ctypes.c_void_p] * 4 + [ctypes.c_size_t, ctypes.c_void_p],
     ),
+    "tmw_generate": (
+        ctypes.c_int,
+        [ctypes.POINTER(StackDesc), ctypes.POINTER(Block), ctypes.c_void_p, ctypes.c_int32] + [ctypes.c_void_p] * 3
+        + [ctypes.c_int64, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p],
+    ),
     "tmw_halo_push": (
         ctypes.c_int,
         [ctypes.POINTER(HaloCopy), ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
@@ -462,7 +467,9 @@ class RingCache:
     """K/V ring of ``window + 1`` slots per (sequence, head) plus the batch-shared persistent K/V."""
 
     def __init__(self, batch: int, heads: int, head_dim: int, window: int, n_persistent: int,
-                 dtype: torch.dtype, device: torch.device, scale: float = 0.0):
+                 dtype: torch.dtype, device: torch.device, scale: float = 0.0,
+                 storage: Optional[torch.Tensor] = None):
+        """``storage``: ``elements(...)`` zeros to live in (the caches of several layers from one allocation)."""
         if dtype not in _DTYPES:
             raise TypeError("dtype must be float32, bfloat16 or float16")
         if window < 0:
@@ -472,19 +479,26 @@ class RingCache:
         self.slots = window + 1
         self.dtype, self.device, self.scale = dtype, torch.device(device), scale
         self.geometry = (batch, heads, head_dim, window, n_persistent, dtype)
-        nbytes = lib().tmw_cache_ring_bytes(_DTYPES[dtype], batch, heads, head_dim, window)
-        elems = nbytes // torch.empty((), dtype=dtype).element_size()
-        assert elems == batch * heads * self.slots * head_dim
-        self.k_ring = torch.zeros((batch, heads, self.slots, head_dim), dtype=dtype, device=device)
-        self.v_ring = torch.zeros_like(self.k_ring)
-        self.k_pers = torch.zeros((heads, n_persistent, head_dim), dtype=dtype, device=device)
-        self.v_pers = torch.zeros_like(self.k_pers)
+        elems, pers = batch * heads * self.slots * head_dim, heads * n_persistent * head_dim
+        assert elems * dtype.itemsize == lib().tmw_cache_ring_bytes(_DTYPES[dtype], batch, heads, head_dim, window)
+        if storage is None:
+            storage = torch.zeros(2 * elems + 2 * pers, dtype=dtype, device=device)
+        k_ring, v_ring, k_pers, v_pers = storage.split((elems, elems, pers, pers))
+        self.k_ring = k_ring.view(batch, heads, self.slots, head_dim)
+        self.v_ring = v_ring.view(batch, heads, self.slots, head_dim)
+        self.k_pers = k_pers.view(heads, n_persistent, head_dim)
+        self.v_pers = v_pers.view(heads, n_persistent, head_dim)
         # A handful of (sequence, head) pairs with a long window cannot fill the GPU with one CTA per pair:
         # then every pair's keys are split over several CTAs (tmw_decode_split) through a scratch buffer
         # owned by this object.  Measured on B200: it wins from about 2000 keys per pair and fewer pairs than
         # half the SMs; at window 512 the unsplit launch is faster for every batch size.
         self.splits = self.pick_splits(batch * heads, self.slots, self.device)
         self._scratch = None
+
+    @staticmethod
+    def elements(batch: int, heads: int, head_dim: int, window: int, n_persistent: int) -> int:
+        """Elements of one cache: both rings, both persistent arrays."""
+        return 2 * heads * head_dim * (batch * (window + 1) + n_persistent)
 
     @staticmethod
     def pick_splits(pairs: int, slots: int, device) -> int:

@@ -244,30 +244,63 @@ def forward(table: ModelTable, token_ids: torch.Tensor, caches=None) -> Optional
     return logits
 
 
+def _step_arguments(table: ModelTable, batch: int, caches):
+    """``(StackDesc, blocks with the caches, workspace)`` of a decode step, or None where the table or the caches are not what
+    the step takes."""
+    device = table.device
+    if not table.decodes or batch == 0 or len(caches) != len(table.blocks):
+        return None
+    blocks = type(table.blocks).from_buffer_copy(table.blocks)  # (the table is shared by all threads)
+    if not _attach(blocks, caches, (batch,) + table.geometry, device):
+        return None
+    d = _native.StackDesc.from_buffer_copy(table.desc)
+    d.batch = batch
+    nbytes = table.workspace_bytes.get((batch, -1))
+    if nbytes is None:
+        nbytes = table.workspace_bytes[batch, -1] = _native.lib().tmw_decode_step_workspace(ctypes.byref(d))
+    return d, blocks, torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
 def decode_step(table: ModelTable, token_ids: torch.Tensor, pos: torch.Tensor, caches) -> Optional[torch.Tensor]:
     """``tmw_decode_step``; None where the arguments are not what that call takes."""
     B = token_ids.shape[0]
     device = table.device
-    if (not table.decodes or B == 0 or token_ids.dtype != torch.int64 or pos.dtype != torch.int32 or token_ids.dim() != 1 or pos.shape != (B,)
-            or token_ids.device != device or pos.device != device or len(caches) != len(table.blocks)):
+    if (token_ids.dtype != torch.int64 or pos.dtype != torch.int32 or token_ids.dim() != 1 or pos.shape != (B,)
+            or token_ids.device != device or pos.device != device):
         return None
+    arguments = _step_arguments(table, B, caches)
+    if arguments is None:
+        return None
+    d, blocks, workspace = arguments
     token_ids, pos = token_ids.contiguous(), pos.contiguous()
-    geometry = (B,) + table.geometry
-    blocks = type(table.blocks).from_buffer_copy(table.blocks)  # (the table is shared by all threads)
-    if not _attach(blocks, caches, geometry, device):
-        return None
-    d = _native.StackDesc.from_buffer_copy(table.desc)
-    d.batch = B
-    lib = _native.lib()
-    nbytes = table.workspace_bytes.get((B, -1))
-    if nbytes is None:
-        nbytes = table.workspace_bytes[B, -1] = lib.tmw_decode_step_workspace(ctypes.byref(d))
-    workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
     logits = torch.empty((B, d.vocab), dtype=table.dtype, device=device)
     with _native._on(device):
-        _native.check(lib.tmw_decode_step(ctypes.byref(d), blocks, token_ids.data_ptr(), pos.data_ptr(),
-                                          logits.data_ptr(), workspace.data_ptr(), nbytes, _native._stream_ptr(device)))
+        _native.check(_native.lib().tmw_decode_step(ctypes.byref(d), blocks, token_ids.data_ptr(), pos.data_ptr(), logits.data_ptr(),
+                                                    workspace.data_ptr(), workspace.numel(), _native._stream_ptr(device)))
     return logits
+
+
+def generate(table: ModelTable, input_ids: torch.Tensor, logits: torch.Tensor, caches, new_tokens: int) -> Optional[torch.Tensor]:
+    """The prompt and its greedy continuation (``tmw_generate``) from the logits of its last token; None where the arguments
+    are not what that call takes."""
+    B, T = input_ids.shape
+    device = table.device
+    if input_ids.dtype != torch.int64 or input_ids.device != device or new_tokens < 0 or not logits.is_contiguous() \
+            or logits.dtype != table.dtype:
+        return None
+    arguments = _step_arguments(table, B, caches)
+    if arguments is None:
+        return None
+    d, blocks, workspace = arguments
+    out = torch.empty((B, T + new_tokens), dtype=torch.int64, device=device)
+    out[:, :T] = input_ids
+    token = torch.empty(B, dtype=torch.int64, device=device)
+    pos = torch.full((B,), T, dtype=torch.int32, device=device)
+    with _native._on(device):
+        _native.check(_native.lib().tmw_generate(ctypes.byref(d), blocks, logits.data_ptr(), new_tokens, token.data_ptr(),
+                                                 pos.data_ptr(), out.data_ptr() + 8 * T, T + new_tokens, workspace.data_ptr(),
+                                                 workspace.numel(), _native._stream_ptr(device)))
+    return out
 
 
 def _plain_weight(mod: nn.Module, kind, dtype: torch.dtype) -> Optional[torch.Tensor]:
@@ -313,7 +346,7 @@ def attention_forward(attn: nn.Module, x: torch.Tensor, n_persistent: int, block
     ref = ctypes.byref(d)
     device = x.device
     nbytes = lib.tmw_attention_workspace(ref)
-    y = torch.empty_like(x)
+    y = torch.empty(x.shape, dtype=x.dtype, device=device)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
     conv_ptrs = tuple(w.data_ptr() for w in conv) if conv else (None, None, None)
     with _native._on(device):

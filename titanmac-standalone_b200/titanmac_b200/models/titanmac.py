@@ -122,8 +122,11 @@ class TitanMAC(nn.Module):
     def new_caches(self, batch: int, device, dtype) -> List[_native.RingCache]:
         self._need_windowed()
         c = self.config
-        return [_native.RingCache(batch, c.n_heads, c.d_head, c.window_size, c.n_persistent, dtype, device)
-                for _ in self.layers]
+        geometry = (batch, c.n_heads, c.d_head, c.window_size, c.n_persistent)
+        if dtype not in _native._DTYPES or c.window_size < 0:
+            return [_native.RingCache(*geometry, dtype, device)]  # (raises)
+        storage = torch.zeros((len(self.layers), _native.RingCache.elements(*geometry)), dtype=dtype, device=device)
+        return [_native.RingCache(*geometry, dtype, device, storage=storage[i]) for i in range(len(self.layers))]
 
     @torch.no_grad()
     def prefill(self, input_ids: torch.Tensor, caches: Optional[List[_native.RingCache]] = None):
@@ -194,13 +197,19 @@ class TitanMAC(nn.Module):
     def generate(self, input_ids: torch.Tensor, max_new_tokens: int, use_cuda_graph: bool = True) -> torch.Tensor:
         """Greedy continuation of ``input_ids [B, T]``; returns ``[B, T + max_new_tokens]``.
 
-        The decode step is launch-bound (a dozen small kernels per layer), so it is captured once in a
-        CUDA graph and replayed; token ids and positions live in static device buffers.
+        On the whole-model path all steps are issued by one library call.  Otherwise a step is launch-bound (a dozen small
+        kernels per layer), so it is captured once in a CUDA graph and replayed (``use_cuda_graph``); token ids and
+        positions live in static device buffers.
         """
         B, T = input_ids.shape
         if T + max_new_tokens > self.config.max_seq_len:
             raise ValueError("prompt + new tokens exceed max_seq_len (the position-embedding table)")
         logits, caches = self.prefill(input_ids)
+        table = _stack.table_of(self)
+        if table is not None:  # every choice and step from one call (tmw_generate)
+            tokens = _stack.generate(table, input_ids, logits, caches, max_new_tokens)
+            if tokens is not None:
+                return tokens
         tok = logits.argmax(dim=-1)
         pos = torch.full((B,), T, dtype=torch.int32, device=input_ids.device)
         out = [input_ids, tok[:, None]]
