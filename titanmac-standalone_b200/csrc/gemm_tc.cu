@@ -667,12 +667,12 @@ struct Variant {
 constexpr Variant kVariants[] = {{2 * GM, 256, 6.1f, 0.28f, 0.46f}, {GM, 256, 5.0f, 0.305f, 0.54f}, {GM, 128, 4.2f, 0.167f, 0.306f},
                                  {GM, 64, 3.7f, 0.128f, 0.186f},    {GM, 32, 3.5f, 0.117f, 0.135f}};
 
-float variant_cost(int i, const GemmCall& g, int splits) {
+float variant_cost(int i, const GemmCall& g, int splits, int sms) {
     const Variant& v = kVariants[i];
     const float slices = (float)((g.k + GK - 1) / GK) / (float)splits;
     // (the pair kernel's last tile of a row multiplies only the columns that exist)
     const float cols = i == 0 ? (float)((g.n + 31) / 32) / 8.f : (float)((g.n + v.cols - 1) / v.cols);
-    const float load = (float)((g.m + v.rows - 1) / v.rows) * cols * (float)splits / (float)(i == 0 ? sm_count() / 2 : sm_count());
+    const float load = (float)((g.m + v.rows - 1) / v.rows) * cols * (float)splits / (float)(i == 0 ? sms / 2 : sms);
     return v.launch + slices * (load <= 1.f ? v.alone + (v.full - v.alone) * load : v.full * ceilf(load));
 }
 
@@ -690,16 +690,17 @@ int launch_variant(int i, const GemmCall& g, cudaStream_t stream) {
 
 int launch_gemm_call(const GemmCall& call, cudaStream_t stream) {
     GemmCall g = call;
+    const int sms = sm_count();
     g.splits = 1;
     // a long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 6.5 us against 8.2)
-    if (!g.a_mn && !g.b_mn && g.epilogue <= GEMM_ADD && g.k >= 16 * GK && 2 * ((g.m + GM - 1) / GM) * ((g.n + 31) / 32) <= sm_count() &&
+    if (!g.a_mn && !g.b_mn && g.epilogue <= GEMM_ADD && g.k >= 16 * GK && 2 * ((g.m + GM - 1) / GM) * ((g.n + 31) / 32) <= sms &&
         g.lda == g.k && g.ldb == g.k && g.ldc == g.n && (g.epilogue != GEMM_ADD || g.aux == g.c))
         return launch_rows_tc(g.dtype, g.m, g.n, g.k, g.a, g.b, g.bias, g.c, g.epilogue, stream, g.chain & kChainDependent);
     int best = -1;
     float least = 0.f;
     for (int i = 0; i < 5; ++i) {
         if ((g.a_mn || g.b_mn) && (i == 1 || i == 4)) continue;  // built for the layouts of a backward pass: 256 x 256, 128, 64
-        const float t = variant_cost(i, g, 1);
+        const float t = variant_cost(i, g, 1, sms);
         if (best < 0 || t < least) {
             best = i;
             least = t;
@@ -713,13 +714,14 @@ int launch_gemm_call(const GemmCall& call, cudaStream_t stream) {
 // costs a trip of m x n fp32 values through memory and back, at about 4 TB/s, and a launch.
 int launch_gemm_splitk(const GemmCall& call, size_t partial_bytes, int* splits, cudaStream_t stream) {
     GemmCall g = call;
+    const int sms = sm_count();
     const size_t out = (size_t)g.m * g.n * sizeof(float);
     int best = 0, best_s = 1;
     float least = 0.f;
     for (int i = 0; i < 4; ++i) {
         if (i == 1) continue;
         for (int s = 1; s <= 32 && (s == 1 || (s * out <= partial_bytes && g.k >= s * 4 * GK)); ++s) {
-            const float t = variant_cost(i, g, s) + (s > 1 ? 2.5f + 2.f * (float)(s * out) / 4e6f : 0.f);
+            const float t = variant_cost(i, g, s, sms) + (s > 1 ? 2.5f + 2.f * (float)(s * out) / 4e6f : 0.f);
             if ((i == 0 && s == 1) || t < least) {
                 best = i;
                 best_s = s;

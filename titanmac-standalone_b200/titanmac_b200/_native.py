@@ -321,7 +321,15 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
             raise RuntimeError("libtmw works on CUDA tensors only; there is no CPU path")
 
 
+# (the raw calls where this build of torch has them: the public ones build a Stream object and look the device up twice,
+# about 2 us a call)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
 def _stream_ptr(device: torch.device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -330,7 +338,7 @@ _no_guard = contextlib.nullcontext()
 
 def _on(device: torch.device):
     """``torch.cuda.device(device)``, for nothing where that device is the current one already."""
-    return _no_guard if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+    return _no_guard if device.index == _raw_device() else torch.cuda.device(device)
 
 
 def _bhrd_strides(t: torch.Tensor) -> Sequence[int]:
@@ -382,7 +390,7 @@ def prefill(
     d.k_stride[:] = _bhrd_strides(k)
     d.v_stride[:] = _bhrd_strides(v)
     d.o_stride[:] = _bhrd_strides(out)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         if halo_wait is not None:
             if lse is not None or window_block > 0:
                 raise ValueError("halo_wait goes with the plain windowed prefill only")
@@ -430,7 +438,7 @@ def prefill_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch
     d.k_stride[:] = _bhrd_strides(k)
     d.v_stride[:] = _bhrd_strides(v)
     d.o_stride[:] = _bhrd_strides(o)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         if window_block > 0:
             check(lib().tmw_prefill_block_sparse_backward(ctypes.byref(d), window_block, q.data_ptr(), k.data_ptr(),
                                                           v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(),
@@ -457,7 +465,7 @@ def causal_dwconv(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     B, T, C = x.shape
     if B == 0 or T == 0:
         return y
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib().tmw_causal_dwconv(_DTYPES[x.dtype], B, T, C, weight.shape[1], x.data_ptr(), weight.data_ptr(),
                                       y.data_ptr(), _stream_ptr(x.device)))
     return y
@@ -530,7 +538,7 @@ class RingCache:
         c = self.desc()
         ks = (ctypes.c_int64 * 3)(*_bhrd_strides(k))
         vs = (ctypes.c_int64 * 3)(*_bhrd_strides(v))
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib().tmw_cache_fill(ctypes.byref(c), k.data_ptr(), v.data_ptr(), ks, vs, k.shape[2], t0,
                                        _stream_ptr(self.device)))
 
@@ -551,7 +559,7 @@ class RingCache:
         qs = (ctypes.c_int64 * 2)(q.stride(0), q.stride(1))
         ns = (ctypes.c_int64 * 2)(k_new.stride(0), k_new.stride(1))
         os_ = (ctypes.c_int64 * 2)(out.stride(0), out.stride(1))
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             if self.splits > 0:
                 if self._scratch is None:
                     nbytes = lib().tmw_decode_split_scratch_bytes(ctypes.byref(c), self.splits)
@@ -578,7 +586,7 @@ def causal_dwconv_backward(x: torch.Tensor, weight: torch.Tensor, dy: torch.Tens
     dx = torch.empty_like(x)
     dw = torch.zeros((C, weight.shape[1]), dtype=torch.float32, device=x.device)
     if B and T:
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             check(lib().tmw_causal_dwconv_backward(_DTYPES[x.dtype], B, T, C, weight.shape[1], x.data_ptr(),
                                                    weight.data_ptr(), dy.data_ptr(), dx.data_ptr(), dw.data_ptr(),
                                                    _stream_ptr(x.device)))
@@ -597,7 +605,7 @@ def gelu(x: torch.Tensor, inplace: bool = False) -> torch.Tensor:
     y = x if inplace else torch.empty_like(x)
     if x.numel() == 0:
         return y
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib().tmw_gelu(_DTYPES[x.dtype], x.numel(), x.data_ptr(), y.data_ptr(), _stream_ptr(x.device)))
     return y
 
@@ -678,7 +686,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         raise ValueError("linear: out must be contiguous, of x's dtype and shaped like x with n columns")
     desc = LinearDesc(dtype=_DTYPES[x.dtype], m=m, n=n, k=k, epilogue=EPILOGUE_GELU if gelu else EPILOGUE_NONE,
                       lda=x2.stride(0), ldw=weight.stride(0), ldc=n)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib().tmw_linear(ctypes.byref(desc), x2.data_ptr(), weight.data_ptr(),
                                bias.data_ptr() if bias is not None else None, out.data_ptr(),
                                _stream_ptr(x.device)))
@@ -733,7 +741,7 @@ def add_rmsnorm(x: torch.Tensor, residual: Optional[torch.Tensor], scale: torch.
     rows = x.numel() // dim if dim else 0
     if rows == 0:  # nothing to do (and an empty tensor has no address to pass)
         return h, y
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib().tmw_add_rmsnorm(_DTYPES[x.dtype], rows, dim, x.data_ptr(),
                                     residual.data_ptr() if residual is not None else None, scale.data_ptr(),
                                     float(eps), h.data_ptr() if residual is not None else None, y.data_ptr(),

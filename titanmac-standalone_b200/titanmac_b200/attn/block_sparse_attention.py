@@ -102,6 +102,8 @@ class BlockSparseAttention(nn.Module):
     def forward(self, x: torch.Tensor, attn_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return self._forward_train(x)
+        if not torch.is_grad_enabled():
+            return self._forward(x)
         with torch.no_grad():
             return self._forward(x)
 
@@ -139,7 +141,7 @@ class BlockSparseAttention(nn.Module):
             raise ValueError(f"n_persistent ({self.n_persistent}) must be < seq_len ({L})")
         y = _stack.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)  # the module as one call
         if y is not None:
-            return self.dropout(y)
+            return y if type(self.dropout) is nn.Identity else self.dropout(y)
         qkv = _native.project(self.qkv_proj, x)
         if self.use_conv:
             qkv = _native.causal_dwconv(qkv, self.stacked_conv_weight())

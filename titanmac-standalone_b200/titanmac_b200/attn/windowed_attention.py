@@ -130,14 +130,14 @@ class WindowedAttention(nn.Module):
             qkv = self.qkv_proj(x).view(B, L, 3, self.n_heads, self.d_head)
             o = _WindowedCore.apply(qkv, self.window_size, self.num_persistent, self.algo)
             return self.dropout(self.out_proj(o.view(B, L, D)))
+        y = _stack.attention_forward(self, x, self.num_persistent, 0, 0.0)  # the module as one call
+        if y is not None:
+            return y if type(self.dropout) is nn.Identity else self.dropout(y)
         with torch.no_grad():
             return self._forward_no_grad(x)
 
     def _forward_no_grad(self, x: torch.Tensor) -> torch.Tensor:
         B, L, D = x.shape
-        y = _stack.attention_forward(self, x, self.num_persistent, 0, 0.0)  # the module as one call
-        if y is not None:
-            return self.dropout(y)
         qkv = _native.project(self.qkv_proj, x)  # tmw_linear: [B, L, 3, H, dh] is just its row-major output
         q, k, v = self.split_qkv(qkv)
         # the output is allocated as [B, L, H, dh] so that "concat heads" is a view
