@@ -1,0 +1,44 @@
+"""Forward cores at the edges of their tiles: the register-tiled fp32 kernel (32 rows x 64 keys, two groups of threads that
+take the key tiles in turn) and the kernel of the block-sparse class's persistent rows (16 rows, keys split over a cluster)."""
+
+import math
+
+import pytest
+import torch
+
+from oracle import block_sparse_oracle as bo
+from oracle import windowed_oracle as wo
+from titanmac_b200 import _native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dh", [64, 128])
+@pytest.mark.parametrize("L,w,n_p", [
+    (1, 0, 0), (32, 31, 0), (33, 0, 1),      # one key, one full tile of rows, self-only windows behind a persistent key
+    (64, 63, 0), (65, 64, 1), (129, 500, 0), # one and two key tiles exactly, and one key more
+    (200, 40, 64), (230, 100, 130),          # rows that see persistent keys only, one tile and more of them
+])
+def test_fp32_core_at_tile_edges(dh, L, w, n_p):
+    q, k, v = wo.qkv_inputs(2, 3, L, dh, seed=dh + L)
+    ref = wo.attention_core_dense(q, k, v, w, n_p)
+    lse = torch.empty(2, 3, L, device=DEV)
+    o = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), w, n_p, lse=lse)
+    assert (o.cpu() - ref).abs().max().item() <= 1e-5
+    s = (q.double() @ k.double().transpose(-1, -2)) / dh ** 0.5
+    s = s.masked_fill(~wo.band_mask(L, w, n_p), float("-inf"))
+    assert (lse.cpu() - torch.logsumexp(s, -1) / math.log(2.0)).abs().max().item() <= 2e-5
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2), (torch.float16, 2e-2)])
+@pytest.mark.parametrize("dh,L,w,block,n_p", [
+    (64, 40, 64, 64, 1), (64, 257, 64, 64, 16), (64, 300, 128, 32, 17),   # 1, 16 and 17 persistent rows
+    (128, 500, 96, 32, 33), (128, 129, 64, 64, 128), (128, 1040, 512, 64, 16),
+])
+def test_block_sparse_core_with_persistent_rows(dtype, tol, dh, L, w, block, n_p):
+    q, k, v = (t.to(dtype) for t in wo.qkv_inputs(2, 3, L, dh, seed=dh + L))
+    ref = bo.attention_core(q.float(), k.float(), v.float(), w, block, n_p)
+    o = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), w, n_p, window_block=block)
+    _native.poll_status()
+    assert (o.float().cpu() - ref).abs().max().item() <= tol

@@ -201,9 +201,13 @@ int launch_dh(const SimtParams& p, int batch, int heads, int dh, cudaStream_t st
         case 8: return launch_t<T, 8>(p, batch, heads, stream);
         case 16: return launch_t<T, 16>(p, batch, heads, stream);
         case 32: return launch_t<T, 32>(p, batch, heads, stream);
-        case 64: return launch_t<T, 64>(p, batch, heads, stream);
+        case 64:
+            if constexpr (sizeof(T) == 2) return launch_t<T, 64>(p, batch, heads, stream);
+            return TMW_ERR_UNSUPPORTED;  // prefill_fp32.cu
         case 96: return launch_t<T, 96>(p, batch, heads, stream);
-        case 128: return launch_t<T, 128>(p, batch, heads, stream);
+        case 128:
+            if constexpr (sizeof(T) == 2) return launch_t<T, 128>(p, batch, heads, stream);
+            return TMW_ERR_UNSUPPORTED;
         case 256: return launch_t<T, 256>(p, batch, heads, stream);
         default: return TMW_ERR_UNSUPPORTED;
     }
@@ -213,6 +217,8 @@ int launch_dh(const SimtParams& p, int batch, int heads, int dh, cudaStream_t st
 
 int launch_prefill_simt(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
                         cudaStream_t stream, int window_block, bool all_keys, float* lse) {
+    if (prefill_fp32_supports(d) && d.batch <= 65535 && d.heads <= 65535)
+        return launch_prefill_fp32(d, q, k, v, o, stream, window_block, all_keys, lse);
     SimtParams p;
     p.lse = lse;
     p.block = window_block;

@@ -242,6 +242,10 @@ int validate_decode_call(const tmw_cache_desc* cache, const void* q, const void*
 // score * scale * log2(e) - what the backward pass needs to rebuild the probabilities
 int launch_prefill_simt(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
                         cudaStream_t stream, int window_block = 0, bool all_keys = false, float* lse = nullptr);
+// fp32, head_dim 64 / 128: register-tiled kernel (prefill_fp32.cu), which launch_prefill_simt hands those calls to
+bool prefill_fp32_supports(const tmw_prefill_desc& d);
+int launch_prefill_fp32(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o, cudaStream_t stream,
+                        int window_block, bool all_keys, float* lse);
 int launch_prefill_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o,
                       cudaStream_t stream, int window_block = 0, float* lse = nullptr, const tmw_halo_wait* wait = nullptr,
                       int chain = 0);
