@@ -84,9 +84,9 @@ struct BwdSmem {
     static constexpr int kTotal = kBars + 256 + 1024;
 };
 
-// barrier slots: R_FULL | C_FULL[4] | C_EMPTY[4] | XY_FULL | PDS_READY | ACC_DONE | V_FULL[4]
-enum { BAR_R_FULL = 0, BAR_C_FULL = 1, BAR_C_EMPTY = 5, BAR_XY_FULL = 9, BAR_PDS_READY = 10, BAR_ACC_DONE = 11, BAR_V_FULL = 12,
-       BAR_N = 16 };
+// barrier slots: R_FULL | C_FULL[4] | C_EMPTY[4] | XY_FULL[2] | PDS_READY[2] | ACC_DONE | V_FULL[4]
+enum { BAR_R_FULL = 0, BAR_C_FULL = 1, BAR_C_EMPTY = 5, BAR_XY_FULL = 9, BAR_PDS_READY = 11, BAR_ACC_DONE = 13, BAR_V_FULL = 14,
+       BAR_N = 18 };
 
 // D = dO . O of one query row (fp32), straight from global memory (two rows of head_dim 16-bit values)
 template <int DH, bool BF16>
@@ -216,8 +216,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             mbar_init(bar(BAR_C_EMPTY + s), 2);  // both issuing warps
         }
         for (int s = 0; s < kColStages; ++s) mbar_init(bar(BAR_V_FULL + s), 1);
-        mbar_init(bar(BAR_XY_FULL), 2);    // X by one issuing warp, Y by the other
-        mbar_init(bar(BAR_PDS_READY), 8);  // the eight element-wise warps
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(bar(BAR_XY_FULL + h), 2);    // X by one issuing warp, Y by the other
+            mbar_init(bar(BAR_PDS_READY + h), 4);  // the four element-wise warps of the half
+        }
         mbar_init(bar(BAR_ACC_DONE), 2);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -293,47 +295,55 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         if (elect_one()) {  // one thread runs the whole role
         const bool second = warp == 2;
         const uint32_t fmt = BF16 ? 1u : 0u;
-        const uint32_t idesc_xy = idesc_kmajor(fmt, CW);
+        constexpr int HC = CW / 2;
+        const uint32_t idesc_xy = idesc_kmajor(fmt, HC);
         const uint32_t idesc_acc = idesc_b_mnmajor(fmt, DH);
         const bool has_acc = second || ROWS_ARE_KEYS;
-        // the 16-bit intermediates of 16 columns (one k-step) sit in 8 tensor-memory columns; each half of the
-        // column tile keeps its packed values inside its own half (see the element-wise warps)
-        auto packed_col = [](int kk) -> uint32_t { return (uint32_t)((kk / (CW / 32)) * (CW / 2) + (kk % (CW / 32)) * 8); };
-        mbar_wait(bar(BAR_R_FULL), 0, abort_flag, p.status);
-        for (int n = 0; n < n_cols; ++n) {
-            const int s = n % kColStages;
-            const uint32_t c_addr = smem_base + L::kC + s * 2 * L::kCTile;
-            mbar_wait(bar(BAR_C_FULL + s), (n / kColStages) & 1, abort_flag, p.status);
-            tc_fence_after();
-            // both operands K-major over head_dim
-            const uint32_t r_addr = smem_base + (second ? L::kR2 : L::kR1);
-            const uint32_t c_tile = c_addr + (second ? L::kCTile : 0);
+        const uint32_t xy = tmem_base + (second ? kY : kX);
+        const uint32_t r_addr = smem_base + (second ? L::kR2 : L::kR1);
+        // X or Y of half h of the column tile n: both operands K-major over head_dim
+        auto issue_xy = [&](int n, int h) {
+            const uint32_t c_tile = smem_base + L::kC + (n % kColStages) * 2 * L::kCTile + (second ? L::kCTile : 0) + h * HC * 128;
 #pragma unroll
             for (int kk = 0; kk < DH / 16; ++kk) {
                 const uint64_t ad = kmajor_desc(r_addr + (kk / 4) * L::kSub + (kk % 4) * 32);
                 const uint64_t bd = kmajor_desc(c_tile + (kk / 4) * L::kCSub + (kk % 4) * 32);
-                mma_ss(tmem_base + (second ? kY : kX), ad, bd, idesc_xy, kk > 0 ? 1u : 0u);
+                mma_ss(xy + h * HC, ad, bd, idesc_xy, kk > 0 ? 1u : 0u);
             }
-            tc_commit(bar(BAR_XY_FULL));
+            tc_commit(bar(BAR_XY_FULL + h));
+        };
+        mbar_wait(bar(BAR_R_FULL), 0, abort_flag, p.status);
+        if (n_cols > 0) {
+            mbar_wait(bar(BAR_C_FULL), 0, abort_flag, p.status);
+            tc_fence_after();
+            issue_xy(0, 0);
+            issue_xy(0, 1);
+        }
+        for (int n = 0; n < n_cols; ++n) {
+            const int s = n % kColStages;
+            const uint32_t c_addr = smem_base + L::kC + s * 2 * L::kCTile;
             // (the next column tile has usually landed: seeing it now takes that wait off the path hand-over ->
             // products of this tile -> X / Y of the next)
             if (n + 1 < n_cols)
                 mbar_wait(bar(BAR_C_FULL + (n + 1) % kColStages), ((n + 1) / kColStages) & 1, abort_flag, p.status);
-            mbar_wait(bar(BAR_PDS_READY), n & 1, abort_flag, p.status);
-            tc_fence_after();
-            if (has_acc) {
-                // A = P or dS from tensor memory, B = the other column tile read MN-major:
-                // warp 1: dV += P^T dO (B = C2);  warp 2: dK += dS^T Q  or  dQ += dS K (B = C1)
-                const uint32_t a_base = tmem_base + (second ? kY : kX);
-                const uint32_t d_acc = tmem_base + ((second && ROWS_ARE_KEYS) ? kAcc2 : kAcc1);
-                const uint64_t b0 = mnmajor_desc(second ? c_addr : c_addr + L::kCTile, L::kCSub);
-                const uint32_t acc = n > 0 ? 1u : 0u;
 #pragma unroll
-                for (int kk = 0; kk < CW / 16; ++kk) {
-                    mma_ts(d_acc, a_base + packed_col(kk), b0 + kk * 128, idesc_acc, kk > 0 ? 1u : acc);
+            for (int h = 0; h < 2; ++h) {
+                mbar_wait(bar(BAR_PDS_READY + h), n & 1, abort_flag, p.status);
+                tc_fence_after();
+                if (has_acc) {
+                    // A = P or dS from tensor memory, B = the other column tile read MN-major:
+                    // warp 1: dV += P^T dO (B = C2);  warp 2: dK += dS^T Q  or  dQ += dS K (B = C1).
+                    // The 16-bit values of 16 columns (one k-step) sit in 8 tensor-memory columns, each half's inside
+                    // its own half.
+                    const uint32_t d_acc = tmem_base + ((second && ROWS_ARE_KEYS) ? kAcc2 : kAcc1);
+                    const uint64_t b0 = mnmajor_desc(second ? c_addr : c_addr + L::kCTile, L::kCSub);
+#pragma unroll
+                    for (int kk = 0; kk < HC / 16; ++kk)
+                        mma_ts(d_acc, xy + h * HC + kk * 8, b0 + (h * (HC / 16) + kk) * 128, idesc_acc, kk + h + n > 0 ? 1u : 0u);
                 }
+                if (h == 1) tc_commit(bar(BAR_C_EMPTY + s));
+                if (n + 1 < n_cols) issue_xy(n + 1, h);
             }
-            tc_commit(bar(BAR_C_EMPTY + s));
             if (n == n_cols - 1) tc_commit(bar(BAR_ACC_DONE));
         }
         }
@@ -403,7 +413,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             const bool vnone = vhi < vlo;
             const int pbase = npc - cbase;                 // column < npc  <=>  (column - cbase) < pbase
 
-            mbar_wait(bar(BAR_XY_FULL), n & 1, abort_flag, p.status);
+            mbar_wait(bar(BAR_XY_FULL + half), n & 1, abort_flag, p.status);
             tc_fence_after();
             // 16 columns at a time.  The body exists twice, with and without the per-element mask, as straight-line
             // code (a run-time test inside it would split it into one basic block per element and serialise the
@@ -484,7 +494,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(BAR_PDS_READY));
+            if (lane == 0) mbar_arrive(bar(BAR_PDS_READY + half));
         }
 
         // ---------------- output: accumulators -> 16 bits -> shared memory (swizzled) -> TMA store ----------------
