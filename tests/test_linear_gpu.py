@@ -49,6 +49,13 @@ def test_ragged_sizes(m, n, k):
     run_case(m, n, k, False, True, seed=m + 1)
 
 
+@pytest.mark.parametrize("m,n,k", [(8320, 640, 72), (8321, 616, 128), (6144, 1000, 64), (16416, 328, 72)])
+def test_column_tiles_narrower_than_256(m, n, k):
+    """Few waves of row bands: the pair kernel cuts N into tiles of 128 to 224 columns."""
+    run_case(m, n, k, True, False, seed=m)
+    run_case(m, n, k, False, True, dtype=torch.float16, seed=n)
+
+
 def test_fp16_and_strided_input():
     run_case(200, 320, 128, True, True, dtype=torch.float16)
     g = torch.Generator(device=DEV).manual_seed(9)

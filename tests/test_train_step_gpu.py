@@ -1,0 +1,90 @@
+"""The training step as two library calls (``tmw_stack_train_*``, ``tmw_cross_entropy``) and the one-call forwards against the
+same computation module by module."""
+
+import pytest
+import torch
+
+from titanmac_b200 import TitanMAC, TitanMACConfig, _native, _stack, _train
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def make(dtype, heads, dh, window, Np, vocab, block_sparse, layers=2, seed=0):
+    D = heads * dh
+    cfg = TitanMACConfig(vocab_size=vocab, d_model=D, n_heads=heads, n_layers=layers, d_ff=2 * D + 96, max_seq_len=1024,
+                         window_size=window, n_persistent=Np, use_block_sparse=block_sparse, block_size=32)
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    with torch.device(DEV):
+        model = TitanMAC(cfg)
+    with torch.no_grad():
+        for name, prm in model.named_parameters():
+            prm.normal_(1.0 if name.endswith("scale") else 0.0, 0.1 if name.endswith(("scale", "bias")) else 0.04, generator=g)
+    return model.to(dtype), g
+
+
+def module_by_module(monkeypatch):
+    monkeypatch.setattr(_stack, "table_of", lambda m: None)
+    monkeypatch.setattr(_stack, "attention_forward", lambda *a: None)
+    for name in ("stack_forward", "attention_forward", "shifted_cross_entropy"):
+        monkeypatch.setattr(_train, name, lambda *a: None)
+
+
+def close(got, want, tol):
+    return ((got.float() - want.float()).norm() / want.float().norm().clamp_min(1e-12)).item() <= tol
+
+
+@pytest.mark.parametrize("B,T,dtype,heads,dh,window,Np,vocab,block_sparse", [
+    (1, 1, torch.bfloat16, 2, 64, 8, 3, 512, False),      # one token: no label is left
+    (2, 61, torch.bfloat16, 2, 64, 16, 16, 1000, False),  # 154 rows: two row tiles, a ragged last one
+    (3, 130, torch.float16, 3, 64, 32, 5, 776, True),     # odd widths (192), the convolutions' strips cut short
+    (2, 200, torch.bfloat16, 1, 128, 40, 0, 4096, False), # no persistent rows
+    (8, 1001, torch.bfloat16, 4, 64, 64, 8, 640, True),   # k = 8072 rows in the weights' gradients: cut into ranges
+    (4, 1024, torch.float16, 5, 128, 100, 16, 2048, False),  # d_model 640: column tiles narrower than 256
+])
+def test_training_step_equals_module_by_module(B, T, dtype, heads, dh, window, Np, vocab, block_sparse, monkeypatch):
+    model, g = make(dtype, heads, dh, window, Np, vocab, block_sparse)
+    ids = torch.randint(0, vocab, (B, T), generator=g, device=DEV)
+    labels = torch.randint(0, vocab, (B, T), generator=g, device=DEV)
+    labels[torch.rand(B, T, generator=g, device=DEV) < 0.2] = -100  # ignored
+    scale = 1.0 if dtype == torch.bfloat16 else 64.0
+
+    def step():
+        model.zero_grad(set_to_none=True)
+        out = model(ids, labels=labels)
+        if T > 1:
+            (out["loss"] * scale).backward()
+        return out["loss"].detach(), out["logits"].detach(), {n: p.grad for n, p in model.named_parameters()}
+
+    loss, logits, grads = step()
+    _native.poll_status(torch.device(DEV))
+    module_by_module(monkeypatch)
+    want_loss, want_logits, want = step()
+    tol = 3e-2 if dtype == torch.bfloat16 else 6e-3
+    assert close(logits, want_logits, tol)
+    if T == 1:
+        return
+    assert abs(loss.item() - want_loss.item()) <= tol * abs(want_loss.item())
+    for name, ref in want.items():
+        assert (grads[name] is None) == (ref is None), name
+        if ref is not None:
+            assert grads[name].dtype == dtype and close(grads[name], ref, 2 * tol), name
+
+
+@pytest.mark.parametrize("B,T,dtype,heads,dh,Np,block_sparse", [
+    (1, 1, torch.bfloat16, 2, 64, 1, False), (2, 33, torch.float16, 3, 64, 0, False), (1, 400, torch.bfloat16, 1, 128, 17, True),
+    (3, 127, torch.bfloat16, 4, 64, 16, True),
+])
+def test_forward_equals_module_by_module(B, T, dtype, heads, dh, Np, block_sparse, monkeypatch):
+    model, g = make(dtype, heads, dh, 48, Np, 520, block_sparse)
+    model.eval()
+    ids = torch.randint(0, 520, (B, T), generator=g, device=DEV)
+    x = torch.randn(B, T + max(Np, 1), heads * dh, generator=g, device=DEV).to(dtype)
+    attn = model.layers[0].attention
+    with torch.no_grad():
+        got = model(ids)["logits"], attn(x)
+        _native.poll_status(torch.device(DEV))
+        module_by_module(monkeypatch)
+        want = model(ids)["logits"], attn(x)
+    tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
+    assert close(got[0], want[0], tol) and close(got[1], want[1], tol)

@@ -55,6 +55,7 @@ struct GemmParams {
     void* aux;           // [m, n] beside the output (see GemmEpilogue), contiguous
     float* partial;      // k cut into `splits` ranges: their fp32 sums go to [splits][m][n] here instead of to the output
     int splits;
+    int width;           // pair kernel: columns of a tile (a multiple of 32)
     int drain;           // a dependent launch follows: the stores have to be complete when the kernel ends
     int* status;
 };
@@ -365,15 +366,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();  // 0: issues the products, 1: partner
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int n_tiles = (p.n + BN - 1) / BN, m_tiles = (p.m + 2 * GM - 1) / (2 * GM);
+    const int n_tiles = (p.n + p.width - 1) / p.width, m_tiles = (p.m + 2 * GM - 1) / (2 * GM);
     const int tiles = n_tiles * m_tiles * p.splits;  // (tile, k range)
     const int k_blocks = (p.k + GK - 1) / GK;
-    // columns a tile multiplies: BN, or for the last tile of a row what is left of N (in steps of 32) - a product
-    // over columns that do not exist would cost its full time
-    auto n_of = [&](int tile) -> int {
-        const int rem = p.n - (tile / p.splits % n_tiles) * BN;
-        return rem >= BN ? BN : (rem + 31) / 32 * 32;
+    auto locate = [&](int tile, int& band, int& col) {  // its band of 256 rows and first column
+        const int mn = tile / p.splits;
+        band = mn / n_tiles;
+        col = (mn % n_tiles) * p.width;
     };
+    // columns a tile multiplies: its width, or for the last tile of a row what is left of N (in steps of 32) - a product
+    // over columns that do not exist would cost its full time
+    auto columns = [&](int col) -> int { return min(p.width, (p.n - col + 31) / 32 * 32); };
+    const int b_boxes = (p.width + 127) / 128;  // boxes of 64 columns that an MN-major half takes
+    const uint32_t stage_bytes = 2 * (L::kStageA + (BMN ? b_boxes * 8192 : p.width * 64));  // both CTAs' bytes
 
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
@@ -405,14 +410,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int s = 0;
             uint32_t parity = 1;
             for (int tile = pair; tile < tiles; tile += pairs) {
-                const int mn = tile / p.splits, split = tile % p.splits;
-                const int row0 = (mn / n_tiles) * (2 * GM) + (int)rank * GM;
-                // each CTA supplies half of the tile's columns (the box is BN / 2 rows; a narrow tile uses its first rows)
-                const int col0 = (mn % n_tiles) * BN + (int)rank * (n_of(tile) / 2);
+                const int split = tile % p.splits;
+                int band, col;
+                locate(tile, band, col);
+                const int row0 = band * (2 * GM) + (int)rank * GM;
+                // each CTA supplies half of the tile's columns (the box is half of p.width; a narrow tile uses its first rows)
+                const int col0 = col + (int)rank * (columns(col) / 2);
                 const int kb1 = k_blocks * (split + 1) / p.splits;
                 for (int kb = k_blocks * split / p.splits; kb < kb1; ++kb) {
                     mbar_wait(empty(s), parity, abort_flag, p.status);
-                    if (rank == 0) mbar_expect_tx(full(s), 2 * L::kStage);  // both CTAs' bytes
+                    if (rank == 0) mbar_expect_tx(full(s), stage_bytes);
                     const uint32_t bar0 = map_to_cta(full(s), 0);
                     const uint32_t dst = smem_base + s * L::kStage;
                     if (AMN) {
@@ -422,8 +429,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         tma_load_2d_pair(dst, &map_a, bar0, kb * GK, row0);
                     }
                     if (BMN) {
-#pragma unroll
-                        for (int c = 0; c < BN / 128; ++c)
+                        for (int c = 0; c < b_boxes; ++c)
                             tma_load_2d_pair(dst + L::kStageA + c * 8192, &map_w, bar0, col0 + c * 64, kb * GK);
                     } else {
                         tma_load_2d_pair(dst + L::kStageA, &map_w, bar0, kb * GK, col0);
@@ -440,7 +446,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             uint32_t parity = 0;
             for (int tile = pair; tile < tiles; tile += pairs, ++t) {
                 const int buf = t & 1;
-                const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, (uint32_t)n_of(tile), 2 * GM) | (AMN ? 1u << 15 : 0u) |
+                int band, col;
+                locate(tile, band, col);
+                const uint32_t idesc = idesc_kmajor(BF16 ? 1u : 0u, (uint32_t)columns(col), 2 * GM) | (AMN ? 1u << 15 : 0u) |
                                        (BMN ? 1u << 16 : 0u);
                 mbar_wait(acc_empty(buf), ((t >> 1) & 1) ^ 1, abort_flag, p.status);
                 tc_fence_after();
@@ -467,16 +475,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int g = warp & 3;
         const int half = (warp - 2) >> 2;
         const int row = g * 32 + lane;
-        constexpr int kPanels = BN / kPanel;
         uint8_t* stage = smem + S * L::kStage;
         const bool epi_leader = warp == 2 && lane == 0;
         int t = 0;
         for (int tile = pair; tile < tiles; tile += pairs, ++t) {
             const int buf = t & 1;
-            const int mn = tile / p.splits;
-            const int row0 = (mn / n_tiles) * (2 * GM) + (int)rank * GM, col0 = (mn % n_tiles) * BN;
+            int band, col0;
+            locate(tile, band, col0);
+            const int row0 = band * (2 * GM) + (int)rank * GM;
             // the tile's panels of 32 columns, split between the two warps of a lane group
-            const int panels = n_of(tile) / kPanel, half_panels = (panels + 1) / 2;
+            const int panels = columns(col0) / kPanel, half_panels = (panels + 1) / 2;
             const int panel0 = half == 0 ? 0 : half_panels;
             const int panel1 = half == 0 ? half_panels : panels;
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
@@ -523,7 +531,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             fence_proxy_async_smem();
             named_barrier_sync(2, kEpiWarps * 32);
             if (epi_leader && row0 < p.m && p.partial == nullptr) {
-                for (int pn = 0; pn < kPanels; ++pn)
+                for (int pn = 0; pn < panels; ++pn)
                     if (col0 + pn * kPanel < p.n)
                         tma_store_2d(&map_c, smem_u32(stage + pn * (GM * 64)), col0 + pn * kPanel, row0);
                 tma_store_commit();
@@ -633,13 +641,14 @@ int max_active_pairs(const void* kern, int smem_bytes) {
 }
 
 template <int BN>
-int launch_gemm_pair(const GemmCall& g, cudaStream_t stream) {
+int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
     using L = PairSmem<BN>;
     CUtensorMap ma, mb, mc;
     GemmParams p;
-    if (!make_maps(g, BN / 2, &ma, &mb, &mc)) return TMW_ERR_CUDA;
+    if (!make_maps(g, width / 2, &ma, &mb, &mc)) return TMW_ERR_CUDA;
     if (gemm_params(g, &p) != TMW_OK) return TMW_ERR_CUDA;
-    const int tiles = ((g.m + 2 * GM - 1) / (2 * GM)) * ((g.n + BN - 1) / BN) * g.splits;
+    p.width = width;
+    const int tiles = ((g.m + 2 * GM - 1) / (2 * GM)) * ((g.n + width - 1) / width) * g.splits;
     auto run = [&](auto kern) -> int {
         const void* fn = reinterpret_cast<const void*>(kern);
         const int rc = allow_shared_memory(fn, L::kTotal);
@@ -656,29 +665,53 @@ int launch_gemm_pair(const GemmCall& g, cudaStream_t stream) {
                              gemm_tc_pair_kernel<BN, false, true, true>, run);
 }
 
-// What a kernel was measured to need (us): a launch without its K, what a 64-wide slice of K takes where a tile is alone on
-// the chip, and where all SMs stream operands.  The pair kernel moves the fewest operand bytes per product and wins
+// What a single-CTA kernel was measured to need (us): a launch without its K, what a 64-wide slice of K takes where a tile is
+// alone on the chip, and where all SMs stream operands.  The pair kernel moves the fewest operand bytes per product and wins
 // wherever it has enough tiles: measured at K = 640 for 1056 | 2528 | 8256 | 32 896 rows of N = 1920, pair | 128 | 64
 // columns: 9.3 | 12.6 | 21.3 | 68.8, 6.3 | 11.4 | 24.1 | 82.5, 7.1 | 11.7 | 29.0 us.
 struct Variant {
     int rows, cols;
     float launch, alone, full;
 };
-constexpr Variant kVariants[] = {{2 * GM, 256, 6.1f, 0.28f, 0.46f}, {GM, 256, 5.0f, 0.305f, 0.54f}, {GM, 128, 4.2f, 0.167f, 0.306f},
-                                 {GM, 64, 3.7f, 0.128f, 0.186f},    {GM, 32, 3.5f, 0.117f, 0.135f}};
+constexpr Variant kVariants[] = {{2 * GM, 256, 6.1f, 0.f, 0.f},  // (see pair_cost)
+                                 {GM, 256, 5.0f, 0.305f, 0.54f}, {GM, 128, 4.2f, 0.167f, 0.306f},
+                                 {GM, 64, 3.7f, 0.128f, 0.186f}, {GM, 32, 3.5f, 0.117f, 0.135f}};
 
-float variant_cost(int i, const GemmCall& g, int splits, int sms) {
+// The pair kernel's cost and tile width.  A 64-wide slice of a tile of w columns takes 0.12 + 0.00105 w us on a busy chip
+// and the chip as a whole 0.465 us per 256 columns of a pair; few waves of wide tiles leave a last one that is nearly empty,
+// which narrower tiles fill.  8320 x 640 x 2560: 33 bands over 74 pairs are two waves at 256 columns and at 160; 33.8 and
+// 28.8 us (64 columns a CTA, single: 38.6).  16416 x 640 x 2560: 47.5 at 256, 50.7 at 160.
+float pair_cost(const GemmCall& g, int splits, int sms, int* width) {
+    const float slices = (float)((g.k + GK - 1) / GK) / (float)splits;
+    const int bands = (g.m + 2 * GM - 1) / (2 * GM), pairs = sms / 2 > 0 ? sms / 2 : 1;
+    const float busy = (float)bands * (float)((g.n + 31) / 32) / 8.f * (float)splits / (float)pairs;
+    auto slice = [](int w) { return 0.12f + 0.00105f * (float)w; };
+    float least = 0.f;
+    for (int w = 256; w >= 128; w -= 32) {
+        const int n_tiles = (g.n + w - 1) / w, last = g.n - (n_tiles - 1) * w;
+        const long long tiles = (long long)n_tiles * bands * splits, waves = (tiles + pairs - 1) / pairs, narrow = waves / n_tiles;
+        float t = (float)(waves - narrow) * slice(w) + (float)narrow * slice(last);
+        if (waves == 1) t *= 0.72f + 0.28f * (float)tiles / (float)pairs;  // operands arrive faster on a chip half idle
+        t = t > 0.465f * busy ? t : 0.465f * busy;
+        if (w == 256 || t < 0.97f * least) {
+            least = t;
+            *width = w;
+        }
+    }
+    return kVariants[0].launch + slices * least;
+}
+
+float variant_cost(int i, const GemmCall& g, int splits, int sms, int* width) {
+    if (i == 0) return pair_cost(g, splits, sms, width);
     const Variant& v = kVariants[i];
     const float slices = (float)((g.k + GK - 1) / GK) / (float)splits;
-    // (the pair kernel's last tile of a row multiplies only the columns that exist)
-    const float cols = i == 0 ? (float)((g.n + 31) / 32) / 8.f : (float)((g.n + v.cols - 1) / v.cols);
-    const float load = (float)((g.m + v.rows - 1) / v.rows) * cols * (float)splits / (float)(i == 0 ? sms / 2 : sms);
+    const float load = (float)((g.m + v.rows - 1) / v.rows) * (float)((g.n + v.cols - 1) / v.cols) * (float)splits / (float)sms;
     return v.launch + slices * (load <= 1.f ? v.alone + (v.full - v.alone) * load : v.full * ceilf(load));
 }
 
-int launch_variant(int i, const GemmCall& g, cudaStream_t stream) {
+int launch_variant(int i, const GemmCall& g, int width, cudaStream_t stream) {
     switch (i) {
-        case 0: return launch_gemm_pair<256>(g, stream);
+        case 0: return launch_gemm_pair<256>(g, width, stream);
         case 1: return launch_gemm<256>(g, stream);
         case 2: return launch_gemm<128>(g, stream);
         case 3: return launch_gemm<64>(g, stream);
@@ -696,17 +729,17 @@ int launch_gemm_call(const GemmCall& call, cudaStream_t stream) {
     if (!g.a_mn && !g.b_mn && g.epilogue <= GEMM_ADD && g.k >= 16 * GK && 2 * ((g.m + GM - 1) / GM) * ((g.n + 31) / 32) <= sms &&
         g.lda == g.k && g.ldb == g.k && g.ldc == g.n && (g.epilogue != GEMM_ADD || g.aux == g.c))
         return launch_rows_tc(g.dtype, g.m, g.n, g.k, g.a, g.b, g.bias, g.c, g.epilogue, stream, g.chain & kChainDependent);
-    int best = -1;
+    int best = -1, width = 256;
     float least = 0.f;
     for (int i = 0; i < 5; ++i) {
         if ((g.a_mn || g.b_mn) && (i == 1 || i == 4)) continue;  // built for the layouts of a backward pass: 256 x 256, 128, 64
-        const float t = variant_cost(i, g, 1, sms);
+        const float t = variant_cost(i, g, 1, sms, &width);
         if (best < 0 || t < least) {
             best = i;
             least = t;
         }
     }
-    return launch_variant(best, g, stream);
+    return launch_variant(best, g, width, stream);
 }
 
 // A product with a long k and a small output (a weight gradient: k = rows of the batch): k is cut into as many ranges as
@@ -716,21 +749,23 @@ int launch_gemm_splitk(const GemmCall& call, size_t partial_bytes, int* splits, 
     GemmCall g = call;
     const int sms = sm_count();
     const size_t out = (size_t)g.m * g.n * sizeof(float);
-    int best = 0, best_s = 1;
+    int best = 0, best_s = 1, best_width = 256;
     float least = 0.f;
     for (int i = 0; i < 4; ++i) {
         if (i == 1) continue;
         for (int s = 1; s <= 32 && (s == 1 || (s * out <= partial_bytes && g.k >= s * 4 * GK)); ++s) {
-            const float t = variant_cost(i, g, s, sms) + (s > 1 ? 2.5f + 2.f * (float)(s * out) / 4e6f : 0.f);
+            int width = 256;
+            const float t = variant_cost(i, g, s, sms, &width) + (s > 1 ? 2.5f + 2.f * (float)(s * out) / 4e6f : 0.f);
             if ((i == 0 && s == 1) || t < least) {
                 best = i;
                 best_s = s;
+                best_width = width;
                 least = t;
             }
         }
     }
     *splits = g.splits = best_s;
-    return launch_variant(best, g, stream);
+    return launch_variant(best, g, best_width, stream);
 }
 
 int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c, cudaStream_t stream,
