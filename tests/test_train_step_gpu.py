@@ -51,9 +51,10 @@ def test_training_step_equals_module_by_module(B, T, dtype, heads, dh, window, N
 
     def step():
         model.zero_grad(set_to_none=True)
-        out = model(ids, labels=labels)
-        if T > 1:
-            (out["loss"] * scale).backward()
+        with torch.enable_grad():  # (other tests may have turned it off)
+            out = model(ids, labels=labels)
+            if T > 1:
+                (out["loss"] * scale).backward()
         return out["loss"].detach(), out["logits"].detach(), {n: p.grad for n, p in model.named_parameters()}
 
     loss, logits, grads = step()

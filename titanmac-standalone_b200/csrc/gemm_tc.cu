@@ -30,8 +30,14 @@ using namespace ptx;
 constexpr int GM = 128;        // rows of an output tile
 constexpr int GK = 64;         // K elements per stage: one 128-byte swizzle row
 constexpr int kPanel = 32;     // columns per staging panel of the output (64 bytes, 64-byte swizzle)
+constexpr int kSlot = 32 * 64; // a warp's 32 rows of a panel
 constexpr int kEpiWarps = 8;
 constexpr int kGemmThreads = 32 * (2 + kEpiWarps);
+// The pair kernel's tiles are ready every 4 to 5 us at K = 640; with GELU the epilogue of one is 128 x 256 x 24 instructions a
+// CTA.  16416 x 2560 x 640 with GELU, us: 75 with eight warps behind block-wide barriers, 72 with sixteen, 58 with sixteen that
+// store their panels themselves and do not wait for one another (QKV, N = 1920, no epilogue: 42 -> 38).
+constexpr int kPairEpiWarps = 16;
+constexpr int kPairThreads = 32 * (2 + kPairEpiWarps);
 
 template <int BN>
 struct GemmSmem {
@@ -41,7 +47,7 @@ struct GemmSmem {
     static constexpr int kStageA = kSlices * GM * GK * 2;
     static constexpr int kStageB = kSlices * BN * GK * 2;
     static constexpr int kStage = kStageA + kStageB;
-    static constexpr int kOut = GM * BN * 2;  // staging of one output tile: BN / 32 panels of 128 rows x 64 bytes
+    static constexpr int kOut = kEpiWarps * 2 * kSlot;
     static constexpr int kStages = (232448 - 2048 - kOut) / kStage;
     static constexpr int kBars = kStages * kStage + kOut;  // offset of the barrier area
     static constexpr int kTotal = kBars + 1024 + 1024;     // barriers, alignment slack
@@ -60,17 +66,51 @@ struct GemmParams {
     int* status;
 };
 
-// 32 accumulator columns of one row -> the values to be stored (bias, then the epilogue)
 template <bool BF16>
-__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, int row, int col) {
+__device__ __forceinline__ uint4 pack8(const float* v) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (BF16) {
+            const __nv_bfloat162 hh = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
+        } else {
+            const __half2 hh = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
+        }
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// What the epilogue of a panel (a warp's 32 rows x 32 columns) reads beside the accumulator (GEMM_ADD, GEMM_GELU_GRAD):
+// columns 8 (lane & 3) .. + 8 of rows 8 i + lane / 4, whole sectors per warp.  Asked for before the accumulator is waited for.
+struct PanelAux { uint4 v[4]; };
+
+__device__ __forceinline__ void load_aux(PanelAux& in, const GemmParams& p, int row0, int col, int lane) {
+    if (p.epilogue != GEMM_ADD && p.epilogue != GEMM_GELU_GRAD) return;
+    const int c = col + (lane & 3) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = row0 + i * 8 + (lane >> 2);
+        in.v[i] = r < p.m && c < p.n ? *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.aux) + (long long)r * p.n + c)
+                                     : make_uint4(0, 0, 0, 0);
+    }
+}
+
+// 32 accumulator columns of one row per lane -> bias, epilogue, the warp's 32 rows of the staging panel (64-byte swizzle).
+// `aux` passes through the same rows of the panel, so that global memory sees whole 64-byte runs: one row per lane there
+// made the epilogue longer than the product (8320 x 2560 x 640, us: GELU_KEEP 62.6, GELU_GRAD 73, no epilogue 28.5).
+template <bool BF16>
+__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, const PanelAux& in, uint8_t* stage, int row0,
+                                             int col, int lane) {
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+    auto slot = [&](int r, int c) { return reinterpret_cast<uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) * 16)); };
     if (p.bias != nullptr) {
-        // bias of 32 columns: 64 bytes, the same for every row (broadcast loads)
 #pragma unroll
         for (int j = 0; j < 32; j += 8)
             if (col + j < p.n) {  // n is a multiple of 8
                 float b8[8];
-                load8<T>(static_cast<const T*>(p.bias) + col + j, b8);
+                load8<T>(static_cast<const T*>(p.bias) + col + j, b8);  // (the same for every lane)
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
             }
@@ -78,26 +118,43 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
     if (p.epilogue == GEMM_GELU) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
-    } else if (p.epilogue > GEMM_GELU && row < p.m) {
-        T* aux = static_cast<T*>(p.aux) + (long long)row * p.n + col;
+    } else if (p.epilogue == GEMM_GELU_KEEP) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 8)
-            if (col + j < p.n) {
-                float x[8];
-                if (p.epilogue == GEMM_GELU_KEEP) {
+        for (int c = 0; c < 4; ++c) {
+            const uint4 raw = pack8<BF16>(v + 8 * c);
+            *slot(lane, c) = raw;
+            float x[8];
+            load8<T>(reinterpret_cast<const T*>(&raw), x);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) x[e] = to_f32<T>(from_f32<T>(v[j + e]));
-                    store8<T>(aux + j, x);
+            for (int e = 0; e < 8; ++e) v[8 * c + e] = gelu_erf(x[e]);
+        }
+        __syncwarp();
+        const int c = lane & 3;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[j + e] = gelu_erf(x[e]);
-                } else {
-                    load8<T>(aux + j, x);
+        for (int i = 0; i < 4; ++i) {
+            const int r = i * 8 + (lane >> 2);
+            if (row0 + r < p.m && col + c * 8 < p.n)
+                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.aux) + (long long)(row0 + r) * p.n + col + c * 8) = *slot(r, c);
+        }
+        __syncwarp();
+    } else if (p.epilogue != GEMM_NONE) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        v[j + e] = p.epilogue == GEMM_ADD ? x[e] + to_f32<T>(from_f32<T>(v[j + e])) : v[j + e] * gelu_slope(x[e]);
-                }
+        for (int i = 0; i < 4; ++i) *slot(i * 8 + (lane >> 2), lane & 3) = in.v[i];
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint4 raw = *slot(lane, c);
+            float x[8];
+            load8<T>(reinterpret_cast<const T*>(&raw), x);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float& y = v[8 * c + e];
+                y = p.epilogue == GEMM_ADD ? x[e] + to_f32<T>(from_f32<T>(y)) : y * gelu_slope(x[e]);
             }
+        }
     }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) *slot(lane, c) = pack8<BF16>(v + 8 * c);
 }
 
 // the fp32 sums of a k range
@@ -107,6 +164,46 @@ __device__ __forceinline__ void store_partial(const float (&v)[32], const GemmPa
 #pragma unroll
     for (int j = 0; j < 32; j += 4)
         if (col + j < p.n) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+}
+
+// A warp's panels (first, first + step, ...) of a finished tile: tensor memory -> the warp's own staging -> TMA store (or, with
+// k cut, fp32 sums to memory).  No warp waits for another: a panel goes out as soon as it is finished, from one of two
+// staging slots of the warp, and a slot is taken again when its last store has read it.  `in` holds the inputs of the first
+// panel; `all_read` is called once the accumulator has been read; `count`: panels that the warp has stored.
+template <bool BF16, typename F>
+__device__ __forceinline__ void epilogue_panels(const GemmParams& p, const CUtensorMap* map_c, PanelAux& in, uint32_t t_addr,
+                                                uint8_t* slots, int& count, int row0, int col0, int first, int panels, int step,
+                                                int split, int lane, F all_read) {
+    if (first >= panels) all_read();
+    for (int pn = first; pn < panels; pn += step) {
+        const int col = col0 + pn * kPanel;
+        uint32_t acc[32];
+        tmem_ld32(t_addr + pn * kPanel, acc);
+        tc_wait_ld();
+        if (pn + step >= panels) {
+            tc_fence_before();
+            __syncwarp();
+            all_read();
+        }
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
+        if (p.partial != nullptr) {
+            store_partial(v, p, split, row0 + lane, col);
+            continue;
+        }
+        uint8_t* stage = slots + (count++ & 1) * kSlot;
+        if (lane == 0) tma_store_wait_read_but_one();
+        __syncwarp();
+        finish_panel<BF16>(v, p, in, stage, row0, col, lane);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            if (row0 < p.m && col < p.n) tma_store_2d(map_c, smem_u32(stage), col, row0);
+            tma_store_commit();
+        }
+        if (pn + step < panels) load_aux(in, p, row0, col + step * kPanel, lane);
+    }
 }
 
 // An operand tile of R rows (of the product: M or N) x 64 k-elements in shared memory, 128 bytes per swizzled row.
@@ -236,72 +333,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else {
         // ---------------- epilogue ----------------
         const int g = warp & 3;             // lane group of tensor memory this warp may read
-        const int half = (warp - 2) >> 2;   // column half
-        const int row = g * 32 + lane;      // row of the tile
+        const int sub = (warp - 2) >> 2;    // its first panel
         constexpr int kPanels = BN / kPanel;
-        constexpr int kHalfPanels = (kPanels + 1) / 2;  // panels of the first half (the second gets the rest)
-        const int panel0 = half == 0 ? 0 : kHalfPanels;
-        const int panel1 = half == 0 ? kHalfPanels : kPanels;
-        uint8_t* stage = smem + S * L::kStage;
-        const bool epi_leader = warp == 2 && lane == 0;
-        int t = 0;
+        uint8_t* slots = smem + S * L::kStage + (warp - 2) * 2 * kSlot;
+        int t = 0, count = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
             const int buf = t & 1;
             const int mn = tile / p.splits, row0 = (mn / n_tiles) * GM, col0 = (mn % n_tiles) * BN;
+            PanelAux in;
+            if (sub < kPanels) load_aux(in, p, row0 + g * 32, col0 + sub * kPanel, lane);
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            // the previous tile's store must have read the staging buffer before it is overwritten
-            if (epi_leader) tma_store_wait_read();
-            named_barrier_sync(1, kEpiWarps * 32);
-            const uint32_t t_addr = tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN;
-            if (panel0 == panel1 && lane == 0) mbar_arrive(acc_empty(buf));  // a tile of one panel: nothing to read
-            for (int pn = panel0; pn < panel1; ++pn) {
-                uint32_t acc[32];
-                tmem_ld32(t_addr + pn * kPanel, acc);
-                tc_wait_ld();
-                if (pn == panel1 - 1) {
-                    // this warp has read all of its columns: hand the accumulator back
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty(buf));
-                }
-                const int col = col0 + pn * kPanel;  // first column of the panel
-                float v[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-                if (p.partial != nullptr) {
-                    store_partial(v, p, tile % p.splits, row0 + row, col);
-                    continue;
-                }
-                finish_panel<BF16>(v, p, row0 + row, col);
-                // 32 columns = 64 bytes = four 16-byte chunks of this row in panel pn (64-byte swizzle)
-                uint8_t* prow = stage + pn * (GM * 64) + row * 64;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (BF16) {
-                            const __nv_bfloat162 hh = __floats2bfloat162_rn(v[c * 8 + 2 * e], v[c * 8 + 2 * e + 1]);
-                            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
-                        } else {
-                            const __half2 hh = __floats2half2_rn(v[c * 8 + 2 * e], v[c * 8 + 2 * e + 1]);
-                            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
-                        }
-                    }
-                    *reinterpret_cast<uint4*>(prow + ((c ^ ((row >> 1) & 3)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            }
-            fence_proxy_async_smem();
-            named_barrier_sync(2, kEpiWarps * 32);
-            if (epi_leader && p.partial == nullptr) {
-                for (int pn = 0; pn < kPanels; ++pn)
-                    if (col0 + pn * kPanel < p.n)
-                        tma_store_2d(&map_c, smem_u32(stage + pn * (GM * 64)), col0 + pn * kPanel, row0);
-                tma_store_commit();
-            }
+            epilogue_panels<BF16>(p, &map_c, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, slots, count, row0 + g * 32, col0,
+                                  sub, kPanels, kEpiWarps / 4, tile % p.splits, lane,
+                                  [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
         }
-        if (epi_leader) {
+        if (lane == 0) {
             if (p.drain) tma_store_wait_all();
             else tma_store_wait_read();  // (the stores themselves complete with the grid)
         }
@@ -334,7 +381,7 @@ struct PairSmem {
     static constexpr int kStageA = GM * GK * 2;
     static constexpr int kStageB = (BN / 2) * GK * 2;
     static constexpr int kStage = kStageA + kStageB;
-    static constexpr int kOut = GM * BN * 2;
+    static constexpr int kOut = kPairEpiWarps * 2 * kSlot;
     static constexpr int kStages = (232448 - 2048 - kOut) / kStage;
     static constexpr int kBars = kStages * kStage + kOut;
     static constexpr int kTotal = kBars + 1024 + 1024;
@@ -343,7 +390,7 @@ struct PairSmem {
 };
 
 template <int BN, bool BF16, bool AMN, bool BMN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
     using L = PairSmem<BN>;
@@ -390,7 +437,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(acc_full(b), 1);
-            mbar_init(acc_empty(b), 2 * kEpiWarps);  // the epilogue warps of both CTAs
+            mbar_init(acc_empty(b), 2 * kPairEpiWarps);  // the epilogue warps of both CTAs
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -473,71 +520,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else {
         // ---------------- epilogue (both CTAs, each its own 128 rows) ----------------
         const int g = warp & 3;
-        const int half = (warp - 2) >> 2;
-        const int row = g * 32 + lane;
-        uint8_t* stage = smem + S * L::kStage;
-        const bool epi_leader = warp == 2 && lane == 0;
-        int t = 0;
+        const int sub = (warp - 2) >> 2;
+        uint8_t* slots = smem + S * L::kStage + (warp - 2) * 2 * kSlot;
+        int t = 0, count = 0;
         for (int tile = pair; tile < tiles; tile += pairs, ++t) {
             const int buf = t & 1;
             int band, col0;
             locate(tile, band, col0);
             const int row0 = band * (2 * GM) + (int)rank * GM;
-            // the tile's panels of 32 columns, split between the two warps of a lane group
-            const int panels = columns(col0) / kPanel, half_panels = (panels + 1) / 2;
-            const int panel0 = half == 0 ? 0 : half_panels;
-            const int panel1 = half == 0 ? half_panels : panels;
+            const int panels = columns(col0) / kPanel;
+            PanelAux in;
+            if (sub < panels) load_aux(in, p, row0 + g * 32, col0 + sub * kPanel, lane);
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            if (epi_leader) tma_store_wait_read();
-            named_barrier_sync(1, kEpiWarps * 32);
-            const uint32_t t_addr = tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN;
-            if (panel0 == panel1 && lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0));
-            for (int pn = panel0; pn < panel1; ++pn) {
-                uint32_t acc[32];
-                tmem_ld32(t_addr + pn * kPanel, acc);
-                tc_wait_ld();
-                if (pn == panel1 - 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0));
-                }
-                const int col = col0 + pn * kPanel;
-                float v[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-                if (p.partial != nullptr) {
-                    store_partial(v, p, tile % p.splits, row0 + row, col);
-                    continue;
-                }
-                finish_panel<BF16>(v, p, row0 + row, col);
-                uint8_t* prow = stage + pn * (GM * 64) + row * 64;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (BF16) {
-                            const __nv_bfloat162 hh = __floats2bfloat162_rn(v[c * 8 + 2 * e], v[c * 8 + 2 * e + 1]);
-                            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
-                        } else {
-                            const __half2 hh = __floats2half2_rn(v[c * 8 + 2 * e], v[c * 8 + 2 * e + 1]);
-                            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
-                        }
-                    }
-                    *reinterpret_cast<uint4*>(prow + ((c ^ ((row >> 1) & 3)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            }
-            fence_proxy_async_smem();
-            named_barrier_sync(2, kEpiWarps * 32);
-            if (epi_leader && row0 < p.m && p.partial == nullptr) {
-                for (int pn = 0; pn < panels; ++pn)
-                    if (col0 + pn * kPanel < p.n)
-                        tma_store_2d(&map_c, smem_u32(stage + pn * (GM * 64)), col0 + pn * kPanel, row0);
-                tma_store_commit();
-            }
+            epilogue_panels<BF16>(p, &map_c, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, slots, count, row0 + g * 32, col0,
+                                  sub, panels, kPairEpiWarps / 4, tile % p.splits, lane,
+                                  [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
         }
-        if (epi_leader) {
+        if (lane == 0) {
             if (p.drain) tma_store_wait_all();
             else tma_store_wait_read();  // (the stores themselves complete with the grid)
         }
@@ -564,7 +564,7 @@ bool make_maps(const GemmCall& g, int b_rows, CUtensorMap* ma, CUtensorMap* mb, 
     return (g.a_mn ? make_map_2d(ma, g.a, g.dtype, g.k, g.m, g.lda, GK, 64, sw) : make_map_2d(ma, g.a, g.dtype, g.m, g.k, g.lda, GM, GK, sw)) &&
            (g.b_mn ? make_map_2d(mb, g.b, g.dtype, g.k, g.n, g.ldb, GK, 64, sw)
                    : make_map_2d(mb, g.b, g.dtype, g.n, g.k, g.ldb, b_rows, GK, sw)) &&
-           make_map_2d(mc, g.c, g.dtype, g.m, g.n, g.ldc, GM, kPanel, CU_TENSOR_MAP_SWIZZLE_64B);
+           make_map_2d(mc, g.c, g.dtype, g.m, g.n, g.ldc, 32, kPanel, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 int gemm_params(const GemmCall& g, GemmParams* p) {
@@ -629,7 +629,7 @@ int max_active_pairs(const void* kern, int smem_bytes) {
     if (e != nullptr && e->pairs[dev] > 0) return e->pairs[dev];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.blockDim = dim3(kPairThreads, 1, 1);
     cfg.dynamicSmemBytes = smem_bytes;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
@@ -655,7 +655,7 @@ int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
         if (rc != TMW_OK) return rc;
         const int resident = max_active_pairs(fn, L::kTotal);
         const int pairs = tiles < resident ? tiles : resident;
-        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kGemmThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, mc, p));
+        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kPairThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, mc, p));
         return TMW_OK;
     };
     return g.dtype == TMW_BF16

@@ -90,31 +90,39 @@ __device__ __forceinline__ void store8<__half>(__half* p, const float (&in)[8]) 
 }
 
 // Exact (erf-based) GELU, 0.5 x (1 + erf(x / sqrt 2)), with erf from the rational approximation 7.1.26 of
-// Abramowitz & Stegun (absolute error below 1.5e-7, i.e. fp32 rounding noise against a 16-bit result): one reciprocal,
-// one exponential and a degree-5 polynomial instead of the library's branchy erff, which is longer than the products
-// or loads it sits behind.
+// Abramowitz & Stegun (absolute error below 1.5e-7, i.e. fp32 rounding noise against a 16-bit result): with z = |x| / sqrt 2
+// and t = 1 / (1 + 0.3275911 z), erf(z) = 1 - Q(t) t exp(-z^2).  In the product's epilogue this is the longest part, so the
+// result is put together from 1 - erf, max(x, 0) - |x| / 2 (1 - erf), and the reciprocal (of 1 or more) and the exponential
+// (zero below 2^-126) take the forms without the care for subnormal numbers: 16416 x 2560 x 640 with GELU, 87 -> 75 us.
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// Q(t) t / 2 and exp(-x^2 / 2)
+__device__ __forceinline__ float half_erfc_poly(float x) {
+    const float t = rcp_ftz(fmaf(0.3275911f * 0.70710678118654752f, fabsf(x), 1.0f));
+    float poly = fmaf(0.5f * 1.061405429f, t, 0.5f * -1.453152027f);
+    poly = fmaf(poly, t, 0.5f * 1.421413741f);
+    poly = fmaf(poly, t, 0.5f * -0.284496736f);
+    poly = fmaf(poly, t, 0.5f * 0.254829592f);
+    return poly * t;
+}
+__device__ __forceinline__ float gauss(float x) { return ex2_ftz(x * -0.72134752044448170f * x); }
 __device__ __forceinline__ float gelu_erf(float x) {
-    const float z = fabsf(x) * 0.70710678118654752f;
-    const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
-    float poly = fmaf(1.061405429f, t, -1.453152027f);
-    poly = fmaf(poly, t, 1.421413741f);
-    poly = fmaf(poly, t, -0.284496736f);
-    poly = fmaf(poly, t, 0.254829592f);
-    const float erf_abs = 1.0f - poly * t * __expf(-z * z);  // erf(|x| / sqrt 2)
-    return 0.5f * x * (1.0f + copysignf(erf_abs, x));
+    // (beyond 16 the exponential is zero: the bound keeps infinity times zero out)
+    return fmaf(-fminf(fabsf(x), 16.0f) * half_erfc_poly(x), gauss(x), fmaxf(x, 0.0f));
 }
 
 // derivative of gelu_erf: Phi(x) + x phi(x)
 __device__ __forceinline__ float gelu_slope(float x) {
-    const float z = fabsf(x) * 0.70710678118654752f;
-    const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
-    float poly = fmaf(1.061405429f, t, -1.453152027f);
-    poly = fmaf(poly, t, 1.421413741f);
-    poly = fmaf(poly, t, -0.284496736f);
-    poly = fmaf(poly, t, 0.254829592f);
-    const float e = __expf(-z * z);  // exp(-x^2 / 2)
-    const float erf_abs = 1.0f - poly * t * e;
-    return 0.5f * (1.0f + copysignf(erf_abs, x)) + 0.3989422804014327f * x * e;
+    const float odd = fmaf(0.3989422804014327f, x, -copysignf(half_erfc_poly(x), x));
+    return fmaf(gauss(x), odd, x > 0.0f ? 1.0f : 0.0f);
 }
 
 __host__ __device__ inline size_t dtype_size(int dtype) { return dtype == TMW_F32 ? 4 : 2; }
