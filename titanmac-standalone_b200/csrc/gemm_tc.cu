@@ -376,6 +376,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // loads; "empty" and "accumulator full" are arrived on in both CTAs by one commit; "accumulator empty" lives in
 // the first CTA and collects the epilogue warps of both.
 // ---------------------------------------------------------------------------------
+// Wide outputs are walked in groups of kGroup row bands, column by column: the tiles in flight then share few rows of W as well
+// as of A (a vocabulary's W is read m / 256 times otherwise, and does not stay in the near half of L2).
+constexpr int kGroup = 8, kGroupFrom = 16;
+
 template <int BN>
 struct PairSmem {
     static constexpr int kStageA = GM * GK * 2;
@@ -418,8 +422,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int k_blocks = (p.k + GK - 1) / GK;
     auto locate = [&](int tile, int& band, int& col) {  // its band of 256 rows and first column
         const int mn = tile / p.splits;
-        band = mn / n_tiles;
-        col = (mn % n_tiles) * p.width;
+        if (n_tiles < kGroupFrom) {
+            band = mn / n_tiles;
+            col = (mn % n_tiles) * p.width;
+        } else {
+            const int first = mn / (kGroup * n_tiles) * kGroup, r = mn - first * n_tiles, bands = min(kGroup, m_tiles - first);
+            band = first + r % bands;
+            col = r / bands * p.width;
+        }
     };
     // columns a tile multiplies: its width, or for the last tile of a row what is left of N (in steps of 32) - a product
     // over columns that do not exist would cost its full time
