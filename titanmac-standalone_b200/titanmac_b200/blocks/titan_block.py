@@ -5,7 +5,8 @@ blocks/mlp.py:28-67 of the reference (same submodule names, so checkpoints load
 unchanged).  The attention is this package's own code, and so is the element-wise work around
 it on a GPU: RMSNorm with the preceding residual add folded in is one kernel
 (``tmw_add_rmsnorm``); the linears are the library's tensor-core product ``tmw_linear`` with bias and the exact GELU
-in its epilogue (a decode step's few rows: library GEMM plus the one-pass ``tmw_gelu``).
+in its epilogue (few rows, module by module: library GEMM plus the one-pass ``tmw_gelu``; a model's decode step is
+``tmw_decode_step``).
 ``use_block_sparse`` selects the attention class exactly as in the reference.
 Under ``torch.no_grad()`` the fused kernels run; with grad mode on, norm and GELU fall back to the
 differentiable PyTorch formulas and the windowed attention core uses its own backward kernel.
@@ -65,7 +66,7 @@ class MLPBlock(nn.Module):
         if torch.is_grad_enabled() and (x.requires_grad or self.fc1.weight.requires_grad):
             return self.dropout(self.fc2(self.activation(self.fc1(x))))
         # inference: bias and the exact-erf GELU ride in the epilogue of the library's tensor-core product
-        # (tmw_linear); few rows (a decode step) take the library GEMM and the one-pass GELU kernel
+        # (tmw_linear); few rows take the library GEMM and the one-pass GELU kernel
         h = _native.project(self.fc1, x, gelu=True)
         return self.dropout(_native.project(self.fc2, h))
 
