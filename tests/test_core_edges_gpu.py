@@ -42,24 +42,3 @@ def test_block_sparse_core_with_persistent_rows(dtype, tol, dh, L, w, block, n_p
     o = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), w, n_p, window_block=block)
     _native.poll_status()
     assert (o.float().cpu() - ref).abs().max().item() <= tol
-
-
-@pytest.mark.parametrize("dh,L,w,block,n_p", [(64, 2100, 64, 0, 16), (128, 1665, 100, 0, 1), (64, 1500, 96, 32, 16), (128, 1300, 64, 64, 40),
-                                              (64, 129, 8, 0, 3)])
-def test_backward_with_a_shared_walk_of_the_persistent_tile(dh, L, w, block, n_p):
-    """One (batch, head) and a long sequence: several CTAs share the row tile that meets every column tile."""
-    q, k, v = (t.to(torch.bfloat16).to(DEV) for t in wo.qkv_inputs(1, 2, L, dh, seed=L))
-    d_o = torch.randn(1, 2, L, dh, generator=torch.Generator().manual_seed(L)).to(torch.bfloat16).to(DEV)
-    lse = torch.empty(1, 2, L, device=DEV)
-    o = torch.empty_like(q)
-    _native.prefill(q, k, v, w, n_p, out=o, lse=lse, window_block=block)
-    grads = []
-    for algo in (_native.ALGO_AUTO, _native.ALGO_SIMT):
-        g = [torch.full_like(q, float("nan")) for _ in range(3)]
-        _native.prefill_backward(q, k, v, o, d_o, lse, *g, w, n_p, algo=algo, window_block=block)
-        grads.append(g)
-    _native.poll_status()
-    for a, b in zip(*grads):
-        a, b = a.float(), b.float()
-        for rows in (slice(None), slice(0, n_p)):
-            assert (a[:, :, rows] - b[:, :, rows]).norm().item() <= 1e-2 * b[:, :, rows].norm().item() + 1e-4

@@ -60,12 +60,7 @@ struct BwdParams {
     // rows of O and dO per column.
     float* stats;
     int rows_pad;
-    int n_bx, heads, batch;      // row tiles per (batch, head); grid = (n_bx + splits - 1) * heads * batch
-    // The row tile with the persistent rows interacts with every column tile.  Where that walk would be longer than the rest
-    // of the launch takes, `splits` CTAs share it and leave fp32 sums in part [batch * heads][splits][2][128][head_dim],
-    // which merge_parts_kernel adds up in a fixed order.
-    int splits;
-    float* part;
+    int n_bx, heads, batch;      // row tiles per (batch, head); grid = n_bx * heads * batch
     // The mask of the block-sparse class (kernels instantiated with GENERAL): block > 0 moves the left edge of a
     // query's window in steps of `block` rows (first_visible_pos), and the persistent QUERY rows see every key;
     // lse then comes in two planes, [batch, heads, rows - np] for the sequence rows and, at lse_pers,
@@ -156,8 +151,7 @@ __device__ __forceinline__ ColPlan col_plan(int r0, int L, int w, int np, int bl
     return c;
 }
 
-// SHARED: the walk of the first row tile may be cut (p.splits); a kernel of its own, which the others' registers do not pay for
-template <int DH, bool BF16, bool ROWS_ARE_KEYS, bool GENERAL, bool SHARED>
+template <int DH, bool BF16, bool ROWS_ARE_KEYS, bool GENERAL>
 __global__ void __launch_bounds__(kBwdThreads, Geo<DH>::kCtasPerSm)
 bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant__ CUtensorMap map_r2,
               const __grid_constant__ CUtensorMap map_c1, const __grid_constant__ CUtensorMap map_c2,
@@ -180,8 +174,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
     float* vec = reinterpret_cast<float*>(smem + L::kVec);  // [stage][lse | D][column]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int seg = 0;
-    bool shared_walk = false;
     // One-dimensional grid.  The row tile that holds the persistent keys walks over EVERY query tile (all queries
     // see those keys), several times the work of any other tile: those CTAs get the first block indices, so they
     // start first and the short ones fill in around them instead of the long ones forming the tail of the launch.
@@ -190,9 +182,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         const int n_bh = p.heads * p.batch;
         int id = (int)blockIdx.x, bh;
         if ((ROWS_ARE_KEYS || GENERAL) && p.np > 0 && p.n_bx > 1) {
-            const int firsts = SHARED ? n_bh * p.splits : n_bh;
-            if (id < firsts) { tile_x = 0; bh = SHARED ? id % n_bh : id; seg = SHARED ? id / n_bh : 0; shared_walk = SHARED; }
-            else { id -= firsts; tile_x = 1 + id % (p.n_bx - 1); bh = id / (p.n_bx - 1); }
+            if (id < n_bh) { tile_x = 0; bh = id; }
+            else { id -= n_bh; tile_x = 1 + id % (p.n_bx - 1); bh = id / (p.n_bx - 1); }
         } else {
             tile_x = id % p.n_bx;
             bh = id / p.n_bx;
@@ -202,12 +193,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
     }
     const int r0 = tile_x * BT;
     const int wblock = GENERAL ? p.block : 0;
-    ColPlan plan = col_plan<ROWS_ARE_KEYS, CW>(r0, p.rows, p.window, p.np, wblock);
-    if (SHARED && shared_walk) {  // (one segment: every column tile)
-        const int n = plan.n0;
-        plan.a0 = (int)((long long)n * seg / p.splits);
-        plan.n0 = (int)((long long)n * (seg + 1) / p.splits) - plan.a0;
-    }
+    const ColPlan plan = col_plan<ROWS_ARE_KEYS, CW>(r0, p.rows, p.window, p.np, wblock);
     const int n_cols = plan.n0 + plan.n1;
     auto col_tile = [&](int n) -> int { return n < plan.n0 ? plan.a0 + n : plan.a1 + (n - plan.n0); };
     // coordinate order of a tensor map: (dh, rows, heads, batch) or (dh, heads, rows, batch)
@@ -527,14 +513,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
                 const int col0 = half * (DH / 2) + c * 16;
                 tmem_ld16(t_row + (which == 0 ? kAcc1 : kAcc2) + col0, o);
                 tc_wait_ld();
-                if (SHARED && shared_walk) {
-                    float* dst = p.part + (((bh * p.splits + seg) * 2 + which) * BT + row) * DH + col0;
-#pragma unroll
-                    for (int e = 0; e < 16; e += 4)
-                        *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(o[e]), __uint_as_float(o[e + 1]),
-                                                                          __uint_as_float(o[e + 2]), __uint_as_float(o[e + 3]));
-                    continue;
-                }
 #pragma unroll
                 for (int g8 = 0; g8 < 2; ++g8) {
                     uint32_t w[4];
@@ -558,7 +536,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         }
         fence_proxy_async_smem();
         named_barrier_sync(2, 2 * BT);
-        if (tid256 == 0 && !(SHARED && shared_walk)) {
+        if (tid256 == 0) {
             int c1, c2;
             coords(kO1, r0, c1, c2);
             for (int u = 0; u < NSUB; ++u)
@@ -586,54 +564,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
     }
 }
 
-// The first row tile's gradients from the sums of its `splits` CTAs; blockIdx.y: 0 = dV or dQ, 1 = dK
-struct MergeParts {
-    const float* part;
-    void* dst[2];
-    long long stride[2][3];  // {batch, head, row}, elements
-    float mul[2];
-    int rows, heads, splits;
-};
-
-template <int DH, bool BF16>
-__global__ void __launch_bounds__(256) merge_parts_kernel(const MergeParts p) {
-    using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
-    const int bh = blockIdx.x, which = blockIdx.y, batch = bh / p.heads, head = bh % p.heads;
-    T* out = static_cast<T*>(p.dst[which]) + batch * p.stride[which][0] + head * p.stride[which][1];
-    const float* src = p.part + ((long long)bh * p.splits * 2 + which) * BT * DH;
-    for (int i = threadIdx.x; i < BT * DH / 8; i += 256) {
-        const int row = i / (DH / 8), col = i % (DH / 8) * 8;
-        if (row >= p.rows) break;
-        float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int s = 0; s < p.splits; ++s) {
-            float v[8];
-            load8<float>(src + (long long)s * 2 * BT * DH + row * DH + col, v);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sum[e] += v[e];
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sum[e] *= p.mul[which];
-        store8<T>(out + row * p.stride[which][2] + col, sum);
-    }
-}
-
 // ---------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------
-// CTAs for the row tile that walks over every column tile: as many as bring its walk down to what the other CTAs of a slot
-// take together, or to another tile's own walk.  Backward in all, 10 heads x
-// 64, window 512, us: 4112 rows 111 -> 80, 16400 rows 376 -> 195; at batch 8 the walk is shorter than the rest and stays whole.
-int shared_walk_ctas(const tmw_prefill_desc& d, int cw, int slots, int window_block) {
-    const long long n_bh = (long long)d.batch * d.heads, tiles = (d.q_rows + BT - 1) / BT, walk = (d.q_rows + cw - 1) / cw;
-    if (d.n_persistent == 0 || tiles <= 1) return 1;
-    const long long span = d.window < d.q_rows ? d.window : d.q_rows;
-    long long own = (span + window_block + BT) / cw + 1;
-    own = own < walk ? own : walk;
-    const long long rest = (n_bh * ((tiles - 1) * own + walk)) / slots;
-    const long long goal = rest > own ? rest : own, splits = (walk + goal - 1) / goal;
-    return (int)(splits < 1 ? 1 : splits > 16 ? 16 : splits);
-}
-
 // Stream-ordered scratch memory comes from a pool of the library's own (one per device, created on first use,
 // kept for the life of the process): freed blocks stay in the pool, so a call costs no trip to the driver's
 // allocator after the first, and the device's default pool and its settings are left alone.
@@ -701,56 +634,33 @@ int launch_bwd_tc(const tmw_prefill_desc& d, const void* q, const void* k, const
     {
         void* mem = nullptr;
         cudaMemPool_t pool = scratch_pool();
-        p.splits = shared_walk_ctas(d, CW, sm_count() * Geo<DH>::kCtasPerSm, window_block);
-        const size_t stats = (size_t)B * H * 2 * p.rows_pad, parts = p.splits > 1 ? (size_t)B * H * p.splits * 2 * BT * DH : 0;
-        if (pool != nullptr && cudaMallocFromPoolAsync(&mem, (stats + parts) * sizeof(float), pool, stream) == cudaSuccess) {
+        if (pool != nullptr &&
+            cudaMallocFromPoolAsync(&mem, (size_t)B * H * 2 * p.rows_pad * sizeof(float), pool, stream) == cudaSuccess)
             p.stats = static_cast<float*>(mem);
-            p.part = p.stats + stats;  // (rows_pad is a multiple of 128: aligned)
-        } else {
+        else
             (void)cudaGetLastError();
-            p.splits = 1;
-        }
     }
     p.n_bx = (R + BT - 1) / BT; p.heads = H; p.batch = B;
+    const dim3 grid(p.n_bx * H * B, 1, 1);
     auto run = [&](auto kern, const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& c1, const CUtensorMap& c2,
-                   const CUtensorMap& o1, const CUtensorMap& o2, const BwdParams& p) -> int {
+                   const CUtensorMap& o1, const CUtensorMap& o2) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), L::kTotal);
         if (rc != TMW_OK) return rc;
-        kern<<<(p.n_bx + p.splits - 1) * H * B, kBwdThreads, L::kTotal, stream>>>(r1, r2, c1, c2, o1, o2, p);
+        kern<<<grid, kBwdThreads, L::kTotal, stream>>>(r1, r2, c1, c2, o1, o2, p);
         return TMW_OK;
     };
-    auto merge = [&](void* d0, const int64_t* s0, float mul0, void* d1, const int64_t* s1, int outputs) {
-        if (p.splits == 1) return;
-        MergeParts m;
-        m.part = p.part; m.rows = R < BT ? R : BT; m.heads = H; m.splits = p.splits;
-        m.dst[0] = d0; m.dst[1] = d1; m.mul[0] = mul0; m.mul[1] = p.scale;
-        for (int i = 0; i < 3; ++i) { m.stride[0][i] = s0[i]; m.stride[1][i] = s1[i]; }
-        if (d.dtype == TMW_BF16) merge_parts_kernel<DH, true><<<dim3(B * H, outputs), 256, 0, stream>>>(m);
-        else merge_parts_kernel<DH, false><<<dim3(B * H, outputs), 256, 0, stream>>>(m);
-    };
-    BwdParams first = p;  // dQ: only the persistent queries of the block-sparse class see everything
-    if (window_block == 0) first.splits = 1;
     // dQ first: rows are queries (Q, dO), columns are keys (K, V); it also leaves the rows' statistics
     const bool bf16 = d.dtype == TMW_BF16, general = window_block > 0;
-    auto run_first = [&](auto shared) -> int {
-        constexpr bool S = decltype(shared)::value;
-        return bf16 ? run(bwd_tc_kernel<DH, true, false, true, S>, mq, mdo, ck, cv, mdq, mdq, first)
-                    : run(bwd_tc_kernel<DH, false, false, true, S>, mq, mdo, ck, cv, mdq, mdq, first);
-    };
-    int st = !general ? (bf16 ? run(bwd_tc_kernel<DH, true, false, false, false>, mq, mdo, ck, cv, mdq, mdq, first)
-                              : run(bwd_tc_kernel<DH, false, false, false, false>, mq, mdo, ck, cv, mdq, mdq, first))
-             : p.splits > 1 ? run_first(std::true_type{}) : run_first(std::false_type{});
-    if (st == TMW_OK && window_block > 0) merge(dq, d.q_stride, p.scale, dq, d.q_stride, 1);
+    int st = general ? (bf16 ? run(bwd_tc_kernel<DH, true, false, true>, mq, mdo, ck, cv, mdq, mdq)
+                             : run(bwd_tc_kernel<DH, false, false, true>, mq, mdo, ck, cv, mdq, mdq))
+                     : (bf16 ? run(bwd_tc_kernel<DH, true, false, false>, mq, mdo, ck, cv, mdq, mdq)
+                             : run(bwd_tc_kernel<DH, false, false, false>, mq, mdo, ck, cv, mdq, mdq));
     // dK, dV: rows are keys (K, V), columns are queries (Q, dO)
-    auto run_second = [&](auto shared) -> int {
-        constexpr bool S = decltype(shared)::value;
-        return general ? (bf16 ? run(bwd_tc_kernel<DH, true, true, true, S>, mk, mv, cq, cdo, mdv, mdk, p)
-                               : run(bwd_tc_kernel<DH, false, true, true, S>, mk, mv, cq, cdo, mdv, mdk, p))
-                       : (bf16 ? run(bwd_tc_kernel<DH, true, true, false, S>, mk, mv, cq, cdo, mdv, mdk, p)
-                               : run(bwd_tc_kernel<DH, false, true, false, S>, mk, mv, cq, cdo, mdv, mdk, p));
-    };
-    if (st == TMW_OK) st = p.splits > 1 ? run_second(std::true_type{}) : run_second(std::false_type{});
-    if (st == TMW_OK) merge(dv, d.v_stride, 1.0f, dk, d.k_stride, 2);
+    if (st == TMW_OK)
+        st = general ? (bf16 ? run(bwd_tc_kernel<DH, true, true, true>, mk, mv, cq, cdo, mdv, mdk)
+                             : run(bwd_tc_kernel<DH, false, true, true>, mk, mv, cq, cdo, mdv, mdk))
+                     : (bf16 ? run(bwd_tc_kernel<DH, true, true, false>, mk, mv, cq, cdo, mdv, mdk)
+                             : run(bwd_tc_kernel<DH, false, true, false>, mk, mv, cq, cdo, mdv, mdk));
     const cudaError_t launched = cudaGetLastError();
     if (p.stats != nullptr) (void)cudaFreeAsync(p.stats, stream);
     if (st != TMW_OK) return st;
