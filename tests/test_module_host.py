@@ -4,7 +4,7 @@ compatibility and the exceptions the reference raises in the same situations."""
 import pytest
 import torch
 
-from titanmac_b200 import TitanMACConfig, WindowConfig, WindowedAttention, _native
+from titanmac_b200 import BlockSparseAttention, TitanMACConfig, WindowConfig, WindowedAttention, _native, _stack
 
 
 def test_constructor_accepts_both_config_kinds():
@@ -63,3 +63,40 @@ def test_unsupported_modes_and_missing_device_fail_loudly():
         nc(x)
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         _native.prefill(torch.zeros(1, 1, 8, 8), torch.zeros(1, 1, 8, 8), torch.zeros(1, 1, 8, 8), 4, 1)
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+def test_one_call_plan_only_for_inputs_and_weights_of_the_modules_own_shapes(sparse):
+    """The library takes its extents from the module: anything narrower would be read and written out of bounds."""
+    def module():
+        m = BlockSparseAttention(d_model=640, n_heads=10) if sparse else WindowedAttention(TitanMACConfig(d_model=640, n_heads=10))
+        return m.to(torch.bfloat16)
+
+    def plan(m, width=640):
+        x = torch.zeros(2, 24, width, dtype=torch.bfloat16)
+        return _stack.attention_plan(m, x, 0, 64 if sparse else 0, 0.125)
+
+    bf16 = dict(bias=False, dtype=torch.bfloat16)
+    assert plan(module()) is not None
+    for width in (8, 128, 632, 648, 1280):
+        assert plan(module(), width) is None
+    for name, shape in (("qkv_proj", (640, 640)), ("qkv_proj", (640, 1920 - 64)), ("qkv_proj", (640, 1920 + 64)), ("qkv_proj", (128, 1920)),
+                        ("out_proj", (640, 128)), ("out_proj", (640, 648)), ("out_proj", (128, 640))):
+        m = module()
+        setattr(m, name, torch.nn.Linear(*shape, **bf16))
+        assert plan(m) is None, (name, shape)
+    for name in ("qkv_proj", "out_proj"):
+        m = module()
+        getattr(m, name).to("meta")  # (another device than the input's)
+        assert plan(m) is None, name
+    m = module()
+    m.n_heads = 20
+    assert plan(m) is None
+    if sparse:
+        for conv in (torch.nn.Conv1d(64, 64, 4, groups=64, **bf16), torch.nn.Conv1d(640, 640, 3, groups=640, **bf16)):
+            m = module()
+            m.conv_k = conv
+            assert plan(m) is None
+        m = module()
+        m.conv_v.to("meta")
+        assert plan(m) is None

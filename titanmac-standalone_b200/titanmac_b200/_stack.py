@@ -303,34 +303,39 @@ def generate(table: ModelTable, input_ids: torch.Tensor, logits: torch.Tensor, c
     return out
 
 
-def _plain_weight(mod: nn.Module, kind, dtype: torch.dtype) -> Optional[torch.Tensor]:
-    """The weight of a submodule that is nothing but a ``kind`` without bias and hooks, contiguous and of that dtype."""
+def _plain_weight(mod: nn.Module, kind, like: torch.Tensor, shape) -> Optional[torch.Tensor]:
+    """The weight of a submodule that is nothing but a ``kind`` without bias and hooks, contiguous, of that shape, and of
+    ``like``'s dtype and device."""
     if type(mod) is not kind or mod._forward_hooks or mod._forward_pre_hooks:
         return None
     p = mod._parameters
     w = p["weight"]
-    return w if p["bias"] is None and w.dtype is dtype and w.is_contiguous() else None
+    return w if p["bias"] is None and w.dtype is like.dtype and w.shape == shape and w.is_contiguous() \
+        and w.device == like.device else None
 
 
 def attention_plan(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float):
     """``(AttentionDesc, w_qkv, w_out, convolution weights)`` if the module's forward on ``x`` is nothing but what the library
-    computes in one call, else None."""
+    computes in one call, else None.  The library takes every extent from the descriptor, so an input or a weight of another
+    shape goes to the modules, which raise or, where they can, compute it."""
     dtype = x.dtype
     if (dtype is not torch.bfloat16 and dtype is not torch.float16) or attn.algo or attn.core_events is not None \
             or not x.is_contiguous():
         return None
     B, L, D = x.shape
+    if D != attn.n_heads * attn.d_head or B * L == 0 or attn.d_head % 8 or _global_hooks():
+        return None
     mods = attn._modules
-    w_qkv, w_out = _plain_weight(mods["qkv_proj"], nn.Linear, dtype), _plain_weight(mods["out_proj"], nn.Linear, dtype)
-    if w_qkv is None or w_out is None or B * L == 0 or D % 8 or attn.d_head % 8 or _global_hooks():
+    w_qkv, w_out = _plain_weight(mods["qkv_proj"], nn.Linear, x, (3 * D, D)), _plain_weight(mods["out_proj"], nn.Linear, x, (D, D))
+    if w_qkv is None or w_out is None:
         return None
     conv, taps = (), 0
     if block_size and attn.use_conv:
-        conv = tuple(_plain_weight(mods[n], nn.Conv1d, dtype) for n in ("conv_q", "conv_k", "conv_v"))
-        taps = conv[0].shape[2] if conv[0] is not None else 0
-        if not 1 <= taps <= 8 or any(w is None or w.shape != (D, 1, taps) for w in conv):
+        taps = mods["conv_q"].weight.shape[-1]
+        conv = tuple(_plain_weight(mods[n], nn.Conv1d, x, (D, 1, taps)) for n in ("conv_q", "conv_k", "conv_v"))
+        if not 1 <= taps <= 8 or any(w is None for w in conv):
             return None
-    if (x.data_ptr() | w_qkv.data_ptr() | w_out.data_ptr()) % 16 or w_qkv.device != x.device:
+    if (x.data_ptr() | w_qkv.data_ptr() | w_out.data_ptr()) % 16:
         return None
     return _native.AttentionDesc(_native._DTYPES[dtype], B, L, attn.n_heads, attn.d_head, attn.window_size, n_persistent, block_size,
                                  taps, scale), w_qkv, w_out, conv
