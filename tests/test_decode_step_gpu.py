@@ -103,6 +103,23 @@ def test_generate_equals_argmax_over_steps(B, vocab, new):
     assert torch.equal(got, torch.cat(want, dim=1))
 
 
+@pytest.mark.parametrize("B,heads,vocab", [(17, 2, 48000), (64, 2, 20000), (40, 17, 30000), (3, 17, 30000)])
+def test_generate_behind_a_wide_head(B, heads, vocab):
+    """More than 16 rows or a width above 1024: the head is the tcgen05 product, whose output (megabytes, stored through TMA)
+    the choice reads as a dependent launch.  Every token against the ones that steps of their own give."""
+    model, g = make(torch.bfloat16, heads, 64, 20, 3, vocab, layers=1)
+    for _ in range(3):
+        ids = torch.randint(0, vocab, (B, 5), generator=g, device=DEV)
+        got = model.generate(ids, 24)
+        logits, caches = model.prefill(ids)
+        pos = torch.full((B,), 5, dtype=torch.int32, device=DEV)
+        for i in range(24):
+            token = logits.argmax(-1)
+            assert torch.equal(got[:, 5 + i], token), i
+            logits = model.decode_step(token, pos, caches)
+            pos += 1
+
+
 def test_greedy_choice_of_ties_and_nan():
     model, _ = make(torch.bfloat16, 2, 64, 20, 0, 5000, layers=1)
     logits = torch.zeros(4, 5000, dtype=torch.bfloat16, device=DEV)
