@@ -220,15 +220,16 @@ __global__ void __launch_bounds__(256) ce_forward_kernel(const CrossEntropy p) {
                     l *= __expf(m - mx);
                     m = mx;
                 }
+                // (a hidden logit counts nothing also while no other has been seen; a NaN reaches the sum whatever m is)
 #pragma unroll
-                for (int e = 0; e < 8; ++e) l += __expf(f[e] - m);
+                for (int e = 0; e < 8; ++e) l += f[e] > -CUDART_INF_F || f[e] != f[e] ? __expf(f[e] - m) : 0.f;
             }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
         const float mn = fmaxf(m, mo);
-        l = (mn > -CUDART_INF_F) ? l * __expf(m - mn) + lo * __expf(mo - mn) : 0.f;
+        l = (mn > -CUDART_INF_F) ? l * __expf(m - mn) + lo * __expf(mo - mn) : l + lo;  // (zeros, or NaN)
         m = mn;
     }
     if ((tid & 31) == 0) {
@@ -242,8 +243,9 @@ __global__ void __launch_bounds__(256) ce_forward_kernel(const CrossEntropy p) {
         float la = 0.f;
         for (int i = 0; i < 8; ++i) la += sl[i] * __expf(sm[i] - ma);
         const float lse = ma + logf(la);
+        const float loss = lse - to_f32<T>(x[y]);
         p.lse[row] = lse;
-        p.row_loss[row] = fmaxf(lse - to_f32<T>(x[y]), 0.f);
+        p.row_loss[row] = loss < 0.f ? 0.f : loss;  // (by rounding; not fmaxf, which makes 0 of NaN)
     }
 }
 
