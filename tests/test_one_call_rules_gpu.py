@@ -1,0 +1,99 @@
+"""What sends a call from the whole-model and whole-module library calls back to the modules, and what the caller sees of them."""
+
+import pytest
+import torch
+import torch.nn as nn
+from torch.nn.modules import module as nn_module
+
+from titanmac_b200 import TitanMAC, TitanMACConfig, _native, _stack, _train
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+BF16 = torch.bfloat16
+
+
+def make(block_sparse=False, layers=2, vocab=128, heads=2, dh=64, n_p=3, seed=0, **more):
+    cfg = TitanMACConfig(vocab_size=vocab, d_model=heads * dh, n_heads=heads, n_layers=layers, d_ff=3 * heads * dh, max_seq_len=64,
+                         window_size=16, n_persistent=n_p, use_block_sparse=block_sparse, block_size=32, **more)
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    with torch.device(DEV):
+        model = TitanMAC(cfg)
+    with torch.no_grad():
+        for name, prm in model.named_parameters():
+            prm.normal_(1.0 if name.endswith("scale") else 0.0, 0.1 if name.endswith(("scale", "bias")) else 0.04, generator=g)
+    return model.to(BF16), torch.randint(0, vocab, (2, 30), generator=g, device=DEV)
+
+
+def module_by_module(monkeypatch):
+    monkeypatch.setattr(_stack, "table_of", lambda *a, **k: None)
+    monkeypatch.setattr(_stack, "attention_forward", lambda *a: None)
+    for name in ("stack_forward", "attention_forward", "shifted_cross_entropy"):
+        monkeypatch.setattr(_train, name, lambda *a: None)
+
+
+def close(got, want, tol):
+    return ((got.float() - want.float()).norm() / want.float().norm().clamp_min(1e-12)).item() <= tol
+
+
+def step(model, ids):
+    model.zero_grad(set_to_none=True)
+    with torch.enable_grad():  # (other tests may have turned it off)
+        out = model(ids, labels=ids)
+        out["loss"].backward()
+    return out, {n: p.grad for n, p in model.named_parameters()}
+
+
+@pytest.mark.parametrize("place", ["layers.0.attention", "layers.0.attention.qkv_proj", "layers.1.mlp", "layers.1.mlp.fc2",
+                                   "layers.0.norm_mlp", "norm", "lm_head", "embed_tokens"])
+@pytest.mark.parametrize("pre", [False, True])
+def test_backward_hooks_of_submodules_fire(place, pre):
+    model, ids = make()
+    mod, seen = model.get_submodule(place), []
+    # (the residual add and the norm behind it are one call of add_forward: module by module norm_mlp is not called either)
+    register = mod.register_full_backward_pre_hook if pre else mod.register_full_backward_hook
+    handle = register(lambda *a: seen.append(1))
+    with torch.enable_grad():
+        assert _train.stack_forward(model, ids) is None
+    step(model, ids)
+    assert seen or place in ("layers.0.norm_mlp", "norm")
+    handle.remove()
+    with torch.enable_grad():
+        assert _train.stack_forward(model, ids) is not None
+
+
+@pytest.mark.parametrize("register", ["register_module_full_backward_hook", "register_module_full_backward_pre_hook"])
+def test_global_backward_hooks_fire(register):
+    model, ids = make()
+    seen = []
+    handle = getattr(nn_module, register)(lambda mod, *a: seen.append(type(mod)))
+    try:
+        step(model, ids)
+    finally:
+        handle.remove()
+    assert nn.Linear in seen
+
+
+@pytest.mark.parametrize("block_sparse", [False, True])
+def test_backward_hook_inside_an_attention_module(block_sparse):
+    model, _ = make(block_sparse)
+    attn, seen = model.layers[0].attention, []
+    attn.out_proj.register_full_backward_hook(lambda *a: seen.append(1))
+    with torch.enable_grad():
+        x = torch.randn(2, 40, 128, device=DEV, dtype=BF16, requires_grad=True)
+        attn(x).sum().backward()
+    assert seen == [1]
+
+
+@pytest.mark.parametrize("place", ["layers.0.attention", "layers.1.mlp", "layers.0.attention.out_proj"])
+@pytest.mark.parametrize("train", [False, True])
+def test_a_forward_replaced_on_the_instance_is_called(place, train):
+    model, ids = make()
+    mod, seen = model.get_submodule(place), []
+    own = mod.forward
+    mod.forward = lambda *a, **k: (seen.append(1), own(*a, **k))[1]
+    if train:
+        step(model, ids)
+    else:
+        with torch.no_grad():
+            model(ids)
+    assert seen

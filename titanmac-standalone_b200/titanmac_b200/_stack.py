@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import operator
 import weakref
 from typing import List, Optional
 
@@ -21,8 +22,22 @@ from torch.nn.modules import module as _nn_module
 from . import _native
 
 
-def _global_hooks() -> bool:
-    return bool(_nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks)
+# What runs when a module is called beside its class's forward; the second pair only with a gradient to come.  (A forward set
+# on the instance replaces the class's.)
+_FORWARD_HOOKS = ("_forward_hooks", "_forward_pre_hooks")
+_BACKWARD_HOOKS = ("_backward_hooks", "_backward_pre_hooks")
+
+
+def _global_hooks(training: bool) -> bool:
+    return bool(_nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks
+                or (training and (_nn_module._global_backward_hooks or _nn_module._global_backward_pre_hooks)))
+
+
+def _is_plain(mod: nn.Module, training: bool) -> bool:
+    """Whether calling the module does nothing but its class's forward."""
+    d = mod.__dict__
+    return not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d
+                or (training and (d["_backward_hooks"] or d["_backward_pre_hooks"])))
 
 
 class ModelTable:
@@ -36,7 +51,7 @@ class ModelTable:
         self.ok = False
         self._params: list = []    # (parameter dict of a module, name, address)
         self._children: list = []  # (child dict of a module, name, child)
-        self._modules: list = []
+        self._module_dicts: list = []
         self._dropouts: list = []
         self._attentions: list = []
         self._places: list = []
@@ -53,7 +68,7 @@ class ModelTable:
                 return None
             if isinstance(child, nn.Dropout):
                 self._dropouts.append(child)
-            self._modules.append(child)
+            self._module_dicts.append(child.__dict__)
             return child
 
         def address(mod: nn.Module, name: str, shape) -> Optional[int]:
@@ -178,30 +193,33 @@ class ModelTable:
                 return False
         return True
 
-    def plain_call(self) -> bool:
+    def plain_call(self, training: bool) -> bool:
         """Whether calling the modules would do nothing but compute: no hooks, no active dropout."""
-        for m in self._modules:
-            if m._forward_hooks or m._forward_pre_hooks:
+        dicts = self._module_dicts
+        for name in _FORWARD_HOOKS + _BACKWARD_HOOKS if training else _FORWARD_HOOKS:
+            if any(map(operator.itemgetter(name), dicts)):
                 return False
+        if any(["forward" in d for d in dicts]):
+            return False
         for m in self._dropouts:
             if m.training and m.p > 0:
                 return False
         for m in self._attentions:
             if m.algo != _native.ALGO_AUTO or m.core_events is not None or not m.causal or (m.training and m.dropout_p > 0):
                 return False
-        return not _global_hooks()
+        return not _global_hooks(training)
 
 
 # not an attribute of the model: copies and pickles of a model do not carry addresses
 _tables: "weakref.WeakKeyDictionary[nn.Module, ModelTable]" = weakref.WeakKeyDictionary()
 
 
-def table_of(model) -> Optional[ModelTable]:
-    """The model's table if it can be used right now, else None."""
+def table_of(model, training: bool = False) -> Optional[ModelTable]:
+    """The model's table if it can be used right now (``training``: for a call with a gradient to come), else None."""
     table = _tables.get(model)
     if table is None or not table.holds():
         table = _tables[model] = ModelTable(model)
-    return table if table.ok and table.plain_call() else None
+    return table if table.ok and table.plain_call(training) else None
 
 
 def _attach(blocks, caches, geometry, device) -> bool:
@@ -303,10 +321,10 @@ def generate(table: ModelTable, input_ids: torch.Tensor, logits: torch.Tensor, c
     return out
 
 
-def _plain_weight(mod: nn.Module, kind, like: torch.Tensor, shape) -> Optional[torch.Tensor]:
+def _plain_weight(mod: nn.Module, kind, like: torch.Tensor, shape, training: bool) -> Optional[torch.Tensor]:
     """The weight of a submodule that is nothing but a ``kind`` without bias and hooks, contiguous, of that shape, and of
     ``like``'s dtype and device."""
-    if type(mod) is not kind or mod._forward_hooks or mod._forward_pre_hooks:
+    if type(mod) is not kind or not _is_plain(mod, training):
         return None
     p = mod._parameters
     w = p["weight"]
@@ -314,7 +332,7 @@ def _plain_weight(mod: nn.Module, kind, like: torch.Tensor, shape) -> Optional[t
         and w.device == like.device else None
 
 
-def attention_plan(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float):
+def attention_plan(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float, training: bool = False):
     """``(AttentionDesc, w_qkv, w_out, convolution weights)`` if the module's forward on ``x`` is nothing but what the library
     computes in one call, else None.  The library takes every extent from the descriptor, so an input or a weight of another
     shape goes to the modules, which raise or, where they can, compute it."""
@@ -323,16 +341,17 @@ def attention_plan(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_si
             or not x.is_contiguous():
         return None
     B, L, D = x.shape
-    if D != attn.n_heads * attn.d_head or B * L == 0 or attn.d_head % 8 or _global_hooks():
+    if D != attn.n_heads * attn.d_head or B * L == 0 or attn.d_head % 8 or _global_hooks(training):
         return None
     mods = attn._modules
-    w_qkv, w_out = _plain_weight(mods["qkv_proj"], nn.Linear, x, (3 * D, D)), _plain_weight(mods["out_proj"], nn.Linear, x, (D, D))
+    w_qkv = _plain_weight(mods["qkv_proj"], nn.Linear, x, (3 * D, D), training)
+    w_out = _plain_weight(mods["out_proj"], nn.Linear, x, (D, D), training)
     if w_qkv is None or w_out is None:
         return None
     conv, taps = (), 0
     if block_size and attn.use_conv:
         taps = mods["conv_q"].weight.shape[-1]
-        conv = tuple(_plain_weight(mods[n], nn.Conv1d, x, (D, 1, taps)) for n in ("conv_q", "conv_k", "conv_v"))
+        conv = tuple(_plain_weight(mods[n], nn.Conv1d, x, (D, 1, taps), training) for n in ("conv_q", "conv_k", "conv_v"))
         if not 1 <= taps <= 8 or any(w is None for w in conv):
             return None
     if (x.data_ptr() | w_qkv.data_ptr() | w_out.data_ptr()) % 16:

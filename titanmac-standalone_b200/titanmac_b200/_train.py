@@ -70,7 +70,7 @@ class _StackTrain(torch.autograd.Function):
 
 def stack_forward(model, input_ids: torch.Tensor) -> Optional[torch.Tensor]:
     """Logits of every row with a gradient to every parameter, or None where that takes the modules themselves."""
-    table = _stack.table_of(model)
+    table = _stack.table_of(model, training=True)
     if table is None or not table.trains or _autocast() or input_ids.dtype != torch.int64 or input_ids.dim() != 2 \
             or input_ids.device != table.device:
         return None
@@ -172,7 +172,7 @@ def attention_forward(attn, x: torch.Tensor, n_persistent: int, block_size: int,
     if _autocast():
         return None
     x = x.contiguous()
-    plan = _stack.attention_plan(attn, x, n_persistent, block_size, scale)
+    plan = _stack.attention_plan(attn, x, n_persistent, block_size, scale, training=True)
     if plan is None:
         return None
     desc, w_qkv, w_out, conv = plan
