@@ -97,3 +97,55 @@ def test_a_forward_replaced_on_the_instance_is_called(place, train):
         with torch.no_grad():
             model(ids)
     assert seen
+
+
+def _window(m):
+    m.layers[1].attention.window_size = 3
+
+
+def _eps(m):
+    m.layers[1].norm_mlp.eps = 0.5
+
+
+def _append(m):
+    m.layers.append(make(layers=1, seed=5)[0].layers[0])
+
+
+def _bias(m):
+    m.layers[0].attention.qkv_proj.bias = nn.Parameter(torch.full((384,), 0.5, device=DEV, dtype=BF16))
+
+
+def _head_bias(m):
+    m.lm_head.bias = nn.Parameter(torch.linspace(-1, 1, 128, device=DEV, dtype=BF16))
+
+
+def _transposed(m):
+    w = m.layers[0].attention.out_proj.weight
+    w.data = w.data.t()
+
+
+def _retyped(m):
+    for p in m.parameters():
+        p.data = (p.data.float() * 0.25).to(torch.float16).view(BF16).view(torch.float16)
+
+
+def _max_norm(m):
+    m.embed_tokens.max_norm = 0.05
+
+
+@pytest.mark.parametrize("change", [_window, _eps, _append, _bias, _head_bias, _transposed, _retyped, _max_norm],
+                         ids=lambda f: f.__name__[1:])
+def test_the_model_as_it_is_at_the_call(change, monkeypatch):
+    """Changed between two calls: the second gives what a model that never had a first call gives."""
+    model, ids = make(tie_weights=False)
+    model.eval()
+    with torch.no_grad():
+        first = model(ids)["logits"]
+        change(model)
+        got = model(ids)["logits"]
+        module_by_module(monkeypatch)
+        want = model(ids)["logits"]
+    _native.poll_status(torch.device(DEV))
+    assert not torch.equal(first, got)
+    assert got.dtype == want.dtype and close(got, want, 2e-2)
+    assert not close(first.to(want.dtype), want, 2e-2)  # (the change is large enough to be told from rounding)

@@ -1,9 +1,9 @@
 """The model as the flat table that the whole-model calls of libtmw take (``tmw_block`` / ``tmw_stack_desc``).
 
 A step of a few rows is bound by its host work when every norm, product and attention call is issued from Python, so
-``TitanMAC`` hands the library one table per call.  The table is built once and holds addresses only: before every use
-it is checked against the modules it was built from, and rebuilt when a parameter has moved or a module has been
-replaced.  A model that the table cannot describe - another type of module in a known place, hooks, fp32, an active
+``TitanMAC`` hands the library one table per call.  The table is built once and holds addresses and sizes only: before every
+use everything that went into it is compared with the modules as they are, and it is rebuilt when a parameter has moved or
+changed its layout, a module has been replaced or added, or an attribute has another value.  A model that the table cannot describe - another type of module in a known place, hooks, fp32, an active
 dropout - has no table, and its modules are called one by one.
 """
 
@@ -22,6 +22,8 @@ from torch.nn.modules import module as _nn_module
 from . import _native
 
 
+_dtype_of, _nbytes_of = operator.attrgetter("dtype"), operator.attrgetter("nbytes")
+
 # What runs when a module is called beside its class's forward; the second pair only with a gradient to come.  (A forward set
 # on the instance replaces the class's.)
 _FORWARD_HOOKS = ("_forward_hooks", "_forward_pre_hooks")
@@ -33,30 +35,36 @@ def _global_hooks(training: bool) -> bool:
                 or (training and (_nn_module._global_backward_hooks or _nn_module._global_backward_pre_hooks)))
 
 
-def _is_plain(mod: nn.Module, training: bool) -> bool:
-    """Whether calling the module does nothing but its class's forward."""
-    d = mod.__dict__
-    return not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d
-                or (training and (d["_backward_hooks"] or d["_backward_pre_hooks"])))
-
-
 class ModelTable:
     """Addresses of a ``TitanMAC``'s parameters and how to tell that they still hold."""
 
     def __init__(self, model):
-        from .attn.block_sparse_attention import BlockSparseAttention
-        from .attn.windowed_attention import WindowedAttention
-        from .blocks.titan_block import MLPBlock, RMSNorm, TitanBlock
-
         self.ok = False
-        self._params: list = []    # (parameter dict of a module, name, address)
-        self._children: list = []  # (child dict of a module, name, child)
+        # what holds() compares: (parameters of a module, name, address, strides, bytes, dtype), (children of a module, name,
+        # child), (object, attribute, value), (parameters of a module, name, identity) where there should be none, and
+        # (children of a ModuleList, how many); also what keeps the table from being built
+        self._params: list = []
+        self._children: list = []
+        self._attributes: list = []
+        self._absent: list = []
+        self._lists: list = []
         self._module_dicts: list = []
         self._dropouts: list = []
         self._attentions: list = []
         self._places: list = []
         self.dtype = model.embed_tokens.weight.dtype
         self.device = model.embed_tokens.weight.device
+        self.config = model.config
+        self._build(model)
+        columns = (lambda rows, n: tuple(list(col) for col in zip(*rows)) if rows else ([],) * n)  # noqa: E731
+        self._params, self._children = columns(self._params, 6), columns(self._children, 3)
+        self._attributes, self._absent = columns(self._attributes, 3), columns(self._absent, 3)
+
+    def _build(self, model) -> None:
+        from .attn.block_sparse_attention import BlockSparseAttention
+        from .attn.windowed_attention import WindowedAttention
+        from .blocks.titan_block import MLPBlock, RMSNorm, TitanBlock
+
         if self.dtype not in (torch.bfloat16, torch.float16) or self.device.type != "cuda":
             return
         c = model.config
@@ -66,6 +74,8 @@ class ModelTable:
             self._children.append((parent._modules, name, child))
             if type(child) not in types:
                 return None
+            if type(child) is nn.ModuleList:
+                self._lists.append((child._modules, len(child)))
             if isinstance(child, nn.Dropout):
                 self._dropouts.append(child)
             self._module_dicts.append(child.__dict__)
@@ -73,24 +83,38 @@ class ModelTable:
 
         def address(mod: nn.Module, name: str, shape) -> Optional[int]:
             prm = mod._parameters.get(name)
-            if prm is None or prm.dtype != self.dtype or tuple(prm.shape) != tuple(shape) or not prm.is_contiguous() \
+            if prm is None:
+                absent(mod, name)
+                return None
+            self._params.append((mod._parameters, name, prm.data_ptr(), prm.stride(), prm.nbytes, prm.dtype))
+            if prm.dtype != self.dtype or tuple(prm.shape) != tuple(shape) or not prm.is_contiguous() \
                     or prm.device != self.device or prm.data_ptr() % 16:
                 return None
-            self._params.append((mod._parameters, name, prm.data_ptr()))
             return prm.data_ptr()
+
+        def absent(mod: nn.Module, name: str) -> bool:
+            prm = mod._parameters.get(name)
+            self._absent.append((mod._parameters, name, id(prm)))
+            return prm is None
 
         def optional(mod: nn.Module, name: str, shape):
             if mod._parameters.get(name) is None:
-                self._params.append((mod._parameters, name, 0))
+                absent(mod, name)
                 return 0
             return address(mod, name, shape)
+
+        def attributes(obj, *names) -> tuple:
+            values = tuple(getattr(obj, name) for name in names)
+            self._attributes += zip((obj,) * len(names), names, values)
+            return values
 
         D, V = c.d_model, c.vocab_size
         layers = take(model, "layers", nn.ModuleList)
         tops = (take(model, "embed_tokens", nn.Embedding), take(model, "embed_positions", nn.Embedding),
                 take(model, "norm", RMSNorm), take(model, "lm_head", nn.Linear))
-        if layers is None or len(layers) == 0 or any(t is None for t in tops) or tops[3].bias is not None:
+        if layers is None or len(layers) == 0 or any(t is None for t in tops) or not absent(tops[3], "bias"):
             return
+        attributes(c, "d_model", "n_heads", "window_size", "n_persistent", "vocab_size", "max_seq_len", "norm_eps")
         F = layers[0].mlp.d_ff if type(layers[0]) is TitanBlock and type(layers[0].mlp) is MLPBlock else 0
         found: List[Optional[int]] = []
         self.blocks = (_native.Block * len(layers))()
@@ -100,28 +124,28 @@ class ModelTable:
                 return
             attn, mlp = take(block, "attention", WindowedAttention, BlockSparseAttention), take(block, "mlp", MLPBlock)
             norms = (take(block, "norm_attn", RMSNorm), take(block, "norm_mlp", RMSNorm))
-            if attn is None or mlp is None or None in norms or any(n.eps != c.norm_eps for n in norms):
+            if attn is None or mlp is None or None in norms or any(attributes(n, "eps") != (c.norm_eps,) for n in norms):
                 return
             windowed = type(attn) is WindowedAttention
-            np_attn = attn.num_persistent if windowed else attn.n_persistent
-            if (attn.n_heads, attn.d_head, attn.window_size, np_attn) != (c.n_heads, c.d_head, c.window_size,
-                                                                          c.n_persistent) or mlp.d_ff != F:
+            if attributes(attn, "n_heads", "d_head", "window_size", "num_persistent" if windowed else "n_persistent") != (
+                    c.n_heads, c.d_head, c.window_size, c.n_persistent) or mlp.d_ff != F:
                 return
             kind = (0, 0)
             if not windowed:
-                if attn.scale != 1.0 / math.sqrt(c.d_head):
+                scale, block_size, use_conv = attributes(attn, "scale", "block_size", "use_conv")
+                if scale != 1.0 / math.sqrt(c.d_head):
                     return
-                kind = (attn.block_size, attn.conv_q.kernel_size[0] if attn.use_conv else 0)
+                kind = (block_size, attn.conv_q.kernel_size[0] if use_conv else 0)
             if i > 0 and kind != self.kind:
                 return
             self.kind = kind
             self._attentions.append(attn)
             qkv, out = take(attn, "qkv_proj", nn.Linear), take(attn, "out_proj", nn.Linear)
             fc1, fc2 = take(mlp, "fc1", nn.Linear), take(mlp, "fc2", nn.Linear)
-            if None in (qkv, out, fc1, fc2) or qkv.bias is not None or out.bias is not None:
+            if None in (qkv, out, fc1, fc2) or not absent(qkv, "bias") or not absent(out, "bias"):
                 return
             if take(attn, "dropout", nn.Identity, nn.Dropout) is None or take(mlp, "dropout", nn.Identity, nn.Dropout) is None \
-                    or take(mlp, "activation", nn.GELU) is None or mlp.activation.approximate != "none":
+                    or take(mlp, "activation", nn.GELU) is None or attributes(mlp.activation, "approximate") != ("none",):
                 return
             b = self.blocks[i]
             values = dict(norm_attn=address(norms[0], "scale", (D,)), norm_mlp=address(norms[1], "scale", (D,)),
@@ -130,7 +154,7 @@ class ModelTable:
                           b_fc1=optional(fc1, "bias", (F,)), b_fc2=optional(fc2, "bias", (D,)))
             for name in ("conv_q", "conv_k", "conv_v") if kind[1] else ():
                 conv = take(attn, name, nn.Conv1d)
-                if conv is None or conv.bias is not None:
+                if conv is None or not absent(conv, "bias"):
                     return
                 values[name] = address(conv, "weight", (D, 1, kind[1]))
             found += values.values()
@@ -147,8 +171,8 @@ class ModelTable:
         pers = 0
         if c.n_persistent > 0:
             pers = address(model, "persistent_tokens", (c.n_persistent, D))
-        if None in found or None in top or pers is None or tops[2].eps != c.norm_eps or tops[0].max_norm is not None \
-                or tops[1].max_norm is not None:
+        if None in found or None in top or pers is None or attributes(tops[2], "eps") != (c.norm_eps,) \
+                or attributes(tops[0], "max_norm") != (None,) or attributes(tops[1], "max_norm") != (None,):
             return
         d.embed_tokens, d.embed_positions, d.norm, d.head = top
         tops_at = dict(embed_tokens=(tops[0], "weight"), embed_positions=(tops[1], "weight"), norm=(tops[2], "scale"),
@@ -179,19 +203,28 @@ class ModelTable:
         self.ok = True
 
     def holds(self) -> bool:
-        """Whether the modules are still the ones, and their parameters still where, the table says."""
-        dtype = self.dtype
-        for d, name, child in self._children:
-            if d.get(name) is not child:
+        """Whether the modules, the attributes that went into the table and the parameters' places and layouts are still what
+        it says.  Whole columns at a time: a model has some hundreds of each, and this is in front of every call."""
+        get, tensor = dict.get, torch.Tensor
+        dicts, names, children = self._children
+        if not all(map(operator.is_, map(get, dicts, names), children)):
+            return False
+        for listed, n in self._lists:
+            if len(listed) != n:
                 return False
-        for d, name, ptr in self._params:
-            prm = d.get(name)
-            if prm is None:
-                if ptr:
-                    return False
-            elif prm.data_ptr() != ptr or prm.dtype is not dtype:
-                return False
-        return True
+        objects, names, values = self._attributes
+        if list(map(getattr, objects, names)) != values:
+            return False
+        dicts, names, ids = self._absent
+        if list(map(id, map(get, dicts, names))) != ids:
+            return False
+        dicts, names, ptrs, strides, sizes, dtypes = self._params
+        params = list(map(get, dicts, names))
+        try:
+            return (list(map(tensor.data_ptr, params)) == ptrs and list(map(tensor.stride, params)) == strides
+                    and list(map(_nbytes_of, params)) == sizes and list(map(_dtype_of, params)) == dtypes)
+        except TypeError:  # a parameter that is no more
+            return False
 
     def plain_call(self, training: bool) -> bool:
         """Whether calling the modules would do nothing but compute: no hooks, no active dropout."""
@@ -216,8 +249,9 @@ _tables: "weakref.WeakKeyDictionary[nn.Module, ModelTable]" = weakref.WeakKeyDic
 
 def table_of(model, training: bool = False) -> Optional[ModelTable]:
     """The model's table if it can be used right now (``training``: for a call with a gradient to come), else None."""
-    table = _tables.get(model)
-    if table is None or not table.holds():
+    table, weight = _tables.get(model), model.embed_tokens.weight
+    if table is None or weight.dtype is not table.dtype or weight.device != table.device or table.config is not model.config \
+            or not table.holds():
         table = _tables[model] = ModelTable(model)
     return table if table.ok and table.plain_call(training) else None
 
@@ -324,9 +358,11 @@ def generate(table: ModelTable, input_ids: torch.Tensor, logits: torch.Tensor, c
 def _plain_weight(mod: nn.Module, kind, like: torch.Tensor, shape, training: bool) -> Optional[torch.Tensor]:
     """The weight of a submodule that is nothing but a ``kind`` without bias and hooks, contiguous, of that shape, and of
     ``like``'s dtype and device."""
-    if type(mod) is not kind or not _is_plain(mod, training):
+    d = mod.__dict__
+    if type(mod) is not kind or d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d \
+            or (training and (d["_backward_hooks"] or d["_backward_pre_hooks"])):
         return None
-    p = mod._parameters
+    p = d["_parameters"]
     w = p["weight"]
     return w if p["bias"] is None and w.dtype is like.dtype and w.shape == shape and w.is_contiguous() \
         and w.device == like.device else None
