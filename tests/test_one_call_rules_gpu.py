@@ -84,6 +84,16 @@ def test_backward_hook_inside_an_attention_module(block_sparse):
     assert seen == [1]
 
 
+@pytest.mark.parametrize("block_sparse", [False, True])
+def test_forward_hook_of_the_modules_dropout(block_sparse):
+    """(an Identity where the rate is 0; the one call skips it)"""
+    attn, seen = make(block_sparse)[0].layers[0].attention, []
+    attn.dropout.register_forward_hook(lambda *a: seen.append(1))
+    with torch.no_grad():
+        attn(torch.randn(2, 40, 128, device=DEV, dtype=BF16))
+    assert seen == [1]
+
+
 @pytest.mark.parametrize("place", ["layers.0.attention", "layers.1.mlp", "layers.0.attention.out_proj"])
 @pytest.mark.parametrize("train", [False, True])
 def test_a_forward_replaced_on_the_instance_is_called(place, train):

@@ -141,7 +141,8 @@ class BlockSparseAttention(nn.Module):
             raise ValueError(f"n_persistent ({self.n_persistent}) must be < seq_len ({L})")
         y = _stack.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)  # the module as one call
         if y is not None:
-            return y if type(self.dropout) is nn.Identity else self.dropout(y)
+            drop = self._modules["dropout"]
+            return y if type(drop) is nn.Identity and not (drop._forward_hooks or drop._forward_pre_hooks) else drop(y)
         qkv = _native.project(self.qkv_proj, x)
         if self.use_conv:
             qkv = _native.causal_dwconv(qkv, self.stacked_conv_weight())

@@ -132,7 +132,8 @@ class WindowedAttention(nn.Module):
             return self.dropout(self.out_proj(o.view(B, L, D)))
         y = _stack.attention_forward(self, x, self.num_persistent, 0, 0.0)  # the module as one call
         if y is not None:
-            return y if type(self.dropout) is nn.Identity else self.dropout(y)
+            drop = self._modules["dropout"]
+            return y if type(drop) is nn.Identity and not (drop._forward_hooks or drop._forward_pre_hooks) else drop(y)
         with torch.no_grad():
             return self._forward_no_grad(x)
 
