@@ -443,9 +443,9 @@ TMW_API int tmw_cross_entropy(int32_t dtype, int32_t batch, int32_t tokens, int3
  * One decode step of the whole model: token_ids [batch] int64 and pos [batch] int32 (device) -> logits [batch, vocab].
  * Every block runs RMSNorm -> QKV -> tmw_decode on its ring -> output projection + residual -> RMSNorm -> MLP + residual
  * (titan_block.py:92-100, blocks/mlp.py:58-65), then the final norm and the head; what the reference's generation
- * helper gets from a full re-forward per token (examples/train_math.py:146-161).  head_dim 64 or 128, d_ff a multiple of
- * 32.  `workspace`: device memory of tmw_decode_step_workspace() bytes, used until the call's kernels have finished;
- * ids or positions outside the tables are clamped and reported by tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).
+ * helper gets from a full re-forward per token (examples/train_math.py:146-161).  head_dim 64 or 128, d_model at most
+ * 4096, d_ff a multiple of 32, batch at most 65535.  `workspace`: device memory of tmw_decode_step_workspace() bytes, used
+ * until the call's kernels have finished; ids or positions outside the tables are clamped and reported by tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).
  */
 TMW_API size_t tmw_decode_step_workspace(const tmw_stack_desc* desc);
 TMW_API int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, const int32_t* pos,

@@ -146,3 +146,15 @@ def test_split_decode_scratch_size_and_argument_checks():
     assert lib.tmw_decode_split(*args, 0, ok, 1 << 30, None) == _native.TMW_ERR_INVALID_ARGUMENT   # splits
     assert lib.tmw_decode_split(*args, 4, None, 1 << 30, None) == _native.TMW_ERR_INVALID_ARGUMENT  # no scratch
     assert lib.tmw_decode_split(*args, 4, ok, 1024, None) == _native.TMW_ERR_TOO_LARGE            # scratch too small
+
+
+def test_decode_step_sizes_the_library_refuses():
+    """No workspace, and so no call, beyond what every kernel of the step takes (the check is the same in both)."""
+    def workspace(**more):
+        sizes = dict(dtype=_native.TMW_BF16, batch=3, layers=1, d_model=4096, heads=32, head_dim=128, d_ff=64, window=8,
+                     vocab=16, max_positions=4, eps=1e-5)
+        return _native.lib().tmw_decode_step_workspace(ctypes.byref(_native.StackDesc(**dict(sizes, **more))))
+
+    assert workspace() > 0 and workspace(batch=65535) > 0
+    assert workspace(d_model=5120, heads=40) == 0 and workspace(batch=65536) == 0
+    assert workspace(head_dim=32, heads=128) == 0 and workspace(d_ff=48) == 0

@@ -57,6 +57,22 @@ def test_step_equals_module_by_module(B, dtype, heads, dh, window, Np, vocab, t,
             assert ((x.float() - y.float()).norm() / y.float().norm()).item() <= tol
 
 
+@pytest.mark.parametrize("B,heads,one_call", [(2, 32, True), (40, 32, True), (2, 40, False), (40, 40, False)])
+def test_widths_around_the_steps_limit(B, heads, one_call, monkeypatch):
+    """The step's norms keep a row of at most 4096 in registers: a wider model goes to its modules."""
+    model, g = make(torch.bfloat16, heads, 128, 16, 1, 64, layers=1)
+    assert _stack.table_of(model).decodes == one_call
+    ids = torch.randint(0, 64, (B, 6), generator=g, device=DEV)
+    assert model.generate(ids, 3).shape == (B, 9)
+    logits, caches = model.prefill(ids)
+    pos = torch.full((B,), 6, dtype=torch.int32, device=DEV)
+    got = model.decode_step(ids[:, 0], pos, caches)
+    _native.poll_status(torch.device(DEV))
+    monkeypatch.setattr(_stack, "table_of", lambda m: None)
+    want = model.decode_step(ids[:, 0], pos, caches)  # (the step before has written the same keys and values)
+    assert ((got.float() - want.float()).norm() / want.float().norm()).item() <= 2e-2
+
+
 def test_table_follows_the_model():
     """A moved parameter, a replaced module, a hook: the step never uses what the model no longer is."""
     model, g = make(torch.bfloat16, 2, 64, 16, 2, 128)

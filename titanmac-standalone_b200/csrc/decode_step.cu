@@ -611,7 +611,7 @@ int validate_step(const tmw_stack_desc* d) {
     if (d->window < 0) return TMW_ERR_NEGATIVE_WINDOW;
     if (d->head_dim != 64 && d->head_dim != 128) return TMW_ERR_UNSUPPORTED;
     if (d->d_model != d->heads * d->head_dim) return TMW_ERR_INVALID_ARGUMENT;
-    if (d->d_ff % 32 != 0) return TMW_ERR_UNSUPPORTED;
+    if (d->d_ff % 32 != 0 || d->d_model > 4096) return TMW_ERR_UNSUPPORTED;  // (launch_rows_norm keeps a row in registers)
     if (d->batch > 65535) return TMW_ERR_TOO_LARGE;
     return TMW_OK;
 }

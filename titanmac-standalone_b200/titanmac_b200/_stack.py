@@ -196,7 +196,7 @@ class ModelTable:
                     self.roles.append([])
                 self.roles[at[id(prm)]].append(place)
         self.geometry = (c.n_heads, c.d_head, c.window_size, c.n_persistent, self.dtype)
-        self.decodes = c.d_head in (64, 128) and F % 32 == 0 and self.kind == (0, 0)
+        self.decodes = c.d_head in (64, 128) and F % 32 == 0 and D <= 4096 and self.kind == (0, 0)
         self.forwards = V % 8 == 0 and F % 8 == 0 and D % 8 == 0 and c.d_head % 8 == 0 and self.kind[1] <= 8
         self.trains = self.forwards and D <= 2048
         self.workspace_bytes: dict = {}  # (batch, tokens) -> bytes; tokens = -1: a decode step
@@ -300,7 +300,7 @@ def _step_arguments(table: ModelTable, batch: int, caches):
     """``(StackDesc, blocks with the caches, workspace)`` of a decode step, or None where the table or the caches are not what
     the step takes."""
     device = table.device
-    if not table.decodes or batch == 0 or len(caches) != len(table.blocks):
+    if not table.decodes or not 0 < batch <= 65535 or len(caches) != len(table.blocks):
         return None
     blocks = type(table.blocks).from_buffer_copy(table.blocks)  # (the table is shared by all threads)
     if not _attach(blocks, caches, (batch,) + table.geometry, device):
