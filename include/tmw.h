@@ -386,7 +386,7 @@ TMW_API int tmw_attention_forward(const tmw_attention_desc* desc, const void* x,
  * (titans_core/models/titanmac.py:554-619), the blocks, the final norm and the head.  logits: [batch, n_persistent + tokens,
  * vocab], or with last_only [batch, vocab] of the last token.  Blocks whose k_ring is not NULL keep their keys and values
  * as tmw_cache_fill does (and the persistent rows' in k_pers, v_pers): a prompt that decode steps continue.  d_ff and vocab
- * multiples of 8, tokens <= max_positions; ids outside the table are clamped and reported by tmw_poll_status.
+ * multiples of 8, tokens <= max_positions; an id outside the table embeds as NaN and is reported by tmw_poll_status.
  */
 TMW_API size_t tmw_stack_workspace(const tmw_stack_desc* desc, int32_t tokens);
 TMW_API int tmw_stack_forward(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, int32_t tokens,
@@ -433,7 +433,7 @@ TMW_API int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_block
  * sequence predicts labels[t + 1]; label -100 does not count, nor do the persistent rows and the last.  With d_logits
  * NULL: *loss (in dtype) = the mean over the counted rows, `stats` (4 + 2 * rows floats) filled for the backward.  Else the
  * backward: d_logits = softmax gradient times *grad (in dtype), zero on rows that do not count.  vocab a multiple of 8;
- * labels outside the vocabulary do not count and are reported by tmw_poll_status.
+ * a label outside the vocabulary makes the loss, and its row of d_logits, NaN and is reported by tmw_poll_status.
  */
 TMW_API int tmw_cross_entropy(int32_t dtype, int32_t batch, int32_t tokens, int32_t n_persistent, int32_t vocab,
                       const void* logits, const int64_t* labels, void* loss, float* stats, const void* grad, void* d_logits,
@@ -445,7 +445,8 @@ TMW_API int tmw_cross_entropy(int32_t dtype, int32_t batch, int32_t tokens, int3
  * (titan_block.py:92-100, blocks/mlp.py:58-65), then the final norm and the head; what the reference's generation
  * helper gets from a full re-forward per token (examples/train_math.py:146-161).  head_dim 64 or 128, d_model at most
  * 4096, d_ff a multiple of 32, batch at most 65535.  `workspace`: device memory of tmw_decode_step_workspace() bytes, used
- * until the call's kernels have finished; ids or positions outside the tables are clamped and reported by tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).
+ * until the call's kernels have finished; an id or position outside its table embeds as NaN and is reported by
+ * tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).
  */
 TMW_API size_t tmw_decode_step_workspace(const tmw_stack_desc* desc);
 TMW_API int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, const int32_t* pos,
@@ -487,8 +488,9 @@ TMW_API const char* tmw_strerror(int status);
 /* Text of the last CUDA error seen by this thread inside the library ("" if none). */
 TMW_API const char* tmw_last_cuda_error(void);
 /*
- * Device-side status word of the current device: 0, or TMW_ERR_DEVICE_TIMEOUT if a
- * kernel's bounded wait expired since the last poll.  Synchronises the given
+ * Device-side status word of the current device: 0, TMW_ERR_DEVICE_TIMEOUT if a
+ * kernel's bounded wait expired since the last poll, or TMW_ERR_INVALID_ARGUMENT if a
+ * kernel met an id, label or position outside its table.  Synchronises the given
  * stream, then clears the word.
  */
 TMW_API int tmw_poll_status(void* stream);

@@ -422,17 +422,18 @@ int tmw_decode_split(const tmw_cache_desc* cache, const void* q, const void* k_n
 }
 
 int tmw_poll_status(void* stream) {
-    TMW_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
     int* word = tmw::device_status_word();
     if (word == nullptr) return TMW_ERR_CUDA;
     int value[4] = {0, 0, 0, 0};
-    TMW_CUDA_TRY(cudaMemcpy(value, word, sizeof(value), cudaMemcpyDeviceToHost));
+    TMW_CUDA_TRY(cudaMemcpyAsync(value, word, sizeof(value), cudaMemcpyDeviceToHost, s));
+    TMW_CUDA_TRY(cudaStreamSynchronize(s));
     if (value[0] != 0) {
-        const int zero[4] = {0, 0, 0, 0};
-        TMW_CUDA_TRY(cudaMemcpy(word, zero, sizeof(zero), cudaMemcpyHostToDevice));
+        TMW_CUDA_TRY(cudaMemsetAsync(word, 0, sizeof(value), s));
+        TMW_CUDA_TRY(cudaStreamSynchronize(s));
         char text[160];
         if (value[0] == TMW_ERR_INVALID_ARGUMENT) {
-            tmw::set_error_text("a kernel met an invalid device-side argument (a negative entry of pos in a decode call)");
+            tmw::set_error_text("a kernel met an invalid device-side argument (a token id, label or position outside its table, a negative pos)");
             return TMW_ERR_INVALID_ARGUMENT;
         }
         if (value[1] == -1)

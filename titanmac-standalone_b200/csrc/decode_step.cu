@@ -10,6 +10,8 @@
 //     up in a fixed order);
 //   * the kernels are launched as programmatic dependents: a kernel's weights are on their way into registers before
 //     its predecessor has finished.
+#include <math_constants.h>
+
 #include "tmw_common.cuh"
 
 namespace tmw {
@@ -392,11 +394,10 @@ __global__ void __launch_bounds__(128) embed_rows_kernel(const EmbedParams p) {
     if (row >= p.rows) return;
     long long id = p.ids[row];
     int pos = p.pos[row];
-    if (id < 0 || id >= p.vocab || pos < 0 || pos >= p.max_pos) {
-        // outside the tables: the nearest row stands in, and the status word says so
+    const bool bad = id < 0 || id >= p.vocab || pos < 0 || pos >= p.max_pos;
+    if (bad) {  // outside the tables: a row of NaN, and the status word says so
         if (lane == 0) atomicCAS(p.status, 0, (int)TMW_ERR_INVALID_ARGUMENT);
-        id = id < 0 ? 0 : id >= p.vocab ? p.vocab - 1 : id;
-        pos = pos < 0 ? 0 : pos >= p.max_pos ? p.max_pos - 1 : pos;
+        id = pos = 0;
     }
     const T* a = static_cast<const T*>(p.tokens) + id * p.dim;
     const T* b = static_cast<const T*>(p.positions) + (long long)pos * p.dim;
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(128) embed_rows_kernel(const EmbedParams p) {
         load8<T>(b + v * 8, w);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            u[e] = to_f32<T>(from_f32<T>(u[e] + w[e]));
+            u[e] = bad ? CUDART_NAN_F : to_f32<T>(from_f32<T>(u[e] + w[e]));
             ss = fmaf(u[e], u[e], ss);
         }
         store8<T>(x + v * 8, u);

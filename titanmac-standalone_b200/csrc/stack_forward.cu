@@ -2,6 +2,8 @@
 // here as a chain of dependent launches (see pdl_wait) instead of one by one from Python.  With six to eight calls per
 // block at 15 - 20 us of host work each, a 16-layer model took 4 ms to issue - more than the GPU needs below about
 // 8000 rows - and a single layer of 144 rows 80 us for 15 us of kernels.
+#include <math_constants.h>
+
 #include "tmw_common.cuh"
 
 namespace tmw {
@@ -32,11 +34,13 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) embed_seq_kernel(const Embed
         const long long b = row / len;
         const int i = (int)(row - b * len) - p.np;
         const T *src = static_cast<const T*>(p.persistent) + (long long)(i + p.np) * p.dim, *add = nullptr;
+        bool bad = false;
         if (i >= 0) {
             long long id = p.ids[b * p.seq + i];
-            if (id < 0 || id >= p.vocab) {  // outside the table: the nearest row stands in, and the status word says so
+            if (id < 0 || id >= p.vocab) {  // outside the table: a row of NaN, and the status word says so
                 if (lane == 0) atomicCAS(p.status, 0, (int)TMW_ERR_INVALID_ARGUMENT);
-                id = id < 0 ? 0 : p.vocab - 1;
+                bad = true;
+                id = 0;
             }
             src = static_cast<const T*>(p.tokens) + id * p.dim;
             add = static_cast<const T*>(p.positions) + (long long)i * p.dim;
@@ -50,7 +54,7 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) embed_seq_kernel(const Embed
                 float w[8];
                 load8<T>(add + v * 8, w);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) u[e] = to_f32<T>(from_f32<T>(u[e] + w[e]));
+                for (int e = 0; e < 8; ++e) u[e] = bad ? CUDART_NAN_F : to_f32<T>(from_f32<T>(u[e] + w[e]));
             }
 #pragma unroll
             for (int e = 0; e < 8; ++e) ss = fmaf(u[e], u[e], ss);

@@ -178,15 +178,17 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const SumParts p) {
 
 // ---- shifted cross-entropy ---------------------------------------------------------------------------------
 // Row (b, i) of the logits [batch, np + seq, vocab] predicts labels[b, i - np + 1]; rows without a label (the persistent
-// ones, the last, label = ignore) do not count.
+// ones, the last, label = kIgnore) do not count.  A label outside the vocabulary makes loss and gradient NaN, and the status
+// word says so.
+constexpr long long kIgnore = -100, kBadLabel = -1;
 __device__ __forceinline__ long long label_of(const CrossEntropy& p, int row) {
     const int len = p.np + p.seq, b = row / len, t = row - b * len - p.np;
-    if (t < 0 || t + 1 >= p.seq) return -100;
+    if (t < 0 || t + 1 >= p.seq) return kIgnore;
     const long long y = p.labels[(long long)b * p.seq + t + 1];
-    if (y == -100) return y;
+    if (y == kIgnore) return y;
     if (y < 0 || y >= p.vocab) {
         if (threadIdx.x == 0) atomicCAS(p.status, 0, (int)TMW_ERR_INVALID_ARGUMENT);
-        return -100;
+        return kBadLabel;
     }
     return y;
 }
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(256) ce_forward_kernel(const CrossEntropy p) {
     const int row = blockIdx.x, tid = threadIdx.x;
     const long long y = label_of(p, row);
     if (y < 0) {
-        if (tid == 0) p.row_loss[row] = -1.f;  // (a loss is never negative)
+        if (tid == 0) p.row_loss[row] = y == kIgnore ? -1.f : CUDART_NAN_F;  // (a loss is never negative)
         return;
     }
     const T* x = static_cast<const T*>(p.logits) + (long long)row * p.vocab;
@@ -290,7 +292,10 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(const CrossEntropy p) 
     const int nvec = p.vocab / 8;
     const long long y = label_of(p, row);
     if (y < 0) {
-        for (int v = tid; v < nvec; v += 256) *reinterpret_cast<uint4*>(d + (long long)v * 8) = make_uint4(0u, 0u, 0u, 0u);
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = y == kIgnore ? 0.f : CUDART_NAN_F;
+        for (int v = tid; v < nvec; v += 256) store8<T>(d + (long long)v * 8, f);
         return;
     }
     const float scale = to_f32<T>(*static_cast<const T*>(p.grad)) / p.count[0], lse = p.lse[row];

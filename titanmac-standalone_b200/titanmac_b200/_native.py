@@ -750,10 +750,14 @@ def add_rmsnorm(x: torch.Tensor, residual: Optional[torch.Tensor], scale: torch.
 
 
 def poll_status(device: Optional[torch.device] = None) -> None:
-    """Synchronise the current stream and raise if a kernel reported an expired bounded wait."""
+    """Synchronise the current stream and raise if a kernel reported an expired bounded wait or an id, label or position
+    outside its table."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
-        check(lib().tmw_poll_status(_stream_ptr(dev)))
+        status = lib().tmw_poll_status(_stream_ptr(dev))
+    if status == TMW_ERR_INVALID_ARGUMENT:  # (met by a kernel: the text says what)
+        raise TmwError(status, lib().tmw_last_cuda_error().decode())
+    check(status)
 
 
 def default_scale(head_dim: int) -> float:

@@ -18,6 +18,8 @@ from typing import Callable, List, Optional, Sequence
 
 import torch
 
+from . import _native
+
 
 class HostPipeline:
     def __init__(self, fn: Callable[[torch.Tensor], torch.Tensor], shape: Sequence[int], dtype: torch.dtype,
@@ -76,6 +78,10 @@ class HostPipeline:
             stream.wait_stream(s)
 
     def drain(self) -> None:
+        """Wait for everything submitted; raise if a libtmw kernel has reported an error (``tmw_poll_status``)."""
         self.copy_out.synchronize()
         self.compute.synchronize()
         self.copy_in.synchronize()
+        if _native._lib is not None:
+            with torch.cuda.stream(self.compute):
+                _native.poll_status(self.device)

@@ -73,6 +73,11 @@ class TitanMAC(nn.Module):
 
     def forward(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None,
                 attention_mask: Optional[torch.Tensor] = None) -> Dict[str, torch.Tensor]:
+        """``{"logits": [B, T, V]}`` and, with ``labels``, ``"loss"``.
+
+        An id or label outside the vocabulary is met on the device: in 16-bit types its sequence's logits, or the loss and
+        the gradients, are NaN, and ``_native.poll_status`` (which synchronises) raises; otherwise PyTorch's own device-side
+        check ends the process's CUDA context.  ``decode_step`` likewise, for its positions too."""
         Np = self.config.n_persistent
         rows = None  # logits of every row, persistent rows first
         if torch.is_grad_enabled() and any(p.requires_grad for p in self.parameters()):
