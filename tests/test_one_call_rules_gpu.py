@@ -159,3 +159,26 @@ def test_the_model_as_it_is_at_the_call(change, monkeypatch):
     assert not torch.equal(first, got)
     assert got.dtype == want.dtype and close(got, want, 2e-2)
     assert not close(first.to(want.dtype), want, 2e-2)  # (the change is large enough to be told from rounding)
+
+
+def _shared_mlp(m):
+    m.layers[1].mlp.fc1.weight = m.layers[0].mlp.fc1.weight
+
+
+def _shared_block(m):
+    m.layers[1] = m.layers[0]
+
+
+def _shared_norm(m):
+    m.layers[0].norm_mlp = m.layers[0].norm_attn
+
+
+@pytest.mark.parametrize("share", [_shared_mlp, _shared_block, _shared_norm], ids=lambda f: f.__name__[1:])
+def test_gradients_of_shared_parameters_add_up(share, monkeypatch):
+    model, ids = make()
+    share(model)
+    _, got = step(model, ids)
+    module_by_module(monkeypatch)
+    _, want = step(model, ids)
+    for name in want:
+        assert close(got[name], want[name], 6e-2), name
