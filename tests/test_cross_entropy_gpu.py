@@ -46,7 +46,7 @@ def test_logits_that_are_not_ordinary(kind, dtype, V):
     special(kind, x, labels, n_p)
     with torch.enable_grad():  # (other tests may have turned it off)
         a = x.clone().requires_grad_(True)
-        loss = _train.shifted_cross_entropy(a, labels, n_p)
+        loss = _train.shifted_cross_entropy(a, labels, n_p)[1]
         loss.backward()
         b = x.double().requires_grad_(True)
         want = F.cross_entropy(b[:, n_p:-1].reshape(-1, V), labels[:, 1:].reshape(-1), ignore_index=-100)

@@ -182,3 +182,35 @@ def test_gradients_of_shared_parameters_add_up(share, monkeypatch):
     _, want = step(model, ids)
     for name in want:
         assert close(got[name], want[name], 6e-2), name
+
+
+@pytest.mark.parametrize("n_p", [0, 3])
+def test_the_loss_depends_on_the_logits_that_are_returned(n_p):
+    """Their gradient is there to be kept, hooked and added to."""
+    model, ids = make(n_p=n_p)
+    with torch.enable_grad():
+        out = model(ids, labels=ids)
+        logits = out["logits"]
+        logits.retain_grad()
+        out["loss"].backward()
+        a = logits.detach().float().requires_grad_(True)
+        torch.nn.functional.cross_entropy(a[:, :-1].reshape(-1, 128), ids[:, 1:].reshape(-1)).backward()
+        assert close(logits.grad, a.grad, 1e-2)
+
+        def grads(two_terms, factor):
+            model.zero_grad(set_to_none=True)
+            out = model(ids, labels=ids)
+            if factor != 1:
+                out["logits"].register_hook(lambda g: g * factor)
+            total = out["loss"] + (out["logits"].float().square().mean() if two_terms else 0.0)
+            total.backward()
+            return {n: p.grad.clone() for n, p in model.named_parameters()}
+
+        one, doubled = grads(False, 1), grads(False, 2)
+        for name in one:
+            assert close(doubled[name], 2 * one[name].float(), 3e-2), name
+        both = grads(True, 1)
+        model.zero_grad(set_to_none=True)
+        model(ids)["logits"].float().square().mean().backward()
+        for name, prm in model.named_parameters():
+            assert close(both[name], one[name].float() + prm.grad.float(), 3e-2), name

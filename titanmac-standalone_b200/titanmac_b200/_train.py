@@ -83,44 +83,83 @@ def stack_forward(model, input_ids: torch.Tensor) -> Optional[torch.Tensor]:
     return _StackTrain.apply(table, input_ids.contiguous(), *params)
 
 
-class _ShiftedCrossEntropy(torch.autograd.Function):
-    """Mean cross-entropy of ``logits [B, Np + T, V]``, row ``Np + t`` against ``labels[:, t + 1]`` (-100: not counted)."""
+class _SequenceRows(torch.autograd.Function):
+    """``rows [B, Np + T, V]`` → its sequence rows ``[B, T, V]``, the logits that the caller sees and the loss depends on.  Slicing
+    would cost a pass over the gradient of all rows on the way back; where the gradient that arrives is the one the loss's
+    backward has just written inside a gradient of all rows (``whole``), that one is handed on."""
 
     @staticmethod
-    def forward(ctx, logits: torch.Tensor, labels: torch.Tensor, n_persistent: int) -> torch.Tensor:
-        B, L, V = logits.shape
-        loss = torch.empty((), dtype=logits.dtype, device=logits.device)
-        stats = torch.empty(4 + 2 * B * L, dtype=torch.float32, device=logits.device)
-        with _native._on(logits.device):
-            _native.check(_native.lib().tmw_cross_entropy(_native._DTYPES[logits.dtype], B, L - n_persistent, n_persistent, V,
-                                                          logits.data_ptr(), labels.data_ptr(), loss.data_ptr(), stats.data_ptr(),
-                                                          None, None, _native._stream_ptr(logits.device)))
-        ctx.save_for_backward(logits, labels, stats)
-        ctx.n_persistent = n_persistent
+    def forward(ctx, rows: torch.Tensor, n_persistent: int, whole: list) -> torch.Tensor:
+        ctx.n_persistent, ctx.whole = n_persistent, whole
+        return rows[:, n_persistent:].detach()  # (not a view to autograd, which would not let the caller change it)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, d_logits: torch.Tensor):
+        n = ctx.n_persistent
+        if ctx.whole:
+            d_rows = ctx.whole.pop()  # (held until here: no other tensor can have its address)
+            own = d_rows[:, n:]
+            if d_logits.data_ptr() == own.data_ptr() and d_logits.stride() == own.stride() and d_logits.shape == own.shape:
+                return d_rows, None, None
+        B, T, V = d_logits.shape
+        d_rows = d_logits.new_empty((B, n + T, V))
+        d_rows[:, :n] = 0
+        d_rows[:, n:] = d_logits
+        return d_rows, None, None
+
+
+class _ShiftedCrossEntropy(torch.autograd.Function):
+    """Mean cross-entropy of ``rows [B, Np + T, V]``, row ``Np + t`` against ``labels[:, t + 1]`` (-100: not counted).  The
+    gradient goes to ``logits``, the sequence rows; ``whole`` keeps it as part of a gradient of all rows."""
+
+    @staticmethod
+    def forward(ctx, logits: torch.Tensor, rows: torch.Tensor, labels: torch.Tensor, n_persistent: int, whole: list) -> torch.Tensor:
+        B, L, V = rows.shape
+        loss = torch.empty((), dtype=rows.dtype, device=rows.device)
+        stats = torch.empty(4 + 2 * B * L, dtype=torch.float32, device=rows.device)
+        with _native._on(rows.device):
+            _native.check(_native.lib().tmw_cross_entropy(_native._DTYPES[rows.dtype], B, L - n_persistent, n_persistent, V,
+                                                          rows.data_ptr(), labels.data_ptr(), loss.data_ptr(), stats.data_ptr(),
+                                                          None, None, _native._stream_ptr(rows.device)))
+        ctx.save_for_backward(rows, labels, stats)
+        ctx.n_persistent, ctx.whole = n_persistent, whole
         return loss
 
     @staticmethod
     @once_differentiable
     def backward(ctx, grad: torch.Tensor):
-        logits, labels, stats = ctx.saved_tensors
-        B, L, V = logits.shape
-        d_logits = torch.empty_like(logits)
+        rows, labels, stats = ctx.saved_tensors
+        B, L, V = rows.shape
+        n = ctx.n_persistent
+        d_rows = torch.empty_like(rows)
         grad = grad.contiguous()
-        with _native._on(logits.device):
-            _native.check(_native.lib().tmw_cross_entropy(_native._DTYPES[logits.dtype], B, L - ctx.n_persistent, ctx.n_persistent,
-                                                          V, logits.data_ptr(), labels.data_ptr(), None, stats.data_ptr(),
-                                                          grad.data_ptr(), d_logits.data_ptr(), _native._stream_ptr(logits.device)))
-        return d_logits, None, None
+        with _native._on(rows.device):
+            _native.check(_native.lib().tmw_cross_entropy(_native._DTYPES[rows.dtype], B, L - n, n, V, rows.data_ptr(),
+                                                          labels.data_ptr(), None, stats.data_ptr(), grad.data_ptr(),
+                                                          d_rows.data_ptr(), _native._stream_ptr(rows.device)))
+        if n == 0:
+            return d_rows, None, None, None, None
+        ctx.whole[:] = [d_rows]
+        return d_rows[:, n:], None, None, None, None
 
 
-def shifted_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, n_persistent: int) -> Optional[torch.Tensor]:
-    """``logits``: every row, persistent rows first.  None where the library's kernel does not apply."""
-    B, L, V = logits.shape
-    if (logits.dtype not in (torch.bfloat16, torch.float16) or not logits.is_cuda or not logits.is_contiguous() or V % 8
-            or logits.data_ptr() % 16 or labels.dtype != torch.int64 or labels.shape != (B, L - n_persistent)
-            or labels.device != logits.device or B == 0 or L == n_persistent or _autocast()):
+def shifted_cross_entropy(rows: torch.Tensor, labels: torch.Tensor, n_persistent: int):
+    """``(logits, loss)`` of ``rows``, every row's logits, persistent rows first: the sequence rows and their mean shifted
+    cross-entropy, which depends on them.  None where the library's kernel does not apply."""
+    B, L, V = rows.shape
+    if (rows.dtype not in (torch.bfloat16, torch.float16) or not rows.is_cuda or not rows.is_contiguous() or V % 8
+            or rows.data_ptr() % 16 or labels.dtype != torch.int64 or labels.shape != (B, L - n_persistent)
+            or labels.device != rows.device or B == 0 or L == n_persistent or _autocast()):
         return None
-    return _ShiftedCrossEntropy.apply(logits, labels.contiguous(), n_persistent)
+    whole: list = []
+    if n_persistent == 0:
+        logits = rows
+    elif rows.requires_grad and torch.is_grad_enabled():
+        logits = _SequenceRows.apply(rows, n_persistent, whole)
+    else:
+        logits = rows[:, n_persistent:]
+    return logits, _ShiftedCrossEntropy.apply(logits, rows.detach(), labels.contiguous(), n_persistent, whole)
 
 
 class _AttentionTrain(torch.autograd.Function):

@@ -73,7 +73,8 @@ class TitanMAC(nn.Module):
 
     def forward(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None,
                 attention_mask: Optional[torch.Tensor] = None) -> Dict[str, torch.Tensor]:
-        """``{"logits": [B, T, V]}`` and, with ``labels``, ``"loss"``.
+        """``{"logits": [B, T, V]}`` and, with ``labels``, ``"loss"``, whose backward reads the logits: until then change a copy
+        of them, not themselves.
 
         An id or label outside the vocabulary is met on the device: in 16-bit types its sequence's logits, or the loss and
         the gradients, are NaN, and ``_native.poll_status`` (which synchronises) raises; otherwise PyTorch's own device-side
@@ -91,8 +92,10 @@ class TitanMAC(nn.Module):
         logits = rows[:, Np:, :] if Np > 0 else rows
         out = {"logits": logits}
         if labels is not None:
-            loss = _train.shifted_cross_entropy(rows, labels, Np)
-            if loss is None:
+            found = _train.shifted_cross_entropy(rows, labels, Np)
+            if found is not None:
+                out["logits"], loss = found
+            else:
                 shift_logits = logits[..., :-1, :].contiguous()
                 shift_labels = labels[..., 1:].contiguous()
                 loss = F.cross_entropy(shift_logits.reshape(-1, self.config.vocab_size), shift_labels.reshape(-1),
