@@ -214,3 +214,17 @@ def test_the_loss_depends_on_the_logits_that_are_returned(n_p):
         model(ids)["logits"].float().square().mean().backward()
         for name, prm in model.named_parameters():
             assert close(both[name], one[name].float() + prm.grad.float(), 3e-2), name
+
+
+def test_a_gradient_of_the_logits_at_an_odd_address():
+    model, ids = make(n_p=0)
+    with torch.enable_grad():
+        logits = model(ids)["logits"]
+        extra = torch.zeros(3, device=DEV, dtype=BF16, requires_grad=True)
+        g = torch.randn(3 + logits.numel(), device=DEV, dtype=BF16)
+        torch.cat([extra, logits.reshape(-1)]).backward(g)  # the second part of g: contiguous, 6 bytes into it
+        got = {n: p.grad.clone() for n, p in model.named_parameters()}
+        model.zero_grad(set_to_none=True)
+        model(ids)["logits"].backward(g[3:].clone().view_as(logits))
+    for name, prm in model.named_parameters():
+        assert close(got[name], prm.grad, 1e-2), name

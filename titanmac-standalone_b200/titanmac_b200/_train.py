@@ -19,6 +19,12 @@ def _autocast() -> bool:
     return torch.is_autocast_enabled("cuda")
 
 
+def _aligned(grad: torch.Tensor) -> torch.Tensor:
+    """The gradient contiguous and at an address the kernels take (autograd may hand over any part of a larger one)."""
+    grad = grad.contiguous()
+    return grad.clone() if grad.data_ptr() % 16 else grad
+
+
 class _StackTrain(torch.autograd.Function):
     """``ids [B, T]`` → logits of every row ``[B, Np + T, V]``."""
 
@@ -43,7 +49,7 @@ class _StackTrain(torch.autograd.Function):
     def backward(ctx, d_logits: torch.Tensor):
         ids, saved, *params = ctx.saved_tensors
         d = _native.StackDesc.from_buffer_copy(ctx.desc)
-        d_logits = d_logits.contiguous()
+        d_logits = _aligned(d_logits)
         # the parameters' addresses as they are now, and their gradients'
         blocks, block_grads = (_native.Block * d.layers)(), (_native.BlockGrads * d.layers)()
         grads, out = _native.StackGrads(), []
@@ -182,9 +188,7 @@ class _AttentionTrain(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, dy: torch.Tensor):
         x, saved, w_qkv, w_out, *conv = ctx.saved_tensors
-        dy = dy.contiguous()
-        if dy.data_ptr() % 16:
-            dy = dy.clone()
+        dy = _aligned(dy)
         lib, ref, device = _native.lib(), ctypes.byref(ctx.desc), x.device
         nbytes = lib.tmw_attention_train_scratch(ref)
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
