@@ -228,3 +228,17 @@ def test_a_gradient_of_the_logits_at_an_odd_address():
         model(ids)["logits"].backward(g[3:].clone().view_as(logits))
     for name, prm in model.named_parameters():
         assert close(got[name], prm.grad, 1e-2), name
+
+
+def test_options_of_the_embedding_tables(monkeypatch):
+    model, ids = make(tie_weights=False)
+    step(model, ids)
+    model.embed_tokens.padding_idx = int(ids[0, 0])
+    _, got = step(model, ids)
+    assert not got["embed_tokens.weight"][ids[0, 0]].any()
+    model.embed_tokens.padding_idx = None
+    model.embed_tokens.scale_grad_by_freq = True
+    _, got = step(model, ids)
+    module_by_module(monkeypatch)
+    _, want = step(model, ids)
+    assert close(got["embed_tokens.weight"], want["embed_tokens.weight"], 5e-2)

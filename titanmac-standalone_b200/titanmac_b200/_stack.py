@@ -199,7 +199,9 @@ class ModelTable:
         self.decodes = c.d_head in (64, 128) and F % 32 == 0 and D <= 4096 and self.kind == (0, 0)
         self.forwards = V % 8 == 0 and F % 8 == 0 and D % 8 == 0 and c.d_head % 8 == 0 and self.kind[1] <= 8
         # the backward writes a gradient once per place; only for the table that is also the head it adds the places up
-        self.trains = self.forwards and D <= 2048 and all(
+        # (and it knows nothing of an embedding table's options)
+        options = [attributes(t, "padding_idx", "scale_grad_by_freq", "sparse") for t in tops[:2]]
+        self.trains = self.forwards and D <= 2048 and options == [(None, False, False)] * 2 and all(
             len(places) == 1 or set(places) == {(-1, "embed_tokens"), (-1, "head")} for places in self.roles)
         self.workspace_bytes: dict = {}  # (batch, tokens) -> bytes; tokens = -1: a decode step
         self.ok = True
