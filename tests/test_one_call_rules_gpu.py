@@ -242,3 +242,19 @@ def test_options_of_the_embedding_tables(monkeypatch):
     module_by_module(monkeypatch)
     _, want = step(model, ids)
     assert close(got["embed_tokens.weight"], want["embed_tokens.weight"], 5e-2)
+
+
+def test_deterministic_algorithms_when_asked_for():
+    """Tokens that repeat a thousand times: sums in no fixed order would differ between the passes."""
+    model, _ = make(vocab=64)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    ids = torch.randint(0, 4, (300, 60), generator=g, device=DEV)
+    torch.use_deterministic_algorithms(True, warn_only=True)
+    try:
+        with torch.enable_grad():
+            assert _train.stack_forward(model, ids) is None
+        grads = [step(model, ids)[1]["embed_tokens.weight"].clone() for _ in range(4)]
+    finally:
+        torch.use_deterministic_algorithms(False)
+    for g2 in grads[1:]:
+        assert torch.equal(grads[0], g2)

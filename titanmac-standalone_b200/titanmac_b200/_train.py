@@ -77,8 +77,9 @@ class _StackTrain(torch.autograd.Function):
 def stack_forward(model, input_ids: torch.Tensor) -> Optional[torch.Tensor]:
     """Logits of every row with a gradient to every parameter, or None where that takes the modules themselves."""
     table = _stack.table_of(model, training=True)
-    if table is None or not table.trains or _autocast() or input_ids.dtype != torch.int64 or input_ids.dim() != 2 \
-            or input_ids.device != table.device:
+    # (tokens that repeat are added up with atomics: not in a fixed order, as the library's embedding backward does)
+    if table is None or not table.trains or _autocast() or torch.are_deterministic_algorithms_enabled() \
+            or input_ids.dtype != torch.int64 or input_ids.dim() != 2 or input_ids.device != table.device:
         return None
     B, T = input_ids.shape
     if B == 0 or T == 0 or T > table.desc.max_positions or B * (T + table.desc.n_persistent) >= (1 << 31) // 8:
