@@ -158,3 +158,23 @@ def test_decode_step_sizes_the_library_refuses():
     assert workspace() > 0 and workspace(batch=65535) > 0
     assert workspace(d_model=5120, heads=40) == 0 and workspace(batch=65536) == 0
     assert workspace(head_dim=32, heads=128) == 0 and workspace(d_ff=48) == 0
+
+
+def test_scratch_of_a_training_step_follows_its_size():
+    """No room for split products where the rows are too few to be cut; never more than 24 MiB a product."""
+    lib = _native.lib()
+
+    def module(rows, dim=128):
+        d = _native.AttentionDesc(_native.TMW_BF16, 1, rows, dim // 64, 64, 16, 3, 0, 0, 0.0)
+        return lib.tmw_attention_train_scratch(ctypes.byref(d)), 4 * rows * dim * 2
+
+    def stack(tokens, dim=128):
+        d = _native.StackDesc(dtype=_native.TMW_BF16, batch=1, layers=2, d_model=dim, heads=dim // 64, head_dim=64, d_ff=2 * dim,
+                              window=16, n_persistent=0, vocab=512, max_positions=tokens, eps=1e-5)
+        return lib.tmw_stack_train_scratch(ctypes.byref(d), tokens), tokens * dim * 2 * (3 + 2 + 3)
+
+    for size in (module, stack):
+        nbytes, activations = size(128)
+        assert activations <= nbytes <= 4 * activations + (1 << 20)
+        nbytes, activations = size(100000, 1024)
+        assert activations + (8 << 20) <= nbytes <= 4 * activations + (200 << 20)

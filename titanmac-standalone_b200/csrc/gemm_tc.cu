@@ -752,6 +752,8 @@ int launch_gemm_call(const GemmCall& call, cudaStream_t stream) {
     return launch_variant(best, g, width, stream);
 }
 
+int gemm_most_splits(int k) { return k / (4 * GK) < 32 ? k / (4 * GK) : 32; }
+
 // A product with a long k and a small output (a weight gradient: k = rows of the batch): k is cut into as many ranges as
 // pays, each leaving fp32 sums in `partial`, and *splits says how many (1: the output itself was written).  Every range
 // costs a trip of m x n fp32 values through memory and back, at about 4 TB/s, and a launch.
@@ -763,7 +765,7 @@ int launch_gemm_splitk(const GemmCall& call, size_t partial_bytes, int* splits, 
     float least = 0.f;
     for (int i = 0; i < 4; ++i) {
         if (i == 1) continue;
-        for (int s = 1; s <= 32 && (s == 1 || (s * out <= partial_bytes && g.k >= s * 4 * GK)); ++s) {
+        for (int s = 1; s == 1 || (s <= gemm_most_splits(g.k) && s * out <= partial_bytes); ++s) {
             int width = 256;
             const float t = variant_cost(i, g, s, sms, &width) + (s > 1 ? 2.5f + 2.f * (float)(s * out) / 4e6f : 0.f);
             if ((i == 0 && s == 1) || t < least) {

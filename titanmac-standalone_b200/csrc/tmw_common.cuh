@@ -314,6 +314,7 @@ struct GemmCall {
     float* partial = nullptr;
 };
 int launch_gemm_call(const GemmCall& g, cudaStream_t stream);
+int gemm_most_splits(int k);  // into how many ranges launch_gemm_splitk cuts a k at most
 int launch_gemm_splitk(const GemmCall& g, size_t partial_bytes, int* splits, cudaStream_t stream);
 int launch_linear(const tmw_linear_desc& d, const void* a, const void* w, const void* bias, void* c,
                   cudaStream_t stream, int chain = 0);

@@ -13,7 +13,7 @@ namespace {
 int64_t align256(int64_t n) { return (n + 255) & ~(int64_t)255; }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-constexpr int64_t kPartialBytes = 96ll << 20;  // room for the split products of a block (each at most a quarter)
+constexpr int64_t kPartBytes = 24ll << 20;  // what the ranges of one split product may take
 
 struct Dims {
     int dtype, B, L, H, dh, D, F, np, window, block, taps;
@@ -32,6 +32,13 @@ tmw_prefill_desc core_desc(const Dims& d) {
         c.o_stride[i] = out[i];
     }
     return c;
+}
+
+// Room for the ranges of the product whose output is [n, k] and whose sum runs over the rows: what launch_gemm_splitk can ask
+// for at most, so that a small batch does not come with megabytes of scratch.
+int64_t split_room(const Dims& d, int64_t n, int64_t k) {
+    const int64_t splits = gemm_most_splits(d.rows()), bytes = splits * n * k * 4;
+    return splits < 2 ? 0 : align256(bytes < kPartBytes ? bytes : kPartBytes);
 }
 
 // c[m, n] = a[m, k] w[n, k]^T
@@ -68,7 +75,7 @@ struct Pending {
         g.c = dw; g.ldc = k; g.chain = chain;
         g.partial = reinterpret_cast<float*>(base + used);
         int splits = 1;
-        const int64_t left = room - used, most = left < kPartialBytes / 4 ? left : kPartialBytes / 4;
+        const int64_t left = room - used, most = left < kPartBytes ? left : kPartBytes;
         const int rc = launch_gemm_splitk(g, (size_t)(most > 0 ? most : 0), &splits, s);
         if (rc == TMW_OK && splits > 1) sums.add(take((int64_t)splits * n * k), dw, (int64_t)n * k, splits);
         return rc;
@@ -188,6 +195,7 @@ struct StackScratch {
     AttentionScratch attn;
     float *norm_parts[4];
     char* partial;
+    int64_t room;  // of `partial` for the split products; behind it the column sums of fc1's bias
     int* owner;
     float* acc;
     int64_t total;
@@ -210,11 +218,14 @@ StackScratch stack_scratch(const Dims& d, int vocab, int tokens, char* base) {
     t.attn.d_conv = d.taps > 0 ? take(3 * row * d.D) : nullptr;
     t.attn.d_taps = reinterpret_cast<float*>(take((int64_t)3 * d.D * (d.taps > 0 ? d.taps : 1) * 4));
     for (float*& p : t.norm_parts) p = reinterpret_cast<float*>(take((int64_t)norm_bwd_blocks(R) * d.D * 4));
-    t.partial = take(kPartialBytes + (int64_t)colsum_strips((int)R) * d.F * 4);
+    const int64_t layer = 2 * split_room(d, d.F, d.D) + split_room(d, d.D, d.D) + split_room(d, 3 * d.D, d.D);
+    const int64_t head = split_room(d, vocab, d.D);
+    t.room = layer > head ? layer : head;
+    t.partial = take(t.room + (int64_t)colsum_strips((int)R) * d.F * 4);
     t.owner = reinterpret_cast<int*>(take((int64_t)vocab * 4));
     t.acc = reinterpret_cast<float*>(t.partial);  // (the partial results are used up by then)
     const int64_t acc = (int64_t)d.B * tokens * d.D * 4;
-    if (acc > kPartialBytes) t.acc = reinterpret_cast<float*>(take(acc));
+    if (acc > t.room) t.acc = reinterpret_cast<float*>(take(acc));
     t.total = at;
     return t;
 }
@@ -323,7 +334,7 @@ extern "C" int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_bl
     char* y_last = x_last + align256((int64_t)R * 2 * D);
     Pending pending;
     pending.base = t.partial;
-    pending.room = kPartialBytes;
+    pending.room = t.room;
     const int blocks_n = norm_bwd_blocks(R), strips = colsum_strips(R);
     // colsum_parts: column sums of t.g, the gradient of fc2's bias in the layer below
     auto norm_bwd = [&](const void* dy, const void* x, const void* gain, const void* add, void* out, float* dgain_part, float* sum_part,
@@ -350,7 +361,7 @@ extern "C" int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_bl
         if (rc == TMW_OK) rc = input_grad(d, R, D, F, t.pre, b.w_fc1, t.dy, GEMM_NONE, nullptr, kChainLink, s);
         if (rc == TMW_OK) rc = pending.weight_grad(d, R, F, D, t.pre, a.y2, q.w_fc1, kChainLink, s);
         if (rc == TMW_OK && q.b_fc1 != nullptr) {
-            float* part = reinterpret_cast<float*>(t.partial + kPartialBytes);
+            float* part = reinterpret_cast<float*>(t.partial + t.room);
             rc = launch_colsum(d.dtype, t.pre, part, R, F, s);
             pending.sums.add(part, q.b_fc1, F, strips);
         }
@@ -398,7 +409,7 @@ int validate_module(const tmw_attention_desc* a) {
 struct ModuleScratch {
     AttentionScratch attn;
     char* partial;
-    int64_t total;
+    int64_t room, total;
 };
 ModuleScratch module_scratch(const Dims& d, char* base) {
     const int64_t row = (int64_t)d.rows() * d.D * 2;
@@ -409,7 +420,8 @@ ModuleScratch module_scratch(const Dims& d, char* base) {
     char* p = t.attn.d_conv + (d.taps > 0 ? align256(3 * row) : 0);
     t.attn.d_taps = reinterpret_cast<float*>(p);
     t.partial = p + align256((int64_t)3 * d.D * 8 * 4);
-    t.total = t.partial - base + kPartialBytes;
+    t.room = split_room(d, d.D, d.D) + split_room(d, 3 * d.D, d.D);
+    t.total = t.partial - base + t.room;
     return t;
 }
 }  // namespace
@@ -454,7 +466,7 @@ extern "C" int tmw_attention_train_backward(const tmw_attention_desc* desc, cons
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Pending pending;
     pending.base = t.partial;
-    pending.room = kPartialBytes;
+    pending.room = t.room;
     const AttentionWeights w = {w_qkv, w_out, {conv_q, conv_k, conv_v}};
     const AttentionGrads g = {grads->w_qkv, grads->w_out, {grads->conv_q, grads->conv_k, grads->conv_v}};
     rc = attention_backward(d, x, w, attention_saved(d, static_cast<char*>(const_cast<void*>(saved))), dy, dx, g, t.attn, pending, true, s);
