@@ -89,3 +89,45 @@ def test_forward_equals_module_by_module(B, T, dtype, heads, dh, Np, block_spars
         want = model(ids)["logits"], attn(x)
     tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
     assert close(got[0], want[0], tol) and close(got[1], want[1], tol)
+
+
+@pytest.mark.parametrize("block_sparse", [False, True])
+@pytest.mark.parametrize("wanted", [("x",), ("qkv_proj",), ("out_proj",), ("x", "out_proj"), ("qkv_proj", "out_proj"), ("conv_k",),
+                                    ("x", "conv_q", "conv_v")])
+def test_only_the_gradients_that_are_wanted(block_sparse, wanted, monkeypatch):
+    """The attention module's backward asks the library for these alone, and they are what they are with all the others."""
+    if not block_sparse and any(n.startswith("conv") for n in wanted):
+        pytest.skip("no convolutions")
+    model, g = make(torch.bfloat16, 2, 64, 40, 5, 64, block_sparse, layers=1)
+    attn = model.layers[0].attention
+    x = torch.randn(3, 700, 128, generator=g, device=DEV).to(torch.bfloat16)
+    dy = torch.randn(3, 700, 128, generator=g, device=DEV).to(torch.bfloat16)
+
+    def grads(names):
+        out = {"x": x.clone().requires_grad_("x" in names)}
+        for name, prm in attn.named_parameters():
+            prm.grad = None
+            prm.requires_grad_(name.split(".")[0] in names)
+        with torch.enable_grad():
+            attn(out["x"]).backward(dy)
+        _native.poll_status(torch.device(DEV))
+        return {"x": out["x"].grad, **{n.split(".")[0]: p.grad for n, p in attn.named_parameters()}}
+
+    want = grads(["x"] + [n.split(".")[0] for n, _ in attn.named_parameters()])
+    asked, real = [], _native.lib()
+
+    class Spy:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def tmw_attention_train_backward(self, *a):
+            asked.append({n for n, p in [("x", a[9])] + [(n, getattr(a[10]._obj, n)) for n, _ in a[10]._obj._fields_] if p})
+            return real.tmw_attention_train_backward(*a)
+
+    monkeypatch.setattr(_native, "lib", lambda: Spy())
+    got = grads(wanted)
+    assert asked == [{n.replace("qkv_proj", "w_qkv").replace("out_proj", "w_out") for n in wanted}]
+    for name in want:
+        assert (got[name] is None) == (name not in wanted)
+        # (a filter's gradient is added up with atomics: the order of its fp32 sums is not fixed)
+        assert name not in wanted or (close(got[name], want[name], 1e-2) if "conv" in name else torch.equal(got[name], want[name])), name

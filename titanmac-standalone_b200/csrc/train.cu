@@ -141,13 +141,16 @@ struct AttentionScratch {
     float* d_taps;               // [3D, taps]
 };
 
-// dx = gradient of x given dy; weight gradients through `pending`
+// dx = gradient of x given dy; weight gradients through `pending`; none of what is not wanted (dx, g.*: nullptr)
 int attention_backward(const Dims& d, const void* x, const AttentionWeights& w, const AttentionSaved& a, const void* dy, void* dx,
                        const AttentionGrads& g, const AttentionScratch& t, Pending& pending, bool first, cudaStream_t s) {
     const int R = d.rows(), D = d.D;
-    int rc = input_grad(d, R, D, D, dy, w.w_out, t.d_o, GEMM_NONE, nullptr, first ? kChainFollowed : kChainLink, s);
-    if (rc == TMW_OK) rc = pending.weight_grad(d, R, D, D, dy, a.o, g.w_out, kChainLink, s);
-    if (rc != TMW_OK) return rc;
+    const bool through = dx != nullptr || g.w_qkv != nullptr || g.conv[0] != nullptr || g.conv[1] != nullptr || g.conv[2] != nullptr;
+    const int link = first ? kChainFollowed : kChainLink;
+    int rc = TMW_OK;
+    if (through) rc = input_grad(d, R, D, D, dy, w.w_out, t.d_o, GEMM_NONE, nullptr, link, s);
+    if (rc == TMW_OK && g.w_out != nullptr) rc = pending.weight_grad(d, R, D, D, dy, a.o, g.w_out, through ? kChainLink : link, s);
+    if (rc != TMW_OK || !through) return rc;
     const tmw_prefill_desc c = core_desc(d);
     const char *q = a.conv, *k = q + 2ll * D, *v = q + 4ll * D;
     char *dq = d.taps > 0 ? t.d_conv : t.d_qkv, *dk = dq + 2ll * D, *dv = dq + 4ll * D;
@@ -156,11 +159,13 @@ int attention_backward(const Dims& d, const void* x, const AttentionWeights& w, 
     if (rc == TMW_OK && d.taps > 0) {
         TMW_CUDA_TRY(cudaMemsetAsync(t.d_taps, 0, (size_t)3 * D * d.taps * sizeof(float), s));
         rc = launch_dwconv_backward(d.dtype, d.B, d.L, 3 * D, d.taps, a.qkv, w.conv, 3, dq, t.d_qkv, t.d_taps, s);
-        for (int i = 0; i < 3; ++i) pending.sums.add(t.d_taps + (int64_t)i * D * d.taps, g.conv[i], (int64_t)D * d.taps, 1);
+        for (int i = 0; i < 3; ++i)
+            if (g.conv[i] != nullptr) pending.sums.add(t.d_taps + (int64_t)i * D * d.taps, g.conv[i], (int64_t)D * d.taps, 1);
     }
-    // (the kernels in front take no part in chains: ordinary launches behind them)
-    if (rc == TMW_OK) rc = input_grad(d, R, D, 3 * D, t.d_qkv, w.w_qkv, dx, GEMM_NONE, nullptr, kChainFollowed, s);
-    if (rc == TMW_OK) rc = pending.weight_grad(d, R, 3 * D, D, t.d_qkv, x, g.w_qkv, kChainLink, s);
+    // (the kernels in front take no part in chains: an ordinary launch behind them)
+    if (rc == TMW_OK && dx != nullptr) rc = input_grad(d, R, D, 3 * D, t.d_qkv, w.w_qkv, dx, GEMM_NONE, nullptr, kChainFollowed, s);
+    if (rc == TMW_OK && g.w_qkv != nullptr)
+        rc = pending.weight_grad(d, R, 3 * D, D, t.d_qkv, x, g.w_qkv, dx != nullptr ? kChainLink : kChainFollowed, s);
     return rc;
 }
 
@@ -454,12 +459,13 @@ extern "C" int tmw_attention_train_backward(const tmw_attention_desc* desc, cons
     int rc = validate_module(desc);
     if (rc != TMW_OK) return rc;
     if (grads == nullptr) return TMW_ERR_INVALID_ARGUMENT;
-    const void* need[] = {x, w_qkv, w_out, dy, saved, dx, scratch, grads->w_qkv, grads->w_out};
+    const void* need[] = {x, w_qkv, w_out, dy, saved, scratch};
     for (const void* q : need)
         if (q == nullptr || !aligned16(q)) return TMW_ERR_INVALID_ARGUMENT;
-    if (desc->conv_taps > 0 && (conv_q == nullptr || conv_k == nullptr || conv_v == nullptr || grads->conv_q == nullptr ||
-                                grads->conv_k == nullptr || grads->conv_v == nullptr))
-        return TMW_ERR_INVALID_ARGUMENT;
+    const void* wanted[] = {dx, grads->w_qkv, grads->w_out, grads->conv_q, grads->conv_k, grads->conv_v};
+    for (const void* q : wanted)
+        if (!aligned16(q)) return TMW_ERR_INVALID_ARGUMENT;
+    if (desc->conv_taps > 0 && (conv_q == nullptr || conv_k == nullptr || conv_v == nullptr)) return TMW_ERR_INVALID_ARGUMENT;
     const Dims d = dims_of(*desc);
     const ModuleScratch t = module_scratch(d, static_cast<char*>(scratch));
     if (scratch_bytes < (size_t)t.total) return TMW_ERR_TOO_LARGE;
@@ -468,7 +474,9 @@ extern "C" int tmw_attention_train_backward(const tmw_attention_desc* desc, cons
     pending.base = t.partial;
     pending.room = t.room;
     const AttentionWeights w = {w_qkv, w_out, {conv_q, conv_k, conv_v}};
-    const AttentionGrads g = {grads->w_qkv, grads->w_out, {grads->conv_q, grads->conv_k, grads->conv_v}};
+    const bool conv = desc->conv_taps > 0;
+    const AttentionGrads g = {grads->w_qkv, grads->w_out, {conv ? grads->conv_q : nullptr, conv ? grads->conv_k : nullptr,
+                                                           conv ? grads->conv_v : nullptr}};
     rc = attention_backward(d, x, w, attention_saved(d, static_cast<char*>(const_cast<void*>(saved))), dy, dx, g, t.attn, pending, true, s);
     return rc != TMW_OK ? rc : pending.flush(d, s);
 }

@@ -193,18 +193,19 @@ class _AttentionTrain(torch.autograd.Function):
         lib, ref, device = _native.lib(), ctypes.byref(ctx.desc), x.device
         nbytes = lib.tmw_attention_train_scratch(ref)
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        dx = torch.empty_like(x)
-        weights = (w_qkv, w_out, *conv)
-        out = [torch.empty_like(w) for w in weights]
+        need = ctx.needs_input_grad
+        dx = torch.empty_like(x) if need[1] else None
+        out = [torch.empty_like(w) if n else None for w, n in zip((w_qkv, w_out, *conv), need[2:])]
         grads = _native.BlockGrads()
         for name, g in zip(("w_qkv", "w_out", "conv_q", "conv_k", "conv_v"), out):
-            setattr(grads, name, g.data_ptr())
+            if g is not None:  # (the library leaves out what is not wanted)
+                setattr(grads, name, g.data_ptr())
         with _native._on(device):
             _native.check(lib.tmw_attention_train_backward(ref, x.data_ptr(), w_qkv.data_ptr(), *_conv_ptrs(conv), w_out.data_ptr(),
-                                                           dy.data_ptr(), saved.data_ptr(), dx.data_ptr(), ctypes.byref(grads),
-                                                           scratch.data_ptr(), nbytes, _native._stream_ptr(device)))
-        need = ctx.needs_input_grad
-        return (None, dx if need[1] else None, *(g if n else None for g, n in zip(out, need[2:])))
+                                                           dy.data_ptr(), saved.data_ptr(), dx.data_ptr() if need[1] else None,
+                                                           ctypes.byref(grads), scratch.data_ptr(), nbytes,
+                                                           _native._stream_ptr(device)))
+        return (None, dx, *out)
 
 
 def _conv_ptrs(conv):
