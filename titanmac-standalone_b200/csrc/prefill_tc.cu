@@ -426,7 +426,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 }
                 if (more) qk(next);
                 else if (SB == 2 && i == q.n_items - 2) tc_commit(bar(BAR_PV_DONE));
-                else if (i == q.n_items - 1) tc_commit(bar(BAR_O_DONE));
+                else {  // the last item.  (Its V stage is not handed back: behind O_DONE nothing would keep the CTA's shared
+                        // memory until that arrival has come in.)
+                    tc_commit(bar(BAR_O_DONE));
+                    break;
+                }
                 if (!pers) {
                     tc_commit(bar(BAR_V_EMPTY + v_stage));
                     if (++v_stage == VS) { v_stage = 0; v_par ^= 1u; }
