@@ -158,6 +158,10 @@ def test_decode_step_sizes_the_library_refuses():
     assert workspace() > 0 and workspace(batch=65535) > 0
     assert workspace(d_model=5120, heads=40) == 0 and workspace(batch=65536) == 0
     assert workspace(head_dim=32, heads=128) == 0 and workspace(d_ff=48) == 0
+    # a long window over few (sequence, head) pairs is split over more CTAs than a cluster holds, through the workspace
+    few = dict(batch=1, d_model=640, heads=10, head_dim=64)
+    assert workspace(**few, window=4095) > workspace(**few, window=4094) == workspace(**few)
+    assert workspace(**dict(few, batch=64), window=4095) == workspace(**dict(few, batch=64))
 
 
 def test_scratch_of_a_training_step_follows_its_size():

@@ -57,6 +57,41 @@ def test_step_equals_module_by_module(B, dtype, heads, dh, window, Np, vocab, t,
             assert ((x.float() - y.float()).norm() / y.float().norm()).item() <= tol
 
 
+@pytest.mark.parametrize("B,dtype,heads,dh,window,n_p,t", [
+    (1, torch.bfloat16, 2, 64, 4094, 3, 200),     # one slot below the rule: clusters
+    (1, torch.bfloat16, 2, 64, 4095, 3, 0),       # the first token, nothing in the ring
+    (3, torch.float16, 4, 64, 4100, 0, 4000),     # ring not full, no persistent rows
+    (2, torch.bfloat16, 3, 128, 2047, 16, 9001),  # full
+    (24, torch.bfloat16, 2, 64, 5000, 5, 4999),   # 48 pairs; 50 with the next, no longer split on 148 SMs
+    (25, torch.bfloat16, 2, 64, 5000, 5, 5000),
+    (1, torch.float16, 1, 128, 16384, 1, 30000),
+])
+def test_long_windows_with_few_pairs(B, dtype, heads, dh, window, n_p, t, monkeypatch):
+    """The step's split attention, twice in a row (its counters are left as they were found), against the unsplit kernel."""
+    model, g = make(dtype, heads, dh, window, n_p, 128)
+    model.embed_positions = torch.nn.Embedding(t + 2, heads * dh, device=DEV, dtype=dtype)
+    model.config.max_seq_len = t + 2
+    ids = torch.randint(0, 128, (B,), generator=g, device=DEV)
+    pos = torch.full((B,), t, dtype=torch.int32, device=DEV)
+    pos[0] = max(0, t - 2)
+    sets = [model.new_caches(B, DEV, dtype) for _ in range(2)]
+    for a, b in zip(*sets):
+        b.splits = 0
+        for x, y in zip((a.k_ring, a.v_ring, a.k_pers, a.v_pers), (b.k_ring, b.v_ring, b.k_pers, b.v_pers)):
+            x.normal_(0.0, 0.5, generator=g)
+            y.copy_(x)
+    got = [model.decode_step(ids, pos + i, sets[0]) for i in range(2)]
+    _native.poll_status(torch.device(DEV))
+    monkeypatch.setattr(_stack, "table_of", lambda m: None)
+    want = [model.decode_step(ids, pos + i, sets[1]) for i in range(2)]
+    tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
+    for a, b in zip(got, want):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() <= tol
+    for a, b in zip(*sets):
+        for x, y in ((a.k_ring, b.k_ring), (a.v_ring, b.v_ring)):
+            assert ((x.float() - y.float()).norm() / y.float().norm()).item() <= tol
+
+
 @pytest.mark.parametrize("B,heads,one_call", [(2, 32, True), (40, 32, True), (2, 40, False), (40, 40, False)])
 def test_widths_around_the_steps_limit(B, heads, one_call, monkeypatch):
     """The step's norms keep a row of at most 4096 in registers: a wider model goes to its modules."""

@@ -958,6 +958,19 @@ int launch_decode_dh(const DecodeParams& p, int dh, cudaStream_t stream, bool pd
 
 }  // namespace
 
+// Key ranges per pair for a decode step of the whole model, or 0.  With few pairs the clusters of launch_decode_shape hold at
+// most eight CTAs a pair, and from about 2^18 values per pair and tensor (4096 slots of 64, 2048 of 128) their scan is longer
+// than that of the split kernel, which puts up to sixteen on it but takes no part in the chain of dependent launches.  A step
+// of 16 layers, us, clusters -> split: 10 pairs, 4096 slots of 64 498 -> 448, 8192 690 -> 540; 40 pairs 4096 710 -> 587; 8 pairs,
+// 2048 slots of 128 614 -> 562; 32 pairs 831 -> 649; 48 pairs, 4096 of 128 1271 -> 981.  The kernel alone at 70 pairs: 33.7 -> 36.8.
+int decode_step_splits(const tmw_cache_desc& c) {
+    const long long pairs = (long long)c.batch * c.heads, slots = (long long)c.window + 1, sms = sm_count();
+    if (pairs == 0 || 3 * pairs > sms || slots * c.head_dim < (1 << 18)) return 0;
+    long long n = 2 * sms / pairs < slots / 128 ? 2 * sms / pairs : slots / 128;
+    n = n < TMW_MAX_DECODE_SPLITS ? n : TMW_MAX_DECODE_SPLITS;
+    return (int)(n > 2 ? n : 2);
+}
+
 int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, const void* v_new, void* o,
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,
                   int splits, float* scratch, unsigned int* counters, cudaStream_t stream, bool pdl) {

@@ -511,8 +511,16 @@ int launch_argmax(int rows, int vocab, const void* logits, int64_t* token, int64
 
 int64_t align256(int64_t n) { return (n + 255) & ~(int64_t)255; }
 
+tmw_cache_desc cache_of(const tmw_stack_desc& d) {
+    tmw_cache_desc c = {};
+    c.dtype = d.dtype; c.batch = d.batch; c.heads = d.heads; c.head_dim = d.head_dim; c.window = d.window;
+    c.n_persistent = d.n_persistent;
+    return c;
+}
+
 struct StepBuffers {
-    int64_t x, qkv, o, f, y, ss, total;  // byte offsets
+    int64_t x, qkv, o, f, y, ss, parts, counters, total;  // byte offsets
+    int splits;                                           // of the attention (decode_step_splits)
 };
 StepBuffers step_buffers(const tmw_stack_desc& d) {
     StepBuffers s;
@@ -523,8 +531,18 @@ StepBuffers step_buffers(const tmw_stack_desc& d) {
     s.f = s.o + align256(row * d.d_model);
     s.y = s.f + align256(row * d.d_ff);
     s.ss = s.y + align256(row * d.d_model);
-    s.total = s.ss + align256((int64_t)d.batch * ((d.d_model + 7) / 8) * 4);
+    s.parts = s.ss + align256((int64_t)d.batch * ((d.d_model + 7) / 8) * 4);
+    s.splits = decode_step_splits(cache_of(d));
+    s.counters = s.parts + (s.splits > 0 ? align256((int64_t)decode_partials_bytes(d.batch, d.heads, d.head_dim, s.splits)) : 0);
+    s.total = s.counters + (s.splits > 0 ? align256((int64_t)d.batch * d.heads * 4) : 0);
     return s;
+}
+
+// the split attention's counters: zero in front of the first step (every launch leaves them so)
+int clear_counters(const tmw_stack_desc& d, char* ws, cudaStream_t stream) {
+    const StepBuffers off = step_buffers(d);
+    if (off.splits > 0) TMW_CUDA_TRY(cudaMemsetAsync(ws + off.counters, 0, (size_t)(off.total - off.counters), stream));
+    return TMW_OK;
 }
 
 // `followed`: kChainFollowed if a dependent launch reads the logits (the tcgen05 product stores them through TMA), else 0
@@ -573,12 +591,11 @@ int decode_step_t(const tmw_stack_desc& d, const tmw_block* blocks, const int64_
         const tmw_block& b = blocks[l];
         int rc = normed(b.norm_attn, b.w_qkv, nullptr, 3 * D, qkv, EPI_STORE);
         if (rc != TMW_OK) return rc;
-        tmw_cache_desc c;
-        c.dtype = d.dtype; c.batch = B; c.heads = d.heads; c.head_dim = d.head_dim; c.window = d.window;
-        c.n_persistent = d.n_persistent;
+        tmw_cache_desc c = cache_of(d);
         c.k_ring = b.k_ring; c.v_ring = b.v_ring; c.k_pers = b.k_pers; c.v_pers = b.v_pers; c.scale = b.cache_scale;
         const T* q = static_cast<const T*>(qkv);
-        rc = launch_decode(c, q, q + D, q + 2 * D, o, row3, row3, row1, pos, 0, nullptr, nullptr, stream, true);
+        rc = launch_decode(c, q, q + D, q + 2 * D, o, row3, row3, row1, pos, off.splits, reinterpret_cast<float*>(ws + off.parts),
+                           reinterpret_cast<unsigned int*>(ws + off.counters), stream, off.splits == 0);
         if (rc == TMW_OK) rc = back(o, D, b.w_out, nullptr);
         if (rc == TMW_OK) rc = normed(b.norm_mlp, b.w_fc1, b.b_fc1, F, f, EPI_GELU);
         if (rc == TMW_OK) rc = back(f, F, b.w_fc2, b.b_fc2);
@@ -655,6 +672,8 @@ extern "C" int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* bloc
     if (rc != TMW_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
+    rc = clear_counters(*desc, ws, s);
+    if (rc != TMW_OK) return rc;
     return desc->dtype == TMW_BF16 ? decode_step_t<__nv_bfloat16>(*desc, blocks, token_ids, pos, logits, ws, 0, s)
                                    : decode_step_t<__half>(*desc, blocks, token_ids, pos, logits, ws, 0, s);
 }
@@ -670,6 +689,8 @@ extern "C" int tmw_generate(const tmw_stack_desc* desc, const tmw_block* blocks,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
     const tmw_stack_desc& d = *desc;
+    rc = clear_counters(d, ws, s);
+    if (rc != TMW_OK) return rc;
     auto run = [&](auto type) -> int {
         using T = decltype(type);
         // (an ordinary launch first; every step starts with one as well, so that a step's early reads of the rings see

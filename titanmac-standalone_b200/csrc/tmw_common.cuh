@@ -288,6 +288,7 @@ bool prefill_tc_supports(const tmw_prefill_desc& d, const void* q, const void* k
 int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, const void* v_new, void* o,
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,
                   int splits, float* scratch, unsigned int* counters, cudaStream_t stream, bool pdl = false);
+int decode_step_splits(const tmw_cache_desc& c);
 
 // layout of the split-decode scratch memory: partial results, then (16-byte aligned) one counter per pair
 inline size_t decode_partials_bytes(int batch, int heads, int head_dim, int splits) {

@@ -313,7 +313,8 @@ def _step_arguments(table: ModelTable, batch: int, caches):
     d.batch = batch
     nbytes = table.workspace_bytes.get((batch, -1))
     if nbytes is None:
-        nbytes = table.workspace_bytes[batch, -1] = _native.lib().tmw_decode_step_workspace(ctypes.byref(d))
+        with _native._on(device):  # (what it takes depends on the device's SMs)
+            nbytes = table.workspace_bytes[batch, -1] = _native.lib().tmw_decode_step_workspace(ctypes.byref(d))
     return d, blocks, torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
