@@ -3,8 +3,9 @@
 A step of a few rows is bound by its host work when every norm, product and attention call is issued from Python, so
 ``TitanMAC`` hands the library one table per call.  The table is built once and holds addresses and sizes only: before every
 use everything that went into it is compared with the modules as they are, and it is rebuilt when a parameter has moved or
-changed its layout, a module has been replaced or added, or an attribute has another value.  A model that the table cannot describe - another type of module in a known place, hooks, fp32, an active
-dropout - has no table, and its modules are called one by one.
+changed its layout, a module has been replaced or added, or an attribute has another value.  A model that the table cannot
+describe - another type of module in a known place, hooks, a forward set on an instance, fp32, an active dropout - has no
+table, and its modules are called one by one.
 """
 
 from __future__ import annotations
@@ -82,15 +83,15 @@ class ModelTable:
             return child
 
         def address(mod: nn.Module, name: str, shape) -> Optional[int]:
-            prm = mod._parameters.get(name)
+            d = mod._parameters
+            prm = d.get(name)
             if prm is None:
                 absent(mod, name)
                 return None
-            self._params.append((mod._parameters, name, prm.data_ptr(), prm.stride(), prm.nbytes, prm.dtype))
-            if prm.dtype != self.dtype or tuple(prm.shape) != tuple(shape) or not prm.is_contiguous() \
-                    or prm.device != self.device or prm.data_ptr() % 16:
-                return None
-            return prm.data_ptr()
+            ptr, dtype = prm.data_ptr(), prm.dtype
+            self._params.append((d, name, ptr, prm.stride(), prm.nbytes, dtype))
+            ok = dtype is self.dtype and prm.shape == shape and prm.is_contiguous() and prm.device == self.device and ptr % 16 == 0
+            return ptr if ok else None
 
         def absent(mod: nn.Module, name: str) -> bool:
             prm = mod._parameters.get(name)
@@ -108,7 +109,8 @@ class ModelTable:
             self._attributes += zip((obj,) * len(names), names, values)
             return values
 
-        D, V = c.d_model, c.vocab_size
+        D, V, d_head = c.d_model, c.vocab_size, c.d_head
+        sizes = (c.n_heads, d_head, c.window_size, c.n_persistent)
         layers = take(model, "layers", nn.ModuleList)
         tops = (take(model, "embed_tokens", nn.Embedding), take(model, "embed_positions", nn.Embedding),
                 take(model, "norm", RMSNorm), take(model, "lm_head", nn.Linear))
@@ -127,13 +129,13 @@ class ModelTable:
             if attn is None or mlp is None or None in norms or any(attributes(n, "eps") != (c.norm_eps,) for n in norms):
                 return
             windowed = type(attn) is WindowedAttention
-            if attributes(attn, "n_heads", "d_head", "window_size", "num_persistent" if windowed else "n_persistent") != (
-                    c.n_heads, c.d_head, c.window_size, c.n_persistent) or mlp.d_ff != F:
+            if attributes(attn, "n_heads", "d_head", "window_size", "num_persistent" if windowed else "n_persistent") != sizes \
+                    or mlp.d_ff != F:
                 return
             kind = (0, 0)
             if not windowed:
                 scale, block_size, use_conv = attributes(attn, "scale", "block_size", "use_conv")
-                if scale != 1.0 / math.sqrt(c.d_head):
+                if scale != 1.0 / math.sqrt(d_head):
                     return
                 kind = (block_size, attn.conv_q.kernel_size[0] if use_conv else 0)
             if i > 0 and kind != self.kind:
@@ -147,24 +149,20 @@ class ModelTable:
             if take(attn, "dropout", nn.Identity, nn.Dropout) is None or take(mlp, "dropout", nn.Identity, nn.Dropout) is None \
                     or take(mlp, "activation", nn.GELU) is None or attributes(mlp.activation, "approximate") != ("none",):
                 return
-            b = self.blocks[i]
-            values = dict(norm_attn=address(norms[0], "scale", (D,)), norm_mlp=address(norms[1], "scale", (D,)),
-                          w_qkv=address(qkv, "weight", (3 * D, D)), w_out=address(out, "weight", (D, D)),
-                          w_fc1=address(fc1, "weight", (F, D)), w_fc2=address(fc2, "weight", (D, F)),
-                          b_fc1=optional(fc1, "bias", (F,)), b_fc2=optional(fc2, "bias", (D,)))
+            homes = [("norm_attn", norms[0], "scale", (D,)), ("norm_mlp", norms[1], "scale", (D,)), ("w_qkv", qkv, "weight", (3 * D, D)),
+                     ("w_out", out, "weight", (D, D)), ("w_fc1", fc1, "weight", (F, D)), ("w_fc2", fc2, "weight", (D, F)),
+                     ("b_fc1", fc1, "bias", (F,)), ("b_fc2", fc2, "bias", (D,))]
             for name in ("conv_q", "conv_k", "conv_v") if kind[1] else ():
                 conv = take(attn, name, nn.Conv1d)
                 if conv is None or not absent(conv, "bias"):
                     return
-                values[name] = address(conv, "weight", (D, 1, kind[1]))
-            found += values.values()
-            for name, value in values.items():
-                setattr(b, name, value or None)
-            homes = dict(norm_attn=(norms[0], "scale"), norm_mlp=(norms[1], "scale"), w_qkv=(qkv, "weight"), w_out=(out, "weight"),
-                         w_fc1=(fc1, "weight"), w_fc2=(fc2, "weight"), b_fc1=(fc1, "bias"), b_fc2=(fc2, "bias"))
-            for name in ("conv_q", "conv_k", "conv_v") if kind[1] else ():
-                homes[name] = (attn._modules[name], "weight")
-            self._places += [((i, name), (m._parameters, key)) for name, (m, key) in homes.items()]
+                homes.append((name, conv, "weight", (D, 1, kind[1])))
+            b = self.blocks[i]
+            for field, mod, key, shape in homes:
+                value = (optional if key == "bias" else address)(mod, key, shape)
+                found.append(value)
+                setattr(b, field, value or None)
+                self._places.append(((i, field), (mod._parameters, key)))
         d = self.desc = _native.StackDesc()
         top = (address(tops[0], "weight", (V, D)), address(tops[1], "weight", (c.max_seq_len, D)), address(tops[2], "scale", (D,)),
                address(tops[3], "weight", (V, D)))
@@ -183,7 +181,7 @@ class ModelTable:
         d.persistent = pers or None
         d.block_size, d.conv_taps = self.kind
         d.dtype = _native._DTYPES[self.dtype]
-        d.layers, d.d_model, d.heads, d.head_dim, d.d_ff = len(layers), D, c.n_heads, c.d_head, F
+        d.layers, d.d_model, d.heads, d.head_dim, d.d_ff = len(layers), D, c.n_heads, d_head, F
         d.window, d.n_persistent, d.vocab, d.max_positions, d.eps = c.window_size, c.n_persistent, V, c.max_seq_len, c.norm_eps
         # unique parameters as (dictionary, name), and each one's places in the structures: (layer or -1, field)
         self.slots, self.roles, at = [], [], {}
@@ -195,9 +193,9 @@ class ModelTable:
                     self.slots.append((d_, name))
                     self.roles.append([])
                 self.roles[at[id(prm)]].append(place)
-        self.geometry = (c.n_heads, c.d_head, c.window_size, c.n_persistent, self.dtype)
-        self.decodes = c.d_head in (64, 128) and F % 32 == 0 and D <= 4096 and self.kind == (0, 0)
-        self.forwards = V % 8 == 0 and F % 8 == 0 and D % 8 == 0 and c.d_head % 8 == 0 and self.kind[1] <= 8
+        self.geometry = sizes + (self.dtype,)
+        self.decodes = d_head in (64, 128) and F % 32 == 0 and D <= 4096 and self.kind == (0, 0)
+        self.forwards = V % 8 == 0 and F % 8 == 0 and D % 8 == 0 and d_head % 8 == 0 and self.kind[1] <= 8
         # the backward writes a gradient once per place; only for the table that is also the head it adds the places up
         # (and it knows nothing of an embedding table's options)
         options = [attributes(t, "padding_idx", "scale_grad_by_freq", "sparse") for t in tops[:2]]

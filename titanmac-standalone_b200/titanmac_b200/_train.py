@@ -25,11 +25,37 @@ def _aligned(grad: torch.Tensor) -> torch.Tensor:
     return grad.clone() if grad.data_ptr() % 16 else grad
 
 
+class _Rows:
+    """The logits of all rows ``[B, Np + T, V]``, persistent rows first, and their gradient, around the sequence rows ``[B, T, V]``
+    that the caller sees and the loss depends on.  Where the gradient of the sequence rows is the one that the loss's backward
+    has just written inside a gradient of all rows, that one is taken as it is."""
+
+    __slots__ = ("rows", "d_rows")
+
+    def __init__(self, rows: Optional[torch.Tensor] = None):
+        self.rows, self.d_rows = rows, None
+
+    def gradient(self, d_logits: torch.Tensor, n_persistent: int) -> torch.Tensor:
+        """Of all rows, contiguous; the persistent ones' is zero."""
+        if n_persistent == 0:
+            return d_logits
+        d_rows, self.d_rows = self.d_rows, None  # (held until here: no other tensor can have its address)
+        if d_rows is not None:
+            own = d_rows[:, n_persistent:]
+            if d_logits.data_ptr() == own.data_ptr() and d_logits.stride() == own.stride() and d_logits.shape == own.shape:
+                return d_rows
+        B, T, V = d_logits.shape
+        d_rows = d_logits.new_empty((B, n_persistent + T, V))
+        d_rows[:, :n_persistent] = 0
+        d_rows[:, n_persistent:] = d_logits
+        return d_rows
+
+
 class _StackTrain(torch.autograd.Function):
-    """``ids [B, T]`` → logits of every row ``[B, Np + T, V]``."""
+    """``ids [B, T]`` → logits of the sequence rows ``[B, T, V]``; ``held`` gets those of all rows."""
 
     @staticmethod
-    def forward(ctx, table, ids: torch.Tensor, *params: torch.Tensor) -> torch.Tensor:
+    def forward(ctx, table, held: _Rows, ids: torch.Tensor, *params: torch.Tensor) -> torch.Tensor:
         d = _native.StackDesc.from_buffer_copy(table.desc)
         B, T = ids.shape
         d.batch = B
@@ -40,16 +66,17 @@ class _StackTrain(torch.autograd.Function):
         with _native._on(device):
             _native.check(lib.tmw_stack_train_forward(ref, table.blocks, ids.data_ptr(), T, logits.data_ptr(), saved.data_ptr(),
                                                       nbytes, _native._stream_ptr(device)))
-        ctx.desc, ctx.roles = d, table.roles
+        ctx.desc, ctx.roles, ctx.held = d, table.roles, held
         ctx.save_for_backward(ids, saved, *params)
-        return logits
+        held.rows = logits
+        return logits[:, d.n_persistent:].detach() if d.n_persistent else logits  # (not a view to autograd: it may be changed)
 
     @staticmethod
     @once_differentiable
     def backward(ctx, d_logits: torch.Tensor):
         ids, saved, *params = ctx.saved_tensors
         d = _native.StackDesc.from_buffer_copy(ctx.desc)
-        d_logits = _aligned(d_logits)
+        d_logits = _aligned(ctx.held.gradient(d_logits, d.n_persistent))
         # the parameters' addresses as they are now, and their gradients'
         blocks, block_grads = (_native.Block * d.layers)(), (_native.BlockGrads * d.layers)()
         grads, out = _native.StackGrads(), []
@@ -71,11 +98,12 @@ class _StackTrain(torch.autograd.Function):
             _native.check(lib.tmw_stack_train_backward(ref, blocks, ctypes.byref(grads), block_grads, ids.data_ptr(), T,
                                                        d_logits.data_ptr(), saved.data_ptr(), scratch.data_ptr(), nbytes,
                                                        _native._stream_ptr(device)))
-        return (None, None, *out)
+        return (None, None, None, *out)
 
 
-def stack_forward(model, input_ids: torch.Tensor) -> Optional[torch.Tensor]:
-    """Logits of every row with a gradient to every parameter, or None where that takes the modules themselves."""
+def stack_forward(model, input_ids: torch.Tensor):
+    """``(logits of the sequence rows with a gradient to every parameter, _Rows around them)``, or None where that takes the
+    modules themselves."""
     table = _stack.table_of(model, training=True)
     # (tokens that repeat are added up with atomics: not in a fixed order, as the library's embedding backward does)
     if table is None or not table.trains or _autocast() or torch.are_deterministic_algorithms_enabled() \
@@ -87,41 +115,31 @@ def stack_forward(model, input_ids: torch.Tensor) -> Optional[torch.Tensor]:
     params = [d[name] for d, name in table.slots]
     if not all(p.requires_grad for p in params):
         return None
-    return _StackTrain.apply(table, input_ids.contiguous(), *params)
+    held = _Rows()
+    return _StackTrain.apply(table, held, input_ids.contiguous(), *params), held
 
 
 class _SequenceRows(torch.autograd.Function):
-    """``rows [B, Np + T, V]`` → its sequence rows ``[B, T, V]``, the logits that the caller sees and the loss depends on.  Slicing
-    would cost a pass over the gradient of all rows on the way back; where the gradient that arrives is the one the loss's
-    backward has just written inside a gradient of all rows (``whole``), that one is handed on."""
+    """The sequence rows of ``rows [B, Np + T, V]``, which the modules have made; a slice of them would cost a pass over the
+    gradient of all rows on the way back."""
 
     @staticmethod
-    def forward(ctx, rows: torch.Tensor, n_persistent: int, whole: list) -> torch.Tensor:
-        ctx.n_persistent, ctx.whole = n_persistent, whole
-        return rows[:, n_persistent:].detach()  # (not a view to autograd, which would not let the caller change it)
+    def forward(ctx, rows: torch.Tensor, n_persistent: int, held: _Rows) -> torch.Tensor:
+        ctx.n_persistent, ctx.held = n_persistent, held
+        return rows[:, n_persistent:].detach()
 
     @staticmethod
     @once_differentiable
     def backward(ctx, d_logits: torch.Tensor):
-        n = ctx.n_persistent
-        if ctx.whole:
-            d_rows = ctx.whole.pop()  # (held until here: no other tensor can have its address)
-            own = d_rows[:, n:]
-            if d_logits.data_ptr() == own.data_ptr() and d_logits.stride() == own.stride() and d_logits.shape == own.shape:
-                return d_rows, None, None
-        B, T, V = d_logits.shape
-        d_rows = d_logits.new_empty((B, n + T, V))
-        d_rows[:, :n] = 0
-        d_rows[:, n:] = d_logits
-        return d_rows, None, None
+        return ctx.held.gradient(d_logits, ctx.n_persistent), None, None
 
 
 class _ShiftedCrossEntropy(torch.autograd.Function):
     """Mean cross-entropy of ``rows [B, Np + T, V]``, row ``Np + t`` against ``labels[:, t + 1]`` (-100: not counted).  The
-    gradient goes to ``logits``, the sequence rows; ``whole`` keeps it as part of a gradient of all rows."""
+    gradient goes to ``logits``, the sequence rows; ``held`` keeps it as part of a gradient of all rows."""
 
     @staticmethod
-    def forward(ctx, logits: torch.Tensor, rows: torch.Tensor, labels: torch.Tensor, n_persistent: int, whole: list) -> torch.Tensor:
+    def forward(ctx, logits: torch.Tensor, rows: torch.Tensor, labels: torch.Tensor, n_persistent: int, held: _Rows) -> torch.Tensor:
         B, L, V = rows.shape
         loss = torch.empty((), dtype=rows.dtype, device=rows.device)
         stats = torch.empty(4 + 2 * B * L, dtype=torch.float32, device=rows.device)
@@ -130,7 +148,7 @@ class _ShiftedCrossEntropy(torch.autograd.Function):
                                                           rows.data_ptr(), labels.data_ptr(), loss.data_ptr(), stats.data_ptr(),
                                                           None, None, _native._stream_ptr(rows.device)))
         ctx.save_for_backward(rows, labels, stats)
-        ctx.n_persistent, ctx.whole = n_persistent, whole
+        ctx.n_persistent, ctx.held = n_persistent, held
         return loss
 
     @staticmethod
@@ -147,26 +165,30 @@ class _ShiftedCrossEntropy(torch.autograd.Function):
                                                           d_rows.data_ptr(), _native._stream_ptr(rows.device)))
         if n == 0:
             return d_rows, None, None, None, None
-        ctx.whole[:] = [d_rows]
+        ctx.held.d_rows = d_rows
         return d_rows[:, n:], None, None, None, None
 
 
-def shifted_cross_entropy(rows: torch.Tensor, labels: torch.Tensor, n_persistent: int):
+def shifted_cross_entropy(rows: torch.Tensor, labels: torch.Tensor, n_persistent: int, logits: Optional[torch.Tensor] = None,
+                          held: Optional[_Rows] = None):
     """``(logits, loss)`` of ``rows``, every row's logits, persistent rows first: the sequence rows and their mean shifted
-    cross-entropy, which depends on them.  None where the library's kernel does not apply."""
+    cross-entropy, which depends on them (``logits`` and ``held``: from ``stack_forward``, else they are made here).  None
+    where the library's kernel does not apply."""
     B, L, V = rows.shape
     if (rows.dtype not in (torch.bfloat16, torch.float16) or not rows.is_cuda or not rows.is_contiguous() or V % 8
             or rows.data_ptr() % 16 or labels.dtype != torch.int64 or labels.shape != (B, L - n_persistent)
             or labels.device != rows.device or B == 0 or L == n_persistent or _autocast()):
         return None
-    whole: list = []
-    if n_persistent == 0:
-        logits = rows
-    elif rows.requires_grad and torch.is_grad_enabled():
-        logits = _SequenceRows.apply(rows, n_persistent, whole)
-    else:
-        logits = rows[:, n_persistent:]
-    return logits, _ShiftedCrossEntropy.apply(logits, rows.detach(), labels.contiguous(), n_persistent, whole)
+    if held is None:
+        held = _Rows()
+        if n_persistent == 0:
+            logits = rows
+        elif rows.requires_grad and torch.is_grad_enabled():
+            logits = _SequenceRows.apply(rows, n_persistent, held)
+        else:
+            logits = rows[:, n_persistent:]
+        rows = rows.detach()
+    return logits, _ShiftedCrossEntropy.apply(logits, rows, labels.contiguous(), n_persistent, held)
 
 
 class _AttentionTrain(torch.autograd.Function):

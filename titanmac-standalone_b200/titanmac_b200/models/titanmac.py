@@ -6,17 +6,19 @@ tokens prepended to every sequence (:608-619), the block stack (:629-640), final
 norm, tied LM head over all rows and the slice that drops the persistent rows
 (:652-662), optional shifted cross-entropy (:674-684).  Parameter names match the
 reference (``embed_tokens``, ``embed_positions``, ``persistent_tokens``,
-``layers.N...``, ``norm``, ``lm_head``), so its checkpoints load.  Under
-``torch.no_grad()`` the fused inference kernels run; with grad mode on the same call
-is differentiable (the attention cores through their own backward kernels, norms and
-GELU through PyTorch), so ``forward(ids, labels=...)["loss"].backward()`` trains.
+``layers.N...``, ``norm``, ``lm_head``), so its checkpoints load.  In 16-bit types a
+forward, a decode step, a generation and the two halves of a training step
+(``forward(ids, labels=...)["loss"].backward()``) are one library call each
+(``_stack``, ``_train``); fp32, hooks, active dropout, frozen or shared parameters and
+the like go through the modules one by one, where with grad mode on the attention
+cores have their own backward kernels and norms and GELU are PyTorch's.
 
 ``prefill`` / ``decode_step`` / ``generate`` are new: the reference has no KV cache,
 its generation helper re-runs the whole forward for every new token
 (examples/train_math.py:146-161).  Here a prompt is run once, every layer's last
 ``w+1`` keys/values go into a ring cache, the persistent keys/values (which do not
-depend on the prompt) are kept once per layer, and each new token costs one pass of
-``tmw_decode`` per layer.  A decode step returns the logits the reference's
+depend on the prompt) are kept once per layer, and each new token attends to one ring
+per layer.  A decode step returns the logits the reference's
 re-forward would return for its last row.
 """
 
@@ -51,7 +53,6 @@ class TitanMAC(nn.Module):
         if config.tie_weights:
             self.lm_head.weight = self.embed_tokens.weight
         self._init_weights()
-        self._graph = None
 
     def _init_weights(self) -> None:
         # titanmac.py:140-158: only embeddings, persistent tokens and an untied head are re-initialised
@@ -80,22 +81,28 @@ class TitanMAC(nn.Module):
         the gradients, are NaN, and ``_native.poll_status`` (which synchronises) raises; otherwise PyTorch's own device-side
         check ends the process's CUDA context.  ``decode_step`` likewise, for its positions too."""
         Np = self.config.n_persistent
-        rows = None  # logits of every row, persistent rows first
+        rows = logits = held = None  # logits of every row, persistent rows first; of the sequence rows; what holds both
         if torch.is_grad_enabled() and any(p.requires_grad for p in self.parameters()):
-            rows = _train.stack_forward(self, input_ids)  # one autograd node
+            found = _train.stack_forward(self, input_ids)  # one autograd node
+            if found is not None:
+                logits, held = found
+                rows, held.rows = held.rows, None
         else:
             table = _stack.table_of(self)
             if table is not None:  # the whole forward as one call (tmw_stack_forward)
                 rows = _stack.forward(table, input_ids)
         if rows is None:
             rows = self._forward_modules(input_ids)
-        logits = rows[:, Np:, :] if Np > 0 else rows
+        loss = None
+        if labels is not None:
+            found = _train.shifted_cross_entropy(rows, labels, Np, logits, held)
+            if found is not None:
+                logits, loss = found
+        if logits is None:
+            logits = rows[:, Np:, :] if Np > 0 else rows
         out = {"logits": logits}
         if labels is not None:
-            found = _train.shifted_cross_entropy(rows, labels, Np)
-            if found is not None:
-                out["logits"], loss = found
-            else:
+            if loss is None:
                 shift_logits = logits[..., :-1, :].contiguous()
                 shift_labels = labels[..., 1:].contiguous()
                 loss = F.cross_entropy(shift_logits.reshape(-1, self.config.vocab_size), shift_labels.reshape(-1),
