@@ -14,7 +14,8 @@
 // 16-bit caches with head_dim 64 or 128 take one of two other kernels further down: decode_stream_kernel with many
 // pairs - the same arithmetic fed from shared memory, which bulk asynchronous copies keep filled three chunks ahead
 // (measured on B200, 2560 pairs, window 512: 60 us against 68 us; 5120 pairs: 105 us against 129 us, the bandwidth of
-// a plain copy) - and decode_cluster_kernel with few.
+// a plain copy) - and decode_cluster_kernel with few; very long windows over few pairs are split over more CTAs than a cluster
+// holds (tmw_decode_split; a decode step of the whole model by decode_step_splits).
 #include <math_constants.h>
 
 #include <cstdio>

@@ -1,17 +1,17 @@
-// Linear layer on tcgen05: C[M, N] = A[M, K] · W[N, K]ᵀ (+ bias[N]) (+ exact GELU), 16-bit inputs, fp32
-// accumulation in tensor memory, 16-bit output.  The layout of torch.nn.functional.linear: activations
-// row-major, weight [out_features, in_features] - both operands K-major, no transposes anywhere.
+// Products on tcgen05: C[M, N] = epilogue(sum over k of A(m, k) B(n, k)), 16-bit operands, fp32 accumulation in tensor memory,
+// 16-bit output (or, with k cut into ranges, fp32 sums of each).  The linear layer of torch.nn.functional.linear has both
+// operands K-major ([M, K] activations, [N, K] weight); a gradient's operands lie transposed and are read MN-major, B alone
+// for the input's gradient, A and B for the weight's.  No transposes in memory anywhere.  Epilogues: see GemmEpilogue.
 //
-// A persistent CTA per SM walks over 128 x BN output tiles (consecutive tiles share their rows of A, so those
-// stay in L2 while the weight panels change).  Warp roles:
-//   warp 0      TMA producer: A and W tiles of 64 K-elements into a ring of shared-memory stages
+// gemm_tc_kernel: a persistent CTA per SM walks over 128 x BN output tiles (consecutive tiles share their rows of A, so those
+// stay in L2 while the panels of B change).  Warp roles:
+//   warp 0      TMA producer: A and B tiles of 64 K-elements into a ring of shared-memory stages
 //   warp 1      issues the tcgen05.mma of every stage (one elected thread); allocates / frees tensor memory
-//   warps 2-9   epilogue: tensor memory -> registers -> bias / GELU -> 16-bit -> shared memory -> TMA store;
-//               warp w reads the 32 lanes of its number modulo 4, warps 2-5 the first half of the columns,
-//               warps 6-9 the second
+//   warps 2-9   epilogue: tensor memory -> registers -> bias, GELU, ... -> 16-bit -> the warp's own staging -> TMA store;
+//               warp w reads the 32 lanes of its number modulo 4 and takes every second panel of 32 columns
 // The accumulator is double-buffered in tensor memory (2 x BN columns): the epilogue of a tile runs under the
-// matrix products of the next one.  Every mbarrier wait is bounded and reports TMW_ERR_DEVICE_TIMEOUT through
-// the device status word.
+// matrix products of the next one.  gemm_tc_pair_kernel, below, does the same on CTA pairs.  Every mbarrier wait is bounded
+// and reports TMW_ERR_DEVICE_TIMEOUT through the device status word.
 #include <cuda.h>
 
 #include <cmath>

@@ -14,6 +14,7 @@
 //   eight warps, two threads per row, turn X into P and Y into dS (16 columns at a time) and write both back into
 //   tensor memory as 16-bit values OVER X and Y,
 //   then  acc += Pᵀ-or-dS (from tensor memory) · column tile (from shared memory, read as an MN-major operand).
+// The two halves of a column tile are chains of their own: products, barriers and four of the eight warps each.
 // Warps: 0 TMA producer (and the columns' statistics), 1 and 2 issue the tcgen05.mma (one elected thread each, each
 // its own chain of products; warp 1 allocates tensor memory), 3 idle, 4-11 the element-wise work and the output.
 // The first launch leaves every row's (log-sum-exp, D) in scratch memory for the second.  Every mbarrier wait is

@@ -22,8 +22,10 @@
 //   head_dim 128  256 columns (S | S | O): two CTAs per SM, and the next scores are multiplied while these are
 //                 exponentiated
 // Measured before (128-key tiles; two CTAs per SM at head_dim 64, one CTA of two query tiles with one S each at 128) and
-// now, us: 8 x 10 heads x 4112 rows of 64, window 128 | 512 | 2048: 82.2 | 133.8 | 283 and 69.5 | 113 | 254; 16 heads x
-// 131 088 rows of 128, window 1024: 1604 and 1321 (two query tiles sharing K and V in one CTA: 1469).
+// now, us: 8 x 10 heads x 4112 rows of 64, window 128 | 512 | 2048: 82.2 | 133.8 | 283 and 63.4 | 105 | 242 (by itself, one
+// input again or four in turn alike; 120 between the products of a layer, which hold the clock at 1760 MHz); 16 heads x
+// 131 088 rows of 128, window 1024: 1604 and 1314 (two query tiles sharing K and V in one CTA: 1469; a hundred calls in a row,
+// under the power cap: 1513).
 //
 // Every wait on an mbarrier is bounded: on expiry the kernel records
 // TMW_ERR_DEVICE_TIMEOUT in the device status word, stops waiting anywhere and runs

@@ -8,8 +8,8 @@ it on a GPU: RMSNorm with the preceding residual add folded in is one kernel
 in its epilogue (few rows, module by module: library GEMM plus the one-pass ``tmw_gelu``; a model's decode step is
 ``tmw_decode_step``).
 ``use_block_sparse`` selects the attention class exactly as in the reference.
-Under ``torch.no_grad()`` the fused kernels run; with grad mode on, norm and GELU fall back to the
-differentiable PyTorch formulas and the windowed attention core uses its own backward kernel.
+Under ``torch.no_grad()`` the fused kernels run; with grad mode on, a block called by itself takes the differentiable PyTorch
+formulas of norm and GELU and the attention module's own backward kernels (a whole model's training step: ``_train``).
 """
 
 from __future__ import annotations
