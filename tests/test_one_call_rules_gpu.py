@@ -5,7 +5,8 @@ import torch
 import torch.nn as nn
 from torch.nn.modules import module as nn_module
 
-from titanmac_b200 import TitanMAC, TitanMACConfig, _native, _stack, _train
+from titanmac_b200 import (BlockSparseAttention, TitanMAC, TitanMACConfig, WindowConfig, WindowedAttention, _native, _stack,
+                           _train)
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -258,3 +259,72 @@ def test_deterministic_algorithms_when_asked_for():
         torch.use_deterministic_algorithms(False)
     for g2 in grads[1:]:
         assert torch.equal(grads[0], g2)
+
+
+class _Scaled(TitanMAC):
+    def _embed(self, input_ids, first_position=0):
+        return super()._embed(input_ids, first_position) * 3
+
+
+class _Counting(TitanMAC):
+    def decode_step(self, *a):
+        self.steps = getattr(self, "steps", 0) + 1
+        return super().decode_step(*a)
+
+
+class _Swapped(WindowedAttention):
+    def split_qkv(self, qkv):
+        q, k, v = super().split_qkv(qkv)
+        return k, q, v
+
+
+class _Halved(BlockSparseAttention):
+    def stacked_conv_weight(self):
+        return super().stacked_conv_weight() / 2
+
+
+def test_a_subclass_that_embeds_otherwise(monkeypatch):
+    model, ids = make()
+    model.__class__ = _Scaled
+    plain, _ = make()
+    _, got = step(model, ids)
+    with torch.no_grad():
+        fwd, pre = model(ids)["logits"], model.prefill(ids)[0]
+        assert not close(fwd, plain(ids)["logits"], 5e-2)
+        module_by_module(monkeypatch)
+        assert close(fwd, model(ids)["logits"], 2e-2) and close(pre, model.prefill(ids)[0], 2e-2)
+    _, want = step(model, ids)
+    for name in want:
+        assert close(got[name], want[name], 6e-2), name
+
+
+@pytest.mark.parametrize("on_the_instance", [False, True])
+def test_generate_takes_the_steps_of_a_subclass(on_the_instance):
+    model, ids = make()
+    want = model.generate(ids, 5)
+    if on_the_instance:
+        own, model.steps = model.decode_step, 0
+
+        def counted(*a):
+            model.steps += 1
+            return own(*a)
+
+        model.decode_step = counted
+    else:
+        model.__class__ = _Counting
+    got = model.generate(ids, 5, use_cuda_graph=False)
+    assert model.steps == 4 and torch.equal(got, want)
+
+
+def test_attention_modules_with_parts_of_their_own():
+    with torch.device(DEV):
+        win = WindowedAttention(WindowConfig(window_size=16, num_heads=2, head_dim=64, n_persistent=3)).to(BF16)
+        sparse = BlockSparseAttention(128, 2, window_size=32, n_persistent=3).to(BF16)
+        x = torch.randn(2, 40, 128, device=DEV).to(BF16)
+    for mod, sub, train in ((win, _Swapped, False), (sparse, _Halved, False), (sparse, _Halved, True)):
+        with torch.set_grad_enabled(train):
+            base = mod(x)
+            mod.__class__ = sub
+            own = mod(x)
+            mod.__class__ = sub.__bases__[0]
+        assert not close(own, base, 5e-2)

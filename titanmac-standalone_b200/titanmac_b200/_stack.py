@@ -25,6 +25,12 @@ from . import _native
 
 _dtype_of, _nbytes_of = operator.attrgetter("dtype"), operator.attrgetter("nbytes")
 
+def overrides(obj, base: type, *names: str) -> bool:
+    """Whether the object, or the subclass of ``base`` that it is of, has methods of its own under these names."""
+    cls, own = type(obj), obj.__dict__
+    return any([n in own for n in names]) or (cls is not base and any([getattr(cls, n) is not getattr(base, n) for n in names]))
+
+
 # What runs when a module is called beside its class's forward; the second pair only with a gradient to come.  (A forward set
 # on the instance replaces the class's.)
 _FORWARD_HOOKS = ("_forward_hooks", "_forward_pre_hooks")

@@ -99,6 +99,10 @@ class BlockSparseAttention(nn.Module):
         """``[3 * d_model, taps]``: the three depthwise filters in the channel order of the QKV projection."""
         return torch.cat([self.conv_q.weight[:, 0], self.conv_k.weight[:, 0], self.conv_v.weight[:, 0]], dim=0)
 
+    def _own_filters(self) -> bool:
+        """Whether the filters are this class's (a subclass may stack others)."""
+        return type(self) is BlockSparseAttention or not _stack.overrides(self, BlockSparseAttention, "stacked_conv_weight")
+
     def forward(self, x: torch.Tensor, attn_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return self._forward_train(x)
@@ -119,7 +123,9 @@ class BlockSparseAttention(nn.Module):
         B, L, D = x.shape
         if self.n_persistent >= L:
             raise ValueError(f"n_persistent ({self.n_persistent}) must be < seq_len ({L})")
-        y = _train.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)
+        y = None
+        if self._own_filters():
+            y = _train.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)
         if y is not None:
             return self.dropout(y)
         qkv = self.qkv_proj(x)
@@ -139,7 +145,9 @@ class BlockSparseAttention(nn.Module):
         B, L, D = x.shape
         if self.n_persistent >= L:
             raise ValueError(f"n_persistent ({self.n_persistent}) must be < seq_len ({L})")
-        y = _stack.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)  # the module as one call
+        y = None
+        if self._own_filters():  # the module as one call
+            y = _stack.attention_forward(self, x, self.n_persistent, self.block_size, self.scale)
         if y is not None:
             drop = self._modules["dropout"]
             return y if type(drop) is nn.Identity and not (drop._forward_hooks or drop._forward_pre_hooks) else drop(y)

@@ -130,7 +130,9 @@ class WindowedAttention(nn.Module):
             qkv = self.qkv_proj(x).view(B, L, 3, self.n_heads, self.d_head)
             o = _WindowedCore.apply(qkv, self.window_size, self.num_persistent, self.algo)
             return self.dropout(self.out_proj(o.view(B, L, D)))
-        y = _stack.attention_forward(self, x, self.num_persistent, 0, 0.0)  # the module as one call
+        y = None
+        if type(self) is WindowedAttention or not _stack.overrides(self, WindowedAttention, "split_qkv", "_forward_no_grad"):
+            y = _stack.attention_forward(self, x, self.num_persistent, 0, 0.0)  # the module as one call
         if y is not None:
             drop = self._modules["dropout"]
             return y if type(drop) is nn.Identity and not (drop._forward_hooks or drop._forward_pre_hooks) else drop(y)

@@ -72,6 +72,10 @@ class TitanMAC(nn.Module):
             x = torch.cat([self.persistent_tokens[None].expand(B, -1, -1), x], dim=1)
         return x
 
+    def _embeds(self) -> bool:
+        """Whether the one-call paths embed as this model does (a subclass may do it otherwise)."""
+        return not _stack.overrides(self, TitanMAC, "_embed", "_forward_modules")
+
     def forward(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None,
                 attention_mask: Optional[torch.Tensor] = None) -> Dict[str, torch.Tensor]:
         """``{"logits": [B, T, V]}`` and, with ``labels``, ``"loss"``, whose backward reads the logits: until then change a copy
@@ -83,12 +87,12 @@ class TitanMAC(nn.Module):
         Np = self.config.n_persistent
         rows = logits = held = None  # logits of every row, persistent rows first; of the sequence rows; what holds both
         if torch.is_grad_enabled() and any(p.requires_grad for p in self.parameters()):
-            found = _train.stack_forward(self, input_ids)  # one autograd node
+            found = _train.stack_forward(self, input_ids) if self._embeds() else None  # one autograd node
             if found is not None:
                 logits, held = found
                 rows, held.rows = held.rows, None
         else:
-            table = _stack.table_of(self)
+            table = _stack.table_of(self) if self._embeds() else None
             if table is not None:  # the whole forward as one call (tmw_stack_forward)
                 rows = _stack.forward(table, input_ids)
         if rows is None:
@@ -151,7 +155,7 @@ class TitanMAC(nn.Module):
         Np = self.config.n_persistent
         if caches is None:
             caches = self.new_caches(B, input_ids.device, self.embed_tokens.weight.dtype)
-        table = _stack.table_of(self)
+        table = _stack.table_of(self) if self._embeds() else None
         if table is not None:  # the prompt as one call (tmw_stack_forward)
             logits = _stack.forward(table, input_ids, caches)
             if logits is not None:
@@ -220,7 +224,7 @@ class TitanMAC(nn.Module):
         if T + max_new_tokens > self.config.max_seq_len:
             raise ValueError("prompt + new tokens exceed max_seq_len (the position-embedding table)")
         logits, caches = self.prefill(input_ids)
-        table = _stack.table_of(self)
+        table = None if _stack.overrides(self, TitanMAC, "decode_step") else _stack.table_of(self)
         if table is not None:  # every choice and step from one call (tmw_generate)
             tokens = _stack.generate(table, input_ids, logits, caches, max_new_tokens)
             if tokens is not None:
