@@ -328,3 +328,21 @@ def test_attention_modules_with_parts_of_their_own():
             own = mod(x)
             mod.__class__ = sub.__bases__[0]
         assert not close(own, base, 5e-2)
+
+
+def test_tables_of_another_type_than_the_layers():
+    """A 16-bit token table in an fp32 model: the embedded rows, and so the keys in the caches, are fp32."""
+    model, ids = make(tie_weights=False)
+    model = model.float().eval()
+    pos = torch.full((2,), 30, dtype=torch.int32, device=DEV)
+
+    def run():
+        logits, caches = model.prefill(ids)
+        assert caches[0].dtype == torch.float32
+        return logits, model.decode_step(ids[:, 0], pos, caches)
+
+    want = run()  # (the table's values are 16-bit ones: the model came from bf16)
+    model.embed_tokens.to(BF16)
+    got = run()
+    for a, b in zip(got, want):
+        assert close(a, b, 1e-5)

@@ -153,14 +153,16 @@ class TitanMAC(nn.Module):
         self._need_windowed()
         B, T = input_ids.shape
         Np = self.config.n_persistent
-        if caches is None:
-            caches = self.new_caches(B, input_ids.device, self.embed_tokens.weight.dtype)
         table = _stack.table_of(self) if self._embeds() else None
         if table is not None:  # the prompt as one call (tmw_stack_forward)
+            if caches is None:
+                caches = self.new_caches(B, input_ids.device, table.dtype)
             logits = _stack.forward(table, input_ids, caches)
             if logits is not None:
                 return logits, caches
         x = self._embed(input_ids)
+        if caches is None:  # (the keys' type is that of the embedded rows, not of one table)
+            caches = self.new_caches(B, x.device, x.dtype)
         pending = None
         for layer, cache in zip(self.layers, caches):
             attn = layer.attention
