@@ -330,6 +330,18 @@ def test_attention_modules_with_parts_of_their_own():
         assert not close(own, base, 5e-2)
 
 
+def test_another_kind_of_embedding():
+    model, ids = make(tie_weights=False)
+    model.eval()
+    with torch.no_grad():
+        want, cont = model(ids)["logits"], model.generate(ids, 4)
+        model.embed_tokens = nn.Sequential(model.embed_tokens)  # has no weight of its own
+        assert close(model(ids)["logits"], want, 2e-2)
+        assert torch.equal(model.generate(ids, 4)[:, :30], cont[:, :30])
+    step(model, ids)
+    assert model.embed_tokens[0].weight.grad is not None
+
+
 def test_tables_of_another_type_than_the_layers():
     """A 16-bit token table in an fp32 model: the embedded rows, and so the keys in the caches, are fp32."""
     model, ids = make(tie_weights=False)

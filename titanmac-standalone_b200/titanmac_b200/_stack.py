@@ -257,7 +257,9 @@ _tables: "weakref.WeakKeyDictionary[nn.Module, ModelTable]" = weakref.WeakKeyDic
 
 def table_of(model, training: bool = False) -> Optional[ModelTable]:
     """The model's table if it can be used right now (``training``: for a call with a gradient to come), else None."""
-    table, weight = _tables.get(model), model.embed_tokens.weight
+    table, weight = _tables.get(model), getattr(model.embed_tokens, "weight", None)
+    if not isinstance(weight, torch.Tensor):  # another kind of embedding
+        return None
     if table is None or weight.dtype is not table.dtype or weight.device != table.device or table.config is not model.config \
             or not table.holds():
         table = _tables[model] = ModelTable(model)
