@@ -89,6 +89,13 @@ def test_one_call_plan_only_for_inputs_and_weights_of_the_modules_own_shapes(spa
         m = module()
         getattr(m, name).to("meta")  # (another device than the input's)
         assert plan(m) is None, name
+    for name in ("qkv_proj", "out_proj"):
+        m = module()
+        lin = getattr(m, name)
+        w = lin.weight.detach()
+        del lin.weight
+        lin.weight = w  # a plain tensor, as wrappers that flatten parameters leave it
+        assert plan(m) is None, name
     m = module()
     m.n_heads = 20
     assert plan(m) is None

@@ -374,9 +374,9 @@ def _plain_weight(mod: nn.Module, kind, like: torch.Tensor, shape, training: boo
             or (training and (d["_backward_hooks"] or d["_backward_pre_hooks"])):
         return None
     p = d["_parameters"]
-    w = p["weight"]
-    return w if p["bias"] is None and w.dtype is like.dtype and w.shape == shape and w.is_contiguous() \
-        and w.device == like.device else None
+    w = p.get("weight")  # (a tensor that is no parameter stands elsewhere)
+    return w if w is not None and p.get("bias") is None and "bias" in p and w.dtype is like.dtype and w.shape == shape \
+        and w.is_contiguous() and w.device == like.device else None
 
 
 def attention_plan(attn: nn.Module, x: torch.Tensor, n_persistent: int, block_size: int, scale: float, training: bool = False):
