@@ -222,9 +222,10 @@ __global__ void __launch_bounds__(256) ce_forward_kernel(const CrossEntropy p) {
                     l *= __expf(m - mx);
                     m = mx;
                 }
-                // (a hidden logit counts nothing also while no other has been seen; a NaN reaches the sum whatever m is)
+                // while only hidden logits (-inf) or NaN have been seen, the former count nothing; a NaN reaches the sum anyway
+                const float base = m > -CUDART_INF_F ? m : 0.f;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) l += f[e] > -CUDART_INF_F || f[e] != f[e] ? __expf(f[e] - m) : 0.f;
+                for (int e = 0; e < 8; ++e) l += __expf(f[e] - base);
             }
     }
 #pragma unroll
