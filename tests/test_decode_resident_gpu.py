@@ -1,0 +1,118 @@
+"""The decode step as one resident kernel (up to eight sequences, head_dim 64) against the step module by module: the sizes at
+which its phases change shape, what must stay in its own sequence, generation, and the step under stream capture."""
+
+import pytest
+import torch
+
+from titanmac_b200 import TitanMAC, TitanMACConfig, _native, _stack
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def make(dtype, heads, window, n_p, vocab, layers=2, d_ff=None, positions=256, seed=0):
+    D = heads * 64
+    cfg = TitanMACConfig(vocab_size=vocab, d_model=D, n_heads=heads, n_layers=layers, d_ff=d_ff or 4 * D, max_seq_len=positions,
+                         window_size=window, n_persistent=n_p, use_block_sparse=False)
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    with torch.device(DEV):
+        model = TitanMAC(cfg).eval()
+    with torch.no_grad():
+        for name, prm in model.named_parameters():
+            prm.normal_(1.0 if name.endswith("scale") else 0.0, 0.1 if name.endswith(("scale", "bias")) else 0.04, generator=g)
+    return model.to(dtype), g
+
+
+def filled(model, B, dtype, g, sets=2):
+    caches = [model.new_caches(B, DEV, dtype) for _ in range(sets)]
+    for group in zip(*caches):
+        for tensors in zip(*((c.k_ring, c.v_ring, c.k_pers, c.v_pers) for c in group)):
+            tensors[0].normal_(0.0, 0.5, generator=g)
+            for t in tensors[1:]:
+                t.copy_(tensors[0])
+    return caches
+
+
+def relative(a, b):
+    return ((a.float() - b.float()).norm() / b.float().norm()).item()
+
+
+@pytest.mark.parametrize("B,dtype,heads,window,n_p,vocab,t,layers,d_ff", [
+    (1, torch.bfloat16, 1, 0, 0, 7, 0, 1, 32),            # the smallest: one key, fewer chunks of k than warps
+    (8, torch.float16, 1, 5, 3, 9, 2, 3, 96),             # ring not full, fewer keys than warps
+    (8, torch.bfloat16, 10, 512, 16, 50000, 600, 2, None),  # the default geometry
+    (7, torch.float16, 8, 250, 5, 1003, 1000, 2, None),   # 16 keys per warp
+    (3, torch.bfloat16, 5, 251, 5, 1000, 300, 2, 1056),   # 17: one key in the second tile; a width that is no multiple of 128
+    (2, torch.bfloat16, 10, 751, 16, 512, 800, 2, None),  # 48 keys per warp: what it holds at once
+    (8, torch.float16, 10, 752, 16, 512, 2000, 2, None),  # 49: twice
+    (1, torch.bfloat16, 12, 3000, 1, 520, 3100, 2, 3072),  # several times; the widest hidden layer
+    (5, torch.bfloat16, 12, 64, 16, 8000, 90, 32, None),  # the most layers
+])
+def test_against_the_modules(B, dtype, heads, window, n_p, vocab, t, layers, d_ff, monkeypatch):
+    model, g = make(dtype, heads, window, n_p, vocab, layers, d_ff, positions=t + 4)
+    ids = torch.randint(0, vocab, (B,), generator=g, device=DEV)
+    pos = torch.randint(max(0, t - 3), t + 1, (B,), generator=g, device=DEV, dtype=torch.int32)
+    got_caches, want_caches = filled(model, B, dtype, g)
+    got = [model.decode_step(ids, pos + i, got_caches) for i in range(2)]  # (the second reads what the first has written)
+    _native.poll_status(torch.device(DEV))
+    monkeypatch.setattr(_stack, "table_of", lambda m: None)
+    want = [model.decode_step(ids, pos + i, want_caches) for i in range(2)]
+    # rounding to 16 bits through `layers` layers, as between any two kernels of the step
+    tol = (2e-2 if dtype == torch.bfloat16 else 4e-3) * max(1.0, (layers / 8) ** 0.5)
+    for a, b in zip(got, want):
+        assert relative(a, b) <= tol, relative(a, b)
+    for a, b in zip(got_caches, want_caches):
+        assert relative(a.k_ring, b.k_ring) <= tol and relative(a.v_ring, b.v_ring) <= tol
+        same = a.k_ring == b.k_ring
+        assert same.all(-1).float().mean() >= 1 - 3 / (window + 1)  # nothing but the new rows was written
+
+
+def test_a_sequence_keeps_its_nan_to_itself():
+    """An id outside the table, and a NaN in one sequence's cache, reach that sequence's logits and no others."""
+    model, g = make(torch.bfloat16, 4, 40, 3, 256)
+    ids = torch.randint(0, 256, (6,), generator=g, device=DEV)
+    pos = torch.full((6,), 50, dtype=torch.int32, device=DEV)
+    clean, dirty = filled(model, 6, torch.bfloat16, g)
+    want = model.decode_step(ids, pos, clean)
+    dirty[0].v_ring[4, 1, 7, 9] = float("nan")
+    bad = ids.clone()
+    bad[2] = 256
+    got = model.decode_step(bad, pos, dirty)
+    with pytest.raises(_native.TmwError):
+        _native.poll_status(torch.device(DEV))
+    for b in range(6):
+        if b in (2, 4):
+            assert torch.isnan(got[b]).all()
+        else:
+            assert torch.equal(got[b], want[b])
+
+
+@pytest.mark.parametrize("B,dtype,vocab,new", [(1, torch.bfloat16, 1003, 30), (8, torch.float16, 4001, 9), (5, torch.bfloat16, 8, 2)])
+def test_generation_equals_steps(B, dtype, vocab, new):
+    model, g = make(dtype, 6, 20, 3, vocab, layers=3)
+    ids = torch.randint(0, vocab, (B, 11), generator=g, device=DEV)
+    got = model.generate(ids, new)
+    logits, caches = model.prefill(ids)
+    pos = torch.full((B,), 11, dtype=torch.int32, device=DEV)
+    for i in range(new):
+        token = logits.argmax(-1)
+        assert torch.equal(got[:, 11 + i], token), i
+        logits = model.decode_step(token, pos, caches)
+        pos += 1
+
+
+def test_step_under_capture():
+    model, g = make(torch.bfloat16, 4, 30, 2, 256)
+    ids = torch.randint(0, 256, (3,), generator=g, device=DEV)
+    pos = torch.full((3,), 40, dtype=torch.int32, device=DEV)
+    eager, captured = filled(model, 3, torch.bfloat16, g)
+    want = [model.decode_step(ids, pos + i, eager) for i in range(3)]
+    graph = torch.cuda.CUDAGraph()
+    static = pos.clone()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        logits = model.decode_step(ids, static, captured)
+    for i in range(3):
+        graph.replay()
+        assert torch.equal(logits, want[i]), i
+        static += 1

@@ -10,6 +10,7 @@
 //     up in a fixed order);
 //   * the kernels are launched as programmatic dependents: a kernel's weights are on their way into registers before
 //     its predecessor has finished.
+// Up to eight sequences with heads of 64 the step is one kernel instead (decode_resident.cu).
 #include <math_constants.h>
 
 #include "tmw_common.cuh"
@@ -535,6 +536,10 @@ StepBuffers step_buffers(const tmw_stack_desc& d) {
     s.splits = decode_step_splits(cache_of(d));
     s.counters = s.parts + (s.splits > 0 ? align256((int64_t)decode_partials_bytes(d.batch, d.heads, d.head_dim, s.splits)) : 0);
     s.total = s.counters + (s.splits > 0 ? align256((int64_t)d.batch * d.heads * 4) : 0);
+    if (decode_step_is_resident(d, nullptr)) {  // (which needs nothing of the above)
+        const int64_t resident = (int64_t)decode_resident_workspace(d);
+        s.total = s.total > resident ? s.total : resident;
+    }
     return s;
 }
 
@@ -672,6 +677,11 @@ extern "C" int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* bloc
     if (rc != TMW_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
+    if (decode_step_is_resident(*desc, blocks)) {
+        rc = decode_resident_begin(*desc, ws, s);
+        if (rc == TMW_OK) rc = launch_decode_resident(*desc, blocks, token_ids, pos, logits, 0, false, nullptr, 0, ws, s);
+        if (rc != TMW_ERR_UNSUPPORTED) return rc;
+    }
     rc = clear_counters(*desc, ws, s);
     if (rc != TMW_OK) return rc;
     return desc->dtype == TMW_BF16 ? decode_step_t<__nv_bfloat16>(*desc, blocks, token_ids, pos, logits, ws, 0, s)
@@ -689,6 +699,18 @@ extern "C" int tmw_generate(const tmw_stack_desc* desc, const tmw_block* blocks,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
     const tmw_stack_desc& d = *desc;
+    // (a tag is used once: 32 bits of them)
+    if (tokens > 1 && (int64_t)tokens * (d.layers + 1) < 0x7fffffff && decode_step_is_resident(d, blocks)) {
+        rc = d.dtype == TMW_BF16 ? launch_argmax<__nv_bfloat16>(d.batch, d.vocab, logits, token_ids, out, out_stride, pos, 0, false, s)
+                                 : launch_argmax<__half>(d.batch, d.vocab, logits, token_ids, out, out_stride, pos, 0, false, s);
+        if (rc == TMW_OK) rc = decode_resident_begin(d, ws, s);
+        if (rc != TMW_OK) return rc;
+        int step = 0;
+        for (; step < tokens - 1 && rc == TMW_OK; ++step)
+            rc = launch_decode_resident(d, blocks, token_ids, pos, logits, step, true, out + step, out_stride, ws, s);
+        if (rc == TMW_OK) return launch_decode_choice(d, step, token_ids, out + step, out_stride, pos, ws, s);
+        if (rc != TMW_ERR_UNSUPPORTED || step != 1) return rc;  // (refused: the first launch was; `step` counts it)
+    }
     rc = clear_counters(d, ws, s);
     if (rc != TMW_OK) return rc;
     auto run = [&](auto type) -> int {

@@ -289,6 +289,16 @@ int launch_decode(const tmw_cache_desc& c, const void* q, const void* k_new, con
                   const int64_t qs[2], const int64_t ns[2], const int64_t os[2], const int32_t* pos,
                   int splits, float* scratch, unsigned int* counters, cudaStream_t stream, bool pdl = false);
 int decode_step_splits(const tmw_cache_desc& c);
+// A decode step as one kernel (decode_resident.cu).  decode_resident_begin once, then steps 0, 1, ... in a row: `choose`: a step
+// leaves what its greedy choice needs, and a step behind it takes its tokens from there (and writes them to out), at the
+// positions pos + step; launch_decode_choice settles the last one.  TMW_ERR_UNSUPPORTED: the device cannot hold the kernel.
+bool decode_step_is_resident(const tmw_stack_desc& d, const tmw_block* blocks);
+size_t decode_resident_workspace(const tmw_stack_desc& d);
+int decode_resident_begin(const tmw_stack_desc& d, void* workspace, cudaStream_t stream);
+int launch_decode_resident(const tmw_stack_desc& d, const tmw_block* blocks, const int64_t* ids, const int32_t* pos, void* logits,
+                           int step, bool choose, int64_t* out, int64_t out_stride, void* workspace, cudaStream_t stream);
+int launch_decode_choice(const tmw_stack_desc& d, int steps, int64_t* tokens, int64_t* out, int64_t out_stride, int32_t* pos,
+                         void* workspace, cudaStream_t stream);
 
 // layout of the split-decode scratch memory: partial results, then (16-byte aligned) one counter per pair
 inline size_t decode_partials_bytes(int batch, int heads, int head_dim, int splits) {
