@@ -41,11 +41,13 @@ def relative(a, b):
     (1, torch.bfloat16, 1, 0, 0, 7, 0, 1, 32),            # the smallest: one key, fewer chunks of k than warps
     (8, torch.float16, 1, 5, 3, 9, 2, 3, 96),             # ring not full, fewer keys than warps
     (8, torch.bfloat16, 10, 512, 16, 50000, 600, 2, None),  # the default geometry
-    (7, torch.float16, 8, 250, 5, 1003, 1000, 2, None),   # 16 keys per warp
-    (3, torch.bfloat16, 5, 251, 5, 1000, 300, 2, 1056),   # 17: one key in the second tile; a width that is no multiple of 128
-    (2, torch.bfloat16, 10, 751, 16, 512, 800, 2, None),  # 48 keys per warp: what it holds at once
-    (8, torch.float16, 10, 752, 16, 512, 2000, 2, None),  # 49: twice
-    (1, torch.bfloat16, 12, 3000, 1, 520, 3100, 2, 3072),  # several times; the widest hidden layer
+    (7, torch.float16, 8, 186, 5, 1003, 1000, 2, None),   # 16 keys per warp: one tile
+    (3, torch.bfloat16, 5, 187, 5, 1000, 300, 2, 1056),   # 17: one key in the second; a width that is no multiple of 128
+    (2, torch.bfloat16, 10, 751, 16, 512, 800, 2, None),  # 64 keys per warp: four tiles, what it holds at once
+    (8, torch.float16, 10, 752, 16, 512, 2000, 2, None),  # 65: twice
+    (1, torch.bfloat16, 12, 3000, 1, 520, 3100, 2, 3072),  # several times; the widest that it takes
+    (4, torch.bfloat16, 13, 40, 2, 512, 60, 2, None),     # the next width: the chain
+    (8, torch.bfloat16, 2, 40, 2, 512, 60, 2, 3104),      # the next hidden width: the chain
     (5, torch.bfloat16, 12, 64, 16, 8000, 90, 32, None),  # the most layers
 ])
 def test_against_the_modules(B, dtype, heads, window, n_p, vocab, t, layers, d_ff, monkeypatch):

@@ -17,14 +17,17 @@
 // cannot hold it gets the chain of launches.  Every wait is bounded; when one expires, the polls of all CTAs end, the status
 // word says so, and the copies in flight are still waited for.
 //
-// What bounds it: instructions.  A layer is about 19 000 cycles for five exchanges of 500 to 900 (store to load, within a die
-// and across); the rest is what 16 warps issue between a poll that succeeds and the words that they send, about 10 cycles per
+// What bounds it: instructions.  A layer is about 17 000 cycles for five exchanges of 500 to 900 (store to load, within a die
+// and across); the rest is what the warps issue between a poll that succeeds and the words that they send, about 10 cycles per
 // instruction and warp, a third of them waiting for the slowest warp at a barrier.  So the code of a phase stands once, in a
 // loop over the half layers (separate code for each of the four products: 220 us instead of 207 for the model below), sums of
-// squares and scores are mma, and nothing is computed twice.  CUDA-core scores and weighted sums took 5000 cycles per layer,
-// these 3200, the most of it shared memory (135 KB per pair).
+// squares and scores are mma, and nothing is computed twice.  Twelve warps, three per scheduler, without register spills: 165 us
+// for 16 layers with a vocabulary of 8000, sixteen 184, ten 183, eight 177.  CUDA-core scores and weighted sums took 5000 cycles
+// per layer, these 3200, the most of it shared memory (135 KB per pair).  No gain: a phase's weights loaded a phase ahead, pauses
+// between polls, a poll of one word in front of the full one (164 us against 152), a barrier behind every send.
 //
-// 16 layers of width 640, vocabulary 50 000, window 512, one sequence: 313 us as a chain of launches, 204 as one kernel.
+// 16 layers of width 640, vocabulary 50 000, window 512, one sequence: 313 us as a chain of launches, 170 as one kernel; eight
+// prompts of 300 continued by 48 tokens: 17.2 and 10.9 ms.
 #include <math_constants.h>
 
 #include "tc_ptx.cuh"
@@ -33,11 +36,12 @@
 namespace tmw {
 namespace {
 
-constexpr int kThreads = 512, kWarps = 16, kRows = 8;  // kRows: sequences at most, half an mma's rows
+constexpr int kWarps = 12, kThreads = 32 * kWarps, kRows = 8;  // kRows: sequences at most, half an mma's rows
 constexpr int kHeadDim = 64, kRowBytes = kHeadDim * 2;
 constexpr int kMaxLayers = 32;                       // the table travels as a kernel parameter (4 KB)
-constexpr int kMaxDim = 1024, kMaxHidden = 3072;     // chunks of 32 elements that a warp holds: 2 and 8
-constexpr int kMaxGroup = 48;                        // keys that a warp has on chip: three tiles of 16
+constexpr int kMaxDim = 768, kMaxHidden = 3072;
+constexpr int kInChunks = (kMaxDim / 32 + kWarps - 1) / kWarps;  // chunks of 32 elements of k that a warp has, at most
+constexpr int kMaxGroup = (768 / kWarps + 15) / 16 * 16;                        // keys that a warp has on chip: three tiles of 16
 constexpr int kSmemLimit = 227 * 1024;
 
 struct HalfLayer {  // norm -> product -> (attention | GELU) -> product + residual
@@ -80,8 +84,8 @@ __device__ __forceinline__ void ld_words(const uint64_t* p, uint64_t& a, uint64_
     asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 }
 // Rows that all CTAs wait for are sent to kCopies places, `copy` words apart, and a CTA polls one of them, so that fewer poll the
-// same lines of L2 (16 layers, vocabulary 8000: one sequence 214 -> 206 us, four 240 -> 229; eight copies are no better).
-constexpr int kCopies = 4;
+// same lines of L2 (16 layers, vocabulary 8000, one | eight sequences: one copy 158 | 205 us, four 152 | 211, eight 156 | 218).
+constexpr int kCopies = 2;
 __device__ __forceinline__ void st_word(uint64_t* p, uint32_t bits, uint32_t tag) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(((uint64_t)tag << 32) | bits) : "memory");
 }
@@ -96,12 +100,13 @@ constexpr int kMaxPairs = 4;  // (sequence, head) pairs of a CTA
 struct KeyRange {  // a warp's keys of a pair
     int lo, hi, slot_new, sequence, head;
 };
+constexpr int kSums = (kWarps + 3) / 4 * 4;
 struct Shared {
     LayerTable layer[kMaxLayers];  // (out of the parameters: a first touch in the constant cache is a trip to L2, every layer)
     long long id[kRows];
     int pos[kRows], bad[kRows];
     unsigned long long best[kRows];
-    __align__(16) float ss[kRows][kWarps];
+    __align__(16) float ss[kRows][kSums];
     __align__(16) float part[kWarps][kHeadDim + 2];
     KeyRange range[kMaxPairs][kWarps];
     int abort;
@@ -129,15 +134,6 @@ __device__ __forceinline__ void receive(uint4 (&out)[N], const uint64_t* src, in
     uint64_t v[N][4] = {};
     long long t0 = 0;
     uint32_t spins = 0;
-    // first for one pair of words: a poll of few instructions, which leaves the SM's issue slots to the warps that still compute
-#pragma unroll 1
-    for (;;) {
-        uint64_t a = (uint64_t)tag << 32, b = a;
-        if (n > 0) ld_words(src, a, b);
-        if (!__any_sync(0xffffffffu, (((uint32_t)(a >> 32) ^ tag) | ((uint32_t)(b >> 32) ^ tag)) != 0u)) break;
-        if (++spins == 1u) t0 = clock64();
-        if ((spins & 63u) == 0u && __any_sync(0xffffffffu, patience_over(p.abort, p.status, &sh.abort, t0))) break;
-    }
 #pragma unroll 1
     for (;;) {
 #pragma unroll
@@ -196,7 +192,7 @@ __device__ __forceinline__ float2 unpack(uint32_t raw) {
     return make_float2(to_f32<T>(w[0]), to_f32<T>(w[1]));
 }
 
-// Partial sums of the 16 warps, [warp][row][column], in rows of 24 floats for the products with a norm (up to 24 columns) and of
+// Partial sums of the warps, [warp][row][column], in rows of 24 floats for the products with a norm (up to 24 columns) and of
 // 8 for those with the residual; the 8-byte accesses meet no bank twice.
 // Outputs: a lane has row lane % 8 and two columns of an eight, a warp an eight.
 constexpr int kInStride = 24, kOutStride = 8;
@@ -229,13 +225,16 @@ __device__ __forceinline__ float inv_sqrt(float v) {
 // eight adjacent values of a chunk, the same ones for both operands, so their order does not matter.  The sums of squares are
 // the diagonal of x x^T, two more mma per chunk.
 template <typename T>
-__device__ __forceinline__ void normed_rows(uint4 (&a)[2], const uint4 (&gain)[2], const uint64_t* x, int n, uint32_t tag,
+__device__ __forceinline__ void normed_rows(uint4 (&a)[kInChunks], const uint4 (&gain)[kInChunks], const uint64_t* x, int n, uint32_t tag,
                                             const ResidentParams& p, Shared& sh, int warp, int g, int t) {
-    receive<2>(a, x + ((blockIdx.x % kCopies * p.rows + g) * p.dim + warp * 32 + t * 8) / 2, g < p.rows ? n : 0, tag, p, sh);
+    float gains[kInChunks][8];
+#pragma unroll
+    for (int i = 0; i < kInChunks; ++i) load8<T>(reinterpret_cast<const T*>(&gain[i]), gains[i]);
+    receive<kInChunks>(a, x + ((blockIdx.x % kCopies * p.rows + g) * p.dim + warp * 32 + t * 8) / 2, g < p.rows ? n : 0, tag, p, sh);
     if (n > 0) {
         float c[4] = {};
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < kInChunks; ++i)
             if (i == 0 || i < n) {
                 mma_16816<T>(c, a[i].x, 0u, a[i].y, 0u, a[i].x, a[i].y);
                 mma_16816<T>(c, a[i].z, 0u, a[i].w, 0u, a[i].z, a[i].w);
@@ -246,7 +245,7 @@ __device__ __forceinline__ void normed_rows(uint4 (&a)[2], const uint4 (&gain)[2
     if (n <= 0) return;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);  // (warps without a chunk left zeros at the start)
 #pragma unroll
-    for (int q = 0; q < kWarps / 4; ++q) {
+    for (int q = 0; q < kSums / 4; ++q) {
         const float4 u = *reinterpret_cast<const float4*>(&sh.ss[g][q * 4]);
         s.x += u.x;
         s.y += u.y;
@@ -255,21 +254,21 @@ __device__ __forceinline__ void normed_rows(uint4 (&a)[2], const uint4 (&gain)[2
     }
     const float inv = inv_sqrt(fmaf((s.x + s.y) + (s.z + s.w), p.inv_dim, p.eps));
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < kInChunks; ++i)
         if (i == 0 || i < n) {
-            float v[8], w[8];
+            float v[8];
             load8<T>(reinterpret_cast<const T*>(&a[i]), v);
-            load8<T>(reinterpret_cast<const T*>(&gain[i]), w);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * w[e];
+            for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * gains[i][e];
             store8<T>(reinterpret_cast<T*>(&a[i]), v);
         }
 }
 
-// The weights of a phase are loaded into registers in front of its poll.  In: nt * 8 rows of this CTA, two chunks of k per warp at most; out: eight rows.
+// The weights of a phase are loaded into registers in front of its poll.  In: nt * 8 rows
+// of this CTA; out: eight rows.
 constexpr int kInTiles = 3;
 struct InWeights {
-    uint4 w[2][kInTiles], gain[2];
+    uint4 w[kInChunks][kInTiles], gain[kInChunks];
 };
 template <typename T>
 __device__ __forceinline__ void load_in(InWeights& r, const ResidentParams& p, const HalfLayer& l, int n, int nt) {
@@ -278,7 +277,7 @@ __device__ __forceinline__ void load_in(InWeights& r, const ResidentParams& p, c
     const T* src = static_cast<const T*>(l.w_in) + (n0 + g) * p.dim + k;
     const T* gain = static_cast<const T*>(l.norm) + k;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kInChunks; ++i) {
 #pragma unroll
         for (int j = 0; j < kInTiles; ++j) {
             r.w[i][j] = make_uint4(0u, 0u, 0u, 0u);
@@ -311,14 +310,14 @@ __device__ __forceinline__ void norm_product(const ResidentParams& p, Shared& sh
     const bool out = warp < nt && row < p.rows && n0 + col < n;
     uint32_t bias = 0u;
     if (l.b_in != nullptr && out) bias = *reinterpret_cast<const uint32_t*>(static_cast<const T*>(l.b_in) + n0 + col);
-    uint4 a[2];
+    uint4 a[kInChunks];
     normed_rows<T>(a, in.gain, x, mine, tag_in, p, sh, warp, g, t);
 #pragma unroll
     for (int j = 0; j < kInTiles; ++j)
         if (j < nt) {
             float acc[4] = {};
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < kInChunks; ++i)
                 if (i < mine) {
                     mma_16816<T>(acc, a[i].x, 0u, a[i].y, 0u, in.w[i][j].x, in.w[i][j].y);
                     mma_16816<T>(acc, a[i].z, 0u, a[i].w, 0u, in.w[i][j].z, in.w[i][j].w);
@@ -342,7 +341,7 @@ __device__ __forceinline__ void norm_product(const ResidentParams& p, Shared& sh
 }
 
 // x' = x + round(a w^T + bias) for eight columns of every row; x stays in the thread that computes it
-constexpr int kOutChunks = kMaxHidden / 32 / kWarps;  // chunks of k that a warp has at most
+constexpr int kOutChunks = (kMaxHidden / 32 + kWarps - 1) / kWarps;  // chunks of k that a warp has at most
 template <typename T>
 __device__ __forceinline__ void residual_product(const ResidentParams& p, Shared& sh, float* red, const uint4 (&w)[kOutChunks],
                                                  const HalfLayer& l, const uint64_t* src, int k, uint64_t* dst, uint32_t tag, uint32_t& x) {
@@ -372,7 +371,7 @@ __device__ __forceinline__ void residual_product(const ResidentParams& p, Shared
     }
 }
 
-// The keys of a (sequence, head) pair - persistent rows, then the ring slots in use - are cut into 16 ranges, one per warp.
+// The keys of a (sequence, head) pair - persistent rows, then the ring slots in use - are cut into a range per warp.
 // A warp has up to kMaxGroup keys and values of its range in shared memory of its own and, once it is done with them, fetches
 // the next: of the same range where it is longer, else of its next pair, else of the next layer, whose rows are then on their
 // way while the products of this one run.
@@ -535,14 +534,14 @@ __device__ __forceinline__ void attention(const ResidentParams& p, Shared& sh, i
         if (lane == 0) *reinterpret_cast<float2*>(&sh.part[warp][kHeadDim]) = make_float2(m, sum);
         __syncthreads();
         if (warp == 0) {
-            const float2 ml = *reinterpret_cast<const float2*>(&sh.part[lane & 15][kHeadDim]);
+            const float2 ml = lane < kWarps ? *reinterpret_cast<const float2*>(&sh.part[lane][kHeadDim]) : make_float2(-CUDART_INF_F, 0.f);
             float top = ml.x;
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
             const float w = exp2f(ml.x - (top > -CUDART_INF_F ? top : 0.f));
             float all = ml.y * w;
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+            for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
             float2 r = make_float2(0.f, 0.f);
 #pragma unroll
             for (int i = 0; i < kWarps; ++i) {
@@ -588,7 +587,9 @@ __device__ __forceinline__ long long chosen(const unsigned long long* best, int 
 
 // logits = norm(x) head^T: the rows, normalised, in shared memory for all warps; a warp takes tiles of eight vocabulary rows
 // with the whole of k, kHeadDepth loads of 16 bytes per lane in flight
-constexpr int kHeadDepth = 16;
+// half layers in front of the head under which its weights go into L2 (under all of them: 170 us instead of 167)
+constexpr int kHeadSteps = 8;
+constexpr int kHeadDepth = 20;
 
 template <typename T>
 __device__ __forceinline__ void head_product(const ResidentParams& p, Shared& sh, unsigned char* mem, uint32_t tag) {
@@ -608,16 +609,16 @@ __device__ __forceinline__ void head_product(const ResidentParams& p, Shared& sh
     }
     const int stride = p.dim * 2 + 64;  // bytes of a row: eight lanes of a 16-byte access fall on different banks
     {
-        uint4 gain[2], a[2];
+        uint4 gain[kInChunks], a[kInChunks];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kInChunks; ++i) {
             gain[i] = make_uint4(0u, 0u, 0u, 0u);
             if (warp + kWarps * i < chunks)
                 gain[i] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.norm) + (warp + kWarps * i) * 32 + t * 8);
         }
         normed_rows<T>(a, gain, p.x, (chunks - warp + kWarps - 1) / kWarps, tag, p, sh, warp, g, t);
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < kInChunks; ++i)
             if (warp + kWarps * i < chunks) *reinterpret_cast<uint4*>(mem + g * stride + (warp + kWarps * i) * 64 + t * 16) = a[i];
     }
     __syncthreads();
@@ -683,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __gr
         reinterpret_cast<uint64_t*>(sh.layer)[i] = reinterpret_cast<const uint64_t*>(p.layer)[i];
     if (tid == 0) sh.abort = 0;
     if (tid < kRows) sh.best[tid] = 0ull;
-    if (tid < kRows * kWarps) sh.ss[tid / kWarps][tid % kWarps] = 0.f;
+    for (int i = tid; i < kRows * kSums; i += kThreads) sh.ss[i / kSums][i % kSums] = 0.f;
     if (warp < p.rows) {
         long long id = 0;
         if (p.best_in != nullptr) {
@@ -746,7 +747,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __gr
         prefetch(sh.layer[0].half[1], true);
     }
     __syncwarp();
-    const long long head_part = ((long long)p.vocab * p.dim * 2 / ((long long)ctas * 2 * p.layers)) & ~15ll;
+    const int head_from = max(0, 2 * p.layers - kHeadSteps);
+    const long long head_part = ((long long)p.vocab * p.dim * 2 / ((long long)ctas * (2 * p.layers - head_from))) & ~15ll;
     // (one loop over the halves of all layers: each phase's code once, which the instruction caches hold)
 #pragma unroll 1
     for (int step = 0; step < 2 * p.layers; ++step) {
@@ -763,7 +765,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __gr
         if (!mlp) attention<T>(p, sh, first, units, mem, l, tag);
         if (warp == kWarps - 1 && ptx::elect_one()) {  // this half of the next layer, and a part of the head
             if (l + 1 < p.layers) prefetch(sh.layer[l + 1].half[mlp], mlp);
-            prefetch_l2(static_cast<const char*>(p.head) + ((long long)step * ctas + cta) * head_part, head_part);
+            if (step >= head_from)
+                prefetch_l2(static_cast<const char*>(p.head) + ((long long)(step - head_from) * ctas + cta) * head_part, head_part);
         }
         __syncwarp();
         {
@@ -843,12 +846,13 @@ int launch(const ResidentParams& p, int ctas, int smem, cudaStream_t stream) {
 
 }  // namespace
 
-// The line is where the registers and the mma's rows end: eight sequences, three tiles of eight columns per CTA, chunks of k as
-// declared above.  us per step as one kernel / as a chain (8 layers of width 640, vocabulary 8000, 16 persistent rows):
-//   window   64: 1 sequence  91 / 155, 8: 114 / 160        512: 1: 106 / 157, 4: 117 / 176, 8: 139 / 184
-//   window 1024: 1: 127 / 169, 4: 150 / 202, 8: 178 / 208  3000: 1: 192 / 212, 4: 214 / 297, 8: 260 / 304
-// With the mma's other eight rows in use: 9 sequences 162 / 187 and 16 208 / 190 at window 512, 274 / 216 at 1024: not kept.
-// Windows that the chain splits over the chip (decode_step_splits) stay with it.
+// The line is where the registers and the used half of the mma's rows end: eight sequences, three tiles of eight columns per
+// CTA, chunks of k as declared above.  us per step as one kernel / as a chain (8 layers, vocabulary 8000, 16 persistent rows):
+//   width 640, window 64: 1 sequence 78 / 155, 4: 84 / 156, 8: 93 / 160       512: 1: 82 / 155, 4: 90 / 175, 8: 110 / 183
+//              window 1024: 1: 106 / 169, 4: 127 / 203, 8: 144 / 208           3000: 1: 171 / 211, 4: 190 / 297, 8: 221 / 304
+//   width 512, window 512: 1: 77 / 149, 8: 94 / 170                            width 768: 8: 122 / 205
+// With the mma's other eight rows in use (sixteen warps): 9 sequences 162 / 187 and 16 208 / 190 at window 512, 274 / 216 at
+// 1024: not kept.  Windows that the chain splits over the chip (decode_step_splits) stay with it.
 bool decode_step_is_resident(const tmw_stack_desc& d, const tmw_block* blocks) {
     const int sms = sm_count();
     if (d.batch < 1 || d.batch > kRows || d.layers < 1 || d.layers > kMaxLayers || d.head_dim != kHeadDim || d.d_model > kMaxDim ||
