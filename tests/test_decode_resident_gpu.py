@@ -91,6 +91,31 @@ def test_a_sequence_keeps_its_nan_to_itself():
             assert torch.equal(got[b], want[b])
 
 
+@pytest.mark.parametrize("bad", [2 ** 31 - 1, 2 ** 31 - 2, 256, -1, -2 ** 31])
+def test_positions_outside_the_table(bad):
+    """Such a sequence's logits are NaN and its new key and value (NaN too) go to the slot of that position
+    (of position 0, if negative); the others are as without it."""
+    model, g = make(torch.bfloat16, 4, 40, 3, 256)
+    ids = torch.randint(0, 256, (3,), generator=g, device=DEV)
+    pos = torch.full((3,), 50, dtype=torch.int32, device=DEV)
+    clean, dirty = filled(model, 3, torch.bfloat16, g)
+    before = [(c.k_ring.clone(), c.v_ring.clone()) for c in dirty]
+    want = model.decode_step(ids, pos, clean)
+    _native.poll_status(torch.device(DEV))
+    pos[1] = bad
+    got = model.decode_step(ids, pos, dirty)
+    with pytest.raises(_native.TmwError):
+        _native.poll_status(torch.device(DEV))
+    assert torch.isnan(got[1]).all() and torch.equal(got[0::2], want[0::2])
+    slot = max(bad, 0) % 41
+    for a, b, (k, v) in zip(dirty, clean, before):
+        for ring, other, old in ((a.k_ring, b.k_ring, k), (a.v_ring, b.v_ring, v)):
+            assert torch.equal(ring[0::2], other[0::2])
+            assert torch.isnan(ring[1, :, slot]).all()
+            old[1, :, slot] = ring[1, :, slot]
+            assert torch.equal(ring[1].view(torch.int16), old[1].view(torch.int16))
+
+
 @pytest.mark.parametrize("B,dtype,vocab,new", [(1, torch.bfloat16, 1003, 30), (8, torch.float16, 4001, 9), (5, torch.bfloat16, 8, 2)])
 def test_generation_equals_steps(B, dtype, vocab, new):
     model, g = make(dtype, 6, 20, 3, vocab, layers=3)

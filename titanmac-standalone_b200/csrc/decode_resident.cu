@@ -380,7 +380,7 @@ __device__ __forceinline__ KeyRange key_range(const ResidentParams& p, const Sha
     r.sequence = pair / p.heads;
     r.head = pair - r.sequence * p.heads;
     const int t = max(sh.pos[r.sequence], 0);
-    const int n = p.np + min(t + 1, p.slots), per = (n + kWarps - 1) / kWarps;
+    const int n = p.np + min(t, p.slots - 1) + 1, per = (n + kWarps - 1) / kWarps;  // (t may be 2^31 - 1: no t + 1)
     r.lo = min(n, warp * per);
     r.hi = min(n, r.lo + per);
     r.slot_new = t % p.slots;
