@@ -166,3 +166,29 @@ def test_negative_position_is_reported_not_written_out_of_bounds():
     changed = (cache.k_ring != guard_k).any(dim=-1).any(dim=1)  # [B, slots]
     assert changed.nonzero().tolist() == [[0, 5], [1, 0], [2, 2]]
     _native.poll_status(torch.device(DEV))  # the status word was cleared
+
+
+@pytest.mark.parametrize("B,H,dh,dtype,splits", [
+    (2, 2, 64, torch.float32, 0),       # register kernel
+    (2, 2, 64, torch.bfloat16, 0),      # clusters
+    (120, 8, 64, torch.bfloat16, 0),    # streaming, two warps per pair
+    (170, 8, 128, torch.float16, 0),    # streaming, one warp per pair
+    (1, 2, 64, torch.bfloat16, 3),      # split
+])
+def test_the_last_position(B, H, dh, dtype, splits):
+    """A step at position 2^31 - 1 is one at any other position of the same slot behind the first round of the ring."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    outs = []
+    last = 2 ** 31 - 1
+    for t in (last, last % 41 + 41):
+        g.manual_seed(3)
+        cache = _native.RingCache(B, H, dh, 40, 3, dtype, DEV)
+        for ring in (cache.k_ring, cache.v_ring, cache.k_pers, cache.v_pers):
+            ring.normal_(0.0, 0.5, generator=g)
+        cache.splits = splits
+        q, k, v = (torch.empty((B, H, dh), dtype=dtype, device=DEV).normal_(generator=g) for _ in range(3))
+        pos = torch.full((B,), t, dtype=torch.int32, device=DEV)
+        outs.append((cache.decode(q, k, v, pos), cache.k_ring, cache.v_ring))
+    _native.poll_status(torch.device(DEV))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)

@@ -138,7 +138,7 @@ decode_kernel(const DecodeParams p) {
         t = 0;
     }
     const int slot_new = t % p.slots;
-    const int count = min(t + 1, p.slots);
+    const int count = min(t, p.slots - 1) + 1;  // (t may be 2^31 - 1)
     const long long ring_bh = ((long long)b * p.heads + h) * p.slots * DH;
     T* kr = static_cast<T*>(p.k_ring) + ring_bh;
     T* vr = static_cast<T*>(p.v_ring) + ring_bh;
@@ -423,7 +423,7 @@ decode_stream_kernel(const DecodeParams p) {
         t = 0;
     }
     const int slot_new = t % p.slots;
-    const int count = min(t + 1, p.slots);
+    const int count = min(t, p.slots - 1) + 1;  // (t may be 2^31 - 1)
     const long long ring_bh = ((long long)b * p.heads + h) * p.slots * DH;
     T* kr = static_cast<T*>(p.k_ring) + ring_bh;
     T* vr = static_cast<T*>(p.v_ring) + ring_bh;
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kClusterWarps * 32, 5) decode_cluster_kernel(c
         t = 0;
     }
     const int slot_new = t % p.slots;
-    const int n_keys = p.np + min(t + 1, p.slots) - 1;  // persistent rows, then the older ring slots in slot order
+    const int n_keys = p.np + min(t, p.slots - 1);  // persistent rows, then the older ring slots in slot order
     const long long ring_bh = ((long long)b * p.heads + h) * p.slots * DH;
     T* kr = static_cast<T*>(p.k_ring) + ring_bh;
     T* vr = static_cast<T*>(p.v_ring) + ring_bh;
