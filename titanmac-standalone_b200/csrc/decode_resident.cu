@@ -96,7 +96,6 @@ __device__ __forceinline__ void st_copies(uint64_t* p, int copy, uint32_t bits, 
 }
 
 // what a CTA shares; the variable part (partial sums, ring rows) follows in dynamic shared memory
-constexpr int kMaxPairs = 4;  // (sequence, head) pairs of a CTA
 struct KeyRange {  // a warp's keys of a pair
     int lo, hi, slot_new, sequence, head;
 };
@@ -108,7 +107,7 @@ struct Shared {
     unsigned long long best[kRows];
     __align__(16) float ss[kRows][kSums];
     __align__(16) float part[kWarps][kHeadDim + 2];
-    KeyRange range[kMaxPairs][kWarps];
+    KeyRange range[kWarps];
     int abort;
 };
 
@@ -373,8 +372,8 @@ __device__ __forceinline__ void residual_product(const ResidentParams& p, Shared
 
 // The keys of a (sequence, head) pair - persistent rows, then the ring slots in use - are cut into a range per warp.
 // A warp has up to kMaxGroup keys and values of its range in shared memory of its own and, once it is done with them, fetches
-// the next: of the same range where it is longer, else of its next pair, else of the next layer, whose rows are then on their
-// way while the products of this one run.
+// the next: of the same range where it is longer, else of the next layer, whose rows are then on their way while the products of
+// this one run.  A CTA has one pair or none.
 __device__ __forceinline__ KeyRange key_range(const ResidentParams& p, const Shared& sh, int pair, int warp) {
     KeyRange r;
     r.sequence = pair / p.heads;
@@ -429,155 +428,146 @@ struct Parts<__half> {
     static constexpr float kRaise = 15.f, kNext = 2048.f;
 };
 template <typename T>
-__device__ __forceinline__ void attention(const ResidentParams& p, Shared& sh, int first, int units, unsigned char* mem, int layer, uint32_t tag) {
+__device__ __forceinline__ void attention(const ResidentParams& p, Shared& sh, int pair, unsigned char* mem, int layer, uint32_t tag) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const LayerTable& l = sh.layer[layer];
     const uint32_t k_mem = ptx::smem_u32(mem), v_mem = k_mem + p.group_keys * kRowBytes;
     const float part1 = g >= 1 ? -1.f : 0.f, part2 = g >= 2 ? -1.f : 0.f;  // what a lane's column leaves out of a weight
     const float raise1 = g >= 1 ? Parts<T>::kNext : 1.f, raise2 = g >= 2 ? Parts<T>::kNext : 1.f;
     const uint32_t mask = g <= 2 ? 0xffffffffu : 0u;
-#pragma unroll 1
-    for (int unit = 0; unit < units; ++unit) {
-        const KeyRange range = sh.range[unit][warp];
-        const int i_new = p.np + range.slot_new;
-        const bool brings = i_new >= range.lo && i_new < range.hi;
-        // query and, in the warp whose range holds the new token's slot, its key and value: two elements per lane
-        uint32_t got[3];
-        receive_words<3>(got, p.qkv + (range.sequence * 3 * p.dim + range.head * kHeadDim) / 2 + lane, p.dim / 2, brings, tag, p, sh);
-        uint32_t q[4][2];
+    const KeyRange range = sh.range[warp];
+    const int i_new = p.np + range.slot_new;
+    const bool brings = i_new >= range.lo && i_new < range.hi;
+    // query and, in the warp whose range holds the new token's slot, its key and value: two elements per lane
+    uint32_t got[3];
+    receive_words<3>(got, p.qkv + (range.sequence * 3 * p.dim + range.head * kHeadDim) / 2 + lane, p.dim / 2, brings, tag, p, sh);
+    uint32_t q[4][2];
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            q[kk][0] = __shfl_sync(0xffffffffu, got[0], kk * 8 + t);
-            q[kk][1] = __shfl_sync(0xffffffffu, got[0], kk * 8 + 4 + t);
-        }
-        float m = -CUDART_INF_F, sum = 0.f, acc[4][4] = {};
-        int at = range.lo;
-        do {
-            const int n = min(p.group_keys, range.hi - at);
-            asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int kk = 0; kk < 4; ++kk) {
+        q[kk][0] = __shfl_sync(0xffffffffu, got[0], kk * 8 + t);
+        q[kk][1] = __shfl_sync(0xffffffffu, got[0], kk * 8 + 4 + t);
+    }
+    float m = -CUDART_INF_F, sum = 0.f, acc[4][4] = {};
+    int at = range.lo;
+    do {
+        const int n = min(p.group_keys, range.hi - at);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (brings && i_new >= at && i_new < at + n) {  // the copy brought what falls out of the window
+            const uint32_t to = unit_offset(i_new - at, lane >> 2) + (lane & 3) * 4;
+            *reinterpret_cast<uint32_t*>(mem + to) = got[1];
+            *reinterpret_cast<uint32_t*>(mem + p.group_keys * kRowBytes + to) = got[2];
             __syncwarp();
-            if (brings && i_new >= at && i_new < at + n) {  // the copy brought what falls out of the window
-                const uint32_t to = unit_offset(i_new - at, lane >> 2) + (lane & 3) * 4;
-                *reinterpret_cast<uint32_t*>(mem + to) = got[1];
-                *reinterpret_cast<uint32_t*>(mem + p.group_keys * kRowBytes + to) = got[2];
-                __syncwarp();
-            }
-            uint32_t off[kMaxGroup / 16];
-            float s[kMaxGroup / 16][4], top = -CUDART_INF_F;
-            bool any = false;
+        }
+        uint32_t off[kMaxGroup / 16];
+        float s[kMaxGroup / 16][4], top = -CUDART_INF_F;
+        bool any = false;
 #pragma unroll
-            for (int c = 0; c < kMaxGroup / 16; ++c)
-                if (c * 16 < n) {
-                    const int row = min(c * 16 + (lane & 7) + (lane >> 4) * 8, n - 1);  // (no key of its own: the last one, at weight zero)
-                    off[c] = unit_offset(row, (lane >> 3) & 1);
-                    float lo[4] = {}, hi[4] = {};
+        for (int c = 0; c < kMaxGroup / 16; ++c)
+            if (c * 16 < n) {
+                const int row = min(c * 16 + (lane & 7) + (lane >> 4) * 8, n - 1);  // (no key of its own: the last one, at weight zero)
+                off[c] = unit_offset(row, (lane >> 3) & 1);
+                float lo[4] = {}, hi[4] = {};
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        uint32_t k[4];
-                        ldmatrix(k, k_mem + (off[c] ^ (kk << 5)));
-                        mma_16816<T>(lo, q[kk][0], 0u, q[kk][1], 0u, k[0], k[1]);
-                        mma_16816<T>(hi, q[kk][0], 0u, q[kk][1], 0u, k[2], k[3]);
-                    }
-                    const int left = n - c * 16 - 2 * t;
-                    s[c][0] = left > 0 ? lo[0] * l.scale_log2 : -CUDART_INF_F;
-                    s[c][1] = left > 1 ? lo[1] * l.scale_log2 : -CUDART_INF_F;
-                    s[c][2] = left > 8 ? hi[0] * l.scale_log2 : -CUDART_INF_F;
-                    s[c][3] = left > 9 ? hi[1] * l.scale_log2 : -CUDART_INF_F;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        top = fmaxf(top, s[c][e]);
-                        any = any || s[c][e] != -CUDART_INF_F;  // (NaN too)
-                    }
+                for (int kk = 0; kk < 4; ++kk) {
+                    uint32_t k[4];
+                    ldmatrix(k, k_mem + (off[c] ^ (kk << 5)));
+                    mma_16816<T>(lo, q[kk][0], 0u, q[kk][1], 0u, k[0], k[1]);
+                    mma_16816<T>(hi, q[kk][0], 0u, q[kk][1], 0u, k[2], k[3]);
                 }
-            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
-            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-            any = __any_sync(0xffffffffu, any);
-            const float m_new = fmaxf(m, top), base = any ? m_new - Parts<T>::kRaise : 0.f;
-            if (at > range.lo) {
-                const float alpha = any ? exp2f(m - m_new) : 1.f;
-                sum *= alpha;
+                const int left = n - c * 16 - 2 * t;
+                s[c][0] = left > 0 ? lo[0] * l.scale_log2 : -CUDART_INF_F;
+                s[c][1] = left > 1 ? lo[1] * l.scale_log2 : -CUDART_INF_F;
+                s[c][2] = left > 8 ? hi[0] * l.scale_log2 : -CUDART_INF_F;
+                s[c][3] = left > 9 ? hi[1] * l.scale_log2 : -CUDART_INF_F;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[j][e] *= alpha;
-            }
-            m = m_new;
-#pragma unroll
-            for (int c = 0; c < kMaxGroup / 16; ++c)
-                if (c * 16 < n) {
-                    uint32_t b[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        float2 w = make_float2(exp2f(s[c][2 * e] - base), exp2f(s[c][2 * e + 1] - base));
-                        sum += w.x + w.y;
-                        float2 h = unpack<T>(pack<T>(w.x, w.y));
-                        w = make_float2(fmaf(h.x, part1, w.x) * raise1, fmaf(h.y, part1, w.y) * raise1);
-                        h = unpack<T>(pack<T>(w.x, w.y));
-                        b[e] = pack<T>(fmaf(h.x, part2, w.x) * raise2, fmaf(h.y, part2, w.y) * raise2) & mask;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint32_t v[4];
-                        ldmatrix_trans(v, v_mem + (off[c] ^ (j << 5)));
-                        mma_16816<T>(acc[j], v[0], v[1], v[2], v[3], b[0], b[1]);
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    top = fmaxf(top, s[c][e]);
+                    any = any || s[c][e] != -CUDART_INF_F;  // (NaN too)
                 }
-            at += p.group_keys;
-            if (at < range.hi) {  // more of this range
-                __syncwarp();
-                fetch_rows(p, l.k_ring, l.k_pers, range, first + unit * gridDim.x, at, k_mem, lane);
-                fetch_rows(p, l.v_ring, l.v_pers, range, first + unit * gridDim.x, at, v_mem, lane);
             }
-        } while (at < range.hi);
-        // merge the warps
-        if (unit > 0) __syncthreads();  // (the pair before has been merged)
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        any = __any_sync(0xffffffffu, any);
+        const float m_new = fmaxf(m, top), base = any ? m_new - Parts<T>::kRaise : 0.f;
+        if (at > range.lo) {
+            const float alpha = any ? exp2f(m - m_new) : 1.f;
+            sum *= alpha;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float lower0 = t == 0 ? 1.f : 1.f / (Parts<T>::kNext * Parts<T>::kNext), lower1 = 1.f / Parts<T>::kNext;
-            float2 v = make_float2(fmaf(acc[j][1], lower1, acc[j][0] * lower0), fmaf(acc[j][3], lower1, acc[j][2] * lower0));
-            v.x += __shfl_xor_sync(0xffffffffu, v.x, 1);
-            v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
-            if (t == 0) {
-                sh.part[warp][j * 16 + g] = v.x;
-                sh.part[warp][j * 16 + 8 + g] = v.y;
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] *= alpha;
+        }
+        m = m_new;
+#pragma unroll
+        for (int c = 0; c < kMaxGroup / 16; ++c)
+            if (c * 16 < n) {
+                uint32_t b[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float2 w = make_float2(exp2f(s[c][2 * e] - base), exp2f(s[c][2 * e + 1] - base));
+                    sum += w.x + w.y;
+                    float2 h = unpack<T>(pack<T>(w.x, w.y));
+                    w = make_float2(fmaf(h.x, part1, w.x) * raise1, fmaf(h.y, part1, w.y) * raise1);
+                    h = unpack<T>(pack<T>(w.x, w.y));
+                    b[e] = pack<T>(fmaf(h.x, part2, w.x) * raise2, fmaf(h.y, part2, w.y) * raise2) & mask;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t v[4];
+                    ldmatrix_trans(v, v_mem + (off[c] ^ (j << 5)));
+                    mma_16816<T>(acc[j], v[0], v[1], v[2], v[3], b[0], b[1]);
+                }
             }
+        at += p.group_keys;
+        if (at < range.hi) {  // more of this range
+            __syncwarp();
+            fetch_rows(p, l.k_ring, l.k_pers, range, pair, at, k_mem, lane);
+            fetch_rows(p, l.v_ring, l.v_pers, range, pair, at, v_mem, lane);
         }
-        if (lane == 0) *reinterpret_cast<float2*>(&sh.part[warp][kHeadDim]) = make_float2(m, sum);
-        __syncthreads();
-        if (warp == 0) {
-            const float2 ml = lane < kWarps ? *reinterpret_cast<const float2*>(&sh.part[lane][kHeadDim]) : make_float2(-CUDART_INF_F, 0.f);
-            float top = ml.x;
+    } while (at < range.hi);
+    // merge the warps (the sums of the layer before have been read: this layer's query depends on what came of them)
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-            const float w = exp2f(ml.x - (top > -CUDART_INF_F ? top : 0.f));
-            float all = ml.y * w;
+    for (int j = 0; j < 4; ++j) {
+        const float lower0 = t == 0 ? 1.f : 1.f / (Parts<T>::kNext * Parts<T>::kNext), lower1 = 1.f / Parts<T>::kNext;
+        float2 v = make_float2(fmaf(acc[j][1], lower1, acc[j][0] * lower0), fmaf(acc[j][3], lower1, acc[j][2] * lower0));
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, 1);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
+        if (t == 0) {
+            sh.part[warp][j * 16 + g] = v.x;
+            sh.part[warp][j * 16 + 8 + g] = v.y;
+        }
+    }
+    if (lane == 0) *reinterpret_cast<float2*>(&sh.part[warp][kHeadDim]) = make_float2(m, sum);
+    __syncthreads();
+    if (warp == 0) {
+        const float2 ml = lane < kWarps ? *reinterpret_cast<const float2*>(&sh.part[lane][kHeadDim]) : make_float2(-CUDART_INF_F, 0.f);
+        float top = ml.x;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-            float2 r = make_float2(0.f, 0.f);
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float w = exp2f(ml.x - (top > -CUDART_INF_F ? top : 0.f));
+        float all = ml.y * w;
 #pragma unroll
-            for (int i = 0; i < kWarps; ++i) {
-                const float w_i = __shfl_sync(0xffffffffu, w, i);
-                const float2 v = *reinterpret_cast<const float2*>(&sh.part[i][lane * 2]);
-                r.x = fmaf(v.x, w_i, r.x);
-                r.y = fmaf(v.y, w_i, r.y);
-            }
-            const float inv = all == 0.f ? 0.f : 1.f / all;
-            st_copies(p.o + (range.sequence * p.dim + range.head * kHeadDim) / 2 + lane, p.rows * p.dim / 2, pack<T>(r.x * inv, r.y * inv),
-                      tag);
+        for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+        float2 r = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) {
+            const float w_i = __shfl_sync(0xffffffffu, w, i);
+            const float2 v = *reinterpret_cast<const float2*>(&sh.part[i][lane * 2]);
+            r.x = fmaf(v.x, w_i, r.x);
+            r.y = fmaf(v.y, w_i, r.y);
         }
-        // nobody waits for the rest: the new token's row for the steps behind, and this warp's rows of the next pair
-        if (brings) {
-            const long long to = ((long long)(first + unit * gridDim.x) * p.slots + range.slot_new) * (kHeadDim / 2) + lane;
-            static_cast<uint32_t*>(l.k_ring)[to] = got[1];
-            static_cast<uint32_t*>(l.v_ring)[to] = got[2];
-        }
-        if (unit + 1 < units) {  // (the next layer's first rows: see the kernel)
-            const KeyRange r = sh.range[unit + 1][warp];
-            fetch_rows(p, l.k_ring, l.k_pers, r, first + (unit + 1) * gridDim.x, r.lo, k_mem, lane);
-            fetch_rows(p, l.v_ring, l.v_pers, r, first + (unit + 1) * gridDim.x, r.lo, v_mem, lane);
-        }
+        const float inv = all == 0.f ? 0.f : 1.f / all;
+        st_copies(p.o + (range.sequence * p.dim + range.head * kHeadDim) / 2 + lane, p.rows * p.dim / 2, pack<T>(r.x * inv, r.y * inv),
+                  tag);
+    }
+    // nobody waits for the rest: the new token's row for the steps behind (the next layer's first rows: see the kernel)
+    if (brings) {
+        const long long to = ((long long)pair * p.slots + range.slot_new) * (kHeadDim / 2) + lane;
+        static_cast<uint32_t*>(l.k_ring)[to] = got[1];
+        static_cast<uint32_t*>(l.v_ring)[to] = got[2];
     }
 }
 
@@ -687,7 +677,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __grid_constant__ ResidentParams p) {
     extern __shared__ __align__(128) unsigned char dynamic[];
     __shared__ Shared sh;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, ctas = gridDim.x, pairs = p.rows * p.heads;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, ctas = gridDim.x;
     // Partial sums: one buffer for the products with a norm (whose sums of squares bring a barrier between the last readers and
     // the next writes), one each for the two with the residual (each has the other's barrier in between).  Then the ring rows.
     float *red = reinterpret_cast<float*>(dynamic), *red_out = red + kWarps * kRows * kInStride, *red_fc2 = red_out + kWarps * kRows * kOutStride;
@@ -729,15 +719,14 @@ __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __gr
         }
     }
     // (the pairs from the last CTA on: the first ones have the residual's columns as well)
-    const int first = ctas - 1 - cta, units = first < pairs ? (pairs - first + ctas - 1) / ctas : 0;
-    for (int u = 0; u < units; ++u) {
-        const KeyRange r = key_range(p, sh, first + u * ctas, warp);
-        if (u == 0) {
-            const LayerTable& l = sh.layer[0];
-            fetch_rows(p, l.k_ring, l.k_pers, r, first, r.lo, ptx::smem_u32(mem), lane);
-            fetch_rows(p, l.v_ring, l.v_pers, r, first, r.lo, ptx::smem_u32(mem) + p.group_keys * kRowBytes, lane);
-        }
-        if (lane == 0) sh.range[u][warp] = r;
+    const int pair = ctas - 1 - cta;
+    const bool attends = pair < p.rows * p.heads;
+    if (attends) {
+        const KeyRange r = key_range(p, sh, pair, warp);
+        const LayerTable& l = sh.layer[0];
+        fetch_rows(p, l.k_ring, l.k_pers, r, pair, r.lo, ptx::smem_u32(mem), lane);
+        fetch_rows(p, l.v_ring, l.v_pers, r, pair, r.lo, ptx::smem_u32(mem) + p.group_keys * kRowBytes, lane);
+        if (lane == 0) sh.range[warp] = r;
     }
     __syncwarp();
 
@@ -775,7 +764,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __gr
             norm_product<T>(p, sh, red, in, half, mlp ? p.hidden : 3 * p.dim, mlp ? p.nt_fc1 : p.nt_qkv, mlp, mlp ? p.y : p.x,
                                 mlp ? tag : tag - 1, mlp ? p.f : p.qkv, tag);
         }
-        if (!mlp) attention<T>(p, sh, first, units, mem, l, tag);
+        if (!mlp && attends) attention<T>(p, sh, pair, mem, l, tag);
         if (warp == kWarps - 1 && ptx::elect_one()) {  // this half of the next layer, and a part of the head
             if (l + 1 < p.layers) prefetch(sh.layer[l + 1].half[mlp], mlp);
             if (step >= head_from)
@@ -789,10 +778,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_resident_kernel(const __gr
         }
         // the next layer's keys, then its values, at times when the rows of the next phase are on their way (135 KB keep the load
         // path of an SM busy for 2700 cycles)
-        if (units > 0 && l + 1 < p.layers) {
+        if (attends && l + 1 < p.layers) {
             const LayerTable& next = sh.layer[l + 1];
-            const KeyRange r = sh.range[0][warp];
-            fetch_rows(p, mlp ? next.v_ring : next.k_ring, mlp ? next.v_pers : next.k_pers, r, first, r.lo,
+            const KeyRange r = sh.range[warp];
+            fetch_rows(p, mlp ? next.v_ring : next.k_ring, mlp ? next.v_pers : next.k_pers, r, pair, r.lo,
                        ptx::smem_u32(mem) + (mlp ? p.group_keys * kRowBytes : 0), lane);
         }
     }
@@ -868,8 +857,9 @@ int launch(const ResidentParams& p, int ctas, int smem, cudaStream_t stream) {
 // 1024: not kept.  Windows that the chain splits over the chip (decode_step_splits) stay with it.
 bool decode_step_is_resident(const tmw_stack_desc& d, const tmw_block* blocks) {
     const int sms = sm_count();
+    static_assert(kRows * 8 <= kHeadDim, "a CTA per eight columns of the model is a CTA per pair: 8 heads = d_model / 8");
     if (d.batch < 1 || d.batch > kRows || d.layers < 1 || d.layers > kMaxLayers || d.head_dim != kHeadDim || d.d_model > kMaxDim ||
-        d.d_ff > kMaxHidden || d.d_ff % 32 != 0 || d.d_model / 8 > sms || d.batch * d.heads > kMaxPairs * sms || columns_per_cta(3 * d.d_model) > kInTiles ||
+        d.d_ff > kMaxHidden || d.d_ff % 32 != 0 || d.d_model / 8 > sms || columns_per_cta(3 * d.d_model) > kInTiles ||
         columns_per_cta(d.d_ff) > kInTiles)
         return false;
     tmw_cache_desc c = {};
