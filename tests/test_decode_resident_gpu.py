@@ -116,6 +116,30 @@ def test_positions_outside_the_table(bad):
             assert torch.equal(ring[1].view(torch.int16), old[1].view(torch.int16))
 
 
+@pytest.mark.parametrize("dtype,scale", [(torch.bfloat16, 2.0 ** -40), (torch.float16, 2.0 ** -9), (torch.bfloat16, 0.3), (torch.float16, 3.0),
+                                         (torch.float16, 2.0 ** 13), (torch.bfloat16, 2.0 ** 55)])
+@pytest.mark.parametrize("heads", [1, 10])
+def test_norm_of_the_head(dtype, scale, heads):
+    """Layers that add nothing and a head that is the identity: the logits are the embedded rows, normalised."""
+    D = heads * 64
+    model, g = make(dtype, heads, 8, 0, D, layers=1)
+    with torch.no_grad():
+        for lin in (model.layers[0].attention.out_proj, model.layers[0].mlp.fc2):
+            for prm in lin.parameters():
+                prm.zero_()
+        model.embed_positions.weight.zero_()
+        model.embed_tokens.weight.normal_(0.0, scale, generator=g)
+        model.norm.scale.fill_(1.0)
+        model.lm_head.weight = torch.nn.Parameter(torch.eye(D, dtype=dtype, device=DEV))
+    ids = torch.arange(8, device=DEV) % D
+    got = model.decode_step(ids, torch.zeros(8, dtype=torch.int32, device=DEV), model.new_caches(8, DEV, dtype)).double()
+    x = model.embed_tokens.weight[ids].double()
+    want = x / torch.sqrt(x.square().mean(-1, keepdim=True) + model.config.norm_eps)
+    # one rounding to 16 bits (at most u, or half of fp16's smallest step), in front of it a few of 32 bits
+    u, floor = (2.0 ** -8, 0.0) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -25)
+    assert ((got - want).abs() <= (u + 2.0 ** -20) * want.abs() + floor).all()
+
+
 @pytest.mark.parametrize("B,dtype,vocab,new", [(1, torch.bfloat16, 1003, 30), (8, torch.float16, 4001, 9), (5, torch.bfloat16, 8, 2)])
 def test_generation_equals_steps(B, dtype, vocab, new):
     model, g = make(dtype, 6, 20, 3, vocab, layers=3)
