@@ -1,10 +1,14 @@
-"""The decode step as one resident kernel (up to eight sequences, head_dim 64) against the step module by module: the sizes at
-which its phases change shape, what must stay in its own sequence, generation, and the step under stream capture."""
+"""The decode step as one resident kernel (up to eight sequences, head_dim 64) against the step module by module and against the
+chain of launches that it stands in for: the sizes at which its phases change shape, what must stay in its own sequence,
+generation, the step under stream capture and from two threads.  Which kernels ran is read from the profiler."""
 
+import ctypes
 import math
+import threading
 
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 from titanmac_b200 import TitanMAC, TitanMACConfig, _native, _stack
 
@@ -39,36 +43,88 @@ def relative(a, b):
     return ((a.float() - b.float()).norm() / b.float().norm()).item()
 
 
-@pytest.mark.parametrize("B,dtype,heads,window,n_p,vocab,t,layers,d_ff", [
-    (1, torch.bfloat16, 1, 0, 0, 7, 0, 1, 32),            # the smallest: one key, fewer chunks of k than warps
-    (8, torch.float16, 1, 5, 3, 9, 2, 3, 96),             # ring not full, fewer keys than warps
-    (8, torch.bfloat16, 10, 512, 16, 50000, 600, 2, None),  # the default geometry
-    (7, torch.float16, 8, 186, 5, 1003, 1000, 2, None),   # 16 keys per warp: one tile
-    (3, torch.bfloat16, 5, 187, 5, 1000, 300, 2, 1056),   # 17: one key in the second; a width that is no multiple of 128
-    (2, torch.bfloat16, 10, 751, 16, 512, 800, 2, None),  # 64 keys per warp: four tiles, what it holds at once
-    (8, torch.float16, 10, 752, 16, 512, 2000, 2, None),  # 65: twice
-    (1, torch.bfloat16, 12, 3000, 1, 520, 3100, 2, 3072),  # several times; the widest that it takes
-    (4, torch.bfloat16, 13, 40, 2, 512, 60, 2, None),     # the next width: the chain
-    (8, torch.bfloat16, 2, 40, 2, 512, 60, 2, 3104),      # the next hidden width: the chain
-    (5, torch.bfloat16, 12, 64, 16, 8000, 90, 32, None),  # the most layers
+def is_resident(call):
+    """``call()``, and whether the resident kernel ran in it (else the chain did)."""
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        out = call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    resident, chain = (any(part in n for n in names) for part in ("decode_resident_kernel", "rows_gemm_kernel"))
+    assert resident != chain, names
+    return out, resident
+
+
+@pytest.fixture
+def take_chain(monkeypatch):
+    """Switches the decode calls to the chain of launches: biases that are not aligned to 16 bytes, which the resident kernel
+    does not take."""
+    kept = []
+    arguments = _stack._step_arguments
+
+    def misaligned(table, batch, caches):
+        d, blocks, workspace = arguments(table, batch, caches)
+        for b, layer in zip(blocks, table.layers_of_test):
+            bias = layer.mlp.fc1.bias.detach()
+            kept.append(torch.cat([bias.new_zeros(1), bias]))
+            b.b_fc1 = ctypes.c_void_p(kept[-1].data_ptr() + bias.element_size())
+        return d, blocks, workspace
+
+    def switch(model):
+        _stack.table_of(model).layers_of_test = model.layers
+        monkeypatch.setattr(_stack, "_step_arguments", misaligned)
+
+    yield switch
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("B,dtype,heads,window,n_p,vocab,t,layers,d_ff,resident", [
+    (1, torch.bfloat16, 1, 0, 0, 7, 0, 1, 32, True),            # the smallest: one key, fewer chunks of k than warps
+    (8, torch.float16, 1, 5, 3, 9, 2, 3, 96, True),             # ring not full, fewer keys than warps
+    (8, torch.bfloat16, 10, 512, 16, 50000, 600, 2, None, True),  # the default geometry
+    (7, torch.float16, 8, 186, 5, 1003, 1000, 2, None, True),   # 16 keys per warp: one tile
+    (3, torch.bfloat16, 5, 187, 5, 1000, 300, 2, 1056, True),   # 17: one key in the second; a width that is no multiple of 128
+    (2, torch.bfloat16, 10, 751, 16, 512, 800, 2, None, True),  # 64 keys per warp: four tiles, what it holds at once
+    (8, torch.float16, 10, 752, 16, 512, 2000, 2, None, True),  # 65: twice
+    (1, torch.bfloat16, 2, 4094, 3, 1000, 5000, 2, None, True),  # the longest of few heads: one slot more is split over the chip
+    (1, torch.bfloat16, 12, 3000, 1, 520, 3100, 2, 3072, True),  # several times; the widest that it takes
+    (4, torch.bfloat16, 13, 40, 2, 512, 60, 2, None, False),    # the next width: the chain
+    (8, torch.bfloat16, 2, 40, 2, 512, 60, 2, 3104, False),     # the next hidden width: the chain
+    (9, torch.bfloat16, 2, 40, 2, 512, 60, 2, None, False),     # the next number of sequences: the chain
+    (2, torch.bfloat16, 1, 20, 2, 512, 30, 33, 64, False),      # the next number of layers: the chain
+    (5, torch.bfloat16, 12, 64, 16, 8000, 90, 32, None, True),  # the most layers
 ])
-def test_against_the_modules(B, dtype, heads, window, n_p, vocab, t, layers, d_ff, monkeypatch):
+def test_against_the_modules_and_the_chain(B, dtype, heads, window, n_p, vocab, t, layers, d_ff, resident, monkeypatch, take_chain):
     model, g = make(dtype, heads, window, n_p, vocab, layers, d_ff, positions=t + 4)
     ids = torch.randint(0, vocab, (B,), generator=g, device=DEV)
     pos = torch.randint(max(0, t - 3), t + 1, (B,), generator=g, device=DEV, dtype=torch.int32)
-    got_caches, want_caches = filled(model, B, dtype, g)
-    got = [model.decode_step(ids, pos + i, got_caches) for i in range(2)]  # (the second reads what the first has written)
+    got_caches, chain_caches, want_caches, before = filled(model, B, dtype, g, sets=4)
+
+    def steps(caches):  # (the second reads what the first has written)
+        return [model.decode_step(ids, pos + i, caches) for i in range(2)]
+
+    got, ran = is_resident(lambda: steps(got_caches))
+    assert ran == resident
+    take_chain(model)
+    chain, ran = is_resident(lambda: steps(chain_caches))
+    assert not ran
     _native.poll_status(torch.device(DEV))
     monkeypatch.setattr(_stack, "table_of", lambda m: None)
-    want = [model.decode_step(ids, pos + i, want_caches) for i in range(2)]
+    want = steps(want_caches)
     # rounding to 16 bits through `layers` layers, as between any two kernels of the step
     tol = (2e-2 if dtype == torch.bfloat16 else 4e-3) * max(1.0, (layers / 8) ** 0.5)
-    for a, b in zip(got, want):
-        assert relative(a, b) <= tol, relative(a, b)
-    for a, b in zip(got_caches, want_caches):
-        assert relative(a.k_ring, b.k_ring) <= tol and relative(a.v_ring, b.v_ring) <= tol
-        same = a.k_ring == b.k_ring
-        assert same.all(-1).float().mean() >= 1 - 3 / (window + 1)  # nothing but the new rows was written
+    written = torch.zeros((B, window + 1), dtype=torch.bool, device=DEV)
+    for i in range(2):
+        written[torch.arange(B, device=DEV), (pos.long() + i) % (window + 1)] = True
+    for logits, caches in ((got, got_caches), (chain, chain_caches)):
+        for a, b in zip(logits, want):
+            assert relative(a, b) <= tol, relative(a, b)
+        for a, b, old in zip(caches, want_caches, before):
+            assert torch.equal(a.k_pers, old.k_pers) and torch.equal(a.v_pers, old.v_pers)
+            for ring, other, was in ((a.k_ring, b.k_ring, old.k_ring), (a.v_ring, b.v_ring, old.v_ring)):
+                ring, other, was = (r.transpose(1, 2) for r in (ring, other, was))
+                assert torch.equal(ring[~written], was[~written])  # nothing but the new rows was written
+                assert relative(ring[written], other[written]) <= tol
 
 
 def test_a_sequence_keeps_its_nan_to_itself():
@@ -140,11 +196,15 @@ def test_norm_of_the_head(dtype, scale, heads):
     assert ((got - want).abs() <= (u + 2.0 ** -20) * want.abs() + floor).all()
 
 
+@pytest.mark.parametrize("chain", [False, True])
 @pytest.mark.parametrize("B,dtype,vocab,new", [(1, torch.bfloat16, 1003, 30), (8, torch.float16, 4001, 9), (5, torch.bfloat16, 8, 2)])
-def test_generation_equals_steps(B, dtype, vocab, new):
+def test_generation_equals_steps(B, dtype, vocab, new, chain, take_chain):
     model, g = make(dtype, 6, 20, 3, vocab, layers=3)
     ids = torch.randint(0, vocab, (B, 11), generator=g, device=DEV)
-    got = model.generate(ids, new)
+    if chain:
+        take_chain(model)
+    got, resident = is_resident(lambda: model.generate(ids, new))
+    assert resident != chain
     logits, caches = model.prefill(ids)
     pos = torch.full((B,), 11, dtype=torch.int32, device=DEV)
     for i in range(new):
@@ -152,6 +212,36 @@ def test_generation_equals_steps(B, dtype, vocab, new):
         assert torch.equal(got[:, 11 + i], token), i
         logits = model.decode_step(token, pos, caches)
         pos += 1
+
+
+def test_steps_from_two_threads():
+    """Each thread on a stream of its own, with its own caches: what the steps give one after the other."""
+    model, g = make(torch.bfloat16, 10, 100, 3, 3000, layers=4)
+    ids = torch.randint(0, 3000, (2, 4), generator=g, device=DEV)
+    pos = torch.full((4,), 150, dtype=torch.int32, device=DEV)
+    alone, together = filled(model, 4, torch.bfloat16, g), [model.new_caches(4, DEV, torch.bfloat16) for _ in range(2)]
+    for a, b in zip(alone, together):
+        for x, y in zip(a, b):
+            for name in ("k_ring", "v_ring", "k_pers", "v_pers"):
+                getattr(y, name).copy_(getattr(x, name))
+    positions = [pos + i for i in range(40)]
+    want = [[model.decode_step(ids[k], p, alone[k]) for p in positions] for k in range(2)]
+    torch.cuda.synchronize()
+    got, streams = [None, None], [torch.cuda.Stream(DEV) for _ in range(2)]
+
+    def work(k):
+        with torch.cuda.stream(streams[k]):
+            got[k] = [model.decode_step(ids[k], p, together[k]) for p in positions]
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    torch.cuda.synchronize()
+    _native.poll_status(torch.device(DEV))
+    for k in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(got[k], want[k]))
 
 
 def test_step_under_capture():

@@ -58,7 +58,8 @@ def test_step_equals_module_by_module(B, dtype, heads, dh, window, Np, vocab, t,
 
 
 @pytest.mark.parametrize("B,dtype,heads,dh,window,n_p,t", [
-    (1, torch.bfloat16, 2, 64, 4094, 3, 200),     # one slot below the rule: clusters
+    (1, torch.bfloat16, 2, 64, 4094, 3, 200),     # one slot below the rule: the resident kernel
+    (3, torch.bfloat16, 2, 128, 2046, 3, 2100),   # one slot below the rule: clusters
     (1, torch.bfloat16, 2, 64, 4095, 3, 0),       # the first token, nothing in the ring
     (3, torch.float16, 4, 64, 4100, 0, 4000),     # ring not full, no persistent rows
     (2, torch.bfloat16, 3, 128, 2047, 16, 9001),  # full
