@@ -447,8 +447,10 @@ TMW_API int tmw_cross_entropy(int32_t dtype, int32_t batch, int32_t tokens, int3
  * helper gets from a full re-forward per token (examples/train_math.py:146-161).  head_dim 64 or 128, d_model at most
  * 4096, d_ff a multiple of 32, batch at most 65535.  `workspace`: device memory of tmw_decode_step_workspace() bytes, used
  * until the call's kernels have finished; an id or position outside its table embeds as NaN and is reported by
- * tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).  Up to eight sequences with head_dim 64 and d_model at most 768 the step is one
- * cooperative kernel with a CTA on every SM: it starts when all of them have room.
+ * tmw_poll_status (TMW_ERR_INVALID_ARGUMENT).  With head_dim 64, up to eight sequences, 32 layers, d_model at most 768, d_ff at
+ * most 3072, biases aligned to 16 bytes, and a window below 4095 or more than a third as many (sequence, head) pairs as SMs, the
+ * step is one cooperative kernel with a CTA on every SM: it starts when all of them have room, so steps of two streams run one
+ * after the other.  Everything else is a chain of launches.
  */
 TMW_API size_t tmw_decode_step_workspace(const tmw_stack_desc* desc);
 TMW_API int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* blocks, const int64_t* token_ids, const int32_t* pos,

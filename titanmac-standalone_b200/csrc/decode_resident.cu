@@ -20,14 +20,15 @@
 // What bounds it: instructions.  A layer is about 17 000 cycles for five exchanges of 500 to 900 (store to load, within a die
 // and across); the rest is what the warps issue between a poll that succeeds and the words that they send, about 10 cycles per
 // instruction and warp, a third of them waiting for the slowest warp at a barrier.  So the code of a phase stands once, in a
-// loop over the half layers (separate code for each of the four products: 220 us instead of 207 for the model below), sums of
-// squares and scores are mma, and nothing is computed twice.  Twelve warps, three per scheduler, without register spills: 165 us
-// for 16 layers with a vocabulary of 8000, sixteen 184, ten 183, eight 177.  CUDA-core scores and weighted sums took 5000 cycles
-// per layer, these 3200, the most of it shared memory (135 KB per pair).  No gain: a phase's weights loaded a phase ahead, pauses
-// between polls, a poll of one word in front of the full one (164 us against 152), a barrier behind every send.
+// loop over the half layers, sums of squares and scores are mma, and nothing is computed twice.  Twelve warps, three per
+// scheduler, without register spills: 159 us for 16 layers with a vocabulary of 8000 and one sequence, 211 with eight; sixteen
+// warps (which spill) 171 and 220, ten 183 and 235, eight 175 and 228.  Tried in an earlier form with sixteen warps: scores and
+// weighted sums on CUDA cores took 5000 cycles per layer, as mma 3200, the most of it shared memory (135 KB per pair); code of
+// its own for each of the four products, a phase's weights loaded a phase ahead, pauses between polls, a poll of one word in
+// front of the full one and a barrier behind every send gained nothing or lost.
 //
-// 16 layers of width 640, vocabulary 50 000, window 512, one sequence: 313 us as a chain of launches, 170 as one kernel; eight
-// prompts of 300 continued by 48 tokens: 17.2 and 10.9 ms.
+// 16 layers of width 640, vocabulary 50 000, window 512, one sequence: 313 us as a chain of launches, 172 as one kernel; eight
+// prompts of 300 continued by 48 tokens: 17.3 and 10.9 ms.
 #include <math_constants.h>
 
 #include "tc_ptx.cuh"
@@ -41,7 +42,7 @@ constexpr int kHeadDim = 64, kRowBytes = kHeadDim * 2;
 constexpr int kMaxLayers = 32;                       // the table travels as a kernel parameter (4 KB)
 constexpr int kMaxDim = 768, kMaxHidden = 3072;
 constexpr int kInChunks = (kMaxDim / 32 + kWarps - 1) / kWarps;  // chunks of 32 elements of k that a warp has, at most
-constexpr int kMaxGroup = (768 / kWarps + 15) / 16 * 16;                        // keys that a warp has on chip: three tiles of 16
+constexpr int kMaxGroup = (768 / kWarps + 15) / 16 * 16;                        // keys that a warp has on chip: four tiles of 16
 constexpr int kSmemLimit = 227 * 1024;
 
 struct HalfLayer {  // norm -> product -> (attention | GELU) -> product + residual
@@ -84,7 +85,8 @@ __device__ __forceinline__ void ld_words(const uint64_t* p, uint64_t& a, uint64_
     asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 }
 // Rows that all CTAs wait for are sent to kCopies places, `copy` words apart, and a CTA polls one of them, so that fewer poll the
-// same lines of L2 (16 layers, vocabulary 8000, one | eight sequences: one copy 158 | 205 us, four 152 | 211, eight 156 | 218).
+// same lines of L2 (16 layers, one | eight sequences, us: with a vocabulary of 8000 one copy 163 | 211, two 159 | 211, four
+// 160 | 212; with 50 000 172 | 222, 175 | 222, 176 | 223).
 constexpr int kCopies = 2;
 __device__ __forceinline__ void st_word(uint64_t* p, uint32_t bits, uint32_t tag) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(((uint64_t)tag << 32) | bits) : "memory");
@@ -583,7 +585,7 @@ __device__ __forceinline__ long long chosen(const unsigned long long* best, int 
 
 // logits = norm(x) head^T: the rows, normalised, in shared memory for all warps; a warp takes tiles of eight vocabulary rows
 // with the whole of k, kHeadDepth loads of 16 bytes per lane in flight
-// half layers in front of the head under which its weights go into L2 (under all of them: 170 us instead of 167)
+// half layers in front of the head under which its weights go into L2 (under all of them: 178 us instead of 175)
 constexpr int kHeadSteps = 8;
 constexpr int kHeadDepth = 20;
 
@@ -843,11 +845,11 @@ int launch(const ResidentParams& p, int ctas, int smem, cudaStream_t stream) {
 
 // The line is where the registers and the used half of the mma's rows end: eight sequences, three tiles of eight columns per
 // CTA, chunks of k as declared above.  us per step as one kernel / as a chain (8 layers, vocabulary 8000, 16 persistent rows):
-//   width 640, window 64: 1 sequence 78 / 155, 4: 84 / 156, 8: 93 / 160       512: 1: 82 / 155, 4: 90 / 175, 8: 110 / 183
-//              window 1024: 1: 106 / 169, 4: 127 / 203, 8: 144 / 208           3000: 1: 171 / 211, 4: 190 / 297, 8: 221 / 304
-//   width 512, window 512: 1: 77 / 149, 8: 94 / 170                            width 768: 8: 122 / 205
-// With the mma's other eight rows in use (sixteen warps): 9 sequences 162 / 187 and 16 208 / 190 at window 512, 274 / 216 at
-// 1024: not kept.  Windows that the chain splits over the chip (decode_step_splits) stay with it.
+//   width 640, window 64: 1 sequence 79 / 162, 4: 84 / 162, 8: 95 / 163       512: 1: 84 / 170, 4: 92 / 178, 8: 113 / 186
+//              window 1024: 1: 108 / 171, 4: 130 / 205, 8: 147 / 211           3000: 1: 172 / 214, 4: 194 / 299, 8: 225 / 307
+//   width 512, window 512: 1: 79 / 161, 8: 93 / 173                            width 768: 8: 124 / 207
+// With the mma's other eight rows in use (tried with sixteen warps only): 9 sequences 162 / 187 and 16 208 / 190 at window 512,
+// 274 / 216 at 1024: not kept.  Windows that the chain splits over the chip (decode_step_splits) stay with it.
 bool decode_step_is_resident(const tmw_stack_desc& d, const tmw_block* blocks) {
     const int sms = sm_count();
     static_assert(kRows * 8 <= kHeadDim, "a CTA per eight columns of the model is a CTA per pair: 8 heads = d_model / 8");
