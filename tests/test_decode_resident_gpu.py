@@ -261,12 +261,10 @@ def test_step_under_capture():
         static += 1
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("window,exponent", [(300, -12.6), (300, -18.6), (300, -23.4), (1500, -23.4), (300, -31.3)])
-def test_small_weights_with_large_values(dtype, window, exponent):
-    """Every eighth key has score 0 and value 0, the others weigh 2^exponent and carry large values: the output is nothing but
-    small weights, each of which counts with the precision of fp32 (a 16-bit part of its own has none left of them in fp16)."""
-    D, g = 64, torch.Generator(device=DEV).manual_seed(1)
+def one_head(dtype, window, query):
+    """A model of one layer and one head whose query is ``query`` e_0, whose new key and value are zeros and whose logits are the
+    normalised row 64 e_0 + attention; and its cache of zeros."""
+    D = 64
     cfg = TitanMACConfig(vocab_size=D, d_model=D, n_heads=1, n_layers=1, d_ff=4 * D, max_seq_len=2 * window, window_size=window,
                          n_persistent=0, use_block_sparse=False)
     with torch.device(DEV):
@@ -274,31 +272,61 @@ def test_small_weights_with_large_values(dtype, window, exponent):
     with torch.no_grad():
         for name, prm in model.named_parameters():
             prm.fill_(1.0 if name.endswith("scale") else 0.0)
-        # x = 64 e_0, so its norm is 8 e_0; the query is that, the new key and value are zeros; the head gives the row itself
-        model.embed_tokens.weight[:, 0] = 64.0
+        model.embed_tokens.weight[:, 0] = 64.0  # whose norm is 8 e_0
         attn = model.layers[0].attention
-        attn.qkv_proj.weight[0, 0] = 1.0
+        attn.qkv_proj.weight[0, 0] = query / 8
         attn.out_proj.weight.copy_(torch.eye(D))
         model.lm_head.weight = torch.nn.Parameter(torch.eye(D, dtype=dtype, device=DEV))
     caches = model.new_caches(1, DEV, dtype)
+    caches[0].k_ring.zero_()
+    caches[0].v_ring.zero_()
+    return model, caches
+
+
+def check_row(model, caches, t, row):
+    """The step's logits against those of the attention's output ``row`` (64 bits, first element zero)."""
+    row = row + 64.0 * torch.nn.functional.one_hot(torch.tensor(0, device=DEV), 64)
+    want = row / torch.sqrt(row.square().mean() + model.config.norm_eps)
+    got = model.decode_step(torch.tensor([3], device=DEV), torch.tensor([t], dtype=torch.int32, device=DEV), caches)[0].double()
+    # Roundings to 16 bits, u each, of the attention's output, the normalised row and the logit (the query and all sums with one
+    # nonzero term are exact), and one u for the rest; in fp16 each of them may lie below 2^-14, where the spacing is 2^-24
+    fp16 = caches[0].dtype == torch.float16
+    u = 2.0 ** (-11 if fp16 else -8)
+    floor = 2.0 ** -25 * (want[1:].abs() / row[1:].abs() + 2) if fp16 else 0.0
+    assert ((got[1:] - want[1:]).abs() <= 4 * u * want[1:].abs() + floor).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("window,exponent", [(300, -12.6), (300, -18.6), (300, -23.4), (1500, -23.4), (300, -31.3)])
+def test_small_weights_with_large_values(dtype, window, exponent):
+    """Every eighth key has score 0 and value 0, the others weigh 2^exponent and carry large values: the output is nothing but
+    small weights, each of which counts with the precision of fp32 (a 16-bit part of its own has none left of them in fp16)."""
+    model, caches = one_head(dtype, window, 8.0)
     k, v = caches[0].k_ring, caches[0].v_ring
     small = torch.arange(window + 1, device=DEV) % 8 != 0
-    score = torch.full((window + 1,), exponent * math.log(2.0), device=DEV)  # q k / sqrt(64) = k[0]
-    k.zero_()
-    k[0, 0, :, 0] = torch.where(small, score, torch.zeros_like(score)).to(dtype)
+    k[0, 0, :, 0] = small * exponent * math.log(2.0)  # q k / sqrt(64) = k[0]
     top = 6e4 if dtype == torch.float16 else 2.0 ** 40  # (bf16: so that the smallest weights matter there too)
-    v.uniform_(0.25, 1.0, generator=g).mul_(top).mul_(small[:, None])
+    v.uniform_(0.25, 1.0, generator=torch.Generator(device=DEV).manual_seed(1)).mul_(top).mul_(small[:, None])
     v[..., 0] = 0.0
     t = 2 * window - 3
-    weight = torch.exp(k[0, 0, :, 0].double())
-    values = v[0, 0].double()
+    weight, values = torch.exp(k[0, 0, :, 0].double()), v[0, 0].double()
     weight[t % (window + 1)], values[t % (window + 1)] = 1.0, 0.0  # the new token
-    row = (weight @ values) / weight.sum()
-    row[0] += 64.0
-    want = row / torch.sqrt(row.square().mean() + cfg.norm_eps)
-    got = model.decode_step(torch.tensor([3], device=DEV), torch.tensor([t], dtype=torch.int32, device=DEV), caches)[0].double()
-    # Roundings to 16 bits, u each, of the attention's output, the normalised row and the logit (the query, 8, and all sums
-    # with one nonzero term are exact), and one u for the rest; in fp16 each of them may lie below 2^-14, where the spacing is 2^-24
-    u = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
-    floor = 2.0 ** -25 * (want[1:].abs() / row[1:].abs() + 2) if dtype == torch.float16 else 0.0
-    assert ((got[1:] - want[1:]).abs() <= 4 * u * want[1:].abs() + floor).all()
+    check_row(model, caches, t, (weight @ values) / weight.sum())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("window,query,key", [(300, 512.0, 32768.0), (300, 2048.0, 41000.0), (1500, 8192.0, 50000.0), (300, 32768.0, 32768.0),
+                                              (300, 32768.0, 60000.0)])
+def test_large_scores(dtype, window, query, key):
+    """Scores up to 2^28, where fp32 has steps of 32: the keys that share the largest one count alike and alone, whichever warp
+    has them."""
+    model, caches = one_head(dtype, window, query)
+    k, v = caches[0].k_ring, caches[0].v_ring
+    g = torch.Generator(device=DEV).manual_seed(2)
+    first = torch.rand(window + 1, generator=g, device=DEV) < 0.1
+    k[0, 0, :, 0] = torch.where(first, key, key / 2)
+    v.uniform_(0.25, 1.0, generator=g)
+    v[..., 0] = 0.0
+    t = 2 * window - 3
+    first[t % (window + 1)] = False  # (the new token, whose score is 0)
+    check_row(model, caches, t, v[0, 0].double()[first].mean(0))
