@@ -66,6 +66,28 @@ def test_fp16_and_strided_input():
     assert (y.float() - reference(x, w, None, False)).abs().max().item() <= 2e-2
 
 
+@pytest.mark.parametrize("m,n", [(300, 648), (8320, 664), (97, 40)])
+@pytest.mark.parametrize("shift", [0, 8])
+def test_output_rows_off_the_32_byte_boundary(m, n, shift):
+    """Rows of 16 n + 8 values, or an output 16 bytes into its allocation, go out in halves of sectors; what surrounds them
+    stays untouched.  Tolerance: one rounding of values below 8 to bf16, and the order of 128 fp32 sums."""
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    x = torch.randn(m, 128, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(n, 128, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    room = torch.full((m * n + 32,), 7.0, device=DEV, dtype=torch.bfloat16)
+    out = room[shift:shift + m * n].view(m, n)
+    _native.linear(x, w, out=out)
+    assert (out.float() - reference(x, w, None, False)).abs().max().item() <= 2 ** -6 + 1e-3
+    assert (room[:shift] == 7).all() and (room[shift + m * n:] == 7).all()
+
+
+def test_output_off_the_16_byte_boundary_is_refused():
+    x, w = torch.zeros(300, 64, device=DEV, dtype=torch.bfloat16), torch.zeros(64, 64, device=DEV, dtype=torch.bfloat16)
+    room = torch.zeros(300 * 64 + 8, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(_native.TmwError):
+        _native.linear(x, w, out=room[4:4 + 300 * 64].view(300, 64))
+
+
 def test_rejects_what_it_cannot_do():
     x = torch.zeros(4, 12, device=DEV, dtype=torch.bfloat16)
     w = torch.zeros(8, 12, device=DEV, dtype=torch.bfloat16)

@@ -7,8 +7,8 @@
 // stay in L2 while the panels of B change).  Warp roles:
 //   warp 0      TMA producer: A and B tiles of 64 K-elements into a ring of shared-memory stages
 //   warp 1      issues the tcgen05.mma of every stage (one elected thread); allocates / frees tensor memory
-//   warps 2-9   epilogue: tensor memory -> registers -> bias, GELU, ... -> 16-bit -> the warp's own staging -> TMA store;
-//               warp w reads the 32 lanes of its number modulo 4 and takes every second panel of 32 columns
+//   warps 2-9   epilogue: tensor memory -> registers -> bias, GELU, ... -> 16-bit -> global memory, a row per lane in whole
+//               32-byte sectors; warp w reads the 32 lanes of its number modulo 4 and takes every second panel of 32 columns
 // The accumulator is double-buffered in tensor memory (2 x BN columns): the epilogue of a tile runs under the
 // matrix products of the next one.  gemm_tc_pair_kernel, below, does the same on CTA pairs.  Every mbarrier wait is bounded
 // and reports TMW_ERR_DEVICE_TIMEOUT through the device status word.
@@ -29,13 +29,12 @@ using namespace ptx;
 
 constexpr int GM = 128;        // rows of an output tile
 constexpr int GK = 64;         // K elements per stage: one 128-byte swizzle row
-constexpr int kPanel = 32;     // columns per staging panel of the output (64 bytes, 64-byte swizzle)
-constexpr int kSlot = 32 * 64; // a warp's 32 rows of a panel
+constexpr int kPanel = 32;     // columns that an epilogue warp finishes at a time
 constexpr int kEpiWarps = 8;
 constexpr int kGemmThreads = 32 * (2 + kEpiWarps);
 // The pair kernel's tiles are ready every 4 to 5 us at K = 640; with GELU the epilogue of one is 128 x 256 x 24 instructions a
 // CTA.  16416 x 2560 x 640 with GELU, us: 75 with eight warps behind block-wide barriers, 72 with sixteen, 58 with sixteen that
-// store their panels themselves and do not wait for one another (QKV, N = 1920, no epilogue: 42 -> 38).
+// do not wait for one another (QKV, N = 1920, no epilogue: 42 -> 38).
 constexpr int kPairEpiWarps = 16;
 constexpr int kPairThreads = 32 * (2 + kPairEpiWarps);
 
@@ -47,10 +46,9 @@ struct GemmSmem {
     static constexpr int kStageA = kSlices * GM * GK * 2;
     static constexpr int kStageB = kSlices * BN * GK * 2;
     static constexpr int kStage = kStageA + kStageB;
-    static constexpr int kOut = kEpiWarps * 2 * kSlot;
-    static constexpr int kStages = (232448 - 2048 - kOut) / kStage;
-    static constexpr int kBars = kStages * kStage + kOut;  // offset of the barrier area
-    static constexpr int kTotal = kBars + 1024 + 1024;     // barriers, alignment slack
+    static constexpr int kStages = (232448 - 2048) / kStage;
+    static constexpr int kBars = kStages * kStage;      // offset of the barrier area
+    static constexpr int kTotal = kBars + 1024 + 1024;  // barriers, alignment slack
     static_assert(kStages >= 3, "pipeline depth");
 };
 
@@ -62,7 +60,9 @@ struct GemmParams {
     float* partial;      // k cut into `splits` ranges: their fp32 sums go to [splits][m][n] here instead of to the output
     int splits;
     int width;           // pair kernel: columns of a tile (a multiple of 32)
-    int drain;           // a dependent launch follows: the stores have to be complete when the kernel ends
+    void* c;             // the output, rows of ldc elements
+    long long ldc;
+    int wide;            // rows of c and aux start on 32-byte boundaries
     int* status;
 };
 
@@ -82,29 +82,50 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// What the epilogue of a panel (a warp's 32 rows x 32 columns) reads beside the accumulator (GEMM_ADD, GEMM_GELU_GRAD):
-// columns 8 (lane & 3) .. + 8 of rows 8 i + lane / 4, whole sectors per warp.  Asked for before the accumulator is waited for.
-struct PanelAux { uint4 v[4]; };
-
-__device__ __forceinline__ void load_aux(PanelAux& in, const GemmParams& p, int row0, int col, int lane) {
-    if (p.epilogue != GEMM_ADD && p.epilogue != GEMM_GELU_GRAD) return;
-    const int c = col + (lane & 3) * 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = row0 + i * 8 + (lane >> 2);
-        in.v[i] = r < p.m && c < p.n ? *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.aux) + (long long)r * p.n + c)
-                                     : make_uint4(0, 0, 0, 0);
+// 16 values of a row, of which the first `left` columns exist (a multiple of 8), to and from global memory: one whole sector
+// where the row is aligned to it.  Half a sector per instruction costs L2 a second pass over it.
+__device__ __forceinline__ void store16(void* row, int col, int left, bool wide, const uint4& a, const uint4& b) {
+    uint16_t* dst = static_cast<uint16_t*>(row) + col;
+    if (wide && left >= 16) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                     : "memory");
+        return;
     }
+    if (left > 0) *reinterpret_cast<uint4*>(dst) = a;
+    if (left > 8) *reinterpret_cast<uint4*>(dst + 8) = b;
+}
+__device__ __forceinline__ void load16(const void* row, int col, int left, bool wide, uint4& a, uint4& b) {
+    const uint16_t* src = static_cast<const uint16_t*>(row) + col;
+    if (wide && left >= 16) {
+        asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                     : "l"(src)
+                     : "memory");
+        return;
+    }
+    a = left > 0 ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
+    b = left > 8 ? *reinterpret_cast<const uint4*>(src + 8) : make_uint4(0, 0, 0, 0);
 }
 
-// 32 accumulator columns of one row per lane -> bias, epilogue, the warp's 32 rows of the staging panel (64-byte swizzle).
-// `aux` passes through the same rows of the panel, so that global memory sees whole 64-byte runs: one row per lane there
-// made the epilogue longer than the product (8320 x 2560 x 640, us: GELU_KEEP 62.6, GELU_GRAD 73, no epilogue 28.5).
+// What the epilogue of a panel reads beside the accumulator (GEMM_ADD, GEMM_GELU_GRAD): a lane's row of its 32 columns.
+// Asked for before the accumulator is waited for.
+struct PanelAux { uint4 v[4]; };
+
+__device__ __forceinline__ void load_aux(PanelAux& in, const GemmParams& p, int row, int col) {
+    if ((p.epilogue != GEMM_ADD && p.epilogue != GEMM_GELU_GRAD) || row >= p.m) return;
+    const uint16_t* src = static_cast<const uint16_t*>(p.aux) + (long long)row * p.n;
+    load16(src, col, p.n - col, p.wide, in.v[0], in.v[1]);
+    load16(src, col + 16, p.n - col - 16, p.wide, in.v[2], in.v[3]);
+}
+
+// 32 accumulator columns of one row per lane -> bias, epilogue -> the output.  A row per lane and 32 bytes per access: every
+// sector is written once and whole, without a detour through shared memory, which leaves that to two more stages of operands.
+// Against panels of 32 x 32 staged for TMA stores, us, K = 640: 16416 x 50000 863 -> 800, 16416 x 2560 46.6 -> 43.5, 32896 x 1920
+// 66.4 -> 64.8, 32896 x 640 30.5 -> 28.5; 8320 x 640 x 2560 28.0 -> 25.0; 8192^3 718 -> 715.
 template <bool BF16>
-__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, const PanelAux& in, uint8_t* stage, int row0,
-                                             int col, int lane) {
+__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, const PanelAux& in, int row, int col) {
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
-    auto slot = [&](int r, int c) { return reinterpret_cast<uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) * 16)); };
     if (p.bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 32; j += 8)
@@ -115,37 +136,29 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
                 for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
             }
     }
+    if (row >= p.m) return;
     if (p.epilogue == GEMM_GELU) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
     } else if (p.epilogue == GEMM_GELU_KEEP) {
+        uint16_t* keep = static_cast<uint16_t*>(p.aux) + (long long)row * p.n;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const uint4 raw = pack8<BF16>(v + 8 * c);
-            *slot(lane, c) = raw;
-            float x[8];
-            load8<T>(reinterpret_cast<const T*>(&raw), x);
+        for (int j = 0; j < 32; j += 16) {
+            const uint4 raw[2] = {pack8<BF16>(v + j), pack8<BF16>(v + j + 8)};
+            store16(keep, col + j, p.n - col - j, p.wide, raw[0], raw[1]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[8 * c + e] = gelu_erf(x[e]);
+            for (int h = 0; h < 2; ++h) {
+                float x[8];
+                load8<T>(reinterpret_cast<const T*>(&raw[h]), x);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[j + 8 * h + e] = gelu_erf(x[e]);
+            }
         }
-        __syncwarp();
-        const int c = lane & 3;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = i * 8 + (lane >> 2);
-            if (row0 + r < p.m && col + c * 8 < p.n)
-                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.aux) + (long long)(row0 + r) * p.n + col + c * 8) = *slot(r, c);
-        }
-        __syncwarp();
     } else if (p.epilogue != GEMM_NONE) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *slot(i * 8 + (lane >> 2), lane & 3) = in.v[i];
-        __syncwarp();
-#pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const uint4 raw = *slot(lane, c);
             float x[8];
-            load8<T>(reinterpret_cast<const T*>(&raw), x);
+            load8<T>(reinterpret_cast<const T*>(&in.v[c]), x);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 float& y = v[8 * c + e];
@@ -153,31 +166,34 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
             }
         }
     }
+    uint16_t* out = static_cast<uint16_t*>(p.c) + (long long)row * p.ldc;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) *slot(lane, c) = pack8<BF16>(v + 8 * c);
+    for (int j = 0; j < 32; j += 16) store16(out, col + j, p.n - col - j, p.wide, pack8<BF16>(v + j), pack8<BF16>(v + j + 8));
 }
 
-// the fp32 sums of a k range
-__device__ __forceinline__ void store_partial(const float (&v)[32], const GemmParams& p, int split, int row, int col) {
+// the fp32 sums of a k range, whole sectors too (n is a multiple of 8, `partial` aligned)
+__device__ __forceinline__ void store_partial(const uint32_t (&v)[32], const GemmParams& p, int split, int row, int col) {
     if (row >= p.m) return;
     float* dst = p.partial + ((long long)split * p.m + row) * p.n + col;
 #pragma unroll
-    for (int j = 0; j < 32; j += 4)
-        if (col + j < p.n) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    for (int j = 0; j < 32; j += 8)
+        if (col + j < p.n)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                         ::"l"(dst + j), "r"(v[j]), "r"(v[j + 1]), "r"(v[j + 2]), "r"(v[j + 3]), "r"(v[j + 4]), "r"(v[j + 5]),
+                           "r"(v[j + 6]), "r"(v[j + 7])
+                         : "memory");
 }
 
-// A warp's panels (first, first + step, ...) of a finished tile: tensor memory -> the warp's own staging -> TMA store (or, with
-// k cut, fp32 sums to memory).  No warp waits for another: a panel goes out as soon as it is finished, from one of two
-// staging slots of the warp, and a slot is taken again when its last store has read it.  `in` holds the inputs of the first
-// panel; `all_read` is called once the accumulator has been read; `count`: panels that the warp has stored.
+// A warp's panels (first, first + step, ...) of a finished tile: tensor memory -> global memory.  No warp waits for another.
+// `in` holds the inputs of the first panel; `all_read` is called once the accumulator has been read.
 template <bool BF16, typename F>
-__device__ __forceinline__ void epilogue_panels(const GemmParams& p, const CUtensorMap* map_c, PanelAux& in, uint32_t t_addr,
-                                                uint8_t* slots, int& count, int row0, int col0, int first, int panels, int step,
-                                                int split, int lane, F all_read) {
+__device__ __forceinline__ void epilogue_panels(const GemmParams& p, PanelAux& in, uint32_t t_addr, int row, int col0, int first,
+                                                int panels, int step, int split, F all_read) {
     if (first >= panels) all_read();
     for (int pn = first; pn < panels; pn += step) {
         const int col = col0 + pn * kPanel;
         uint32_t acc[32];
+        __syncwarp();
         tmem_ld32(t_addr + pn * kPanel, acc);
         tc_wait_ld();
         if (pn + step >= panels) {
@@ -185,24 +201,15 @@ __device__ __forceinline__ void epilogue_panels(const GemmParams& p, const CUten
             __syncwarp();
             all_read();
         }
+        if (p.partial != nullptr) {
+            store_partial(acc, p, split, row, col);
+            continue;
+        }
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-        if (p.partial != nullptr) {
-            store_partial(v, p, split, row0 + lane, col);
-            continue;
-        }
-        uint8_t* stage = slots + (count++ & 1) * kSlot;
-        if (lane == 0) tma_store_wait_read_but_one();
-        __syncwarp();
-        finish_panel<BF16>(v, p, in, stage, row0, col, lane);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-            if (row0 < p.m && col < p.n) tma_store_2d(map_c, smem_u32(stage), col, row0);
-            tma_store_commit();
-        }
-        if (pn + step < panels) load_aux(in, p, row0, col + step * kPanel, lane);
+        finish_panel<BF16>(v, p, in, row, col);
+        if (pn + step < panels) load_aux(in, p, row, col + step * kPanel);
     }
 }
 
@@ -218,8 +225,7 @@ constexpr uint64_t kStepDesc = MN ? 128 : 2;  // 16 k-elements on, in units of 1
 
 template <int BN, bool BF16, bool AMN, bool BMN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-               const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
     using L = GemmSmem<BN>;
     constexpr int S = L::kStages;
     constexpr uint32_t kTmemCols = 512;  // two accumulators of BN <= 256 columns
@@ -244,7 +250,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
         for (int s = 0; s < S; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
@@ -335,22 +340,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int g = warp & 3;             // lane group of tensor memory this warp may read
         const int sub = (warp - 2) >> 2;    // its first panel
         constexpr int kPanels = BN / kPanel;
-        uint8_t* slots = smem + S * L::kStage + (warp - 2) * 2 * kSlot;
-        int t = 0, count = 0;
+        int t = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
             const int buf = t & 1;
-            const int mn = tile / p.splits, row0 = (mn / n_tiles) * GM, col0 = (mn % n_tiles) * BN;
+            const int mn = tile / p.splits, row = (mn / n_tiles) * GM + g * 32 + lane, col0 = (mn % n_tiles) * BN;
             PanelAux in;
-            if (sub < kPanels) load_aux(in, p, row0 + g * 32, col0 + sub * kPanel, lane);
+            if (sub < kPanels) load_aux(in, p, row, col0 + sub * kPanel);
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            epilogue_panels<BF16>(p, &map_c, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, slots, count, row0 + g * 32, col0,
-                                  sub, kPanels, kEpiWarps / 4, tile % p.splits, lane,
-                                  [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
-        }
-        if (lane == 0) {
-            if (p.drain) tma_store_wait_all();
-            else tma_store_wait_read();  // (the stores themselves complete with the grid)
+            epilogue_panels<BF16>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, row, col0, sub, kPanels, kEpiWarps / 4,
+                                  tile % p.splits, [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
         }
     }
 
@@ -380,25 +379,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // as of A (a vocabulary's W is read m / 256 times otherwise, and does not stay in the near half of L2).
 constexpr int kGroup = 8, kGroupFrom = 16;
 
-template <int BN>
+// Shared memory of the pair kernel is a ring of as many stages as fit at the tile's width (256 columns: 7, 160: 8).  The bytes
+// in flight are what the rate hangs on: 16416 x 50000 x 640 takes 976 | 875 | 847 | 823 us with 3 | 4 | 5 | 6 stages.
 struct PairSmem {
     static constexpr int kStageA = GM * GK * 2;
-    static constexpr int kStageB = (BN / 2) * GK * 2;
-    static constexpr int kStage = kStageA + kStageB;
-    static constexpr int kOut = kPairEpiWarps * 2 * kSlot;
-    static constexpr int kStages = (232448 - 2048 - kOut) / kStage;
-    static constexpr int kBars = kStages * kStage + kOut;
-    static constexpr int kTotal = kBars + 1024 + 1024;
-    static_assert(kStages >= 3, "pipeline depth");
-    static_assert(kStage % 1024 == 0 && kStageA % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
+    static constexpr int kMost = 10;  // stages (barriers)
+    static constexpr int kBars = 232448 - 1024 - 1024;
+    static constexpr int kTotal = kBars + 1024 + 1024;  // barriers, alignment slack
 };
 
 template <int BN, bool BF16, bool AMN, bool BMN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                    const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
-    using L = PairSmem<BN>;
-    constexpr int S = L::kStages;
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
+    using L = PairSmem;
+    constexpr int M = L::kMost;
     constexpr uint32_t kTmemCols = 512;
     extern __shared__ uint8_t smem_raw[];
     // the same offsets in both CTAs of the pair (the dynamic shared memory of a kernel starts at the same
@@ -408,11 +402,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint8_t* bar_area = smem + L::kBars;
     const uint32_t bar_base = smem_base + L::kBars;
     auto full = [&](int s) -> uint32_t { return bar_base + 8 * s; };
-    auto empty = [&](int s) -> uint32_t { return bar_base + 8 * (S + s); };
-    auto acc_full = [&](int b) -> uint32_t { return bar_base + 8 * (2 * S + b); };
-    auto acc_empty = [&](int b) -> uint32_t { return bar_base + 8 * (2 * S + 2 + b); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_area + 8 * (2 * S + 4));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_area + 8 * (2 * S + 4) + 8);
+    auto empty = [&](int s) -> uint32_t { return bar_base + 8 * (M + s); };
+    auto acc_full = [&](int b) -> uint32_t { return bar_base + 8 * (2 * M + b); };
+    auto acc_empty = [&](int b) -> uint32_t { return bar_base + 8 * (2 * M + 2 + b); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_area + 8 * (2 * M + 4));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_area + 8 * (2 * M + 4) + 8);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();  // 0: issues the products, 1: partner
@@ -435,13 +429,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // over columns that do not exist would cost its full time
     auto columns = [&](int col) -> int { return min(p.width, (p.n - col + 31) / 32 * 32); };
     const int b_boxes = (p.width + 127) / 128;  // boxes of 64 columns that an MN-major half takes
-    const uint32_t stage_bytes = 2 * (L::kStageA + (BMN ? b_boxes * 8192 : p.width * 64));  // both CTAs' bytes
+    const uint32_t stage = L::kStageA + (BMN ? b_boxes * 8192 : p.width * 64);  // (a multiple of 1024: swizzled tiles)
+    const int S = min(M, (int)(L::kBars / stage));
 
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
-        for (int s = 0; s < S; ++s) {
+        for (int s = 0; s < M; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
         }
@@ -465,7 +459,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ---------------- producer (both CTAs) ----------------
         if (elect_one()) {
             int s = 0;
-            uint32_t parity = 1;
+            uint32_t parity = 1, dst = smem_base;
             for (int tile = pair; tile < tiles; tile += pairs) {
                 const int split = tile % p.splits;
                 int band, col;
@@ -476,9 +470,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int kb1 = k_blocks * (split + 1) / p.splits;
                 for (int kb = k_blocks * split / p.splits; kb < kb1; ++kb) {
                     mbar_wait(empty(s), parity, abort_flag, p.status);
-                    if (rank == 0) mbar_expect_tx(full(s), stage_bytes);
+                    if (rank == 0) mbar_expect_tx(full(s), 2 * stage);  // both CTAs' bytes
                     const uint32_t bar0 = map_to_cta(full(s), 0);
-                    const uint32_t dst = smem_base + s * L::kStage;
                     if (AMN) {
 #pragma unroll
                         for (int c = 0; c < GM / 64; ++c) tma_load_2d_pair(dst + c * 8192, &map_a, bar0, row0 + c * 64, kb * GK);
@@ -491,7 +484,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     } else {
                         tma_load_2d_pair(dst + L::kStageA, &map_w, bar0, kb * GK, col0);
                     }
-                    if (++s == S) { s = 0; parity ^= 1u; }
+                    dst += stage;
+                    if (++s == S) { s = 0; dst = smem_base; parity ^= 1u; }
                 }
             }
         }
@@ -500,7 +494,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ---------------- tensor-core issue (first CTA of the pair only) ----------------
         if (rank == 0 && elect_one()) {
             int s = 0, t = 0;
-            uint32_t parity = 0;
+            uint32_t parity = 0, src = smem_base;
             for (int tile = pair; tile < tiles; tile += pairs, ++t) {
                 const int buf = t & 1;
                 int band, col;
@@ -514,15 +508,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 for (int kb = kb0; kb < kb1; ++kb) {
                     mbar_wait(full(s), parity, abort_flag, p.status);
                     tc_fence_after();
-                    const uint64_t a_desc = tile_desc<GM, AMN>(smem_base + s * L::kStage);
-                    const uint64_t b_desc = tile_desc<BN / 2, BMN>(smem_base + s * L::kStage + L::kStageA);
+                    const uint64_t a_desc = tile_desc<GM, AMN>(src);
+                    const uint64_t b_desc = tile_desc<BN / 2, BMN>(src + L::kStageA);
 #pragma unroll
                     for (int kk = 0; kk < GK / 16; ++kk)
                         mma_ss_pair(d_tmem, a_desc + kStepDesc<AMN> * kk, b_desc + kStepDesc<BMN> * kk, idesc,
                                     (kb > kb0 || kk) ? 1u : 0u);
                     tc_commit_pair(empty(s));
                     if (kb == kb1 - 1) tc_commit_pair(acc_full(buf));
-                    if (++s == S) { s = 0; parity ^= 1u; }
+                    src += stage;
+                    if (++s == S) { s = 0; src = smem_base; parity ^= 1u; }
                 }
             }
         }
@@ -531,25 +526,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ---------------- epilogue (both CTAs, each its own 128 rows) ----------------
         const int g = warp & 3;
         const int sub = (warp - 2) >> 2;
-        uint8_t* slots = smem + S * L::kStage + (warp - 2) * 2 * kSlot;
-        int t = 0, count = 0;
+        int t = 0;
         for (int tile = pair; tile < tiles; tile += pairs, ++t) {
             const int buf = t & 1;
             int band, col0;
             locate(tile, band, col0);
-            const int row0 = band * (2 * GM) + (int)rank * GM;
+            const int row = band * (2 * GM) + (int)rank * GM + g * 32 + lane;
             const int panels = columns(col0) / kPanel;
             PanelAux in;
-            if (sub < panels) load_aux(in, p, row0 + g * 32, col0 + sub * kPanel, lane);
+            if (sub < panels) load_aux(in, p, row, col0 + sub * kPanel);
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            epilogue_panels<BF16>(p, &map_c, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, slots, count, row0 + g * 32, col0,
-                                  sub, panels, kPairEpiWarps / 4, tile % p.splits, lane,
-                                  [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
-        }
-        if (lane == 0) {
-            if (p.drain) tma_store_wait_all();
-            else tma_store_wait_read();  // (the stores themselves complete with the grid)
+            epilogue_panels<BF16>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, row, col0, sub, panels, kPairEpiWarps / 4,
+                                  tile % p.splits, [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
         }
     }
 
@@ -569,12 +558,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // ---------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------
-bool make_maps(const GemmCall& g, int b_rows, CUtensorMap* ma, CUtensorMap* mb, CUtensorMap* mc) {
+bool make_maps(const GemmCall& g, int b_rows, CUtensorMap* ma, CUtensorMap* mb) {
     const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
     return (g.a_mn ? make_map_2d(ma, g.a, g.dtype, g.k, g.m, g.lda, GK, 64, sw) : make_map_2d(ma, g.a, g.dtype, g.m, g.k, g.lda, GM, GK, sw)) &&
            (g.b_mn ? make_map_2d(mb, g.b, g.dtype, g.k, g.n, g.ldb, GK, 64, sw)
-                   : make_map_2d(mb, g.b, g.dtype, g.n, g.k, g.ldb, b_rows, GK, sw)) &&
-           make_map_2d(mc, g.c, g.dtype, g.m, g.n, g.ldc, 32, kPanel, CU_TENSOR_MAP_SWIZZLE_64B);
+                   : make_map_2d(mb, g.b, g.dtype, g.n, g.k, g.ldb, b_rows, GK, sw));
 }
 
 int gemm_params(const GemmCall& g, GemmParams* p) {
@@ -584,9 +572,18 @@ int gemm_params(const GemmCall& g, GemmParams* p) {
     p->aux = g.aux;
     p->splits = g.splits;
     p->partial = g.splits > 1 ? g.partial : nullptr;
-    p->drain = g.chain & kChainFollowed;
+    p->c = g.c;
+    p->ldc = g.ldc;
+    auto on32 = [](const void* q, int64_t ld) { return (reinterpret_cast<uintptr_t>(q) & 31u) == 0 && ld % 16 == 0; };
+    p->wide = on32(g.c, g.ldc) && (g.aux == nullptr || on32(g.aux, g.n));
     p->status = device_status_word();
-    return p->status == nullptr ? TMW_ERR_CUDA : TMW_OK;
+    if (p->status == nullptr) return TMW_ERR_CUDA;
+    auto on16 = [](const void* q, int64_t ld) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0 && ld % 8 == 0; };
+    if (!on16(g.c, g.ldc) || (g.aux != nullptr && !on16(g.aux, g.n))) {
+        set_error_text("product: rows of the output and of what the epilogue reads must start on 16-byte boundaries");
+        return TMW_ERR_INVALID_ARGUMENT;
+    }
+    return TMW_OK;
 }
 
 // `with` is called with the kernel of the call's data type and operand layouts
@@ -599,16 +596,16 @@ int with_layout(const GemmCall& g, K00 k00, K01 k01, K11 k11, F with) {
 template <int BN>
 int launch_gemm(const GemmCall& g, cudaStream_t stream) {
     using L = GemmSmem<BN>;
-    CUtensorMap ma, mb, mc;
+    CUtensorMap ma, mb;
     GemmParams p;
-    if (!make_maps(g, BN, &ma, &mb, &mc)) return TMW_ERR_CUDA;
-    if (gemm_params(g, &p) != TMW_OK) return TMW_ERR_CUDA;
+    if (!make_maps(g, BN, &ma, &mb)) return TMW_ERR_CUDA;
+    if (const int rc = gemm_params(g, &p); rc != TMW_OK) return rc;
     const int tiles = ((g.m + GM - 1) / GM) * ((g.n + BN - 1) / BN) * g.splits;
     const int grid = tiles < sm_count() ? tiles : sm_count();
     auto run = [&](auto kern) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), L::kTotal);
         if (rc != TMW_OK) return rc;
-        TMW_CUDA_TRY(launch_ex(kern, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, mc, p));
+        TMW_CUDA_TRY(launch_ex(kern, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, p));
         return TMW_OK;
     };
     if constexpr (BN == 64 || BN == 128) {
@@ -652,11 +649,11 @@ int max_active_pairs(const void* kern, int smem_bytes) {
 
 template <int BN>
 int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
-    using L = PairSmem<BN>;
-    CUtensorMap ma, mb, mc;
+    using L = PairSmem;
+    CUtensorMap ma, mb;
     GemmParams p;
-    if (!make_maps(g, width / 2, &ma, &mb, &mc)) return TMW_ERR_CUDA;
-    if (gemm_params(g, &p) != TMW_OK) return TMW_ERR_CUDA;
+    if (!make_maps(g, width / 2, &ma, &mb)) return TMW_ERR_CUDA;
+    if (const int rc = gemm_params(g, &p); rc != TMW_OK) return rc;
     p.width = width;
     const int tiles = ((g.m + 2 * GM - 1) / (2 * GM)) * ((g.n + width - 1) / width) * g.splits;
     auto run = [&](auto kern) -> int {
@@ -665,7 +662,7 @@ int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
         if (rc != TMW_OK) return rc;
         const int resident = max_active_pairs(fn, L::kTotal);
         const int pairs = tiles < resident ? tiles : resident;
-        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kPairThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, mc, p));
+        TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kPairThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, p));
         return TMW_OK;
     };
     return g.dtype == TMW_BF16
