@@ -56,7 +56,7 @@ struct BwdParams {
     long long os[3];             // {batch, head, row} strides of o and d_o, elements
     const float* lse;            // [batch, heads, rows]
     // Scratch memory [batch * heads][2][rows_pad] (fp32; rows_pad a multiple of 128), or nullptr.  The launch whose
-    // rows are queries computes every row's D anyway and leaves (lse, D) here; the launch whose rows are keys,
+    // rows are queries computes every row's D anyway and leaves (-lse, -D) here; the launch whose rows are keys,
     // run after it, then fetches its column statistics with one 16-byte load per lane instead of reading two
     // rows of O and dO per column.
     float* stats;
@@ -80,7 +80,7 @@ struct BwdSmem {
     static constexpr int kCSub = CW * 128;
     static constexpr int kR1 = 0, kR2 = kTile;                  // row tiles (later: staging of the outputs)
     static constexpr int kC = 2 * kTile;                        // S x (C1 | C2)
-    static constexpr int kVec = kC + S * 2 * kCTile;            // per stage and column: lse and D (fp32)
+    static constexpr int kVec = kC + S * 2 * kCTile;            // per stage and column: -lse and -D (fp32)
     static constexpr int kBars = kVec + S * 2 * CW * 4;
     static constexpr int kTotal = kBars + 256 + 1024;
 };
@@ -116,6 +116,13 @@ struct ColPlan {
     int a0, n0;  // first segment (tiles that hold persistent rows / all query tiles)
     int a1, n1;  // second segment
 };
+
+// bits lo .. hi of a word (none if hi < lo)
+__device__ __forceinline__ uint32_t bits(int lo, int hi) {
+    lo = max(lo, 0);
+    hi = min(hi, 31);
+    return hi < lo ? 0u : (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo);
+}
 
 // last query that sees sequence key k through its window (block > 0: the window's left edge is block-aligned)
 __device__ __forceinline__ int last_query_of_key(int k, int np, int w, int block) {
@@ -172,7 +179,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
     auto bar = [&](int slot) -> uint32_t { return bar_base + slot * 8; };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_area + BAR_N * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_area + BAR_N * 8 + 8);
-    float* vec = reinterpret_cast<float*>(smem + L::kVec);  // [stage][lse | D][column]
+    float* vec = reinterpret_cast<float*>(smem + L::kVec);  // [stage][-lse | -D][column]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // One-dimensional grid.  The row tile that holds the persistent keys walks over EVERY query tile (all queries
@@ -264,7 +271,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
                 float* v_lse = vec + s * 2 * CW;
                 const long long bh = (long long)batch * p.heads + head;
                 if (p.stats != nullptr) {
-                    // [lse | D] of the tile's CW columns: 2 * CW / 4 loads of 16 bytes
+                    // [-lse | -D] of the tile's CW columns: 2 * CW / 4 loads of 16 bytes
                     const float* src = p.stats + bh * 2 * p.rows_pad + col_tile(n) * CW;
                     for (int i = lane; i < 2 * CW / 4; i += 32) {
                         const int half = i / (CW / 4), c4 = i % (CW / 4);
@@ -275,9 +282,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
                     for (int i = lane; i < CW; i += 32) {
                         const int qrow = col_tile(n) * CW + i;
                         v_lse[i] = qrow >= p.rows ? 0.f
-                                   : !GENERAL ? p.lse[bh * p.rows + qrow]
-                                   : qrow >= p.np ? p.lse[bh * (p.rows - p.np) + (qrow - p.np)] : p.lse_pers[bh * p.np + qrow];
-                        v_lse[CW + i] = delta_of<DH, BF16>(p, batch, head, qrow);
+                                   : !GENERAL ? -p.lse[bh * p.rows + qrow]
+                                   : qrow >= p.np ? -p.lse[bh * (p.rows - p.np) + (qrow - p.np)] : -p.lse_pers[bh * p.np + qrow];
+                        v_lse[CW + i] = -delta_of<DH, BF16>(p, batch, head, qrow);
                     }
                 }
                 __syncwarp();
@@ -357,25 +364,26 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
         const int pos_row = r0 + row;              // position of this thread's key (ROWS_ARE_KEYS) or query
         const uint32_t t_row = tmem_base + ((uint32_t)(g * 32) << 16);
         const long long bh = (long long)batch * p.heads + head;
-        // log-sum-exp of a query row (GENERAL: the persistent rows have a plane of their own)
-        auto lse_of = [&](int q) -> float {
+        // minus the log-sum-exp of a query row (GENERAL: the persistent rows have a plane of their own)
+        auto neg_lse_of = [&](int q) -> float {
             if (q >= p.rows) return 0.f;
-            if (GENERAL) return q >= p.np ? p.lse[bh * (p.rows - p.np) + (q - p.np)] : p.lse_pers[bh * p.np + q];
-            return p.lse[bh * p.rows + q];
+            if (GENERAL) return q >= p.np ? -p.lse[bh * (p.rows - p.np) + (q - p.np)] : -p.lse_pers[bh * p.np + q];
+            return -p.lse[bh * p.rows + q];
         };
         constexpr int HC = CW / 2;                 // columns per thread and tile
         const int cbase = half * HC;
 
         // rows are queries: this thread's own statistics, once
-        float lse_own = 0.f, d_own = 0.f;
+        float nl_own = 0.f, nd_own = 0.f;
         if (!ROWS_ARE_KEYS) {
-            lse_own = lse_of(pos_row);
-            d_own = delta_of<DH, BF16>(p, batch, head, pos_row);
+            nl_own = neg_lse_of(pos_row);
+            nd_own = -delta_of<DH, BF16>(p, batch, head, pos_row);
             if (p.stats != nullptr && half == 0) {  // rows beyond the sequence get (0, 0), like the bounds-checked path
-                p.stats[bh * 2 * p.rows_pad + pos_row] = lse_own;
-                p.stats[bh * 2 * p.rows_pad + p.rows_pad + pos_row] = d_own;
+                p.stats[bh * 2 * p.rows_pad + pos_row] = nl_own;
+                p.stats[bh * 2 * p.rows_pad + p.rows_pad + pos_row] = nd_own;
             }
         }
+        const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
 
         for (int n = 0; n < n_cols; ++n) {
             const int c0 = col_tile(n) * CW;  // position of column 0
@@ -394,29 +402,43 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
                        (chi < p.np || (GENERAL && rhi < p.np) ||
                         (clo >= p.np && rlo >= p.np && chi <= rlo && clo >= first_visible_pos(rhi, p.np, p.window, wblock)));
 
-            // Columns of this tile that this thread's row sees: [vlo, vhi] (relative to the tile) and the columns
-            // below npc - the persistent keys when the rows are queries, the persistent queries (block-sparse
-            // class: they see every key) when the rows are keys.  Two instructions per element.
-            int vlo = 1, vhi = 0, npc = 0;
-            if (pos_row < p.rows) {
-                if (ROWS_ARE_KEYS) {
-                    if (GENERAL) npc = p.np - c0;
-                    if (pos_row < p.np) { vlo = 0; vhi = p.rows - 1 - c0; }
-                    else { vlo = pos_row - c0; vhi = min(last_query_of_key(pos_row, p.np, p.window, wblock), p.rows - 1) - c0; }
-                } else {
-                    npc = p.np - c0;
-                    if (pos_row >= p.np) { vlo = first_visible_pos(pos_row, p.np, p.window, wblock) - c0; vhi = pos_row - c0; }
-                    else if (GENERAL) { vlo = 0; vhi = p.rows - 1 - c0; }
+            // Which of its columns this thread's row sees, a bit each: [vlo, vhi] (relative to the half tile) and the columns
+            // below npc - the persistent keys when the rows are queries, the persistent queries (block-sparse class:
+            // they see every key) when the rows are keys.
+            uint32_t vis[HC / 32];
+            int seen = 2;  // columns that the rows of this warp see: 0 none, 1 some, 2 all
+            if (!full) {
+                int vlo = 1, vhi = 0, npc = 0;
+                const int h0 = c0 + cbase;
+                if (pos_row < p.rows) {
+                    if (ROWS_ARE_KEYS) {
+                        if (GENERAL) npc = p.np - h0;
+                        if (pos_row < p.np) { vlo = 0; vhi = p.rows - 1 - h0; }
+                        else { vlo = pos_row - h0; vhi = min(last_query_of_key(pos_row, p.np, p.window, wblock), p.rows - 1) - h0; }
+                    } else {
+                        npc = p.np - h0;
+                        if (pos_row >= p.np) { vlo = first_visible_pos(pos_row, p.np, p.window, wblock) - h0; vhi = pos_row - h0; }
+                        else if (GENERAL) { vlo = 0; vhi = p.rows - 1 - h0; }
+                    }
                 }
+                bool none = true, all = true;
+#pragma unroll
+                for (int k = 0; k < HC / 32; ++k) {
+                    vis[k] = bits(vlo - 32 * k, vhi - 32 * k);
+                    if (!ROWS_ARE_KEYS || GENERAL) vis[k] |= bits(0, npc - 1 - 32 * k);
+                    none &= vis[k] == 0u;
+                    all &= vis[k] == 0xffffffffu;
+                }
+                if (__all_sync(0xffffffffu, none)) seen = 0;
+                else if (!__all_sync(0xffffffffu, all)) seen = 1;
             }
-            const int vbase = cbase - vlo;                 // column - vlo = vbase + (column - cbase)
-            const unsigned vspan = (unsigned)max(vhi - vlo, -1);   // vhi < vlo: empty (0xffffffff would mean everything)
-            const bool vnone = vhi < vlo;
-            const int pbase = npc - cbase;                 // column < npc  <=>  (column - cbase) < pbase
 
             mbar_wait(bar(BAR_XY_FULL + half), n & 1, abort_flag, p.status);
             tc_fence_after();
-            // 16 columns at a time.  The body exists twice, with and without the per-element mask, as straight-line
+            // 16 columns at a time, two values per instruction where there is one (fma, add, mul of f32x2), and a mask only in
+            // warps that need one: the tile pairs on an edge are five of eleven, the warps that see a part of their half
+            // tile a fifth (8 x 10 heads x 4112 rows of 64, window 512: 338 -> 324 us for both launches; 4 x 10 heads x 2064, block-granular: 133.8 -> 122.8).
+            // The body exists twice, with and without the per-element mask, as straight-line
             // code (a run-time test inside it would split it into one basic block per element and serialise the
             // elements' dependency chains).  The 16-bit results go back OVER the fp32 inputs, each thread's inside
             // its own half of the columns: chunk j's 8 packed columns lie in columns this thread has already read.
@@ -431,44 +453,40 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
                     uint32_t pp[8], ds[8];
 #pragma unroll
                     for (int e4 = 0; e4 < 16; e4 += 4) {
-                        float l[4], dd[4];
-                        if (ROWS_ARE_KEYS) {  // the columns' statistics, four columns per shared-memory load
+                        uint64_t nl[2], nd[2];  // minus log-sum-exp and D, two columns each
+                        if (ROWS_ARE_KEYS) {    // the columns' statistics, four columns per shared-memory load
                             const float4 l4 = *reinterpret_cast<const float4*>(v_lse + cbase + j * 16 + e4);
                             const float4 d4 = *reinterpret_cast<const float4*>(v_d + cbase + j * 16 + e4);
-                            l[0] = l4.x; l[1] = l4.y; l[2] = l4.z; l[3] = l4.w;
-                            dd[0] = d4.x; dd[1] = d4.y; dd[2] = d4.z; dd[3] = d4.w;
+                            nl[0] = pack2(l4.x, l4.y); nl[1] = pack2(l4.z, l4.w);
+                            nd[0] = pack2(d4.x, d4.y); nd[1] = pack2(d4.z, d4.w);
                         } else {
-                            l[0] = l[1] = l[2] = l[3] = lse_own;
-                            dd[0] = dd[1] = dd[2] = dd[3] = d_own;
-                        }
-                        float pv[4], dv[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float pr = fast_exp2(fmaf(__uint_as_float(x[e4 + e]), p.scale_log2, -l[e]));
-                            const float dsv = pr * (__uint_as_float(y[e4 + e]) - dd[e]);
-                            if (MASKED) {
-                                const int rel = j * 16 + e4 + e;  // column - cbase, a compile-time constant
-                                bool vis = ((unsigned)(vbase + rel) <= vspan) & !vnone;
-                                if (!ROWS_ARE_KEYS || GENERAL) vis |= rel < pbase;
-                                pv[e] = vis ? pr : 0.f;
-                                dv[e] = vis ? dsv : 0.f;
-                            } else {
-                                pv[e] = pr;
-                                dv[e] = dsv;
-                            }
+                            nl[0] = nl[1] = pack2(nl_own, nl_own);
+                            nd[0] = nd[1] = pack2(nd_own, nd_own);
                         }
 #pragma unroll
                         for (int e = 0; e < 4; e += 2) {
+                            const int at = e4 + e;
+                            float p0, p1, d0, d1;
+                            unpack2(fma2(pack2(__uint_as_float(x[at]), __uint_as_float(x[at + 1])), scale2, nl[e / 2]), p0, p1);
+                            p0 = fast_exp2(p0);
+                            p1 = fast_exp2(p1);
+                            const uint64_t yd = add2(pack2(__uint_as_float(y[at]), __uint_as_float(y[at + 1])), nd[e / 2]);
+                            unpack2(mul2(pack2(p0, p1), yd), d0, d1);
+                            if (MASKED) {  // (a bit of the half tile's columns: its number is a constant)
+                                const uint32_t w = vis[(j * 16 + at) / 32] >> ((j * 16 + at) % 32);
+                                if (!(w & 1u)) p0 = d0 = 0.f;
+                                if (!(w & 2u)) p1 = d1 = 0.f;
+                            }
                             if (BF16) {
-                                const __nv_bfloat162 a2 = __floats2bfloat162_rn(pv[e], pv[e + 1]);
-                                const __nv_bfloat162 b2 = __floats2bfloat162_rn(dv[e], dv[e + 1]);
-                                pp[(e4 + e) / 2] = *reinterpret_cast<const uint32_t*>(&a2);
-                                ds[(e4 + e) / 2] = *reinterpret_cast<const uint32_t*>(&b2);
+                                const __nv_bfloat162 a2 = __floats2bfloat162_rn(p0, p1);
+                                const __nv_bfloat162 b2 = __floats2bfloat162_rn(d0, d1);
+                                pp[at / 2] = *reinterpret_cast<const uint32_t*>(&a2);
+                                ds[at / 2] = *reinterpret_cast<const uint32_t*>(&b2);
                             } else {
-                                const __half2 a2 = __floats2half2_rn(pv[e], pv[e + 1]);
-                                const __half2 b2 = __floats2half2_rn(dv[e], dv[e + 1]);
-                                pp[(e4 + e) / 2] = *reinterpret_cast<const uint32_t*>(&a2);
-                                ds[(e4 + e) / 2] = *reinterpret_cast<const uint32_t*>(&b2);
+                                const __half2 a2 = __floats2half2_rn(p0, p1);
+                                const __half2 b2 = __floats2half2_rn(d0, d1);
+                                pp[at / 2] = *reinterpret_cast<const uint32_t*>(&a2);
+                                ds[at / 2] = *reinterpret_cast<const uint32_t*>(&b2);
                             }
                         }
                     }
@@ -478,16 +496,14 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             };
             // a warp none of whose rows sees any of its columns (rows beyond the diagonal or the window's edge, or the
             // sequence keys of a tile that far queries only reach through the persistent keys) writes zeros unread
-            const bool mine_empty = vnone || vhi < cbase || vlo >= cbase + HC;
-            const bool nothing = !full && __all_sync(0xffffffffu, mine_empty && ((ROWS_ARE_KEYS && !GENERAL) || pbase <= 0 || pos_row >= p.rows));
-            if (nothing) {
+            if (seen == 0) {
                 const uint32_t zero[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll
                 for (int j = 0; j < HC / 16; ++j) {
                     if (ROWS_ARE_KEYS) tmem_st8(t_row + kX + cbase + j * 8, zero);
                     tmem_st8(t_row + kY + cbase + j * 8, zero);
                 }
-            } else if (full) {
+            } else if (seen == 2) {
                 process(std::false_type{});
             } else {
                 process(std::true_type{});
