@@ -85,9 +85,9 @@ struct BwdSmem {
     static constexpr int kTotal = kBars + 256 + 1024;
 };
 
-// barrier slots: R_FULL | C_FULL[4] | C_EMPTY[4] | XY_FULL[2] | PDS_READY[2] | ACC_DONE | V_FULL[4]
+// barrier slots: R_FULL | C_FULL[4] | C_EMPTY[4] | XY_FULL[2] | PDS_READY[2] | ACC_DONE | V_FULL[4] | ROWS_READY
 enum { BAR_R_FULL = 0, BAR_C_FULL = 1, BAR_C_EMPTY = 5, BAR_XY_FULL = 9, BAR_PDS_READY = 11, BAR_ACC_DONE = 13, BAR_V_FULL = 14,
-       BAR_N = 18 };
+       BAR_ROWS_READY = 18, BAR_N = 19 };
 
 // D = dO . O of one query row (fp32), straight from global memory (two rows of head_dim 16-bit values)
 template <int DH, bool BF16>
@@ -169,7 +169,13 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
     constexpr int NSUB = DH / 64;
     constexpr int CW = Geo<DH>::kCW, kColStages = Geo<DH>::kStages;
     constexpr uint32_t kX = 0, kY = CW, kAcc1 = 2 * CW, kAcc2 = 2 * CW + DH;
-    constexpr uint32_t kNeed = 2 * CW + (ROWS_ARE_KEYS ? 2 : 1) * DH;
+    // Rows that are queries have room for their own tiles in tensor memory too (16-bit pairs: DH / 2 columns each), as the first
+    // operands of X and Y.  From shared memory these would be read again, 4 KB, for every product of 32 or 64 columns, which
+    // takes longer than the product (8 x 10 heads x 4112 rows of 64, window 512, both launches: 325 -> 315 us).
+    constexpr bool kRowsInTmem = !ROWS_ARE_KEYS;
+    constexpr uint32_t kRows = 2 * CW + DH;
+    constexpr uint32_t kNeed = 2 * CW + 2 * DH;
+    static_assert(kNeed <= 512 / Geo<DH>::kCtasPerSm, "tensor memory");
     constexpr uint32_t kTmemCols = kNeed <= 256 ? 256 : 512;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -229,6 +235,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             mbar_init(bar(BAR_PDS_READY + h), 4);  // the four element-wise warps of the half
         }
         mbar_init(bar(BAR_ACC_DONE), 2);
+        mbar_init(bar(BAR_ROWS_READY), 8);  // the element-wise warps
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -314,13 +321,15 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             const uint32_t c_tile = smem_base + L::kC + (n % kColStages) * 2 * L::kCTile + (second ? L::kCTile : 0) + h * HC * 128;
 #pragma unroll
             for (int kk = 0; kk < DH / 16; ++kk) {
-                const uint64_t ad = kmajor_desc(r_addr + (kk / 4) * L::kSub + (kk % 4) * 32);
                 const uint64_t bd = kmajor_desc(c_tile + (kk / 4) * L::kCSub + (kk % 4) * 32);
-                mma_ss(xy + h * HC, ad, bd, idesc_xy, kk > 0 ? 1u : 0u);
+                if (kRowsInTmem)
+                    mma_ts(xy + h * HC, tmem_base + kRows + (second ? DH / 2 : 0) + kk * 8, bd, idesc_xy, kk > 0 ? 1u : 0u);
+                else
+                    mma_ss(xy + h * HC, kmajor_desc(r_addr + (kk / 4) * L::kSub + (kk % 4) * 32), bd, idesc_xy, kk > 0 ? 1u : 0u);
             }
             tc_commit(bar(BAR_XY_FULL + h));
         };
-        mbar_wait(bar(BAR_R_FULL), 0, abort_flag, p.status);
+        mbar_wait(bar(kRowsInTmem ? BAR_ROWS_READY : BAR_R_FULL), 0, abort_flag, p.status);
         if (n_cols > 0) {
             mbar_wait(bar(BAR_C_FULL), 0, abort_flag, p.status);
             tc_fence_after();
@@ -384,6 +393,25 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant_
             }
         }
         const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
+        if (kRowsInTmem) {  // this thread's row of the first (half 0) or second tile: shared -> tensor memory
+            mbar_wait(bar(BAR_R_FULL), 0, abort_flag, p.status);
+            const uint8_t* src = smem + (half ? L::kR2 : L::kR1) + row * 128;
+#pragma unroll
+            for (int c = 0; c < DH / 16; ++c) {
+                uint32_t r[8];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int chunk = (2 * c + e) % 8;  // of 16 bytes, swizzled inside the row
+                    const uint4 v = *reinterpret_cast<const uint4*>(src + (2 * c + e) / 8 * L::kSub + ((chunk ^ (row & 7)) * 16));
+                    r[4 * e] = v.x; r[4 * e + 1] = v.y; r[4 * e + 2] = v.z; r[4 * e + 3] = v.w;
+                }
+                tmem_st8(t_row + kRows + half * (DH / 2) + c * 8, r);
+            }
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(BAR_ROWS_READY));
+        }
 
         for (int n = 0; n < n_cols; ++n) {
             const int c0 = col_tile(n) * CW;  // position of column 0
