@@ -41,6 +41,9 @@ def close(got, want, tol):
     (2, 200, torch.bfloat16, 1, 128, 40, 0, 4096, False), # no persistent rows
     (8, 1001, torch.bfloat16, 4, 64, 64, 8, 640, True),   # k = 8072 rows in the weights' gradients: cut into ranges
     (4, 1024, torch.float16, 5, 128, 100, 16, 2048, False),  # d_model 640: column tiles narrower than 256
+    (5, 1000, torch.bfloat16, 8, 64, 40, 8, 512, False),     # norms of 512 columns, three rows to a warp
+    (5, 1000, torch.bfloat16, 8, 128, 40, 8, 512, False),    # 1024 columns
+    (2, 150, torch.float16, 16, 128, 40, 4, 512, False),     # 2048 columns, the widest
 ])
 def test_training_step_equals_module_by_module(B, T, dtype, heads, dh, window, Np, vocab, block_sparse, monkeypatch):
     model, g = make(dtype, heads, dh, window, Np, vocab, block_sparse)

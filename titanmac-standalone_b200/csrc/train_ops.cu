@@ -14,10 +14,13 @@ constexpr int kNormWarps = 8;
 // y = x inv gain with inv = 1 / sqrt(mean(x^2) + eps).  Given dy: dx = inv (dy gain - x̂ mean(dy gain x̂)), x̂ = x inv, and
 // out = add + dx (the residual branch's gradient rides along).  A warp walks over rows with its columns of the two column
 // sums - dgain = sum dy x̂, and sum out, the bias gradient of the linear whose output the residual stream is - in registers;
-// the CTA adds its warps' up and leaves one partial row of each.
+// the CTA adds its warps' up and leaves one partial row of each.  Bound by HBM and, with three or four rows to a warp, by the
+// first row's latency and the tail; 8320 rows of 640 (32 MB in, 11 MB out: 6.5 us), cold caches, us: 21.1 -> 15.2 with both sums,
+// 17.6 -> 14.6 with dgain alone, since the warps' sums are added up side by side and not one warp after the other, and the
+// next row loads under a row.
 template <typename T, int NV, bool SUMS>
-__global__ void __launch_bounds__(kNormWarps * 32) rmsnorm_bwd_kernel(const NormBwd p) {
-    extern __shared__ float sums[];  // [2][dim]
+__global__ void __launch_bounds__(kNormWarps * 32, NV <= 3 ? 2 : 1) rmsnorm_bwd_kernel(const NormBwd p) {
+    extern __shared__ float sums[];  // [dgain | sum of out][warp][dim]
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = p.dim / 8;
@@ -30,24 +33,36 @@ __global__ void __launch_bounds__(kNormWarps * 32) rmsnorm_bwd_kernel(const Norm
             if (SUMS) os[j][e] = 0.f;
         }
     const long long warps = (long long)gridDim.x * kNormWarps;
-    for (long long row = (long long)blockIdx.x * kNormWarps + warp; row < p.rows; row += warps) {
-        const long long at = row * p.dim;
-        Vec8<T> xv[NV], dv[NV], av[NV];
+    // the next row loads under this one, where the registers hold two rows beside the sums at two CTAs per SM
+    constexpr bool AHEAD = NV <= 2 || (NV == 3 && !SUMS);
+    Vec8<T> xv[NV], dv[NV], av[NV];
+    auto fetch = [&](long long row) {
+        if (row >= p.rows) return;
 #pragma unroll
         for (int j = 0; j < NV; ++j)
             if (lane + j * 32 < nvec) {
-                const long long o = at + (lane + j * 32) * 8;
+                const long long o = row * p.dim + (lane + j * 32) * 8;
                 xv[j].load(static_cast<const T*>(p.x) + o);
                 dv[j].load(static_cast<const T*>(p.dy) + o);
                 if (p.add != nullptr) av[j].load(static_cast<const T*>(p.add) + o);
             }
+    };
+    const long long first = (long long)blockIdx.x * kNormWarps + warp;
+    if (AHEAD) fetch(first);
+    for (long long row = first; row < p.rows; row += warps) {
+        const long long at = row * p.dim;
+        if (!AHEAD) fetch(row);
+        Vec8<T> x0[NV], d0[NV], a0[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) { x0[j] = xv[j]; d0[j] = dv[j]; a0[j] = av[j]; }
+        if (AHEAD) fetch(row + warps);
         float ss = 0.f, dot = 0.f;
 #pragma unroll
         for (int j = 0; j < NV; ++j)
             if (lane + j * 32 < nvec) {
                 float x[8], d[8], g[8];
-                xv[j].unpack(x);
-                dv[j].unpack(d);
+                x0[j].unpack(x);
+                d0[j].unpack(d);
                 load8<T>(static_cast<const T*>(p.gain) + (lane + j * 32) * 8, g);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
@@ -66,10 +81,10 @@ __global__ void __launch_bounds__(kNormWarps * 32) rmsnorm_bwd_kernel(const Norm
         for (int j = 0; j < NV; ++j)
             if (lane + j * 32 < nvec) {
                 float x[8], d[8], g[8], a[8];
-                xv[j].unpack(x);
-                dv[j].unpack(d);
+                x0[j].unpack(x);
+                d0[j].unpack(d);
                 load8<T>(static_cast<const T*>(p.gain) + (lane + j * 32) * 8, g);
-                if (p.add != nullptr) av[j].unpack(a);
+                if (p.add != nullptr) a0[j].unpack(a);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     ds[j][e] = fmaf(d[e], x[e] * inv, ds[j][e]);
@@ -81,27 +96,29 @@ __global__ void __launch_bounds__(kNormWarps * 32) rmsnorm_bwd_kernel(const Norm
                 store8<T>(static_cast<T*>(p.out) + at + (lane + j * 32) * 8, a);
             }
     }
-    // one warp after the other adds its columns: the order of the sum is fixed (8320 rows of 640 with both sums, us: 25.5 with a
-    // lane's eight columns side by side, 21 with neighbouring lanes in neighbouring banks)
-    for (int w = 0; w < kNormWarps; ++w) {
-        if (warp == w) {
+    // every warp leaves its columns, then each column's eight values are added up in the order of the warps (neighbouring lanes
+    // in neighbouring banks)
 #pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (lane + j * 32 < nvec) {
+    for (int j = 0; j < NV; ++j)
+        if (lane + j * 32 < nvec) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int col = e * nvec + lane + j * 32;
-                        sums[col] = (w ? sums[col] : 0.f) + ds[j][e];
-                        if (SUMS) sums[p.dim + col] = (w ? sums[p.dim + col] : 0.f) + os[j][e];
-                    }
-                }
+            for (int e = 0; e < 8; ++e) {
+                const int col = e * nvec + lane + j * 32;
+                sums[warp * p.dim + col] = ds[j][e];
+                if (SUMS) sums[(kNormWarps + warp) * p.dim + col] = os[j][e];
+            }
         }
-        __syncthreads();
-    }
+    __syncthreads();
     for (int i = threadIdx.x; i < p.dim; i += kNormWarps * 32) {
         const int at = (i & 7) * nvec + (i >> 3);
-        p.dgain_part[(long long)blockIdx.x * p.dim + i] = sums[at];
-        if (SUMS) p.sum_part[(long long)blockIdx.x * p.dim + i] = sums[p.dim + at];
+        float a = 0.f, b = 0.f;
+#pragma unroll
+        for (int w = 0; w < kNormWarps; ++w) {
+            a += sums[w * p.dim + at];
+            if (SUMS) b += sums[(kNormWarps + w) * p.dim + at];
+        }
+        p.dgain_part[(long long)blockIdx.x * p.dim + i] = a;
+        if (SUMS) p.sum_part[(long long)blockIdx.x * p.dim + i] = b;
     }
 }
 
@@ -137,33 +154,37 @@ __global__ void __launch_bounds__(256) colsum_kernel(const void* src, float* par
     }
 }
 
-// dst[j] = round(sum over parts of src[part][j]) for several arrays at once (blockIdx.y).  Many parts (column sums): 32
-// groups of four columns x 8 threads per group; few parts (split products): a thread per group of four columns.
+// dst[j] = round(sum over parts of src[part][j]) for several arrays at once (blockIdx.y).  Few parts (split products): a thread
+// per group of four columns.  Many parts (column sums): eight groups x 32 threads per group, so that a thread's chain of loads
+// is short - 296 parts of 640 columns are a matter of latency, 14 us with eight threads per group and 5.6 with 32.
+constexpr int kManyParts = 16, kManyGroups = 8, kManyLanes = 32;
 template <typename T>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const SumParts p) {
-    __shared__ float4 s[8][32];
+    __shared__ float4 s[kManyLanes][kManyGroups];
     pdl_trigger();
     pdl_wait();
     const SumParts::Item it = p.item[blockIdx.y];
-    const bool many = it.parts > 16;
+    const bool many = it.parts > kManyParts;
     const long long groups = (it.n + 3) / 4;
-    const int lanes = many ? 32 : 256, sub = many ? threadIdx.x >> 5 : 0, step = many ? 8 : 1;
+    const int lanes = many ? kManyGroups : 256, at = many ? threadIdx.x % kManyGroups : threadIdx.x;
+    const int sub = many ? threadIdx.x / kManyGroups : 0, step = many ? kManyLanes : 1;
     for (long long g0 = (long long)blockIdx.x * lanes; g0 < groups; g0 += (long long)gridDim.x * lanes) {
-        const long long g = g0 + (many ? threadIdx.x & 31 : threadIdx.x);
+        const long long g = g0 + at;
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
         if (g < groups) {
-#pragma unroll 4
+#pragma unroll 8
             for (int q = sub; q < it.parts; q += step) {
                 const float4 v = *reinterpret_cast<const float4*>(it.src + (long long)q * it.n + g * 4);
                 t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
             }
         }
         if (many) {
-            s[sub][threadIdx.x & 31] = t;
+            s[sub][at] = t;
             __syncthreads();
             if (sub == 0) {
-                for (int q = 1; q < 8; ++q) {
-                    const float4 v = s[q][threadIdx.x];
+#pragma unroll
+                for (int q = 1; q < kManyLanes; ++q) {
+                    const float4 v = s[q][at];
                     t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
                 }
             }
@@ -389,11 +410,17 @@ __global__ void __launch_bounds__(256) embed_rows_bwd_kernel(const EmbedBwd p) {
 
 template <typename T, int NV>
 int launch_rmsnorm_bwd_nv(const NormBwd& p, int blocks, cudaStream_t stream) {
-    const int smem = 2 * p.dim * (int)sizeof(float);
     const dim3 grid(blocks), block(kNormWarps * 32);
-    if (p.sum_part != nullptr) TMW_CUDA_TRY(launch_ex(rmsnorm_bwd_kernel<T, NV, true>, grid, block, smem, stream, true, 1, p));
-    else TMW_CUDA_TRY(launch_ex(rmsnorm_bwd_kernel<T, NV, false>, grid, block, smem, stream, true, 1, p));
-    return TMW_OK;
+    auto run = [&](auto kern, int sums) -> int {
+        const int smem = sums * kNormWarps * p.dim * (int)sizeof(float);
+        if (smem > 48 * 1024) {  // (the default limit)
+            const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), smem);
+            if (rc != TMW_OK) return rc;
+        }
+        TMW_CUDA_TRY(launch_ex(kern, grid, block, smem, stream, true, 1, p));
+        return TMW_OK;
+    };
+    return p.sum_part != nullptr ? run(rmsnorm_bwd_kernel<T, NV, true>, 2) : run(rmsnorm_bwd_kernel<T, NV, false>, 1);
 }
 
 template <typename T>
@@ -434,7 +461,7 @@ int launch_sum_parts(int dtype, const SumParts& p, cudaStream_t stream) {
     if (p.count == 0) return TMW_OK;
     long long most = 1;
     for (int i = 0; i < p.count; ++i) {
-        const long long lanes = p.item[i].parts > 16 ? 32 : 256, blocks = ((p.item[i].n + 3) / 4 + lanes - 1) / lanes;
+        const long long lanes = p.item[i].parts > kManyParts ? kManyGroups : 256, blocks = ((p.item[i].n + 3) / 4 + lanes - 1) / lanes;
         most = blocks > most ? blocks : most;
     }
     const dim3 grid((unsigned)(most < 8 * sm_count() ? most : 8 * sm_count()), p.count), block(256);
