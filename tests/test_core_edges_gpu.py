@@ -42,3 +42,23 @@ def test_block_sparse_core_with_persistent_rows(dtype, tol, dh, L, w, block, n_p
     o = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), w, n_p, window_block=block)
     _native.poll_status()
     assert (o.float().cpu() - ref).abs().max().item() <= tol
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,w,n_p,block", [
+    (700, 511, 16, 0), (700, 512, 16, 0),     # either side of the rule: the general body alone, whole tiles on their own
+    (641, 512, 0, 0), (1100, 513, 128, 0),    # no persistent keys: the first tile sets the maximum; a ragged left edge
+    (1500, 700, 5, 64), (129, 4000, 16, 0),   # block-granular left edge; a window wider than the sequence
+])
+@pytest.mark.parametrize("spread", [1.0, 8.0])
+def test_wide_heads_with_long_windows(dtype, L, w, n_p, block, spread):
+    """Whole key tiles without a mask (head_dim 128, windows from 512 on).  ``spread`` 8 makes scores of up to about 100, whose
+    running maximum grows by more than 2^8 inside such tiles.  Tolerance: probabilities rounded to bf16 (2^-9) weight values
+    of up to 5."""
+    q, k, v = (t.to(dtype) for t in wo.qkv_inputs(1, 2, L, 128, seed=L + w))
+    q = (q.float() * spread).to(dtype)
+    ref = (bo.attention_core(q.float(), k.float(), v.float(), w, block, n_p) if block
+           else wo.attention_core_dense(q.float(), k.float(), v.float(), w, n_p))
+    o = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), w, n_p, window_block=block)
+    _native.poll_status()
+    assert (o.float().cpu() - ref).abs().max().item() <= 2e-2

@@ -24,8 +24,8 @@
 // Measured before (128-key tiles; two CTAs per SM at head_dim 64, one CTA of two query tiles with one S each at 128) and
 // now, us: 8 x 10 heads x 4112 rows of 64, window 128 | 512 | 2048: 82.2 | 133.8 | 283 and 63.4 | 105 | 242 (by itself, one
 // input again or four in turn alike; 120 between the products of a layer, which hold the clock at 1760 MHz); 16 heads x
-// 131 088 rows of 128, window 1024: 1604 and 1314 (two query tiles sharing K and V in one CTA: 1469; a hundred calls in a row,
-// under the power cap: 1513).
+// 131 088 rows of 128, window 1024: 1604 and 1290 (two query tiles sharing K and V in one CTA: 1469; a hundred calls in a row,
+// under the power cap: 1466, 1515 without the straight body below).
 //
 // Every wait on an mbarrier is bounded: on expiry the kernel records
 // TMW_ERR_DEVICE_TIMEOUT in the device status word, stops waiting anywhere and runs
@@ -210,7 +210,12 @@ enum BarSlot {
 
 // GENERAL = false: the plain windowed mask (per-token);
 // GENERAL = true: block-granular window, read from the parameters.
-template <int DH, bool BF16, bool GENERAL>
+// STRAIGHT: key tiles that every row sees in full have a body of their own without mask and chunk tests, one run of
+// instructions (head_dim 128; at head_dim 64 the 96 registers of a softmax thread do not hold it).  It pays where most tiles of
+// a window are such: 8 heads x 30 000 rows, us, windows 200 | 300 | 400 | 512 | 640 | 1024 | 2048: 84.7 | 94.2 | 110.5 | 121.0 |
+// 136.4 | 183.5 | 307.6 without and 86.7 | 96.6 | 110.8 | 119.8 | 134.1 | 178.2 | 296.0 with it.
+constexpr int kStraightFrom = 512;  // window
+template <int DH, bool BF16, bool GENERAL, bool STRAIGHT>
 __global__ void __launch_bounds__(kTcThreads, Budget<DH>::kCtasPerSm)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -432,7 +437,65 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         float m_used = -INFINITY;  // maximum the stored P and O are relative to (log2 domain)
         float l_sum = 0.f;
 
+        // window tiles that every row of the query tile sees in full: items [full0, full1)
+        int full0 = 0, full1 = 0;
+        if (STRAIGHT && q.p_lo >= p.np) {
+            const int lo = max(p.np, first_visible_pos(q.p_lo + BM - 1, p.np, p.window, wblock)) - q.anchor;
+            full0 = max(1, q.n_pers + max(0, (lo + BN - 1) / BN - q.a));
+            full1 = min(q.n_items, q.n_pers + floor_div(q.p_lo + 1 - q.anchor, BN) - q.a);
+        }
+
         for (int item = 0; item < q.n_items; ++item) {
+            if (STRAIGHT && item >= full0 && item < full1) {
+                const int buf = SB == 2 ? (item & 1) : 0;
+                const uint32_t s_addr = s_base + buf * BN;
+                mbar_wait(bar(BAR_S_FULL + buf), (SB == 2 ? item >> 1 : item) & 1, abort_flag, p.status);
+                tc_fence_after();
+                const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+                const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), negm2 = pack2(neg_m, neg_m);
+                uint64_t lacc[2] = {0ull, 0ull};
+                uint32_t s[NCH][32];
+#pragma unroll
+                for (int c = 0; c < NCH; ++c) tmem_ld32(s_addr + c * 32, s[c]);
+                tc_wait_ld();
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int c = 0; c < NCH; ++c)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) mx[i & 3] = max3(mx[i & 3], __uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1]));
+                const float tile_max = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]) * p.scale_log2;
+                if (!__any_sync(0xffffffffu, tile_max > m_used + 8.0f)) {  // (otherwise the general body does it all over again)
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) {
+                        uint32_t packed[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float s0 = __uint_as_float(s[c][2 * i]), s1 = __uint_as_float(s[c][2 * i + 1]);
+                            float x0, x1;
+                        unpack2(fma2(pack2(s0, s1), scale2, negm2), x0, x1);
+                        const float e0 = fast_exp2(x0), e1 = fast_exp2(x1);
+                        lacc[i & 1] = add2(lacc[i & 1], pack2(e0, e1));
+                        if (BF16) {
+                            const __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
+                            packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+                        } else {
+                            const __half2 h = __floats2half2_rn(e0, e1);
+                            packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+                        }
+                        }
+                        tmem_st16(s_addr + c * 16, packed);
+                    }
+                    float a0, a1, a2, a3;
+                    unpack2(lacc[0], a0, a1);
+                    unpack2(lacc[1], a2, a3);
+                    l_sum += (a0 + a1) + (a2 + a3);
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(BAR_P_READY + buf));
+                    continue;
+                }
+            }
             // visible columns of this row inside the tile: [j_lo, j_hi]
             int j_lo, j_hi, ncols;
             bool full;
@@ -690,19 +753,19 @@ int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const voi
     if (p.status == nullptr) return TMW_ERR_CUDA;
     const int smem_bytes = L::total_bytes(np_pad);
     dim3 grid((d.q_rows + BM - 1) / BM, d.heads, d.batch);
-    const bool general = window_block > 0;
     auto run = [&](auto kern) -> int {
         const int rc = allow_shared_memory(reinterpret_cast<const void*>(kern), smem_bytes);
         if (rc != TMW_OK) return rc;
         TMW_CUDA_TRY(launch_ex(kern, grid, dim3(kTcThreads), smem_bytes, stream, chain & kChainDependent, 1, mq, mk, mv, mo, mkp, mvp, p));
         return TMW_OK;
     };
-    int st;
-    if (d.dtype == TMW_BF16)
-        st = general ? run(prefill_tc_kernel<DH, true, true>) : run(prefill_tc_kernel<DH, true, false>);
-    else
-        st = general ? run(prefill_tc_kernel<DH, false, true>) : run(prefill_tc_kernel<DH, false, false>);
-    return st;
+    auto pick = [&](auto bf16, auto general) -> int {
+        constexpr bool BF16 = decltype(bf16)::value, GENERAL = decltype(general)::value;
+        if (DH == 128 && d.window >= kStraightFrom) return run(prefill_tc_kernel<DH, BF16, GENERAL, DH == 128>);
+        return run(prefill_tc_kernel<DH, BF16, GENERAL, false>);
+    };
+    if (d.dtype == TMW_BF16) return window_block > 0 ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
+    return window_block > 0 ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{});
 }
 
 constexpr int kMaxDynamicSmem = 232448;  // 227 KB per CTA on sm_100
