@@ -189,7 +189,7 @@ int attention(const tmw_attention_desc& a, const void* x, const void* w_qkv, con
     int rc = linear(a.dtype, rows, 3 * D, D, x, w_qkv, nullptr, qkv, TMW_EPILOGUE_NONE, stream,
                     first ? kChainFollowed : kChainLink);
     if (rc == TMW_OK && a.conv_taps > 0) {
-        rc = launch_dwconv(a.dtype, a.batch, a.rows, 3 * D, a.conv_taps, qkv, conv, 3, conv_out, stream);
+        rc = launch_dwconv(a.dtype, a.batch, a.rows, 3 * D, a.conv_taps, qkv, conv, 3, conv_out, stream, true);
         qkv = conv_out;
     }
     bool dependent = false;

@@ -333,7 +333,7 @@ int launch_add_rmsnorm(int dtype, long long rows, int dim, const void* x, const 
                        void* sum_out, void* y, cudaStream_t stream, bool pdl = false);
 // w: the filters of channels [0, c/n), [c/n, 2c/n), ... in n arrays [c/n, taps]
 int launch_dwconv(int dtype, int batch, int rows, int channels, int taps, const void* x, const void* const* w, int n_w, void* y,
-                  cudaStream_t stream);
+                  cudaStream_t stream, bool pdl = false);
 // links of a chain of dependent launches (see pdl_wait): a product of up to a few hundred rows (epi: 0 = store, 1 = GELU,
 // 2 = added to c, which is read and written; n and k multiples of 8, contiguous rows), and the RMSNorm in front of it
 int launch_rows_tc(int dtype, int m, int n, int k, const void* a, const void* w, const void* bias, void* c, int epi,

@@ -123,7 +123,7 @@ int attention_forward(const Dims& d, const void* x, const AttentionWeights& w, c
                       int first, cudaStream_t s) {
     const int R = d.rows(), D = d.D;
     int rc = product(d, R, 3 * D, D, x, w.w_qkv, nullptr, a.qkv, GEMM_NONE, nullptr, first ? kChainFollowed : kChainLink, s);
-    if (rc == TMW_OK && d.taps > 0) rc = launch_dwconv(d.dtype, d.B, d.L, 3 * D, d.taps, a.qkv, w.conv, 3, a.conv, s);
+    if (rc == TMW_OK && d.taps > 0) rc = launch_dwconv(d.dtype, d.B, d.L, 3 * D, d.taps, a.qkv, w.conv, 3, a.conv, s, true);
     if (rc != TMW_OK) return rc;
     const tmw_prefill_desc c = core_desc(d);
     const char *q = a.conv, *k = q + 2ll * D, *v = q + 4ll * D;
