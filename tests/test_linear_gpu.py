@@ -56,6 +56,12 @@ def test_column_tiles_narrower_than_256(m, n, k):
     run_case(m, n, k, False, True, dtype=torch.float16, seed=n)
 
 
+@pytest.mark.parametrize("m,n,k", [(12544, 4096, 64), (12545, 4104, 72), (2300, 4360, 4096), (2048, 4096, 8200)])
+def test_wide_outputs_in_groups_of_row_bands(m, n, k):
+    """Sixteen column tiles and more: 49 and 50 bands in groups of 48, 9 in one of 16, 8 of the least size."""
+    run_case(m, n, k, False, False, seed=m + n)
+
+
 def test_fp16_and_strided_input():
     run_case(200, 320, 128, True, True, dtype=torch.float16)
     g = torch.Generator(device=DEV).manual_seed(9)

@@ -60,6 +60,7 @@ struct GemmParams {
     float* partial;      // k cut into `splits` ranges: their fp32 sums go to [splits][m][n] here instead of to the output
     int splits;
     int width;           // pair kernel: columns of a tile (a multiple of 32)
+    int group;           // pair kernel: row bands that a wide output is walked in (group_bands)
     void* c;             // the output, rows of ldc elements
     long long ldc;
     int wide;            // rows of c and aux start on 32-byte boundaries
@@ -375,9 +376,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // loads; "empty" and "accumulator full" are arrived on in both CTAs by one commit; "accumulator empty" lives in
 // the first CTA and collects the epilogue warps of both.
 // ---------------------------------------------------------------------------------
-// Wide outputs are walked in groups of kGroup row bands, column by column: the tiles in flight then share few rows of W as well
-// as of A (a vocabulary's W is read m / 256 times otherwise, and does not stay in the near half of L2).
-constexpr int kGroup = 8, kGroupFrom = 16;
+// Outputs of kGroupFrom or more column tiles are walked in groups of row bands, column by column: the tiles in flight then share
+// few rows of W as well as of A.  W is read once per group, so a group is as large as its rows of A stay in L2 beside the rest:
+// 32 MiB of them, from 8 up to 48 bands (of 256 rows).  us with groups of 8 | 16 | 24 | 32 | 48 | 128: 16416 x 50000 x 640
+// 777 | 762 | 755 | 755 | 753 | 754; 32896 x 50000 x 640 1583 | 1550 | 1538 | 1535 | 1533 | 1632; 16384^2 x 4096
+// 1385 | 1350 | 1373 | 1447 | 1534 | 1650; 8192^3 695 | 698 | 713 | 740 | 739 | 738.
+constexpr int kGroupFrom = 16;
+int group_bands(int k) {
+    const int bands = (32 << 20) / (2 * GM * 2) / k;
+    return bands < 8 ? 8 : bands > 48 ? 48 : bands;
+}
 
 // Shared memory of the pair kernel is a ring of as many stages as fit at the tile's width (256 columns: 7, 160: 8).  The bytes
 // in flight are what the rate hangs on: 16416 x 50000 x 640 takes 976 | 875 | 847 | 823 us with 3 | 4 | 5 | 6 stages.
@@ -420,7 +428,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             band = mn / n_tiles;
             col = (mn % n_tiles) * p.width;
         } else {
-            const int first = mn / (kGroup * n_tiles) * kGroup, r = mn - first * n_tiles, bands = min(kGroup, m_tiles - first);
+            const int first = mn / (p.group * n_tiles) * p.group, r = mn - first * n_tiles, bands = min(p.group, m_tiles - first);
             band = first + r % bands;
             col = r / bands * p.width;
         }
@@ -655,6 +663,7 @@ int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
     if (!make_maps(g, width / 2, &ma, &mb)) return TMW_ERR_CUDA;
     if (const int rc = gemm_params(g, &p); rc != TMW_OK) return rc;
     p.width = width;
+    p.group = group_bands(g.k);
     const int tiles = ((g.m + 2 * GM - 1) / (2 * GM)) * ((g.n + width - 1) / width) * g.splits;
     auto run = [&](auto kern) -> int {
         const void* fn = reinterpret_cast<const void*>(kern);
