@@ -550,7 +550,7 @@ int clear_counters(const tmw_stack_desc& d, char* ws, cudaStream_t stream) {
     return TMW_OK;
 }
 
-// `followed`: kChainFollowed if a dependent launch reads the logits (the tcgen05 product stores them through TMA), else 0
+// `followed`: kChainFollowed if a dependent launch reads the logits, else 0
 template <typename T>
 int decode_step_t(const tmw_stack_desc& d, const tmw_block* blocks, const int64_t* ids, const int32_t* pos, void* logits,
                   char* ws, int followed, cudaStream_t stream) {
