@@ -1,6 +1,8 @@
 """The training step as two library calls (``tmw_stack_train_*``, ``tmw_cross_entropy``) and the one-call forwards against the
 same computation module by module."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -134,3 +136,36 @@ def test_only_the_gradients_that_are_wanted(block_sparse, wanted, monkeypatch):
         assert (got[name] is None) == (name not in wanted)
         # (a filter's gradient is added up with atomics: the order of its fp32 sums is not fixed)
         assert name not in wanted or (close(got[name], want[name], 1e-2) if "conv" in name else torch.equal(got[name], want[name])), name
+
+
+@pytest.mark.parametrize("rows,taps", [(6000, 0), (6001, 4)])
+def test_scratch_aligned_to_16_bytes(rows, taps):
+    """Scratch and saved activations need 16 bytes of alignment, no more: the weights' gradients (k = rows, cut into ranges whose fp32
+    sums lie in the scratch) are bit for bit what they are with scratch on a 256-byte boundary, and nothing beyond it is touched."""
+    lib, D = _native.lib(), 128
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    desc = _native.AttentionDesc(_native.TMW_BF16, 1, rows, 2, 64, 40, 5, 32 if taps else 0, taps, 0.0)
+    x, dy = (torch.randn(rows, D, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    w_qkv, w_out = ((torch.randn(n, D, generator=g, device=DEV) * 0.1).to(torch.bfloat16) for n in (3 * D, D))
+    conv = [(torch.randn(D, taps, generator=g, device=DEV) * 0.5).to(torch.bfloat16) for _ in range(3 if taps else 0)]
+    convs = [c.data_ptr() for c in conv] or [None] * 3
+    ref, stream = ctypes.byref(desc), _native._stream_ptr(torch.device(DEV))
+    n_saved, n_scratch = lib.tmw_attention_train_saved(ref), lib.tmw_attention_train_scratch(ref)
+
+    def run(shift):
+        room = torch.full((n_scratch + 512,), 77, dtype=torch.uint8, device=DEV)
+        saved = torch.empty(n_saved + 512, dtype=torch.uint8, device=DEV)
+        y, dx = torch.empty_like(x), torch.empty_like(x)
+        out = [torch.empty_like(w) for w in (w_qkv, w_out)]
+        grads = _native.BlockGrads(w_qkv=out[0].data_ptr(), w_out=out[1].data_ptr())
+        _native.check(lib.tmw_attention_train_forward(ref, x.data_ptr(), w_qkv.data_ptr(), *convs, w_out.data_ptr(), y.data_ptr(),
+                                                      saved.data_ptr() + shift, n_saved, stream))
+        _native.check(lib.tmw_attention_train_backward(ref, x.data_ptr(), w_qkv.data_ptr(), *convs, w_out.data_ptr(), dy.data_ptr(),
+                                                       saved.data_ptr() + shift, dx.data_ptr(), ctypes.byref(grads),
+                                                       room.data_ptr() + shift, n_scratch, stream))
+        _native.poll_status(torch.device(DEV))
+        assert (room[:shift] == 77).all() and (room[shift + n_scratch:] == 77).all()
+        return y, dx, *out
+
+    for got, want in zip(run(16), run(0)):
+        assert torch.equal(got, want)

@@ -63,7 +63,7 @@ struct GemmParams {
     int group;           // pair kernel: row bands that a wide output is walked in (group_bands)
     void* c;             // the output, rows of ldc elements
     long long ldc;
-    int wide;            // rows of c and aux start on 32-byte boundaries
+    int wide;            // rows of what is written (c, or the fp32 sums) and of aux start on 32-byte boundaries
     int* status;
 };
 
@@ -172,17 +172,24 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
     for (int j = 0; j < 32; j += 16) store16(out, col + j, p.n - col - j, p.wide, pack8<BF16>(v + j), pack8<BF16>(v + j + 8));
 }
 
-// the fp32 sums of a k range, whole sectors too (n is a multiple of 8, `partial` aligned)
+// the fp32 sums of a k range: whole sectors where `partial` lies on one (n is a multiple of 8), halves where the caller's scratch is
+// aligned to 16 bytes only
 __device__ __forceinline__ void store_partial(const uint32_t (&v)[32], const GemmParams& p, int split, int row, int col) {
     if (row >= p.m) return;
     float* dst = p.partial + ((long long)split * p.m + row) * p.n + col;
 #pragma unroll
-    for (int j = 0; j < 32; j += 8)
-        if (col + j < p.n)
+    for (int j = 0; j < 32; j += 8) {
+        if (col + j >= p.n) continue;
+        if (p.wide) {
             asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                          ::"l"(dst + j), "r"(v[j]), "r"(v[j + 1]), "r"(v[j + 2]), "r"(v[j + 3]), "r"(v[j + 4]), "r"(v[j + 5]),
                            "r"(v[j + 6]), "r"(v[j + 7])
                          : "memory");
+        } else {
+            *reinterpret_cast<uint4*>(dst + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            *reinterpret_cast<uint4*>(dst + j + 4) = make_uint4(v[j + 4], v[j + 5], v[j + 6], v[j + 7]);
+        }
+    }
 }
 
 // A warp's panels (first, first + step, ...) of a finished tile: tensor memory -> global memory.  No warp waits for another.
@@ -583,7 +590,7 @@ int gemm_params(const GemmCall& g, GemmParams* p) {
     p->c = g.c;
     p->ldc = g.ldc;
     auto on32 = [](const void* q, int64_t ld) { return (reinterpret_cast<uintptr_t>(q) & 31u) == 0 && ld % 16 == 0; };
-    p->wide = on32(g.c, g.ldc) && (g.aux == nullptr || on32(g.aux, g.n));
+    p->wide = p->partial != nullptr ? on32(p->partial, 16) : on32(g.c, g.ldc) && (g.aux == nullptr || on32(g.aux, g.n));
     p->status = device_status_word();
     if (p->status == nullptr) return TMW_ERR_CUDA;
     auto on16 = [](const void* q, int64_t ld) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0 && ld % 8 == 0; };
