@@ -169,3 +169,45 @@ def test_scratch_aligned_to_16_bytes(rows, taps):
 
     for got, want in zip(run(16), run(0)):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("B,T,d_ff", [
+    (1, 40, 256),        # 5 partial rows of the norms, 1 of fc1's bias: one chain each
+    (1, 1023, 4096), (1, 1023, 4104),  # 128 partial rows; 16 strips of fc1's bias
+    (2, 604, 4096), (2, 604, 4104),    # 151; 19 strips, either side of the columns that share out the threads differently
+    (8, 1024, 128),      # 296; weight gradients cut into more than 16 ranges
+])
+def test_sums_of_partial_results(B, T, d_ff):
+    """Every row of the batch is the same token at the same (zero) position, so each sum over the rows is their number times the
+    gradient of one row: a part that is missing or counted twice shows.  Tolerance: a part is at least 1/296 of a sum; one rounding
+    to fp16 of each of a gradient's factors, on average over the elements, is below 2^-11."""
+    heads, vocab = 2, 64
+    cfg = TitanMACConfig(vocab_size=vocab, d_model=64 * heads, n_heads=heads, n_layers=1, d_ff=d_ff, max_seq_len=1024, window_size=16,
+                         n_persistent=0, use_block_sparse=False)
+    g = torch.Generator(device=DEV).manual_seed(d_ff)
+    with torch.device(DEV):
+        model = TitanMAC(cfg)
+    with torch.no_grad():
+        for name, prm in model.named_parameters():
+            prm.normal_(1.0 if name.endswith("scale") else 0.0, 0.1 if name.endswith(("scale", "bias")) else 0.04, generator=g)
+            if "pos" in name:
+                prm.zero_()
+    model = model.half()
+    d_row = torch.randn(vocab, generator=g, device=DEV)
+
+    def grads(B, T, scale):
+        model.zero_grad(set_to_none=True)
+        with torch.enable_grad():
+            logits = model(torch.full((B, T), 7, device=DEV))["logits"]
+        assert "_StackTrain" in type(logits.grad_fn).__name__
+        logits.backward((d_row * scale).half().expand(B, T, vocab))
+        _native.poll_status(torch.device(DEV))
+        return {n: p.grad.float() / scale for n, p in model.named_parameters()}
+
+    one, many = grads(1, 1, 1.0), grads(B, T, 2.0 ** -4)
+    checked = [n for n in one if "embed" not in n and "attention" not in n and "norm_attn" not in n]
+    assert len(checked) >= 5
+    for name in checked:
+        want = one[name] * (B * T)
+        if want.norm() > 0:
+            assert ((many[name] - want).norm() / want.norm()).item() <= 2 ** -10, name

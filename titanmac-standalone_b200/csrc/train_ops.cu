@@ -154,46 +154,78 @@ __global__ void __launch_bounds__(256) colsum_kernel(const void* src, float* par
     }
 }
 
-// dst[j] = round(sum over parts of src[part][j]) for several arrays at once (blockIdx.y).  Few parts (split products): a thread
-// per group of four columns.  Many parts (column sums): eight groups x 32 threads per group, so that a thread's chain of loads
-// is short - 296 parts of 640 columns are a matter of latency, 14 us with eight threads per group and 5.6 with 32.
-constexpr int kManyParts = 16, kManyGroups = 8, kManyLanes = 32;
+// dst[j] = round(sum over parts of src[part][j]) for several arrays at once (blockIdx.y).  Up to kManyParts parts (split products): a
+// thread per group of four columns, one chain.  More: eight chains (parts sub, sub + 8, ...), then their sums in the order of sub,
+// whatever the threads are shared out to: 32 groups x 8 threads where the columns fill the chip (weight gradients cut into 17 to
+// 32 ranges), and where they do not - column sums, 296 parts of 640 columns are a matter of latency - 8 groups x 32 threads
+// that bring 128 parts at a time into shared memory for the eight chains.  us, cold caches (back to back), 32 x 8 | 8 x 32: 296 parts
+// of 640 columns 16.4 (6.2) | 9.2 (3.4), 64 of 2560 9.2 (2.8) | 6.2 (2.4); 24 of 400 000 14.4 (5.8) | 28.7 (15.7).
+constexpr int kManyParts = 16, kWide = 32, kNarrow = 8, kChunk = 128;
+constexpr long long kNarrowColumns = 4096;  // (a CTA per 32 of them is less than one per SM)
+__host__ __device__ inline int sum_groups(const SumParts::Item& it) {
+    return it.parts <= kManyParts ? 256 : it.n <= kNarrowColumns ? kNarrow : kWide;
+}
+
+__device__ __forceinline__ void add4(float4& t, const float4& v) { t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
+template <typename T>
+__device__ __forceinline__ void store_sum(const SumParts::Item& it, long long g, const float4& t) {
+    T o[4] = {from_f32<T>(t.x), from_f32<T>(t.y), from_f32<T>(t.z), from_f32<T>(t.w)};
+    *reinterpret_cast<uint2*>(static_cast<T*>(it.dst) + g * 4) = *reinterpret_cast<const uint2*>(o);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const SumParts p) {
-    __shared__ float4 s[kManyLanes][kManyGroups];
+    __shared__ float4 s[kChunk * kNarrow];
     pdl_trigger();
     pdl_wait();
     const SumParts::Item it = p.item[blockIdx.y];
-    const bool many = it.parts > kManyParts;
     const long long groups = (it.n + 3) / 4;
-    const int lanes = many ? kManyGroups : 256, at = many ? threadIdx.x % kManyGroups : threadIdx.x;
-    const int sub = many ? threadIdx.x / kManyGroups : 0, step = many ? kManyLanes : 1;
+    if (sum_groups(it) == kNarrow) {
+        const int at = threadIdx.x % kNarrow, sub = threadIdx.x / kNarrow;
+        for (long long g0 = (long long)blockIdx.x * kNarrow; g0 < groups; g0 += (long long)gridDim.x * kNarrow) {
+            const bool mine = g0 + at < groups;
+            const float* src = it.src + (g0 + at) * 4;
+            float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q0 = 0; q0 < it.parts; q0 += kChunk) {
+                const int n = min(kChunk, it.parts - q0);
+                if (mine)
+                    for (int q = sub; q < n; q += 256 / kNarrow)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                     ::"r"((uint32_t)__cvta_generic_to_shared(s + q * kNarrow + at)), "l"(src + (q0 + q) * it.n) : "memory");
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncthreads();
+                if (mine && sub < 8)
+                    for (int q = sub; q < n; q += 8) add4(t, s[q * kNarrow + at]);
+                __syncthreads();
+            }
+            if (sub < 8) s[sub * kNarrow + at] = t;
+            __syncthreads();
+            if (mine && sub == 0) {
+                for (int q = 1; q < 8; ++q) add4(t, s[q * kNarrow + at]);
+                store_sum<T>(it, g0 + at, t);
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    const bool many = it.parts > kManyParts;
+    const int lanes = many ? kWide : 256, sub = many ? threadIdx.x >> 5 : 0, step = many ? 8 : 1;
     for (long long g0 = (long long)blockIdx.x * lanes; g0 < groups; g0 += (long long)gridDim.x * lanes) {
-        const long long g = g0 + at;
+        const long long g = g0 + (many ? threadIdx.x & 31 : threadIdx.x);
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
         if (g < groups) {
-#pragma unroll 8
-            for (int q = sub; q < it.parts; q += step) {
-                const float4 v = *reinterpret_cast<const float4*>(it.src + (long long)q * it.n + g * 4);
-                t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
-            }
+#pragma unroll 4
+            for (int q = sub; q < it.parts; q += step) add4(t, *reinterpret_cast<const float4*>(it.src + (long long)q * it.n + g * 4));
         }
         if (many) {
-            s[sub][at] = t;
+            s[sub * kWide + (threadIdx.x & 31)] = t;
             __syncthreads();
             if (sub == 0) {
-#pragma unroll
-                for (int q = 1; q < kManyLanes; ++q) {
-                    const float4 v = s[q][at];
-                    t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
-                }
+                for (int q = 1; q < 8; ++q) add4(t, s[q * kWide + threadIdx.x]);
             }
             __syncthreads();
         }
-        if (g < groups && sub == 0) {
-            T o[4] = {from_f32<T>(t.x), from_f32<T>(t.y), from_f32<T>(t.z), from_f32<T>(t.w)};
-            *reinterpret_cast<uint2*>(static_cast<T*>(it.dst) + g * 4) = *reinterpret_cast<const uint2*>(o);
-        }
+        if (g < groups && sub == 0) store_sum<T>(it, g, t);
     }
 }
 
@@ -461,7 +493,7 @@ int launch_sum_parts(int dtype, const SumParts& p, cudaStream_t stream) {
     if (p.count == 0) return TMW_OK;
     long long most = 1;
     for (int i = 0; i < p.count; ++i) {
-        const long long lanes = p.item[i].parts > kManyParts ? kManyGroups : 256, blocks = ((p.item[i].n + 3) / 4 + lanes - 1) / lanes;
+        const long long lanes = sum_groups(p.item[i]), blocks = ((p.item[i].n + 3) / 4 + lanes - 1) / lanes;
         most = blocks > most ? blocks : most;
     }
     const dim3 grid((unsigned)(most < 8 * sm_count() ? most : 8 * sm_count()), p.count), block(256);
