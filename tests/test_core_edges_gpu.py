@@ -45,6 +45,21 @@ def test_block_sparse_core_with_persistent_rows(dtype, tol, dh, L, w, block, n_p
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_persistent_rows_of_many_sequences(dtype):
+    """The two bodies at head_dim 64: K of the next block ahead while all CTAs (here four to a pair) fit the chip three to an SM, not
+    ahead with one pair more.  The sums are the same, so a sequence's rows are, bit for bit; one of them against the oracle, tolerance
+    as above."""
+    most = 3 * torch.cuda.get_device_properties(0).multi_processor_count // 4
+    q, k, v = (t.to(dtype) for t in wo.qkv_inputs(most + 1, 1, 520, 64, seed=3))
+    many = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), 40, 16, window_block=32)
+    few = _native.prefill(q[:most].to(DEV), k[:most].to(DEV), v[:most].to(DEV), 40, 16, window_block=32)
+    _native.poll_status()
+    assert torch.equal(many[:most], few)
+    ref = bo.attention_core(q[-1:].float(), k[-1:].float(), v[-1:].float(), 40, 32, 16)
+    assert (many[-1:].float().cpu() - ref).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("L,w,n_p,block", [
     (700, 511, 16, 0), (700, 512, 16, 0),     # either side of the rule: the general body alone, whole tiles on their own
     (641, 512, 0, 0), (1100, 513, 128, 0),    # no persistent keys: the first tile sets the maximum; a ragged left edge
