@@ -45,6 +45,7 @@ def close(got, want, tol):
     (4, 1024, torch.float16, 5, 128, 100, 16, 2048, False),  # d_model 640: column tiles narrower than 256
     (5, 1000, torch.bfloat16, 8, 64, 40, 8, 512, False),     # norms of 512 columns, three rows to a warp
     (5, 1000, torch.bfloat16, 8, 128, 40, 8, 512, False),    # 1024 columns
+    (5, 1000, torch.float16, 14, 64, 40, 8, 512, False),     # 896
     (2, 150, torch.float16, 16, 128, 40, 4, 512, False),     # 2048 columns, the widest
 ])
 def test_training_step_equals_module_by_module(B, T, dtype, heads, dh, window, Np, vocab, block_sparse, monkeypatch):

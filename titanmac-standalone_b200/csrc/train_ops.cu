@@ -18,8 +18,11 @@ constexpr int kNormWarps = 8;
 // first row's latency and the tail; 8320 rows of 640 (32 MB in, 11 MB out: 6.5 us), cold caches, us: 21.1 -> 15.2 with both sums,
 // 17.6 -> 14.6 with dgain alone, since the warps' sums are added up side by side and not one warp after the other, and the
 // next row loads under a row.
+// Two CTAs to an SM, as many as are launched, up to 768 columns, and up to 1024 without the second sum (32896 rows of 1024, us:
+// 49.8, with one 66.9).  With both sums 1024 columns take 179 registers; at 128 they spill (fp16, 8320 rows: 23.4 against 20.4).
+constexpr bool norm_two_ctas(int nv, bool sums) { return nv <= (sums ? 3 : 4); }
 template <typename T, int NV, bool SUMS>
-__global__ void __launch_bounds__(kNormWarps * 32, NV <= 3 ? 2 : 1) rmsnorm_bwd_kernel(const NormBwd p) {
+__global__ void __launch_bounds__(kNormWarps * 32, norm_two_ctas(NV, SUMS) ? 2 : 1) rmsnorm_bwd_kernel(const NormBwd p) {
     extern __shared__ float sums[];  // [dgain | sum of out][warp][dim]
     pdl_trigger();
     pdl_wait();
@@ -33,7 +36,8 @@ __global__ void __launch_bounds__(kNormWarps * 32, NV <= 3 ? 2 : 1) rmsnorm_bwd_
             if (SUMS) os[j][e] = 0.f;
         }
     const long long warps = (long long)gridDim.x * kNormWarps;
-    // the next row loads under this one, where the registers hold two rows beside the sums at two CTAs per SM
+    // the next row loads under this one, where two rows beside the sums come close to 128 registers (of a thread's, 16 bytes spill at
+    // 520 to 768 columns without the second sum; the bound itself spills 56 there in fp16 with it and 16 up to 1024 without)
     constexpr bool AHEAD = NV <= 2 || (NV == 3 && !SUMS);
     Vec8<T> xv[NV], dv[NV], av[NV];
     auto fetch = [&](long long row) {
