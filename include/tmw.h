@@ -397,7 +397,8 @@ TMW_API int tmw_stack_forward(const tmw_stack_desc* desc, const tmw_block* block
  * *_train_saved call gives, to be handed on unchanged), and backward.  Replaces what autograd records and replays through
  * WindowedAttention / BlockSparseAttention (see tmw_prefill_backward) and, for the whole model, through
  * titans_core/models/titanmac.py:554-662 with its blocks.  `scratch` is used until the call's kernels have finished.
- * Gradients are written (not added to); the bias and convolution entries are NULL where the model has none.  For the
+ * Gradients are written (not added to); the bias and convolution entries are NULL where the model has none; every
+ * other array of the whole model's gradients is needed, on a 16-byte boundary (norms, biases, filters: 8).  For the
  * module alone dx and every entry may be NULL: what is not wanted is not computed.  d_model at most 2048 for the whole
  * model, otherwise the limits of tmw_stack_forward.
  */

@@ -182,3 +182,38 @@ def test_scratch_of_a_training_step_follows_its_size():
         assert activations <= nbytes <= 4 * activations + (1 << 20)
         nbytes, activations = size(100000, 1024)
         assert activations + (8 << 20) <= nbytes <= 4 * activations + (200 << 20)
+
+
+def test_training_backward_checks_where_gradients_go_on_the_host():
+    """A missing or misaligned gradient is refused before anything is launched: products write 16 bytes at a time, sums of partial
+    results 8.  Optional entries (biases, filters) may be NULL."""
+    lib, tokens = _native.lib(), 64
+    ok = 0x1000  # never dereferenced: validation fails first
+    d = _native.StackDesc(dtype=_native.TMW_BF16, batch=1, layers=2, d_model=128, heads=2, head_dim=64, d_ff=256, window=16,
+                          n_persistent=4, vocab=512, max_positions=tokens, block_size=16, conv_taps=4, eps=1e-5,
+                          embed_tokens=ok, embed_positions=ok, persistent=ok, norm=ok, head=ok)
+    nbytes = lib.tmw_stack_train_scratch(ctypes.byref(d), tokens)
+    blocks = (_native.Block * 2)()
+    for b in blocks:
+        b.norm_attn = b.w_qkv = b.w_out = b.norm_mlp = b.w_fc1 = b.w_fc2 = b.conv_q = b.conv_k = b.conv_v = ok
+
+    def refused(layer=None, name=None, at=None, saved=ok):
+        grads, block_grads = _native.StackGrads(*[ok] * 5), (_native.BlockGrads * 2)()
+        for g in block_grads:
+            g.norm_attn = g.w_qkv = g.w_out = g.norm_mlp = g.w_fc1 = g.w_fc2 = ok
+        if name is not None:
+            setattr(grads if layer is None else block_grads[layer], name, at)
+        return lib.tmw_stack_train_backward(ctypes.byref(d), blocks, ctypes.byref(grads), block_grads, ok, tokens, ok, saved, ok, nbytes,
+                                            None) == _native.TMW_ERR_INVALID_ARGUMENT
+
+    for name in ("embed_tokens", "head", "embed_positions", "persistent"):
+        assert refused(None, name, None) and refused(None, name, ok + 8), name
+    assert refused(None, "norm", None) and refused(None, "norm", ok + 4)
+    for layer in range(2):
+        for name in ("w_qkv", "w_out", "w_fc1", "w_fc2"):
+            assert refused(layer, name, None) and refused(layer, name, ok + 8), name
+        for name in ("norm_attn", "norm_mlp"):
+            assert refused(layer, name, None) and refused(layer, name, ok + 4), name
+        for name in ("b_fc1", "b_fc2", "conv_q", "conv_k", "conv_v"):
+            assert refused(layer, name, ok + 4), name
+    assert refused(saved=ok + 8)

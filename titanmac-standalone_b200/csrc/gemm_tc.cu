@@ -594,7 +594,7 @@ int gemm_params(const GemmCall& g, GemmParams* p) {
     p->status = device_status_word();
     if (p->status == nullptr) return TMW_ERR_CUDA;
     auto on16 = [](const void* q, int64_t ld) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0 && ld % 8 == 0; };
-    if (!on16(g.c, g.ldc) || (g.aux != nullptr && !on16(g.aux, g.n))) {
+    if (g.c == nullptr || !on16(g.c, g.ldc) || (g.aux != nullptr && !on16(g.aux, g.n))) {
         set_error_text("product: rows of the output and of what the epilogue reads must start on 16-byte boundaries");
         return TMW_ERR_INVALID_ARGUMENT;
     }

@@ -332,6 +332,20 @@ extern "C" int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_bl
     const Dims d = dims_of(k, tokens);
     const StackScratch t = stack_scratch(d, k.vocab, tokens, static_cast<char*>(scratch));
     if (scratch_bytes < (size_t)t.total) return TMW_ERR_TOO_LARGE;
+    // Where gradients go, before anything is launched: products and the embedding's kernels write 16 bytes at a time, sums of
+    // partial results 8.
+    auto written = [](const void* q, uintptr_t bytes) { return q != nullptr && (reinterpret_cast<uintptr_t>(q) & (bytes - 1)) == 0; };
+    auto optional = [&](const void* q) { return q == nullptr || written(q, 8); };
+    bool ok = aligned16(saved) && written(grads->embed_tokens, 16) && written(grads->head, 16) && written(grads->embed_positions, 16) &&
+              (k.n_persistent == 0 || written(grads->persistent, 16)) && written(grads->norm, 8);
+    for (int l = 0; l < k.layers && ok; ++l) {
+        const tmw_block_grads& q = block_grads[l];
+        for (const void* w : {q.w_qkv, q.w_out, q.w_fc1, q.w_fc2}) ok = ok && written(w, 16);
+        for (const void* n : {q.norm_attn, q.norm_mlp}) ok = ok && written(n, 8);
+        for (const void* o : {q.b_fc1, q.b_fc2}) ok = ok && optional(o);
+        for (const void* o : {q.conv_q, q.conv_k, q.conv_v}) ok = ok && (k.conv_taps == 0 || optional(o));
+    }
+    if (!ok) return TMW_ERR_INVALID_ARGUMENT;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int R = d.rows(), D = d.D, F = d.F, V = k.vocab;
     char* base = static_cast<char*>(const_cast<void*>(saved));
