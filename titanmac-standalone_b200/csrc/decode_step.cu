@@ -550,10 +550,9 @@ int clear_counters(const tmw_stack_desc& d, char* ws, cudaStream_t stream) {
     return TMW_OK;
 }
 
-// `followed`: kChainFollowed if a dependent launch reads the logits, else 0
 template <typename T>
 int decode_step_t(const tmw_stack_desc& d, const tmw_block* blocks, const int64_t* ids, const int32_t* pos, void* logits,
-                  char* ws, int followed, cudaStream_t stream) {
+                  char* ws, cudaStream_t stream) {
     const StepBuffers off = step_buffers(d);
     const int B = d.batch, D = d.d_model, F = d.d_ff;
     void *x = ws + off.x, *qkv = ws + off.qkv, *o = ws + off.o, *f = ws + off.f, *y = ws + off.y;
@@ -620,7 +619,7 @@ int decode_step_t(const tmw_stack_desc& d, const tmw_block* blocks, const int64_
     tmw_linear_desc ld = {};
     ld.dtype = d.dtype; ld.m = B; ld.n = d.vocab; ld.k = D; ld.epilogue = TMW_EPILOGUE_NONE;
     ld.lda = D; ld.ldw = D; ld.ldc = d.vocab;
-    return launch_linear(ld, y, d.head, nullptr, logits, stream, followed);
+    return launch_linear(ld, y, d.head, nullptr, logits, stream);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -684,8 +683,8 @@ extern "C" int tmw_decode_step(const tmw_stack_desc* desc, const tmw_block* bloc
     }
     rc = clear_counters(*desc, ws, s);
     if (rc != TMW_OK) return rc;
-    return desc->dtype == TMW_BF16 ? decode_step_t<__nv_bfloat16>(*desc, blocks, token_ids, pos, logits, ws, 0, s)
-                                   : decode_step_t<__half>(*desc, blocks, token_ids, pos, logits, ws, 0, s);
+    return desc->dtype == TMW_BF16 ? decode_step_t<__nv_bfloat16>(*desc, blocks, token_ids, pos, logits, ws, s)
+                                   : decode_step_t<__half>(*desc, blocks, token_ids, pos, logits, ws, s);
 }
 
 extern "C" int tmw_generate(const tmw_stack_desc* desc, const tmw_block* blocks, void* logits, int32_t tokens, int64_t* token_ids,
@@ -719,7 +718,7 @@ extern "C" int tmw_generate(const tmw_stack_desc* desc, const tmw_block* blocks,
         // what the step before has written)
         int st = launch_argmax<T>(d.batch, d.vocab, logits, token_ids, out, out_stride, pos, 0, false, s);
         for (int i = 1; i < tokens && st == TMW_OK; ++i) {
-            st = decode_step_t<T>(d, blocks, token_ids, pos, logits, ws, kChainFollowed, s);
+            st = decode_step_t<T>(d, blocks, token_ids, pos, logits, ws, s);
             if (st == TMW_OK) st = launch_argmax<T>(d.batch, d.vocab, logits, token_ids, out + i, out_stride, pos, 1, true, s);
         }
         return st;

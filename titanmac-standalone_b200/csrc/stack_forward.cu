@@ -181,20 +181,20 @@ AttentionBuffers attention_buffers(const tmw_attention_desc& a) {
     return b;
 }
 
-// x [rows, D] -> y [rows, D], or added to y (`onto`).  `first`: nothing of this chain is in front; `last`: nothing of it follows.  (Launching as
+// x [rows, D] -> y [rows, D], or added to y (`onto`).  `first`: nothing of this chain is in front.  (Launching as
 // dependents pays at every size: 2 x 8208 rows of 16 layers 5.96 -> 5.83 ms, 3000 rows of one layer 38.9 -> 32.8 us.)
 int attention(const tmw_attention_desc& a, const void* x, const void* w_qkv, const void* const* conv, const void* w_out,
-              void* qkv, void* conv_out, void* o, void* y, bool onto, bool first, bool last, cudaStream_t stream) {
+              void* qkv, void* conv_out, void* o, void* y, bool onto, bool first, cudaStream_t stream) {
     const int rows = a.batch * a.rows, D = a.heads * a.head_dim;
     int rc = linear(a.dtype, rows, 3 * D, D, x, w_qkv, nullptr, qkv, TMW_EPILOGUE_NONE, stream,
-                    first ? kChainFollowed : kChainLink);
+                    first ? 0 : kChainDependent);
     if (rc == TMW_OK && a.conv_taps > 0) {
         rc = launch_dwconv(a.dtype, a.batch, a.rows, 3 * D, a.conv_taps, qkv, conv, 3, conv_out, stream, true);
         qkv = conv_out;
     }
     bool dependent = false;
     if (rc == TMW_OK) rc = core(a, qkv, o, &dependent, stream);
-    const int link = (dependent ? kChainDependent : 0) | (last ? 0 : kChainFollowed);
+    const int link = dependent ? kChainDependent : 0;
     if (rc != TMW_OK) return rc;
     return onto ? linear_onto(a.dtype, rows, D, D, o, w_out, nullptr, y, stream, link)
                 : linear(a.dtype, rows, D, D, o, w_out, nullptr, y, TMW_EPILOGUE_NONE, stream, link);
@@ -270,7 +270,7 @@ extern "C" int tmw_attention_forward(const tmw_attention_desc* desc, const void*
     if (workspace_bytes < (size_t)off.total) return TMW_ERR_TOO_LARGE;
     char* ws = static_cast<char*>(workspace);
     return attention(*desc, x, w_qkv, conv, w_out, ws + off.qkv, ws + off.conv, ws + off.o, y,
-                     false, true, true, static_cast<cudaStream_t>(stream));
+                     false, true, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t tmw_stack_workspace(const tmw_stack_desc* desc, int32_t tokens) {
@@ -317,7 +317,7 @@ extern "C" int tmw_stack_forward(const tmw_stack_desc* desc, const tmw_block* bl
     for (int l = 0; l < d.layers && rc == TMW_OK; ++l) {
         const tmw_block& b = blocks[l];
         const void* conv[3] = {b.conv_q, b.conv_k, b.conv_v};
-        rc = attention(a, y, b.w_qkv, conv, b.w_out, big, ws + off.conv, o, x, true, false, false, s);
+        rc = attention(a, y, b.w_qkv, conv, b.w_out, big, ws + off.conv, o, x, true, false, s);
         if (rc == TMW_OK && b.k_ring != nullptr) {
             // keys and values of the sequence rows into the ring, those of the persistent rows (the same for every
             // sequence) beside it
@@ -333,8 +333,8 @@ extern "C" int tmw_stack_forward(const tmw_stack_desc* desc, const tmw_block* bl
                                    d.n_persistent > 0 ? v : nullptr, true);
         }
         if (rc == TMW_OK) rc = launch_add_rmsnorm(d.dtype, rows, D, x, nullptr, b.norm_mlp, d.eps, nullptr, y, s, true);
-        if (rc == TMW_OK) rc = linear(d.dtype, rows, F, D, y, b.w_fc1, b.b_fc1, big, TMW_EPILOGUE_GELU, s, kChainLink);
-        if (rc == TMW_OK) rc = linear_onto(d.dtype, rows, D, F, big, b.w_fc2, b.b_fc2, x, s, kChainLink);
+        if (rc == TMW_OK) rc = linear(d.dtype, rows, F, D, y, b.w_fc1, b.b_fc1, big, TMW_EPILOGUE_GELU, s, kChainDependent);
+        if (rc == TMW_OK) rc = linear_onto(d.dtype, rows, D, F, big, b.w_fc2, b.b_fc2, x, s, kChainDependent);
         if (rc == TMW_OK && (l + 1 < d.layers || !last_only))
             rc = launch_add_rmsnorm(d.dtype, rows, D, x, nullptr, l + 1 < d.layers ? blocks[l + 1].norm_attn : d.norm, d.eps, nullptr, y, s,
                                     true);

@@ -197,7 +197,8 @@ SideStream* side_stream_of_current_device();  // nullptr if it cannot be made
 // loads for invariant and moves them in front of pdl_wait().
 // A kernel that stores through TMA has to see its stores complete, not just read, before it ends if a dependent follows:
 // what it leaves in flight an ordinary launch waits for, pdl_wait() does not.
-enum : int { kChainDependent = 1, kChainFollowed = 2, kChainLink = 3 };  // a launch's place in a chain (0: none)
+// A launch's place in a chain (0: none).  Products store from registers: kChainFollowed matters to the attention core alone.
+enum : int { kChainDependent = 1, kChainFollowed = 2, kChainLink = 3 };
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

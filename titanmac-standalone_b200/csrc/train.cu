@@ -122,7 +122,7 @@ AttentionSaved attention_saved(const Dims& d, char* p) {
 int attention_forward(const Dims& d, const void* x, const AttentionWeights& w, const AttentionSaved& a, void* y, void* residual,
                       int first, cudaStream_t s) {
     const int R = d.rows(), D = d.D;
-    int rc = product(d, R, 3 * D, D, x, w.w_qkv, nullptr, a.qkv, GEMM_NONE, nullptr, first ? kChainFollowed : kChainLink, s);
+    int rc = product(d, R, 3 * D, D, x, w.w_qkv, nullptr, a.qkv, GEMM_NONE, nullptr, first ? 0 : kChainDependent, s);
     if (rc == TMW_OK && d.taps > 0) rc = launch_dwconv(d.dtype, d.B, d.L, 3 * D, d.taps, a.qkv, w.conv, 3, a.conv, s, true);
     if (rc != TMW_OK) return rc;
     const tmw_prefill_desc c = core_desc(d);
@@ -133,7 +133,7 @@ int attention_forward(const Dims& d, const void* x, const AttentionWeights& w, c
     else rc = tmw_prefill_lse(&c, q, k, v, a.o, a.lse, s);
     if (rc != TMW_OK) return rc;
     return product(d, R, D, D, a.o, w.w_out, nullptr, y, residual != nullptr ? GEMM_ADD : GEMM_NONE, residual,
-                   (link ? kChainDependent : 0) | kChainFollowed, s);
+                   link ? kChainDependent : 0, s);
 }
 
 struct AttentionScratch {
@@ -146,10 +146,10 @@ int attention_backward(const Dims& d, const void* x, const AttentionWeights& w, 
                        const AttentionGrads& g, const AttentionScratch& t, Pending& pending, bool first, cudaStream_t s) {
     const int R = d.rows(), D = d.D;
     const bool through = dx != nullptr || g.w_qkv != nullptr || g.conv[0] != nullptr || g.conv[1] != nullptr || g.conv[2] != nullptr;
-    const int link = first ? kChainFollowed : kChainLink;
+    const int link = first ? 0 : kChainDependent;
     int rc = TMW_OK;
     if (through) rc = input_grad(d, R, D, D, dy, w.w_out, t.d_o, GEMM_NONE, nullptr, link, s);
-    if (rc == TMW_OK && g.w_out != nullptr) rc = pending.weight_grad(d, R, D, D, dy, a.o, g.w_out, through ? kChainLink : link, s);
+    if (rc == TMW_OK && g.w_out != nullptr) rc = pending.weight_grad(d, R, D, D, dy, a.o, g.w_out, through ? kChainDependent : link, s);
     if (rc != TMW_OK || !through) return rc;
     const tmw_prefill_desc c = core_desc(d);
     const char *q = a.conv, *k = q + 2ll * D, *v = q + 4ll * D;
@@ -163,9 +163,9 @@ int attention_backward(const Dims& d, const void* x, const AttentionWeights& w, 
             if (g.conv[i] != nullptr) pending.sums.add(t.d_taps + (int64_t)i * D * d.taps, g.conv[i], (int64_t)D * d.taps, 1);
     }
     // (the kernels in front take no part in chains: an ordinary launch behind them)
-    if (rc == TMW_OK && dx != nullptr) rc = input_grad(d, R, D, 3 * D, t.d_qkv, w.w_qkv, dx, GEMM_NONE, nullptr, kChainFollowed, s);
+    if (rc == TMW_OK && dx != nullptr) rc = input_grad(d, R, D, 3 * D, t.d_qkv, w.w_qkv, dx, GEMM_NONE, nullptr, 0, s);
     if (rc == TMW_OK && g.w_qkv != nullptr)
-        rc = pending.weight_grad(d, R, 3 * D, D, t.d_qkv, x, g.w_qkv, dx != nullptr ? kChainLink : kChainFollowed, s);
+        rc = pending.weight_grad(d, R, 3 * D, D, t.d_qkv, x, g.w_qkv, dx != nullptr ? kChainDependent : 0, s);
     return rc;
 }
 
@@ -308,10 +308,10 @@ extern "C" int tmw_stack_train_forward(const tmw_stack_desc* desc, const tmw_blo
         const LayerSaved a = layer(l);
         rc = attention_forward(d, a.y1, weights_of(b), a.attn, a.x2, a.x, l == 0, s);
         if (rc == TMW_OK) rc = launch_add_rmsnorm(d.dtype, R, D, a.x2, nullptr, b.norm_mlp, d.eps, nullptr, a.y2, s, true);
-        if (rc == TMW_OK) rc = product(d, R, F, D, a.y2, b.w_fc1, b.b_fc1, a.f, GEMM_GELU_KEEP, a.pre, kChainLink, s);
+        if (rc == TMW_OK) rc = product(d, R, F, D, a.y2, b.w_fc1, b.b_fc1, a.f, GEMM_GELU_KEEP, a.pre, kChainDependent, s);
         const bool more = l + 1 < k.layers;
         char* x = more ? layer(l + 1).x : x_last;
-        if (rc == TMW_OK) rc = product(d, R, D, F, a.f, b.w_fc2, b.b_fc2, x, GEMM_ADD, a.x2, kChainLink, s);
+        if (rc == TMW_OK) rc = product(d, R, D, F, a.f, b.w_fc2, b.b_fc2, x, GEMM_ADD, a.x2, kChainDependent, s);
         if (rc == TMW_OK)
             rc = launch_add_rmsnorm(d.dtype, R, D, x, nullptr, more ? blocks[l + 1].norm_attn : k.norm, d.eps, nullptr,
                                     more ? layer(l + 1).y1 : y_last, s, true);
@@ -366,8 +366,8 @@ extern "C" int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_bl
         return st;
     };
 
-    rc = input_grad(d, R, D, V, d_logits, k.head, t.dy, GEMM_NONE, nullptr, kChainFollowed, s);
-    if (rc == TMW_OK) rc = pending.weight_grad(d, R, V, D, d_logits, y_last, grads->head, kChainLink, s);
+    rc = input_grad(d, R, D, V, d_logits, k.head, t.dy, GEMM_NONE, nullptr, 0, s);
+    if (rc == TMW_OK) rc = pending.weight_grad(d, R, V, D, d_logits, y_last, grads->head, kChainDependent, s);
     if (rc == TMW_OK) rc = norm_bwd(t.dy, x_last, k.norm, nullptr, t.g, t.norm_parts[0], t.norm_parts[1], grads->norm);
     if (rc == TMW_OK) rc = pending.flush(d, s);
     for (int l = k.layers - 1; l >= 0 && rc == TMW_OK; --l) {
@@ -375,10 +375,10 @@ extern "C" int tmw_stack_train_backward(const tmw_stack_desc* desc, const tmw_bl
         const tmw_block_grads& q = block_grads[l];
         const LayerSaved a = layer_saved(d, base + l * layer_saved_bytes(d));
         if (q.b_fc2 != nullptr) pending.sums.add(t.norm_parts[1], q.b_fc2, D, blocks_n);
-        rc = input_grad(d, R, F, D, t.g, b.w_fc2, t.pre, GEMM_GELU_GRAD, a.pre, kChainLink, s);
-        if (rc == TMW_OK) rc = pending.weight_grad(d, R, D, F, t.g, a.f, q.w_fc2, kChainLink, s);
-        if (rc == TMW_OK) rc = input_grad(d, R, D, F, t.pre, b.w_fc1, t.dy, GEMM_NONE, nullptr, kChainLink, s);
-        if (rc == TMW_OK) rc = pending.weight_grad(d, R, F, D, t.pre, a.y2, q.w_fc1, kChainLink, s);
+        rc = input_grad(d, R, F, D, t.g, b.w_fc2, t.pre, GEMM_GELU_GRAD, a.pre, kChainDependent, s);
+        if (rc == TMW_OK) rc = pending.weight_grad(d, R, D, F, t.g, a.f, q.w_fc2, kChainDependent, s);
+        if (rc == TMW_OK) rc = input_grad(d, R, D, F, t.pre, b.w_fc1, t.dy, GEMM_NONE, nullptr, kChainDependent, s);
+        if (rc == TMW_OK) rc = pending.weight_grad(d, R, F, D, t.pre, a.y2, q.w_fc1, kChainDependent, s);
         if (rc == TMW_OK && q.b_fc1 != nullptr) {
             float* part = reinterpret_cast<float*>(t.partial + t.room);
             rc = launch_colsum(d.dtype, t.pre, part, R, F, s);
