@@ -87,6 +87,29 @@ def test_output_rows_off_the_32_byte_boundary(m, n, shift):
     assert (room[:shift] == 7).all() and (room[shift + m * n:] == 7).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,n", [(33, 8), (97, 40), (300, 648), (257, 1920), (8320, 664), (2060, 2568)])
+def test_bias_and_gelu_of_rows_off_the_32_byte_boundary(m, n, dtype):
+    """Lanes take their columns eight further on there: the result 16 bytes into its allocation is bit for bit the one at its start,
+    and that within one rounding of fp32 (tolerance as in run_case)."""
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    x = torch.randn(m, 128, generator=g, device=DEV).to(dtype)
+    w = (torch.randn(n, 128, generator=g, device=DEV) * 0.05).to(dtype)
+    b = (torch.randn(n, generator=g, device=DEV) * 0.5).to(dtype)
+    ref = reference(x, w, b, True)
+    tol = (2 ** -8 if dtype == torch.bfloat16 else 2 ** -10) * max(1.0, ref.abs().max().item()) + 1e-3
+    outs = []
+    for shift in (0, 8):
+        room = torch.full((m * n + 32,), 7.0, device=DEV, dtype=dtype)
+        out = room[shift:shift + m * n].view(m, n)
+        _native.linear(x, w, b, gelu=True, out=out)
+        _native.poll_status(torch.device(DEV))
+        assert (out.float() - ref).abs().max().item() <= tol
+        assert (room[:shift] == 7).all() and (room[shift + m * n:] == 7).all()
+        outs.append(out)
+    assert torch.equal(*outs)
+
+
 def test_output_off_the_16_byte_boundary_is_refused():
     x, w = torch.zeros(300, 64, device=DEV, dtype=torch.bfloat16), torch.zeros(64, 64, device=DEV, dtype=torch.bfloat16)
     room = torch.zeros(300 * 64 + 8, device=DEV, dtype=torch.bfloat16)

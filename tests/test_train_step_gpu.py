@@ -212,3 +212,72 @@ def test_sums_of_partial_results(B, T, d_ff):
         want = one[name] * (B * T)
         if want.norm() > 0:
             assert ((many[name] - want).norm() / want.norm()).item() <= 2 ** -10, name
+
+
+@pytest.mark.parametrize("B,T,dtype,heads,dh,d_ff,vocab", [
+    (2, 61, torch.bfloat16, 2, 64, 264, 520),       # hidden rows and logits of 16 n + 8 values
+    (4, 1024, torch.float16, 2, 128, 2568, 1000),   # more rows, tiles of 256
+])
+def test_training_step_of_rows_off_the_sectors(B, T, dtype, heads, dh, d_ff, vocab, monkeypatch):
+    """The epilogues of such rows (kept GELU argument, its derivative) against the same computation module by module; tolerances as
+    above."""
+    D = heads * dh
+    cfg = TitanMACConfig(vocab_size=vocab, d_model=D, n_heads=heads, n_layers=2, d_ff=d_ff, max_seq_len=1024, window_size=32,
+                         n_persistent=5, use_block_sparse=False)
+    g = torch.Generator(device=DEV).manual_seed(d_ff)
+    with torch.device(DEV):
+        model = TitanMAC(cfg)
+    with torch.no_grad():
+        for name, prm in model.named_parameters():
+            prm.normal_(1.0 if name.endswith("scale") else 0.0, 0.1 if name.endswith(("scale", "bias")) else 0.04, generator=g)
+    model = model.to(dtype)
+    ids = torch.randint(0, vocab, (B, T), generator=g, device=DEV)
+    scale = 1.0 if dtype == torch.bfloat16 else 64.0
+
+    def step():
+        model.zero_grad(set_to_none=True)
+        with torch.enable_grad():
+            out = model(ids, labels=ids)
+            (out["loss"] * scale).backward()
+        _native.poll_status(torch.device(DEV))
+        return out["logits"].detach(), {n: p.grad for n, p in model.named_parameters()}
+
+    logits, grads = step()
+    module_by_module(monkeypatch)
+    want_logits, want = step()
+    tol = 3e-2 if dtype == torch.bfloat16 else 6e-3
+    assert close(logits, want_logits, tol)
+    for name, ref in want.items():
+        assert close(grads[name], ref, 2 * tol), name
+
+
+@pytest.mark.parametrize("shifts", [(16, 0), (0, 16), (16, 16)])
+def test_training_step_with_buffers_aligned_to_16_bytes(shifts, monkeypatch):
+    """Saved activations and scratch 16 bytes into their allocations, together and one of them alone (an epilogue then reads rows that
+    start on sectors and writes rows that do not, or the other way round): bit for bit the gradients of aligned ones."""
+    model, g = make(torch.bfloat16, 2, 64, 40, 5, 512, False)
+    ids = torch.randperm(512, generator=g, device=DEV)[:450].view(3, 150)  # (each token once: no sum has an order to choose)
+
+    def step(shifts):
+        left, empty = list(shifts), torch.empty
+
+        def shifted(*size, **kw):
+            if kw.get("dtype") is not torch.uint8:
+                return empty(*size, **kw)
+            off = left.pop(0)
+            return empty(size[0] + 32, **kw)[off:off + size[0]]
+
+        model.zero_grad(set_to_none=True)
+        with monkeypatch.context() as m, torch.enable_grad():
+            m.setattr(torch, "empty", shifted)
+            out = model(ids, labels=ids)
+            out["loss"].backward()
+            assert not left
+        _native.poll_status(torch.device(DEV))
+        return out["logits"].detach(), {n: p.grad for n, p in model.named_parameters()}
+
+    want_logits, want = step((0, 0))
+    logits, grads = step(shifts)
+    assert torch.equal(logits, want_logits)
+    for name, ref in want.items():
+        assert torch.equal(grads[name], ref), name

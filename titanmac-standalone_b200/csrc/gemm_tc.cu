@@ -83,59 +83,85 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// 16 values of a row, of which the first `left` columns exist (a multiple of 8), to and from global memory: one whole sector
-// where the row is aligned to it.  Half a sector per instruction costs L2 a second pass over it.
-__device__ __forceinline__ void store16(void* row, int col, int left, bool wide, const uint4& a, const uint4& b) {
-    uint16_t* dst = static_cast<uint16_t*>(row) + col;
-    if (wide && left >= 16) {
+// Rows that start on a sector (32 bytes; WIDE: all of the output and of what the epilogue reads do) go out as they lie in tensor
+// memory, 32 columns of a row per lane and panel.  Rows that do not (every second one of 16 n + 8 values, all of an output 16 bytes
+// into its allocation) would cost L2 two accesses of half a sector for each sector: their lane takes its columns 8 further on,
+// where sectors start, and the first eight of the tile with the last panel.  (In kernels of their own: another form chosen at run
+// time beside the plain one cost that its registers, 16416 x 2560 x 640 with GELU 54 -> 62 us.)  us, staged for TMA stores as before |
+// halves of sectors | shifted: 16416 x 50008 x 640 1098 | 1390 | 912, 32896 x 1928 x 640 70.8 | 86.1 | 63.8, 16416 x 2568 x 640 with
+// GELU_KEEP 77.6 | 134 | 71.5; an output 16 bytes off, 16416 x 50000 x 640 1234 | 1573 | 925.
+// Columns [c0, c0 + 8) and [c1, c1 + 8) of a row, of which those below n exist (a multiple of 8):
+template <bool WIDE>
+__device__ __forceinline__ bool one_sector(const void* at, int c0, int c1, int n) {
+    return WIDE ? c1 < n : c1 == c0 + 8 && c1 < n && (reinterpret_cast<uintptr_t>(at) & 31u) == 0;
+}
+template <bool WIDE>
+__device__ __forceinline__ void store16(void* row, int c0, int c1, int n, const uint4& a, const uint4& b) {
+    uint16_t *dst = static_cast<uint16_t*>(row) + c0, *dst1 = static_cast<uint16_t*>(row) + c1;
+    if (one_sector<WIDE>(dst, c0, c1, n)) {
         asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                      ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
                      : "memory");
         return;
     }
-    if (left > 0) *reinterpret_cast<uint4*>(dst) = a;
-    if (left > 8) *reinterpret_cast<uint4*>(dst + 8) = b;
+    if (c0 < n) *reinterpret_cast<uint4*>(dst) = a;
+    if (!WIDE && c1 < n) *reinterpret_cast<uint4*>(dst1) = b;
 }
-__device__ __forceinline__ void load16(const void* row, int col, int left, bool wide, uint4& a, uint4& b) {
-    const uint16_t* src = static_cast<const uint16_t*>(row) + col;
-    if (wide && left >= 16) {
+template <bool WIDE>
+__device__ __forceinline__ void load16(const void* row, int c0, int c1, int n, uint4& a, uint4& b) {
+    const uint16_t *src = static_cast<const uint16_t*>(row) + c0, *src1 = static_cast<const uint16_t*>(row) + c1;
+    if (one_sector<WIDE>(src, c0, c1, n)) {
         asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                      : "l"(src)
                      : "memory");
         return;
     }
-    a = left > 0 ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
-    b = left > 8 ? *reinterpret_cast<const uint4*>(src + 8) : make_uint4(0, 0, 0, 0);
+    a = c0 < n ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
+    b = !WIDE && c1 < n ? *reinterpret_cast<const uint4*>(src1) : make_uint4(0, 0, 0, 0);
+}
+
+// The columns that a lane has of a panel: [col, col + 24) and [col3, col3 + 8).
+struct PanelColumns {
+    int col, col3;
+};
+template <bool WIDE>
+__device__ __forceinline__ PanelColumns panel_columns(bool shifted, int col0, int panel, int panels) {
+    const int col = col0 + panel * kPanel;
+    if (WIDE || !shifted) return {col, col + 24};
+    return {col + 8, panel + 1 < panels ? col + 32 : col0};
 }
 
 // What the epilogue of a panel reads beside the accumulator (GEMM_ADD, GEMM_GELU_GRAD): a lane's row of its 32 columns.
 // Asked for before the accumulator is waited for.
 struct PanelAux { uint4 v[4]; };
 
-__device__ __forceinline__ void load_aux(PanelAux& in, const GemmParams& p, int row, int col) {
+template <bool WIDE>
+__device__ __forceinline__ void load_aux(PanelAux& in, const GemmParams& p, int row, const PanelColumns& c) {
     if ((p.epilogue != GEMM_ADD && p.epilogue != GEMM_GELU_GRAD) || row >= p.m) return;
     const uint16_t* src = static_cast<const uint16_t*>(p.aux) + (long long)row * p.n;
-    load16(src, col, p.n - col, p.wide, in.v[0], in.v[1]);
-    load16(src, col + 16, p.n - col - 16, p.wide, in.v[2], in.v[3]);
+    load16<WIDE>(src, c.col, c.col + 8, p.n, in.v[0], in.v[1]);
+    load16<WIDE>(src, c.col + 16, c.col3, p.n, in.v[2], in.v[3]);
 }
 
 // 32 accumulator columns of one row per lane -> bias, epilogue -> the output.  A row per lane and 32 bytes per access: every
 // sector is written once and whole, without a detour through shared memory, which leaves that to two more stages of operands.
 // Against panels of 32 x 32 staged for TMA stores, us, K = 640: 16416 x 50000 863 -> 800, 16416 x 2560 46.6 -> 43.5, 32896 x 1920
 // 66.4 -> 64.8, 32896 x 640 30.5 -> 28.5; 8320 x 640 x 2560 28.0 -> 25.0; 8192^3 718 -> 715.
-template <bool BF16>
-__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, const PanelAux& in, int row, int col) {
+template <bool BF16, bool WIDE>
+__device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, const PanelAux& in, int row, const PanelColumns& c) {
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
     if (p.bias != nullptr) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 8)
-            if (col + j < p.n) {  // n is a multiple of 8
+        for (int j = 0; j < 32; j += 8) {
+            const int at = j < 24 ? c.col + j : c.col3;
+            if (at < p.n) {
                 float b8[8];
-                load8<T>(static_cast<const T*>(p.bias) + col + j, b8);  // (the same for every lane)
+                load8<T>(static_cast<const T*>(p.bias) + at, b8);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
             }
+        }
     }
     if (row >= p.m) return;
     if (p.epilogue == GEMM_GELU) {
@@ -146,7 +172,7 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
 #pragma unroll
         for (int j = 0; j < 32; j += 16) {
             const uint4 raw[2] = {pack8<BF16>(v + j), pack8<BF16>(v + j + 8)};
-            store16(keep, col + j, p.n - col - j, p.wide, raw[0], raw[1]);
+            store16<WIDE>(keep, c.col + j, j ? c.col3 : c.col + 8, p.n, raw[0], raw[1]);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float x[8];
@@ -157,19 +183,20 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
         }
     } else if (p.epilogue != GEMM_NONE) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int i = 0; i < 4; ++i) {
             float x[8];
-            load8<T>(reinterpret_cast<const T*>(&in.v[c]), x);
+            load8<T>(reinterpret_cast<const T*>(&in.v[i]), x);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                float& y = v[8 * c + e];
+                float& y = v[8 * i + e];
                 y = p.epilogue == GEMM_ADD ? x[e] + to_f32<T>(from_f32<T>(y)) : y * gelu_slope(x[e]);
             }
         }
     }
     uint16_t* out = static_cast<uint16_t*>(p.c) + (long long)row * p.ldc;
 #pragma unroll
-    for (int j = 0; j < 32; j += 16) store16(out, col + j, p.n - col - j, p.wide, pack8<BF16>(v + j), pack8<BF16>(v + j + 8));
+    for (int j = 0; j < 32; j += 16)
+        store16<WIDE>(out, c.col + j, j ? c.col3 : c.col + 8, p.n, pack8<BF16>(v + j), pack8<BF16>(v + j + 8));
 }
 
 // the fp32 sums of a k range: whole sectors where `partial` lies on one (n is a multiple of 8), halves where the caller's scratch is
@@ -194,31 +221,36 @@ __device__ __forceinline__ void store_partial(const uint32_t (&v)[32], const Gem
 
 // A warp's panels (first, first + step, ...) of a finished tile: tensor memory -> global memory.  No warp waits for another.
 // `in` holds the inputs of the first panel; `all_read` is called once the accumulator has been read.
-template <bool BF16, typename F>
-__device__ __forceinline__ void epilogue_panels(const GemmParams& p, PanelAux& in, uint32_t t_addr, int row, int col0, int first,
-                                                int panels, int step, int split, F all_read) {
+template <bool BF16, bool WIDE, typename F>
+__device__ __forceinline__ void epilogue_panels(const GemmParams& p, PanelAux& in, uint32_t t_addr, bool shifted, int row, int col0,
+                                                int first, int panels, int step, int split, F all_read) {
     if (first >= panels) all_read();
     for (int pn = first; pn < panels; pn += step) {
-        const int col = col0 + pn * kPanel;
-        uint32_t acc[32];
+        uint32_t acc[32], next[8];
         __syncwarp();
         tmem_ld32(t_addr + pn * kPanel, acc);
+        if (!WIDE) tmem_ld8(t_addr + (pn + 1 < panels ? (pn + 1) * kPanel : 0), next);
         tc_wait_ld();
         if (pn + step >= panels) {
             tc_fence_before();
             __syncwarp();
             all_read();
         }
-        if (p.partial != nullptr) {
-            store_partial(acc, p, split, row, col);
+        if (WIDE && p.partial != nullptr) {
+            store_partial(acc, p, split, row, col0 + pn * kPanel);
             continue;
         }
         float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-        finish_panel<BF16>(v, p, in, row, col);
-        if (pn + step < panels) load_aux(in, p, row, col + step * kPanel);
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(WIDE || !shifted ? acc[j] : j < 24 ? acc[j + 8] : next[j - 24]);
+        finish_panel<BF16, WIDE>(v, p, in, row, panel_columns<WIDE>(shifted, col0, pn, panels));
+        if (pn + step < panels) load_aux<WIDE>(in, p, row, panel_columns<WIDE>(shifted, col0, pn + step, panels));
     }
+}
+// whether a row of the output starts in the middle of a sector (its columns from col0 on, a multiple of 32)
+template <bool WIDE>
+__device__ __forceinline__ bool off_sector(const GemmParams& p, int row) {
+    return !WIDE && (reinterpret_cast<uintptr_t>(static_cast<uint16_t*>(p.c) + (long long)row * p.ldc) & 31u) != 0;
 }
 
 // An operand tile of R rows (of the product: M or N) x 64 k-elements in shared memory, 128 bytes per swizzled row.
@@ -231,7 +263,7 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
 template <bool MN>
 constexpr uint64_t kStepDesc = MN ? 128 : 2;  // 16 k-elements on, in units of 16 bytes
 
-template <int BN, bool BF16, bool AMN, bool BMN>
+template <int BN, bool BF16, bool AMN, bool BMN, bool WIDE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
     using L = GemmSmem<BN>;
@@ -353,11 +385,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int buf = t & 1;
             const int mn = tile / p.splits, row = (mn / n_tiles) * GM + g * 32 + lane, col0 = (mn % n_tiles) * BN;
             PanelAux in;
-            if (sub < kPanels) load_aux(in, p, row, col0 + sub * kPanel);
+            const bool shifted = off_sector<WIDE>(p, row);
+            if (sub < kPanels) load_aux<WIDE>(in, p, row, panel_columns<WIDE>(shifted, col0, sub, kPanels));
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            epilogue_panels<BF16>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, row, col0, sub, kPanels, kEpiWarps / 4,
-                                  tile % p.splits, [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
+            epilogue_panels<BF16, WIDE>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, shifted, row, col0, sub, kPanels,
+                                        kEpiWarps / 4, tile % p.splits, [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
         }
     }
 
@@ -403,7 +436,7 @@ struct PairSmem {
     static constexpr int kTotal = kBars + 1024 + 1024;  // barriers, alignment slack
 };
 
-template <int BN, bool BF16, bool AMN, bool BMN>
+template <int BN, bool BF16, bool AMN, bool BMN, bool WIDE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
     using L = PairSmem;
@@ -549,11 +582,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int row = band * (2 * GM) + (int)rank * GM + g * 32 + lane;
             const int panels = columns(col0) / kPanel;
             PanelAux in;
-            if (sub < panels) load_aux(in, p, row, col0 + sub * kPanel);
+            const bool shifted = off_sector<WIDE>(p, row);
+            if (sub < panels) load_aux<WIDE>(in, p, row, panel_columns<WIDE>(shifted, col0, sub, panels));
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            epilogue_panels<BF16>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, row, col0, sub, panels, kPairEpiWarps / 4,
-                                  tile % p.splits, [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
+            epilogue_panels<BF16, WIDE>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, shifted, row, col0, sub, panels,
+                                        kPairEpiWarps / 4, tile % p.splits, [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
         }
     }
 
@@ -601,11 +635,34 @@ int gemm_params(const GemmCall& g, GemmParams* p) {
     return TMW_OK;
 }
 
-// `with` is called with the kernel of the call's data type and operand layouts
-template <typename K00, typename K01, typename K11, typename F>
-int with_layout(const GemmCall& g, K00 k00, K01 k01, K11 k11, F with) {
-    if (!g.a_mn) return g.b_mn ? with(k01) : with(k00);
-    return g.b_mn ? with(k11) : TMW_ERR_UNSUPPORTED;
+// The kernels by data type, operand layouts (built with MN-major ones: 256 x 256, 128 and 64 columns) and alignment of the rows.
+template <int BN>
+struct Single {
+    static constexpr bool kMn = BN == 64 || BN == 128;
+    template <bool BF16, bool AMN, bool BMN, bool WIDE>
+    static constexpr auto kernel = gemm_tc_kernel<BN, BF16, AMN, BMN, WIDE>;
+};
+template <int BN>
+struct Pair {
+    static constexpr bool kMn = true;
+    template <bool BF16, bool AMN, bool BMN, bool WIDE>
+    static constexpr auto kernel = gemm_tc_pair_kernel<BN, BF16, AMN, BMN, WIDE>;
+};
+// `run` is called with the call's kernel
+template <typename Family, typename F>
+int with_kernel(const GemmCall& g, const GemmParams& p, F run) {
+    auto pick = [&](auto bf16, auto wide) -> int {
+        constexpr bool B = decltype(bf16)::value, W = decltype(wide)::value;
+        if (!g.a_mn && !g.b_mn) return run(Family::template kernel<B, false, false, W>);
+        if constexpr (Family::kMn) {
+            if (g.b_mn && g.a_mn) return run(Family::template kernel<B, true, true, W>);
+            if (g.b_mn) return run(Family::template kernel<B, false, true, W>);
+        }
+        return TMW_ERR_UNSUPPORTED;
+    };
+    const bool wide = p.partial != nullptr || p.wide;  // (fp32 sums have a path of their own)
+    if (g.dtype == TMW_BF16) return wide ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
+    return wide ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{});
 }
 
 template <int BN>
@@ -623,15 +680,7 @@ int launch_gemm(const GemmCall& g, cudaStream_t stream) {
         TMW_CUDA_TRY(launch_ex(kern, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, p));
         return TMW_OK;
     };
-    if constexpr (BN == 64 || BN == 128) {
-        return g.dtype == TMW_BF16 ? with_layout(g, gemm_tc_kernel<BN, true, false, false>, gemm_tc_kernel<BN, true, false, true>,
-                                                 gemm_tc_kernel<BN, true, true, true>, run)
-                                   : with_layout(g, gemm_tc_kernel<BN, false, false, false>, gemm_tc_kernel<BN, false, false, true>,
-                                                 gemm_tc_kernel<BN, false, true, true>, run);
-    } else {
-        if (g.a_mn || g.b_mn) return TMW_ERR_UNSUPPORTED;
-        return g.dtype == TMW_BF16 ? run(gemm_tc_kernel<BN, true, false, false>) : run(gemm_tc_kernel<BN, false, false, false>);
-    }
+    return with_kernel<Single<BN>>(g, p, run);
 }
 
 // How many CTA pairs of the kernel the device runs at once (asked once per kernel and device).
@@ -681,11 +730,7 @@ int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
         TMW_CUDA_TRY(launch_ex(kern, dim3(2 * pairs), dim3(kPairThreads), L::kTotal, stream, g.chain & kChainDependent, 1, ma, mb, p));
         return TMW_OK;
     };
-    return g.dtype == TMW_BF16
-               ? with_layout(g, gemm_tc_pair_kernel<BN, true, false, false>, gemm_tc_pair_kernel<BN, true, false, true>,
-                             gemm_tc_pair_kernel<BN, true, true, true>, run)
-               : with_layout(g, gemm_tc_pair_kernel<BN, false, false, false>, gemm_tc_pair_kernel<BN, false, false, true>,
-                             gemm_tc_pair_kernel<BN, false, true, true>, run);
+    return with_kernel<Pair<BN>>(g, p, run);
 }
 
 // What a single-CTA kernel was measured to need (us): a launch without its K, what a 64-wide slice of K takes where a tile is
