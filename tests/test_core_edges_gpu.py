@@ -46,9 +46,8 @@ def test_block_sparse_core_with_persistent_rows(dtype, tol, dh, L, w, block, n_p
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_persistent_rows_of_many_sequences(dtype):
-    """The two bodies at head_dim 64: K of the next block ahead while all CTAs (here four to a pair) fit the chip three to an SM, not
-    ahead with one pair more.  The sums are the same, so a sequence's rows are, bit for bit; one of them against the oracle, tolerance
-    as above."""
+    """As many sequences as fit the chip three CTAs to an SM (here four to a sequence), and one more: a sequence's rows are the same
+    in both launches, bit for bit; one of them against the oracle, tolerance as above."""
     most = 3 * torch.cuda.get_device_properties(0).multi_processor_count // 4
     q, k, v = (t.to(dtype) for t in wo.qkv_inputs(most + 1, 1, 520, 64, seed=3))
     many = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), 40, 16, window_block=32)

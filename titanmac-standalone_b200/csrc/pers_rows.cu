@@ -6,11 +6,9 @@
 // warp walks over blocks of 32 (head_dim 128: 16) keys with its own running maximum, and the partial results are merged through shared memory
 // and the cluster's.  As a query tile of 128 rows in the tcgen05 kernel the same rows walked 2747 keys one tile after the
 // other, 37 us on a side stream of its own beside 35 us for all other rows.
-// V of a warp's next block loads under this one.  At head_dim 64 so does K (AHEAD), where the launch fits the chip three CTAs to an
-// SM: the second block of K takes 168 registers instead of 126, and four CTAs to an SM do not.  us, back to back, without |
-// with: 8 heads x 1 | 3 | 6 | 12 sequences of 2747 rows 8.6 | 8.4, 10.5 | 10.0, 12.5 | 11.3, 17.1 | 15.1; 7 | 8 | 16 sequences (448
-// and 512 CTAs) 12.7 | 18.7, 12.7 | 19.4, 18.1 | 26.1.  Held at 128 registers it is slower than without throughout (12.5 | 13.4),
-// as it is at head_dim 128, two CTAs to an SM either way (8 heads x 3 sequences: 13.7 | 14.6).
+// V of a warp's next block loads under this one, K does not: at head_dim 64 the second block of K takes 168 registers instead of 126,
+// three CTAs to an SM instead of four, and these leave the attention behind no room to start.  Block-sparse layers of 10 heads, us, K
+// ahead | not: 5 x 1400 rows, window 300 74.6 | 71.3; 5 x 2747, window 512 130.6 | 124.9; 1 x 316 30.0 | 30.3; 3 x 2747 89.7 | 89.7.
 #include <math_constants.h>
 
 #include "tmw_common.cuh"
@@ -45,7 +43,7 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(h);
 }
 
-template <typename T, int DH, bool AHEAD>
+template <typename T, int DH>
 __global__ void __launch_bounds__(kPersWarps * 32) pers_rows_kernel(const PersParams p) {
     constexpr int KEYS = pers_keys(DH), KN = KEYS / 8;  // keys per block, in groups of 8
     constexpr int KC = DH / 32, NT = DH / 8;            // 32-wide chunks of head_dim; 8-wide output columns
@@ -85,33 +83,16 @@ __global__ void __launch_bounds__(kPersWarps * 32) pers_rows_kernel(const PersPa
     for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
-    auto fetch_k = [&](int block, uint4 (&to)[KN][KC]) {
+    if (first < blocks) fetch_v(first, 0);
+    int buf = 0;
+    for (int b = first; b < blocks; b += step, buf ^= 1) {
+        uint4 kb[KN][KC];
 #pragma unroll
         for (int n = 0; n < KN; ++n)
 #pragma unroll
             for (int c = 0; c < KC; ++c)
-                to[n][c] = *reinterpret_cast<const uint4*>(k + min(block * KEYS + n * 8 + g, p.k_rows - 1) * p.ks[2] + c * 32 + t * 8);
-    };
-    uint4 ahead[KN][KC];
-    if (first < blocks) {
-        fetch_v(first, 0);
-        if (AHEAD) fetch_k(first, ahead);
-    }
-    int buf = 0;
-    for (int b = first; b < blocks; b += step, buf ^= 1) {
-        uint4 kb[KN][KC];
-        if (AHEAD) {
-#pragma unroll
-            for (int n = 0; n < KN; ++n)
-#pragma unroll
-                for (int c = 0; c < KC; ++c) kb[n][c] = ahead[n][c];
-        } else {
-            fetch_k(b, kb);
-        }
-        if (b + step < blocks) {
-            fetch_v(b + step, buf ^ 1);
-            if (AHEAD) fetch_k(b + step, ahead);
-        }
+                kb[n][c] = *reinterpret_cast<const uint4*>(k + min(b * KEYS + n * 8 + g, p.k_rows - 1) * p.ks[2] + c * 32 + t * 8);
+        if (b + step < blocks) fetch_v(b + step, buf ^ 1);
         float s[KN][4], mx[2] = {m[0], m[1]};
 #pragma unroll
         for (int n = 0; n < KN; ++n) {
@@ -262,8 +243,8 @@ int launch_pers_rows(const tmw_prefill_desc& d, const void* q, const void* k, co
     }
     p.q_rows = d.q_rows; p.k_rows = d.k_rows;
     p.scale_log2 = (d.scale != 0.f ? d.scale : 1.0f / sqrtf((float)d.head_dim)) * 1.4426950408889634f;
-    // CTAs per (batch, head, 16 rows): up to eight, while they fit the chip four to an SM (head_dim 64 without AHEAD: 126 registers; at
-    // head_dim 128 two are resident and the rest a second wave) and have a block for every warp
+    // CTAs per (batch, head, 16 rows): up to eight, while they fit the chip four to an SM (head_dim 64; at 128 two are resident and the
+    // rest a second wave) and have a block for every warp
     const long long groups = (long long)(d.q_rows + 15) / 16 * d.heads * d.batch;
     p.cluster = 1;
     while (p.cluster < 8 && groups * p.cluster * 2 <= 4 * sm_count() && p.cluster * 2 * kPersWarps * pers_keys(d.head_dim) <= d.k_rows) p.cluster *= 2;
@@ -272,12 +253,9 @@ int launch_pers_rows(const tmw_prefill_desc& d, const void* q, const void* k, co
         TMW_CUDA_TRY(launch_ex(kern, grid, block, 0, stream, pdl, p.cluster, p));
         return TMW_OK;
     };
-    auto pick = [&](auto type) -> int {
-        using T = decltype(type);
-        if (d.head_dim == 128) return run(pers_rows_kernel<T, 128, false>);
-        return groups * p.cluster <= 3 * sm_count() ? run(pers_rows_kernel<T, 64, true>) : run(pers_rows_kernel<T, 64, false>);
-    };
-    return d.dtype == TMW_BF16 ? pick(__nv_bfloat16()) : pick(__half());
+    if (d.head_dim == 64)
+        return d.dtype == TMW_BF16 ? run(pers_rows_kernel<__nv_bfloat16, 64>) : run(pers_rows_kernel<__half, 64>);
+    return d.dtype == TMW_BF16 ? run(pers_rows_kernel<__nv_bfloat16, 128>) : run(pers_rows_kernel<__half, 128>);
 }
 
 }  // namespace tmw
