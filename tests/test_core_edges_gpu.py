@@ -76,3 +76,17 @@ def test_wide_heads_with_long_windows(dtype, L, w, n_p, block, spread):
     o = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), w, n_p, window_block=block)
     _native.poll_status()
     assert (o.float().cpu() - ref).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_whole_key_tiles_either_side_of_the_rule(dtype):
+    """As many sequences of 6 query tiles and two heads as make four tiles to an SM (whole key tiles on their own), and more (the general
+    body): the same sums, so a sequence's rows are the same, bit for bit; one of them against the oracle, tolerance as above."""
+    most = 4 * torch.cuda.get_device_properties(0).multi_processor_count // 12
+    q, k, v = (t.to(dtype) for t in wo.qkv_inputs(most + 2, 2, 700, 128, seed=5))
+    many = _native.prefill(q.to(DEV), k.to(DEV), v.to(DEV), 512, 16)
+    few = _native.prefill(q[:most].to(DEV), k[:most].to(DEV), v[:most].to(DEV), 512, 16)
+    _native.poll_status()
+    assert torch.equal(many[:most], few)
+    ref = wo.attention_core_dense(q[-1:].float(), k[-1:].float(), v[-1:].float(), 512, 16)
+    assert (many[-1:].float().cpu() - ref).abs().max().item() <= 2e-2

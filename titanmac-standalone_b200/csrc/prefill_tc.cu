@@ -211,10 +211,7 @@ enum BarSlot {
 // GENERAL = false: the plain windowed mask (per-token);
 // GENERAL = true: block-granular window, read from the parameters.
 // STRAIGHT: key tiles that every row sees in full have a body of their own without mask and chunk tests, one run of
-// instructions (head_dim 128; at head_dim 64 the 96 registers of a softmax thread do not hold it).  It pays where most tiles of
-// a window are such: 8 heads x 30 000 rows, us, windows 200 | 300 | 400 | 512 | 640 | 1024 | 2048: 84.7 | 94.2 | 110.5 | 121.0 |
-// 136.4 | 183.5 | 307.6 without and 86.7 | 96.6 | 110.8 | 119.8 | 134.1 | 178.2 | 296.0 with it.
-constexpr int kStraightFrom = 512;  // window
+// instructions (head_dim 128; at head_dim 64 the 96 registers of a softmax thread do not hold it).  See straight_pays.
 template <int DH, bool BF16, bool GENERAL, bool STRAIGHT>
 __global__ void __launch_bounds__(kTcThreads, Budget<DH>::kCtasPerSm)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -472,16 +469,16 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                         for (int i = 0; i < 16; ++i) {
                             const float s0 = __uint_as_float(s[c][2 * i]), s1 = __uint_as_float(s[c][2 * i + 1]);
                             float x0, x1;
-                        unpack2(fma2(pack2(s0, s1), scale2, negm2), x0, x1);
-                        const float e0 = fast_exp2(x0), e1 = fast_exp2(x1);
-                        lacc[i & 1] = add2(lacc[i & 1], pack2(e0, e1));
-                        if (BF16) {
-                            const __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
-                            packed[i] = *reinterpret_cast<const uint32_t*>(&h);
-                        } else {
-                            const __half2 h = __floats2half2_rn(e0, e1);
-                            packed[i] = *reinterpret_cast<const uint32_t*>(&h);
-                        }
+                            unpack2(fma2(pack2(s0, s1), scale2, negm2), x0, x1);
+                            const float e0 = fast_exp2(x0), e1 = fast_exp2(x1);
+                            lacc[i & 1] = add2(lacc[i & 1], pack2(e0, e1));
+                            if (BF16) {
+                                const __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
+                                packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+                            } else {
+                                const __half2 h = __floats2half2_rn(e0, e1);
+                                packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+                            }
                         }
                         tmem_st16(s_addr + c * 16, packed);
                     }
@@ -713,6 +710,18 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 // ---------------------------------------------------------------------------------
 int np_pad_of(int np) { return np > 0 ? ((np + 15) / 16) * 16 : 0; }
 
+// Whether the body for whole key tiles pays (never below 512, where few tiles of a window are such: 8 heads x 30 000 rows, window
+// 300, 94.2 us without and 96.6 with it).  It does with block-granular windows (3 x 8 heads x 2747 rows, blocks of 64, windows 512 | 1024:
+// 51.0 | 70.3 and 48.2 | 62.8 us), with windows of 1024 and more (30 000 rows: 169.9 and 162.8), with few query tiles to an SM, where
+// one tile's time counts (1040 rows, window 640: 16.5 and 15.7), and in long sequences (30 000 rows, 512 | 896: 108.9 | 153.5 and
+// 106.6 | 150.0; 4 x 8208, 896: 154.9 and 152.2).  Many sequences of a few windows each are slower with it (8 x 2064 rows, 512 | 640: 60.6 |
+// 66.6 and 62.2 | 67.6; 16 x 2064, 896: 160.4 and 164.0; 8 x 4112, 512: 116.5 and 118.3).
+bool straight_pays(const tmw_prefill_desc& d, bool block_window) {
+    if (d.window < 512) return false;
+    const long long tiles = (long long)((d.q_rows + BM - 1) / BM) * d.heads * d.batch;
+    return block_window || d.window >= 1024 || tiles <= 4 * sm_count() || d.q_rows >= 9ll * d.window;
+}
+
 template <int DH>
 int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const void* v, void* o, cudaStream_t stream,
               int window_block, float* lse, const tmw_halo_wait* wait, int chain) {
@@ -761,7 +770,7 @@ int launch_tc(const tmw_prefill_desc& d, const void* q, const void* k, const voi
     };
     auto pick = [&](auto bf16, auto general) -> int {
         constexpr bool BF16 = decltype(bf16)::value, GENERAL = decltype(general)::value;
-        if (DH == 128 && d.window >= kStraightFrom) return run(prefill_tc_kernel<DH, BF16, GENERAL, DH == 128>);
+        if (DH == 128 && straight_pays(d, GENERAL)) return run(prefill_tc_kernel<DH, BF16, GENERAL, DH == 128>);
         return run(prefill_tc_kernel<DH, BF16, GENERAL, false>);
     };
     if (d.dtype == TMW_BF16) return window_block > 0 ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
