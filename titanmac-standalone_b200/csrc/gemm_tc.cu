@@ -30,6 +30,7 @@ using namespace ptx;
 constexpr int GM = 128;        // rows of an output tile
 constexpr int GK = 64;         // K elements per stage: one 128-byte swizzle row
 constexpr int kPanel = 32;     // columns that an epilogue warp finishes at a time
+constexpr int kBiasSlot = 96;  // bytes: an epilogue warp's bias of a panel and the eight columns behind it
 constexpr int kEpiWarps = 8;
 constexpr int kGemmThreads = 32 * (2 + kEpiWarps);
 // The pair kernel's tiles are ready every 4 to 5 us at K = 640; with GELU the epilogue of one is 128 x 256 x 24 instructions a
@@ -48,7 +49,8 @@ struct GemmSmem {
     static constexpr int kStage = kStageA + kStageB;
     static constexpr int kStages = (232448 - 2048) / kStage;
     static constexpr int kBars = kStages * kStage;      // offset of the barrier area
-    static constexpr int kTotal = kBars + 1024 + 1024;  // barriers, alignment slack
+    static constexpr int kTotal = kBars + 1024 + 1024;  // barriers and, from 256 on, the warps' bias; alignment slack
+    static_assert(256 + kEpiWarps * kBiasSlot <= 1024, "bias slots");
     static_assert(kStages >= 3, "pipeline depth");
 };
 
@@ -136,43 +138,46 @@ __device__ __forceinline__ PanelColumns panel_columns(bool shifted, int col0, in
 // Asked for before the accumulator is waited for.
 struct PanelAux { uint4 v[4]; };
 
-template <bool WIDE>
+template <bool WIDE, bool AUX>
 __device__ __forceinline__ void load_aux(PanelAux& in, const GemmParams& p, int row, const PanelColumns& c) {
-    if ((p.epilogue != GEMM_ADD && p.epilogue != GEMM_GELU_GRAD) || row >= p.m) return;
+    if (!AUX || row >= p.m) return;
     const uint16_t* src = static_cast<const uint16_t*>(p.aux) + (long long)row * p.n;
     load16<WIDE>(src, c.col, c.col + 8, p.n, in.v[0], in.v[1]);
     load16<WIDE>(src, c.col + 16, c.col3, p.n, in.v[2], in.v[3]);
 }
 
-// 32 accumulator columns of one row per lane -> bias, epilogue -> the output.  A row per lane and 32 bytes per access: every
+// The bias of a panel and of the eight columns behind it (at the tile's end: its first eight), two columns for each of 20 lanes.  It is
+// asked for a panel ahead and passes through a slot of the warp's own in shared memory.  Loaded by every lane where it is added, 64
+// bytes four times, it came from L2 - the outputs that the lanes store push it out of L1 - and the warps are at the latency of their
+// instructions as it is.  With GELU, N = 2560, K = 640, rows 8320 | 16416 | 32896, us: 38.1 | 72.5 | 142 so, 38.9 | 75.3 | 147 by
+// shuffles, 33.0 | 62.8 | 120 now (panels staged for TMA stores 33.4 | 62.1 | 119).
+__device__ __forceinline__ uint32_t load_bias(const GemmParams& p, int col0, int panel, int panels, int lane) {
+    if (p.bias == nullptr || lane >= 20) return 0u;
+    const int c = col0 + (lane >= 16 && panel + 1 == panels ? 2 * lane - 32 : panel * kPanel + 2 * lane);
+    return c < p.n ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.bias) + c) : 0u;
+}
+
+// 32 accumulator columns of one row per lane -> epilogue -> the output, sixteen at a time.  A row per lane and 32 bytes per access: every
 // sector is written once and whole, without a detour through shared memory, which leaves that to two more stages of operands.
 // Against panels of 32 x 32 staged for TMA stores, us, K = 640: 16416 x 50000 863 -> 800, 16416 x 2560 46.6 -> 43.5, 32896 x 1920
-// 66.4 -> 64.8, 32896 x 640 30.5 -> 28.5; 8320 x 640 x 2560 28.0 -> 25.0; 8192^3 718 -> 715.
-template <bool BF16, bool WIDE>
+// 66.4 -> 64.8, 32896 x 640 30.5 -> 28.5; 8320 x 640 x 2560 28.0 -> 25.0; 8192^3 718 -> 715.  Sixteen columns at a time, and the epilogues
+// that read a second operand (AUX) in kernels of their own, leave the registers that GELU's instructions overlap in: with GELU and
+// bias, 16416 x 2560 x 640 65.5 us with 32 at a time, 63.7 with one kernel for all, 62.8 so (a chip that is warm).
+template <bool BF16, bool WIDE, bool AUX>
 __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p, const PanelAux& in, int row, const PanelColumns& c) {
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
-    if (p.bias != nullptr) {
+    uint16_t* out = static_cast<uint16_t*>(p.c) + (long long)row * p.ldc;
+    uint16_t* aux = static_cast<uint16_t*>(p.aux) + (long long)row * p.n;
+    const int n = row < p.m ? p.n : 0;  // (nothing of a row beyond the output is stored)
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-            const int at = j < 24 ? c.col + j : c.col3;
-            if (at < p.n) {
-                float b8[8];
-                load8<T>(static_cast<const T*>(p.bias) + at, b8);
+    for (int j = 0; j < 32; j += 16) {
+        const int c0 = c.col + j, c1 = j ? c.col3 : c.col + 8;
+        if (!AUX && p.epilogue == GEMM_GELU) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[j + e] += b8[e];
-            }
-        }
-    }
-    if (row >= p.m) return;
-    if (p.epilogue == GEMM_GELU) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
-    } else if (p.epilogue == GEMM_GELU_KEEP) {
-        uint16_t* keep = static_cast<uint16_t*>(p.aux) + (long long)row * p.n;
-#pragma unroll
-        for (int j = 0; j < 32; j += 16) {
+            for (int e = 0; e < 16; ++e) v[j + e] = gelu_erf(v[j + e]);
+        } else if (!AUX && p.epilogue == GEMM_GELU_KEEP) {
             const uint4 raw[2] = {pack8<BF16>(v + j), pack8<BF16>(v + j + 8)};
-            store16<WIDE>(keep, c.col + j, j ? c.col3 : c.col + 8, p.n, raw[0], raw[1]);
+            store16<WIDE>(aux, c0, c1, n, raw[0], raw[1]);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float x[8];
@@ -180,23 +185,20 @@ __device__ __forceinline__ void finish_panel(float (&v)[32], const GemmParams& p
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[j + 8 * h + e] = gelu_erf(x[e]);
             }
-        }
-    } else if (p.epilogue != GEMM_NONE) {
+        } else if (AUX) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float x[8];
-            load8<T>(reinterpret_cast<const T*>(&in.v[i]), x);
+            for (int h = 0; h < 2; ++h) {
+                float x[8];
+                load8<T>(reinterpret_cast<const T*>(&in.v[j / 8 + h]), x);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                float& y = v[8 * i + e];
-                y = p.epilogue == GEMM_ADD ? x[e] + to_f32<T>(from_f32<T>(y)) : y * gelu_slope(x[e]);
+                for (int e = 0; e < 8; ++e) {
+                    float& y = v[j + 8 * h + e];
+                    y = p.epilogue == GEMM_ADD ? x[e] + to_f32<T>(from_f32<T>(y)) : y * gelu_slope(x[e]);
+                }
             }
         }
+        store16<WIDE>(out, c0, c1, n, pack8<BF16>(v + j), pack8<BF16>(v + j + 8));
     }
-    uint16_t* out = static_cast<uint16_t*>(p.c) + (long long)row * p.ldc;
-#pragma unroll
-    for (int j = 0; j < 32; j += 16)
-        store16<WIDE>(out, c.col + j, j ? c.col3 : c.col + 8, p.n, pack8<BF16>(v + j), pack8<BF16>(v + j + 8));
 }
 
 // the fp32 sums of a k range: whole sectors where `partial` lies on one (n is a multiple of 8), halves where the caller's scratch is
@@ -220,14 +222,20 @@ __device__ __forceinline__ void store_partial(const uint32_t (&v)[32], const Gem
 }
 
 // A warp's panels (first, first + step, ...) of a finished tile: tensor memory -> global memory.  No warp waits for another.
-// `in` holds the inputs of the first panel; `all_read` is called once the accumulator has been read.
-template <bool BF16, bool WIDE, typename F>
-__device__ __forceinline__ void epilogue_panels(const GemmParams& p, PanelAux& in, uint32_t t_addr, bool shifted, int row, int col0,
-                                                int first, int panels, int step, int split, F all_read) {
+// `in` and `bias` hold what the first panel needs; `all_read` is called once the accumulator has been read.
+template <bool BF16, bool WIDE, bool AUX, typename F>
+__device__ __forceinline__ void epilogue_panels(const GemmParams& p, PanelAux& in, uint32_t bias, uint8_t* slot, uint32_t t_addr,
+                                                bool shifted, int row, int col0, int first, int panels, int step, int split, F all_read) {
+    using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+    const int lane = row & 31;
     if (first >= panels) all_read();
     for (int pn = first; pn < panels; pn += step) {
         uint32_t acc[32], next[8];
         __syncwarp();
+        if (p.bias != nullptr) {
+            if (lane < 20) reinterpret_cast<uint32_t*>(slot)[lane] = bias;
+            __syncwarp();
+        }
         tmem_ld32(t_addr + pn * kPanel, acc);
         if (!WIDE) tmem_ld8(t_addr + (pn + 1 < panels ? (pn + 1) * kPanel : 0), next);
         tc_wait_ld();
@@ -243,8 +251,19 @@ __device__ __forceinline__ void epilogue_panels(const GemmParams& p, PanelAux& i
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(WIDE || !shifted ? acc[j] : j < 24 ? acc[j + 8] : next[j - 24]);
-        finish_panel<BF16, WIDE>(v, p, in, row, panel_columns<WIDE>(shifted, col0, pn, panels));
-        if (pn + step < panels) load_aux<WIDE>(in, p, row, panel_columns<WIDE>(shifted, col0, pn + step, panels));
+        if (p.bias != nullptr) {
+            const T* b = reinterpret_cast<const T*>(slot) + (!WIDE && shifted ? 8 : 0);
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+                float x[8];
+                load8<T>(b + i, x);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[i + e] += x[e];
+            }
+            if (pn + step < panels) bias = load_bias(p, col0, pn + step, panels, lane);
+        }
+        finish_panel<BF16, WIDE, AUX>(v, p, in, row, panel_columns<WIDE>(shifted, col0, pn, panels));
+        if (pn + step < panels) load_aux<WIDE, AUX>(in, p, row, panel_columns<WIDE>(shifted, col0, pn + step, panels));
     }
 }
 // whether a row of the output starts in the middle of a sector (its columns from col0 on, a multiple of 32)
@@ -263,7 +282,7 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
 template <bool MN>
 constexpr uint64_t kStepDesc = MN ? 128 : 2;  // 16 k-elements on, in units of 16 bytes
 
-template <int BN, bool BF16, bool AMN, bool BMN, bool WIDE>
+template <int BN, bool BF16, bool AMN, bool BMN, bool WIDE, bool AUX>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
     using L = GemmSmem<BN>;
@@ -386,11 +405,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int mn = tile / p.splits, row = (mn / n_tiles) * GM + g * 32 + lane, col0 = (mn % n_tiles) * BN;
             PanelAux in;
             const bool shifted = off_sector<WIDE>(p, row);
-            if (sub < kPanels) load_aux<WIDE>(in, p, row, panel_columns<WIDE>(shifted, col0, sub, kPanels));
+            if (sub < kPanels) load_aux<WIDE, AUX>(in, p, row, panel_columns<WIDE>(shifted, col0, sub, kPanels));
+            const uint32_t bias = load_bias(p, col0, sub, kPanels, lane);
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            epilogue_panels<BF16, WIDE>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, shifted, row, col0, sub, kPanels,
-                                        kEpiWarps / 4, tile % p.splits, [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
+            epilogue_panels<BF16, WIDE, AUX>(p, in, bias, bar_area + 256 + (warp - 2) * kBiasSlot,
+                                             tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, shifted, row, col0, sub, kPanels,
+                                             kEpiWarps / 4, tile % p.splits, [&] { if (lane == 0) mbar_arrive(acc_empty(buf)); });
         }
     }
 
@@ -428,15 +449,17 @@ int group_bands(int k) {
 }
 
 // Shared memory of the pair kernel is a ring of as many stages as fit at the tile's width (256 columns: 7, 160: 8).  The bytes
-// in flight are what the rate hangs on: 16416 x 50000 x 640 takes 976 | 875 | 847 | 823 us with 3 | 4 | 5 | 6 stages.
+// in flight are what the rate hangs on: 16416 x 50000 x 640 took 976 | 875 | 847 | 823 us with 3 | 4 | 5 | 6 stages of a form on the
+// way to this one, whose seven took 800 (753 since wide outputs are walked in larger groups).
 struct PairSmem {
     static constexpr int kStageA = GM * GK * 2;
     static constexpr int kMost = 10;  // stages (barriers)
-    static constexpr int kBars = 232448 - 1024 - 1024;
-    static constexpr int kTotal = kBars + 1024 + 1024;  // barriers, alignment slack
+    static constexpr int kBars = 229376;  // (what the ring takes at most)
+    static constexpr int kTotal = kBars + 256 + kPairEpiWarps * kBiasSlot + 1024;  // barriers, bias, alignment slack
+    static_assert(kTotal <= 232448, "shared memory");
 };
 
-template <int BN, bool BF16, bool AMN, bool BMN, bool WIDE>
+template <int BN, bool BF16, bool AMN, bool BMN, bool WIDE, bool AUX>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
     using L = PairSmem;
@@ -583,11 +606,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int panels = columns(col0) / kPanel;
             PanelAux in;
             const bool shifted = off_sector<WIDE>(p, row);
-            if (sub < panels) load_aux<WIDE>(in, p, row, panel_columns<WIDE>(shifted, col0, sub, panels));
+            if (sub < panels) load_aux<WIDE, AUX>(in, p, row, panel_columns<WIDE>(shifted, col0, sub, panels));
+            const uint32_t bias = load_bias(p, col0, sub, panels, lane);
             mbar_wait(acc_full(buf), (t >> 1) & 1, abort_flag, p.status);
             tc_fence_after();
-            epilogue_panels<BF16, WIDE>(p, in, tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, shifted, row, col0, sub, panels,
-                                        kPairEpiWarps / 4, tile % p.splits, [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
+            epilogue_panels<BF16, WIDE, AUX>(p, in, bias, bar_area + 256 + (warp - 2) * kBiasSlot,
+                                             tmem_base + ((uint32_t)(g * 32) << 16) + buf * BN, shifted, row, col0, sub, panels,
+                                             kPairEpiWarps / 4, tile % p.splits, [&] { if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(buf), 0)); });
         }
     }
 
@@ -639,30 +664,39 @@ int gemm_params(const GemmCall& g, GemmParams* p) {
 template <int BN>
 struct Single {
     static constexpr bool kMn = BN == 64 || BN == 128;
-    template <bool BF16, bool AMN, bool BMN, bool WIDE>
-    static constexpr auto kernel = gemm_tc_kernel<BN, BF16, AMN, BMN, WIDE>;
+    template <bool BF16, bool AMN, bool BMN, bool WIDE, bool AUX>
+    static auto kernel() { return gemm_tc_kernel<BN, BF16, AMN, BMN, WIDE, AUX>; }
 };
 template <int BN>
 struct Pair {
     static constexpr bool kMn = true;
-    template <bool BF16, bool AMN, bool BMN, bool WIDE>
-    static constexpr auto kernel = gemm_tc_pair_kernel<BN, BF16, AMN, BMN, WIDE>;
+    template <bool BF16, bool AMN, bool BMN, bool WIDE, bool AUX>
+    static auto kernel() { return gemm_tc_pair_kernel<BN, BF16, AMN, BMN, WIDE, AUX>; }
 };
+template <typename F>
+int with_bool(bool value, F f) { return value ? f(std::true_type{}) : f(std::false_type{}); }
 // `run` is called with the call's kernel
 template <typename Family, typename F>
 int with_kernel(const GemmCall& g, const GemmParams& p, F run) {
-    auto pick = [&](auto bf16, auto wide) -> int {
-        constexpr bool B = decltype(bf16)::value, W = decltype(wide)::value;
-        if (!g.a_mn && !g.b_mn) return run(Family::template kernel<B, false, false, W>);
-        if constexpr (Family::kMn) {
-            if (g.b_mn && g.a_mn) return run(Family::template kernel<B, true, true, W>);
-            if (g.b_mn) return run(Family::template kernel<B, false, true, W>);
-        }
-        return TMW_ERR_UNSUPPORTED;
-    };
     const bool wide = p.partial != nullptr || p.wide;  // (fp32 sums have a path of their own)
-    if (g.dtype == TMW_BF16) return wide ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
-    return wide ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{});
+    const bool aux = p.partial == nullptr && (g.epilogue == GEMM_ADD || g.epilogue == GEMM_GELU_GRAD);
+    return with_bool(g.dtype == TMW_BF16, [&](auto bf16) {
+        return with_bool(wide, [&](auto w) {
+            constexpr bool B = decltype(bf16)::value, W = decltype(w)::value;
+            if (g.a_mn) {
+                if constexpr (Family::kMn) {
+                    if (g.b_mn && !aux) return run(Family::template kernel<B, true, true, W, false>());
+                }
+                return (int)TMW_ERR_UNSUPPORTED;
+            }
+            return with_bool(aux, [&](auto a) {
+                constexpr bool A = decltype(a)::value;
+                if (!g.b_mn) return run(Family::template kernel<B, false, false, W, A>());
+                if constexpr (Family::kMn) return run(Family::template kernel<B, false, true, W, A>());
+                return (int)TMW_ERR_UNSUPPORTED;
+            });
+        });
+    });
 }
 
 template <int BN>
@@ -685,7 +719,7 @@ int launch_gemm(const GemmCall& g, cudaStream_t stream) {
 
 // How many CTA pairs of the kernel the device runs at once (asked once per kernel and device).
 int max_active_pairs(const void* kern, int smem_bytes) {
-    constexpr int kMaxDevices = 64, kMaxKernels = 16;
+    constexpr int kMaxDevices = 64, kMaxKernels = 32;
     struct Entry { const void* kern; int pairs[kMaxDevices]; };
     static std::mutex mutex;
     static Entry table[kMaxKernels] = {};
@@ -736,7 +770,10 @@ int launch_gemm_pair(const GemmCall& g, int width, cudaStream_t stream) {
 // What a single-CTA kernel was measured to need (us): a launch without its K, what a 64-wide slice of K takes where a tile is
 // alone on the chip, and where all SMs stream operands.  The pair kernel moves the fewest operand bytes per product and wins
 // wherever it has enough tiles: measured at K = 640 for 1056 | 2528 | 8256 | 32 896 rows of N = 1920, pair | 128 | 64
-// columns: 9.3 | 12.6 | 21.3 | 68.8, 6.3 | 11.4 | 24.1 | 82.5, 7.1 | 11.7 | 29.0 us.
+// columns: 7.8 | 10.0 | 21.1 | 73.8, 6.2 | 11.1 | 24.9 | 102.9, 7.0 | 12.1 | 30.8 | 129.7 us (one after the other, the chip warm).  The
+// constants are older than the present epilogue and ring.  What they choose is within 4 % of the best kernel and width for the four
+// products of a layer of width 640 at 144 to 32 896 rows; elsewhere it is up to a sixth off (2112 x 1024 x 4096, second operand
+// MN-major: 19.1 against 16.5).
 struct Variant {
     int rows, cols;
     float launch, alone, full;
@@ -747,8 +784,8 @@ constexpr Variant kVariants[] = {{2 * GM, 256, 6.1f, 0.f, 0.f},  // (see pair_co
 
 // The pair kernel's cost and tile width.  A 64-wide slice of a tile of w columns takes 0.12 + 0.00105 w us on a busy chip
 // and the chip as a whole 0.465 us per 256 columns of a pair; few waves of wide tiles leave a last one that is nearly empty,
-// which narrower tiles fill.  8320 x 640 x 2560: 33 bands over 74 pairs are two waves at 256 columns and at 160; 33.8 and
-// 28.8 us (64 columns a CTA, single: 38.6).  16416 x 640 x 2560: 47.5 at 256, 50.7 at 160.
+// which narrower tiles fill.  8256 x 640 x 2560: 33 bands over 74 pairs are two waves at 256 columns and at 160; 30.7 and
+// 23.8 us (64 columns a CTA, single: 35.2).  16416 x 640 x 2560: 52.1 at 256, 48.4 at 224, 50.5 at 160 (the chip warm).
 float pair_cost(const GemmCall& g, int splits, int sms, int* width) {
     const float slices = (float)((g.k + GK - 1) / GK) / (float)splits;
     const int bands = (g.m + 2 * GM - 1) / (2 * GM), pairs = sms / 2 > 0 ? sms / 2 : 1;
@@ -793,7 +830,7 @@ int launch_gemm_call(const GemmCall& call, cudaStream_t stream) {
     GemmCall g = call;
     const int sms = sm_count();
     g.splits = 1;
-    // a long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 6.5 us against 8.2)
+    // a long K over few tiles goes to the kernel that cuts K (144 rows, N = 640, K = 2560: 7.6 us against 8.2)
     if (!g.a_mn && !g.b_mn && g.epilogue <= GEMM_ADD && g.k >= 16 * GK && 2 * ((g.m + GM - 1) / GM) * ((g.n + 31) / 32) <= sms &&
         g.lda == g.k && g.ldb == g.k && g.ldc == g.n && (g.epilogue != GEMM_ADD || g.aux == g.c))
         return launch_rows_tc(g.dtype, g.m, g.n, g.k, g.a, g.b, g.bias, g.c, g.epilogue, stream, g.chain & kChainDependent);

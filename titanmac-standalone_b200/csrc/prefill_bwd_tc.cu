@@ -17,7 +17,7 @@
 // The two halves of a column tile are chains of their own: products, barriers and four of the eight warps each.
 // Warps: 0 TMA producer (and the columns' statistics), 1 and 2 issue the tcgen05.mma (one elected thread each, each
 // its own chain of products; warp 1 allocates tensor memory), 3 idle, 4-11 the element-wise work and the output.
-// The first launch leaves every row's (log-sum-exp, D) in scratch memory for the second.  Every mbarrier wait is
+// The first launch leaves every row's (-log-sum-exp, -D) in scratch memory for the second.  Every mbarrier wait is
 // bounded (TMW_ERR_DEVICE_TIMEOUT in the status word).
 #include <cuda.h>
 
@@ -672,7 +672,7 @@ int launch_bwd_tc(const tmw_prefill_desc& d, const void* q, const void* k, const
     p.lse_pers = window_block > 0 ? lse + (size_t)B * H * (R - d.n_persistent) : nullptr;
     p.status = device_status_word();
     if (p.status == nullptr) return TMW_ERR_CUDA;
-    // scratch memory for the rows' (lse, D), ordered on the caller's stream; without it the launch whose rows are
+    // scratch memory for the rows' (-lse, -D), ordered on the caller's stream; without it the launch whose rows are
     // keys computes D itself
     p.rows_pad = (R + BT - 1) / BT * BT;
     p.stats = nullptr;
